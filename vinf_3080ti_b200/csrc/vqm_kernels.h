@@ -1,6 +1,7 @@
 // Host-visible declarations shared by the kernel translation units and the runtime.
 #pragma once
 
+#include <cuda.h>  // CUtensorMap (types only; nothing links against the driver)
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -80,6 +81,16 @@ enum : unsigned { kStatusOk = 0, kStatusWaitExpired = 1, kStatusPeerWaitExpired 
     cudaError_t launch_qmv_fused_##name(const MatvecArgs &a, int m, int sm_count, cudaStream_t stream, int *grid_out);  // honours a.fuse
 VQM_FOR_EACH_TYPE(VQM_DECLARE_LAUNCHER)
 #undef VQM_DECLARE_LAUNCHER
+
+// The tensor-core matvec (vqm_tcmv_type.cu).  maps: per tensor of the launch its tensor maps (tc_encode_maps).
+#define VQM_FOR_EACH_TC_TYPE(X) \
+    X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(20, IQ4_NL) X(23, IQ4_XS)
+#define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
+    cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, \
+                                   cudaStream_t stream);
+VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_TC_LAUNCHER)
+#undef VQM_DECLARE_TC_LAUNCHER
+cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, CUtensorMap *out);
 
 constexpr int kMaxGrid = 4096;  // upper bound on the matvec grid (sizes the argmax partial arrays)
 

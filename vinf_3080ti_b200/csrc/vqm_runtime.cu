@@ -48,6 +48,7 @@ struct Tensor {
     size_t row_bytes = 0, nbytes = 0;
     int argmax_row_base = 0;
     bool owned = true;
+    std::vector<CUtensorMap> maps;  // of the tensor-core matvec, encoded on first use
 };
 
 struct Buffer {
@@ -198,6 +199,38 @@ cudaError_t dispatch_qmv(int type, const vqm::MatvecArgs &a, int m, int sm_count
     }
 }
 
+// Whether a launch runs on the tensor-core matvec.
+bool use_tcmv(int type, const vqm::MatvecArgs &a) {
+    if (a.push.push_slot > 0 || a.push.wait_slot > 0) return false;
+    if ((a.fuse & vqm::kFuseNorm) && a.cols > 128 * 256) return false;
+    switch (type) {
+#define VQM_CASE(id, name) case id: return true;
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+        default: return false;
+    }
+}
+
+cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, cudaStream_t stream) {
+    switch (type) {
+#define VQM_CASE(id, name) \
+    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, m, sm_count, stream);
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+// One tensor in device memory that has no Tensor record.
+cudaError_t dispatch_raw(int type, const vqm::MatvecArgs &a, int m, int sm_count, cudaStream_t stream) {
+    if (!use_tcmv(type, a)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
+    CUtensorMap maps[8];
+    const CUtensorMap *p[1] = {maps};
+    const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, maps);
+    if (err != cudaSuccess) return err;
+    return dispatch_tcmv(type, a, p, 1, m, sm_count, stream);
+}
+
 int check_shape(const char *name, int type, int cols, int rows, size_t *row_bytes) {
     const vqm::Traits t = vqm::traits_of(type);
     if (t.block == 0) return fail(VQM_ERR_VALUE, "unsupported GGUF tensor type id %d for CUDA matvec", type);
@@ -222,9 +255,9 @@ struct Fuse {
     float eps = 0.0f;
 };
 
-int launch_parts(vqm_runtime *rt, int n, const Tensor *const *ts, const float *x, float *const *ys, int m, bool with_argmax,
+int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, float *const *ys, int m, bool with_argmax,
                  const vqm::PushInfo *push = nullptr, const Fuse *fuse = nullptr) {
-    const Tensor &t0 = *ts[0];
+    Tensor &t0 = *ts[0];
     const uint8_t *cb = codebook_for(rt, t0.type);
     if (vqm::grid_is_codebook(t0.type) && cb == nullptr)
         return fail(VQM_ERR_VALUE, "the codebook for GGUF type %d has not been set (vqm_set_codebook)", t0.type);
@@ -267,25 +300,39 @@ int launch_parts(vqm_runtime *rt, int n, const Tensor *const *ts, const float *x
         a.out_val = rt->argmax_vals;
         a.row_base = t0.argmax_row_base;
     }
-    const cudaError_t err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
+    cudaError_t err = cudaSuccess;
+    if (use_tcmv(t0.type, a)) {
+        const CUtensorMap *maps[vqm::kMaxParts];
+        for (int i = 0; i < n && err == cudaSuccess; ++i) {
+            if (ts[i]->maps.empty()) {
+                ts[i]->maps.resize(8);
+                err = vqm::tc_encode_maps(ts[i]->type, ts[i]->data, ts[i]->rows, static_cast<long long>(ts[i]->row_bytes), ts[i]->maps.data());
+                if (err != cudaSuccess) ts[i]->maps.clear();
+            }
+            maps[i] = ts[i]->maps.data();
+        }
+        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, m, rt->sm_count, rt->stream);
+    } else {
+        err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
+    }
     if (err != cudaSuccess) return cuda_fail("qmv launch", err);
     count_launch(rt);
     return VQM_OK;
 }
 
-int launch_group(vqm_runtime *rt, const Tensor &t, const float *x, float *y, int m, bool with_argmax, const vqm::PushInfo *push = nullptr) {
-    const Tensor *ts[1] = {&t};
+int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bool with_argmax, const vqm::PushInfo *push = nullptr) {
+    Tensor *ts[1] = {&t};
     float *ys[1] = {y};
     return launch_parts(rt, 1, ts, x, ys, m, with_argmax, push);
 }
 
 // The tensors and output buffers of a group call, checked: same type and columns, every y large enough.
-int resolve_group(vqm_runtime *rt, int n, const char *const *weights, const char *const *ys, int ntok, const Tensor **ts, float **yps) {
+int resolve_group(vqm_runtime *rt, int n, const char *const *weights, const char *const *ys, int ntok, Tensor **ts, float **yps) {
     if (n < 1 || n > vqm::kMaxParts) return fail(VQM_ERR_VALUE, "a group holds 1 to %d tensors", vqm::kMaxParts);
     if (weights == nullptr || ys == nullptr) return fail(VQM_ERR_VALUE, "null pointer");
     int rc = VQM_OK;
     for (int i = 0; i < n; ++i) {
-        const Tensor *t = find_tensor(rt, weights[i], &rc);
+        Tensor *t = find_tensor(rt, weights[i], &rc);
         if (t == nullptr) return rc;
         if (t->cols % 32 != 0) return fail(VQM_ERR_VALUE, "%s: matvec cols must be a multiple of 32", weights[i]);
         if (i > 0 && (t->type != ts[0]->type || t->cols != ts[0]->cols))
@@ -889,7 +936,7 @@ int vqm_qmv_fused(vqm_runtime *rt, const char *weight, const char *x, const char
         if (!(eps >= 0.0f)) return fail(VQM_ERR_VALUE, "eps must be >= 0");
     }
     if (out_ids != nullptr && (rc = no_capture(rt, "a blocking fused argmax")) != VQM_OK) return rc;
-    const Tensor *ts[1] = {t};
+    Tensor *ts[1] = {t};
     float *ys[1] = {yp};
     if ((rc = launch_parts(rt, 1, ts, xp, ys, ntok, with_argmax, nullptr, &f)) != VQM_OK) return rc;
     if (out_ids != nullptr) {
@@ -930,7 +977,7 @@ int vqm_set_argmax_row_base(vqm_runtime *rt, const char *weight, int row_base) {
 int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t x_bytes, float *y_host, size_t y_bytes) {
     auto it = rt->tensors.find(weight);
     if (it == rt->tensors.end()) return fail(VQM_ERR_KEY, "%s is not resident on the GPU", weight);
-    const Tensor &t = it->second;
+    Tensor &t = it->second;
     if (x_bytes != static_cast<size_t>(t.cols) * sizeof(float))
         return fail(VQM_ERR_VALUE, "%s: x has %zu bytes, expected %d float32", weight, x_bytes, t.cols);
     if (y_bytes < static_cast<size_t>(t.rows) * sizeof(float))
@@ -1164,7 +1211,7 @@ int vqm_set_column_split(vqm_runtime *rt, int enabled) {
 
 int vqm_qmv_group(vqm_runtime *rt, int n, const char *const *weights, const char *x, const char *const *ys, int ntok) {
     if (ntok < 1 || ntok > 8) return fail(VQM_ERR_VALUE, "ntok must be in [1, 8]");
-    const Tensor *ts[vqm::kMaxParts];
+    Tensor *ts[vqm::kMaxParts];
     float *yps[vqm::kMaxParts];
     int rc = resolve_group(rt, n, weights, ys, ntok, ts, yps);
     if (rc != VQM_OK) return rc;
@@ -1180,7 +1227,7 @@ int vqm_qmv_push_group(vqm_runtime *rt, int n, const char *const *weights, const
     if (slot < -1 || slot >= rt->exchange_slots || wait_slot < -1 || wait_slot >= rt->exchange_slots)
         return fail(VQM_ERR_VALUE, "slot out of range");
     if (dst_offs == nullptr || rows_totals == nullptr || row_begins == nullptr) return fail(VQM_ERR_VALUE, "null pointer");
-    const Tensor *ts[vqm::kMaxParts];
+    Tensor *ts[vqm::kMaxParts];
     float *yps[vqm::kMaxParts];
     int rc = resolve_group(rt, n, weights, ys, ntok, ts, yps);
     if (rc != VQM_OK) return rc;
@@ -1221,7 +1268,8 @@ int vqm_qmv_raw(int type, const void *w, int rows, int cols, const float *x, flo
     a.status = status;
     a.cols = cols;
     a.row_bytes = static_cast<long long>(row_bytes);
-    const cudaError_t err = dispatch_qmv(type, a, ntok, sm_count, static_cast<cudaStream_t>(stream), nullptr);
+    a.allow_split = 1;
+    const cudaError_t err = dispatch_raw(type, a, ntok, sm_count, static_cast<cudaStream_t>(stream));
     if (err != cudaSuccess) return cuda_fail("qmv launch", err);
     return VQM_OK;
 }
@@ -1284,8 +1332,8 @@ int vqm_qmv_argmax_static(int type, const void *w, int rows, int cols, const flo
     a.cols = cols;
     a.row_bytes = static_cast<long long>(row_bytes);
     a.max_grid = kStaticMaxBlocks;  // the launch never uses more blocks than the scratch has partial slots for
-    int grid = 0;
-    err = dispatch_qmv(type, a, ntok, sm_count, st, &grid);
+    a.allow_split = 1;
+    err = dispatch_raw(type, a, ntok, sm_count, st);
     if (err != cudaSuccess) return cuda_fail("qmv launch", err);
     return VQM_OK;
 }

@@ -1,0 +1,345 @@
+// Row decoders of the tensor-core matvec (vqm_tcmv.cuh): raw words of one row -> fp16 A columns.
+//
+// begin() reads the scales of half a step (128 columns; `kh` = which half), chunk<CH>() fills the 32 registers (64 fp16
+// values) of chunk CH of the half.  Registers come in core rows of 4 (8 columns); the columns behind them are tc_columns() of
+// the kernel's header.  Masked fields are fp16 subnormals, field * 2^-24 times the field's place value; the multipliers undo
+// the place value, so every A value is (quant - bias) * sub-scale * 2^-24, exactly (at most 11 significant bits).  scale() is
+// the fp16 super-scale times 2^24.
+// The comments give the instructions per 8 weights: integer ones go to a pipe that takes a warp instruction every 2 cycles,
+// and so does packed fp16 arithmetic, but the two run side by side (measured 1.3 cycles per instruction when mixed).
+#pragma once
+
+#include "vqm_tcmv.cuh"
+
+namespace vqm {
+
+constexpr float kTc24 = 16777216.0f;  // 2^24
+
+template <int TYPE>
+struct TcUnit;
+
+// Q4_K / Q5_K: d, dmin, 12 bytes of 6-bit scales and minimums; sub-block pairs (low and high nibbles) of 64 columns.
+// Q4_K: 5 integer + 4 fp16 instructions per 8 weights.  Q5_K adds the fifth bit with its own multiplier: 11 + 8.
+template <int TYPE>
+struct TcUnitK45 {
+    float d, dm;
+    uint32_t sc, mn;  // scales / minimums of the half's four sub-blocks, one per byte
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t, int kh) {
+        const uint4 h = lds128u(line);
+        d = half_bits_to_float(h.x & 0xFFFFu) * kTc24;
+        dm = half_bits_to_float(h.x >> 16);
+        sc = kh == 0 ? h.y & 0x3F3F3F3Fu : (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
+        mn = kh == 0 ? h.z & 0x3F3F3F3Fu : ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
+    }
+    __device__ __forceinline__ float scale(int) const { return d; }
+    template <int G>
+    __device__ __forceinline__ float minimum() const { return dm * byte_to_float<G>(mn); }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
+        constexpr uint32_t kNeg1024 = 0xE400E400u, kNeg64 = 0xD400D400u;
+        const uint32_t k0 = tc::hadd2(tc::byte_h2<2 * CH>(sc, tc::kHi1024), kNeg1024);    // scale of the low nibbles
+        const uint32_t k1 = tc::hadd2(tc::byte_h2<2 * CH + 1>(sc, tc::kHi64), kNeg64);    // of the high ones, / 16
+        uint32_t q[8];
+        tc::words<TYPE, O, (TYPE == kQ4_K ? 16 : 48) + 32 * CH, 8>(line + 64 * kh, sh, q);
+        if constexpr (TYPE == kQ4_K) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t w = q[i], v = w >> 8;
+                a[4 * i] = tc::hmul2(w & 0x000F000Fu, k0);
+                a[4 * i + 1] = tc::hmul2(w & 0x00F000F0u, k1);
+                a[4 * i + 2] = tc::hmul2(v & 0x000F000Fu, k0);
+                a[4 * i + 3] = tc::hmul2(v & 0x00F000F0u, k1);
+            }
+        } else {
+            uint32_t f[8];
+            tc::words<TYPE, O, 16, 8>(line, sh, f);
+            // the fifth bit of sub-block 4 kh + s is bit 4 kh + s of its byte: place value 2^s after the shift, worth 16 * scale
+            constexpr uint32_t e0 = (15 + 4 - 2 * CH) << 10, e1 = (15 + 7 - 2 * CH) << 10;  // 2^(4 - s), and 2^(4 - s) * 16 (k1 is / 16)
+            const uint32_t f0 = tc::hmul2(k0, e0 * 0x10001u), f1 = tc::hmul2(k1, e1 * 0x10001u);
+            constexpr uint32_t m0 = 0x00010001u << (2 * CH), m1 = 0x00010001u << (2 * CH + 1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t w = q[i], v = w >> 8, b = f[i] >> (4 * kh), c = f[i] >> (4 * kh + 8);
+                a[4 * i] = tc::hfma2(w & 0x000F000Fu, k0, tc::hmul2(b & m0, f0));
+                a[4 * i + 1] = tc::hfma2(w & 0x00F000F0u, k1, tc::hmul2(b & m1, f1));
+                a[4 * i + 2] = tc::hfma2(v & 0x000F000Fu, k0, tc::hmul2(c & m0, f0));
+                a[4 * i + 3] = tc::hfma2(v & 0x00F000F0u, k1, tc::hmul2(c & m1, f1));
+            }
+        }
+    }
+};
+template <>
+struct TcUnit<kQ4_K> : TcUnitK45<kQ4_K> {};
+template <>
+struct TcUnit<kQ5_K> : TcUnitK45<kQ5_K> {};
+
+// Q6_K: low nibbles @0, high bit pairs @128, int8 scales @192, d @208.  Quant times scale needs 14 bits, so a weight is two
+// A columns over the same activations: scale * low nibble and 16 * scale * (high bits - 2).  10 + 8 per 8 weights.
+// Chunk CH: byte columns 8 CH .. 8 CH + 7 of each of the half's four 32-column quarters.
+template <>
+struct TcUnit<kQ6_K> {
+    float d;
+    uint32_t sc[2];  // the half's eight scales (quarter * 2 + half of the quarter), one per byte, + 128
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int kh) {
+        tc::words<kQ6_K, O, 192, 2>(line + 8 * kh, sh, sc);
+        sc[0] ^= 0x80808080u, sc[1] ^= 0x80808080u;
+        uint32_t w[1];
+        tc::words<kQ6_K, O, 208, 1>(line, sh, w);
+        d = half_bits_to_float(w[0] & 0xFFFFu) * kTc24;
+    }
+    __device__ __forceinline__ float scale(int) const { return d; }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
+        constexpr int IS = CH >> 1;
+        uint32_t k[4], kh2[4], kb[4];
+        {
+            const uint32_t n1152 = 0xE480E480u;  // -(1024 + 128)
+            k[0] = tc::hadd2(tc::byte_h2<IS>(sc[0], tc::kHi1024), n1152);
+            k[1] = tc::hadd2(tc::byte_h2<2 + IS>(sc[0], tc::kHi1024), n1152);
+            k[2] = tc::hadd2(tc::byte_h2<IS>(sc[1], tc::kHi1024), n1152);
+            k[3] = tc::hadd2(tc::byte_h2<2 + IS>(sc[1], tc::kHi1024), n1152);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kb[i] = tc::hmul2(k[i], 0x80208020u);  // * -2^-19: 16 * -2 * 2^-24
+            kh2[0] = tc::hmul2(k[0], 0x4C004C00u);                             // 16
+            kh2[1] = tc::hmul2(k[1], 0x44004400u);                             // 16 / 4
+            kh2[2] = k[2];                                                     // 16 / 16
+            kh2[3] = tc::hmul2(k[3], 0x34003400u);                             // 16 / 64
+            k[2] = tc::hmul2(k[2], 0x2C002C00u), k[3] = tc::hmul2(k[3], 0x2C002C00u);  // / 16: high nibbles
+        }
+        uint32_t l0[2], l1[2], hb[2];
+        tc::words<kQ6_K, O, 8 * CH, 2>(line + 64 * kh, sh, l0);
+        tc::words<kQ6_K, O, 32 + 8 * CH, 2>(line + 64 * kh, sh, l1);
+        tc::words<kQ6_K, O, 128 + 8 * CH, 2>(line + 32 * kh, sh, hb);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            uint32_t *lo = a + 16 * i, *hi = a + 16 * i + 8;
+            uint32_t w = l0[i], v = w >> 8;
+            lo[0] = tc::hmul2(w & 0x000F000Fu, k[0]);
+            lo[1] = tc::hmul2(w & 0x00F000F0u, k[2]);
+            lo[2] = tc::hmul2(v & 0x000F000Fu, k[0]);
+            lo[3] = tc::hmul2(v & 0x00F000F0u, k[2]);
+            w = l1[i], v = w >> 8;
+            lo[4] = tc::hmul2(w & 0x000F000Fu, k[1]);
+            lo[5] = tc::hmul2(w & 0x00F000F0u, k[3]);
+            lo[6] = tc::hmul2(v & 0x000F000Fu, k[1]);
+            lo[7] = tc::hmul2(v & 0x00F000F0u, k[3]);
+            w = hb[i], v = w >> 8;
+            hi[0] = tc::hfma2(w & 0x00030003u, kh2[0], kb[0]);
+            hi[1] = tc::hfma2(w & 0x00300030u, kh2[2], kb[2]);
+            hi[2] = tc::hfma2(v & 0x00030003u, kh2[0], kb[0]);
+            hi[3] = tc::hfma2(v & 0x00300030u, kh2[2], kb[2]);
+            hi[4] = tc::hfma2(w & 0x000C000Cu, kh2[1], kb[1]);
+            hi[5] = tc::hfma2(w & 0x00C000C0u, kh2[3], kb[3]);
+            hi[6] = tc::hfma2(v & 0x000C000Cu, kh2[1], kb[1]);
+            hi[7] = tc::hfma2(v & 0x00C000C0u, kh2[3], kb[3]);
+        }
+    }
+};
+
+// Q3_K: high-bit mask @0, bit pairs @32, 12 bytes of 6-bit scales @96, d @108; weight = d * (sc - 32) * (q2 + 4 h - 4).
+// Chunk CH: byte columns 16 CH .. 16 CH + 15 of each of the half's four 32-column groups.  10 + 8 per 8 weights.
+template <>
+struct TcUnit<kQ3_K> {
+    float d;
+    uint32_t sc[2];  // the half's eight 6-bit scales: byte 2 (j % 2) + CH of sc[j / 2] belongs to group j
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int kh) {
+        uint32_t s[4];
+        tc::words<kQ3_K, O, 96, 4>(line, sh, s);
+        d = half_bits_to_float(s[3] & 0xFFFFu) * kTc24;
+        if (kh == 0) {
+            sc[0] = (s[0] & 0x0F0F0F0Fu) | ((s[2] << 4) & 0x30303030u);
+            sc[1] = (s[1] & 0x0F0F0F0Fu) | ((s[2] << 2) & 0x30303030u);
+        } else {
+            sc[0] = ((s[0] >> 4) & 0x0F0F0F0Fu) | (s[2] & 0x30303030u);
+            sc[1] = ((s[1] >> 4) & 0x0F0F0F0Fu) | ((s[2] >> 2) & 0x30303030u);
+        }
+    }
+    __device__ __forceinline__ float scale(int) const { return d; }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
+        uint32_t k[4], f[4], b[4];  // multipliers of the bit pair and of the high bit, bias
+        {
+            const uint32_t n1056 = 0xE420E420u;  // -(1024 + 32)
+            const uint32_t s0 = tc::hadd2(tc::byte_h2<CH>(sc[0], tc::kHi1024), n1056), s1 = tc::hadd2(tc::byte_h2<2 + CH>(sc[0], tc::kHi1024), n1056);
+            const uint32_t s2 = tc::hadd2(tc::byte_h2<CH>(sc[1], tc::kHi1024), n1056), s3 = tc::hadd2(tc::byte_h2<2 + CH>(sc[1], tc::kHi1024), n1056);
+            b[0] = tc::hmul2(s0, 0x80048004u), b[1] = tc::hmul2(s1, 0x80048004u);  // * -4 * 2^-24
+            b[2] = tc::hmul2(s2, 0x80048004u), b[3] = tc::hmul2(s3, 0x80048004u);
+            f[0] = tc::hmul2(s0, 0x44004400u), f[1] = tc::hmul2(s1, 0x40004000u), f[2] = s2, f[3] = tc::hmul2(s3, 0x38003800u);  // 4 / 2^j
+            k[0] = s0, k[1] = tc::hmul2(s1, 0x34003400u), k[2] = tc::hmul2(s2, 0x2C002C00u), k[3] = tc::hmul2(s3, 0x24002400u);  // 1 / 4^j
+        }
+        uint32_t h[4], q[4];
+        tc::words<kQ3_K, O, 16 * CH, 4>(line, sh, h);
+        tc::words<kQ3_K, O, 32 + 16 * CH, 4>(line + 32 * kh, sh, q);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t w = q[i], v = w >> 8, m = h[i] >> (4 * kh), n = h[i] >> (4 * kh + 8);
+            uint32_t *r = a + 8 * i;
+            r[0] = tc::hfma2(w & 0x00030003u, k[0], tc::hfma2(m & 0x00010001u, f[0], b[0]));
+            r[1] = tc::hfma2(w & 0x000C000Cu, k[1], tc::hfma2(m & 0x00020002u, f[1], b[1]));
+            r[2] = tc::hfma2(v & 0x00030003u, k[0], tc::hfma2(n & 0x00010001u, f[0], b[0]));
+            r[3] = tc::hfma2(v & 0x000C000Cu, k[1], tc::hfma2(n & 0x00020002u, f[1], b[1]));
+            r[4] = tc::hfma2(w & 0x00300030u, k[2], tc::hfma2(m & 0x00040004u, f[2], b[2]));
+            r[5] = tc::hfma2(w & 0x00C000C0u, k[3], tc::hfma2(m & 0x00080008u, f[3], b[3]));
+            r[6] = tc::hfma2(v & 0x00300030u, k[2], tc::hfma2(n & 0x00040004u, f[2], b[2]));
+            r[7] = tc::hfma2(v & 0x00C000C0u, k[3], tc::hfma2(n & 0x00080008u, f[3], b[3]));
+        }
+    }
+};
+
+// Q2_K: 16 bytes of 4-bit scales and minimums @0, bit pairs @16, d @80, dmin @82.  5 + 4 per 8 weights.
+template <>
+struct TcUnit<kQ2_K> {
+    float d, dm;
+    uint32_t sc[2], mn[2];  // the half's eight scales and minimums, one per byte: 2 j + half of the 32-column group j
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int kh) {
+        uint32_t s[2], w[1];
+        tc::words<kQ2_K, O, 0, 2>(line + 8 * kh, sh, s);
+        tc::words<kQ2_K, O, 80, 1>(line, sh, w);
+        sc[0] = s[0] & 0x0F0F0F0Fu, sc[1] = s[1] & 0x0F0F0F0Fu;
+        mn[0] = (s[0] >> 4) & 0x0F0F0F0Fu, mn[1] = (s[1] >> 4) & 0x0F0F0F0Fu;
+        d = half_bits_to_float(w[0] & 0xFFFFu) * kTc24;
+        dm = half_bits_to_float(w[0] >> 16);
+    }
+    __device__ __forceinline__ float scale(int) const { return d; }
+    template <int G>
+    __device__ __forceinline__ float minimum() const { return dm * byte_to_float<G & 3>(mn[G >> 2]); }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
+        const uint32_t n1024 = 0xE400E400u;
+        uint32_t k[4];
+        k[0] = tc::hadd2(tc::byte_h2<CH>(sc[0], tc::kHi1024), n1024);
+        k[1] = tc::hmul2(tc::hadd2(tc::byte_h2<2 + CH>(sc[0], tc::kHi1024), n1024), 0x34003400u);
+        k[2] = tc::hadd2(tc::byte_h2<CH>(sc[1], tc::kHi64), 0xD400D400u);
+        k[3] = tc::hmul2(tc::hadd2(tc::byte_h2<2 + CH>(sc[1], tc::kHi64), 0xD400D400u), 0x34003400u);
+        uint32_t q[4];
+        tc::words<kQ2_K, O, 16 + 16 * CH, 4>(line + 32 * kh, sh, q);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t w = q[i], v = w >> 8;
+            uint32_t *r = a + 8 * i;
+            r[0] = tc::hmul2(w & 0x00030003u, k[0]);
+            r[1] = tc::hmul2(w & 0x000C000Cu, k[1]);
+            r[2] = tc::hmul2(v & 0x00030003u, k[0]);
+            r[3] = tc::hmul2(v & 0x000C000Cu, k[1]);
+            r[4] = tc::hmul2(w & 0x00300030u, k[2]);
+            r[5] = tc::hmul2(w & 0x00C000C0u, k[3]);
+            r[6] = tc::hmul2(v & 0x00300030u, k[2]);
+            r[7] = tc::hmul2(v & 0x00C000C0u, k[3]);
+        }
+    }
+};
+
+// N words at any even shared address (the same position within 8 bytes for all lanes): aligned 8-byte loads, one select and
+// one funnel shift per word.  For the 34- and 18-byte blocks, whose position changes from block to block.
+template <int N>
+__device__ __forceinline__ void tc_words_at(uint32_t at, uint32_t (&w)[N]) {
+    constexpr int loads = (N + 3) / 2;
+    const uint32_t line = at & ~7u, sh = (at & 2u) * 8u;
+    const bool upper = (at & 4u) != 0;
+    uint32_t r[2 * loads];
+#pragma unroll
+    for (int i = 0; i < loads; ++i) {
+        const unsigned long long v = lds64(line + 8 * i);
+        r[2 * i] = static_cast<uint32_t>(v), r[2 * i + 1] = static_cast<uint32_t>(v >> 32);
+    }
+    uint32_t s[N + 1];
+#pragma unroll
+    for (int i = 0; i < N + 1; ++i) s[i] = upper ? r[i + 1] : r[i];
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(s[i], s[i + 1], sh);
+}
+
+// Q8_0: blocks of 32 int8 behind an fp16 scale; the scale stays outside, one sum per block.
+template <>
+struct TcUnit<kQ8_0> {
+    float d[4];  // the half's four blocks
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t, uint32_t, int) {}
+    __device__ __forceinline__ float scale(int g) const { return d[g]; }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t at = row + 34 * (4 * kh + 2 * CH + g);
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * kTc24;
+            uint32_t q[8];
+            tc_words_at<8>(at + 2, q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t *r = a + 16 * g + 4 * i;  // int8 + 128 is the unsigned byte; 0x8080 is -128 * 2^-24
+                r[0] = tc::hadd2((q[2 * i] ^ 0x80808080u) & 0x00FF00FFu, 0x80808080u);
+                r[1] = tc::hadd2((q[2 * i + 1] ^ 0x80808080u) & 0x00FF00FFu, 0x80808080u);
+                r[2] = tc::hadd2(((q[2 * i] >> 8) ^ 0x00800080u) & 0x00FF00FFu, 0x80808080u);
+                r[3] = tc::hadd2(((q[2 * i + 1] >> 8) ^ 0x00800080u) & 0x00FF00FFu, 0x80808080u);
+            }
+        }
+    }
+};
+
+// The 8 nibbles of a word as a core row: the 16 levels of IQ4_NL / IQ4_XS sit in four registers, plus 128, one per byte.
+__device__ __forceinline__ void tc_iq4_word(uint32_t w, uint32_t *r) {
+    constexpr uint32_t L0 = 0x3F2D1801u, L1 = 0x766A5D4Fu, H0 = 0xA6998D81u, H1 = 0xF1D9C5B5u;
+    const uint32_t sel = w & 0x77777777u;                          // entry within each half of the table
+    const uint32_t pick = ((w >> 1) & 0x44444444u) | 0x32103210u;  // which half
+    const uint32_t x0 = __byte_perm(__byte_perm(L0, L1, sel), __byte_perm(H0, H1, sel), pick);
+    const uint32_t x1 = __byte_perm(__byte_perm(L0, L1, sel >> 16), __byte_perm(H0, H1, sel >> 16), pick >> 16);
+    r[0] = tc::hadd2(x0 & 0x00FF00FFu, 0x80808080u);               // low nibbles of bytes 0 and 1
+    r[1] = tc::hadd2(__byte_perm(x0, 0u, 0x4341), 0x80808080u);    // their high nibbles
+    r[2] = tc::hadd2(x1 & 0x00FF00FFu, 0x80808080u);
+    r[3] = tc::hadd2(__byte_perm(x1, 0u, 0x4341), 0x80808080u);
+}
+
+// IQ4_NL: blocks of 32 nibbles behind an fp16 scale.
+template <>
+struct TcUnit<kIQ4_NL> {
+    float d[4];
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t, uint32_t, int) {}
+    __device__ __forceinline__ float scale(int g) const { return d[g]; }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t at = row + 18 * (4 * kh + 2 * CH + g);
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * kTc24;
+            uint32_t q[4];
+            tc_words_at<4>(at + 2, q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) tc_iq4_word(q[i], a + 16 * g + 4 * i);
+        }
+    }
+};
+
+// IQ4_XS: d @0, high scale bits @2, low scale nibbles @4, nibbles @8; 32-column groups with a 6-bit scale.
+template <>
+struct TcUnit<kIQ4_XS> {
+    float d, dl[4];
+    uint32_t sl, sh6;  // the half's four scale nibbles (16 bits) and bit pairs (8 bits)
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t, int kh) {
+        const unsigned long long h = lds64(line);
+        d = half_bits_to_float(static_cast<uint32_t>(h) & 0xFFFFu) * kTc24;
+        sl = static_cast<uint32_t>(h >> 32) >> (16 * kh);
+        sh6 = static_cast<uint32_t>(h) >> (16 + 8 * kh);
+    }
+    __device__ __forceinline__ float scale(int g) const { return dl[g]; }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) {
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int i = 2 * CH + g;
+            const uint32_t ls = ((sl >> (4 * i)) & 15u) | (((sh6 >> (2 * i)) & 3u) << 4);
+            dl[i] = d * (__uint_as_float(0x4B000000u | ls) - (8388608.0f + 32.0f));
+        }
+        uint32_t q[8];
+        tc::words<kIQ4_XS, false, 8 + 32 * CH, 8>(line + 64 * kh, sh, q);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tc_iq4_word(q[i], a + 4 * i);
+    }
+};
+
+}  // namespace vqm

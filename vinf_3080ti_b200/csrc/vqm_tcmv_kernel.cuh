@@ -1,0 +1,670 @@
+// The kernel of the tensor-core matvec; vqm_tcmv.cuh has the description.
+#pragma once
+
+#include "vqm_tcmv_decoders.cuh"
+
+namespace vqm {
+
+template <int N>
+struct TcInt {
+    static constexpr int value = N;
+};
+
+// First columns of the two 4-column words a and b whose 8 columns make core row `l` (0..31) of a step's B operand.
+template <int TYPE>
+__device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
+    if constexpr (TYPE == kQ4_K || TYPE == kQ5_K) {  // chunk of 64 columns, word of its 32 bytes
+        a = 64 * (l >> 3) + 4 * (l & 7), b = a + 32;
+    } else if constexpr (TYPE == kQ6_K) {            // half, word, pair of quarters
+        a = 128 * (l >> 4) + 32 * (l & 1) + 4 * ((l >> 1) & 7), b = a + 64;
+    } else if constexpr (TYPE == kQ3_K || TYPE == kQ2_K) {
+        a = 128 * (l >> 4) + 64 * (l & 1) + 4 * ((l >> 1) & 7), b = a + 32;
+    } else if constexpr (TYPE == kIQ4_NL || TYPE == kIQ4_XS) {
+        a = 32 * (l >> 2) + 4 * (l & 3), b = a + 16;
+    } else {
+        a = 8 * l, b = a + 4;
+    }
+}
+
+// Converts activation row t's 256 columns of a step into the B operand: called by a whole warp, lane = core row.
+//   xs: the row's columns in the stage; cols_here: how many exist; info: where the row's scale and group sums go (floats
+//   [MC] scales, padded to 4, then [groups][MC]); norm_part: where the row's sum of squares goes (0: nowhere)
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, int t, int col0, int cols_here, uint32_t b_stage, uint32_t info,
+                                           uint32_t norm_part, int lane) {
+    int ca, cb;
+    tc_columns<TYPE>(lane, ca, cb);
+    float v[8];
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(xs + ca * 4));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(xs + cb * 4));
+    const bool has_a = ca < cols_here, has_b = cb < cols_here;  // cols are multiples of 32: a word exists as a whole
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        v[i] = has_a ? v[i] : 0.0f;
+        v[4 + i] = has_b ? v[4 + i] : 0.0f;
+    }
+    if (args.fuse & (kFuseSiluMul | kFuseNorm)) {
+        if (args.fuse & kFuseSiluMul) {
+            const float *x2 = args.x2 + static_cast<size_t>(t) * args.cols + col0;
+            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 ga = has_a ? *reinterpret_cast<const float4 *>(x2 + ca) : z, gb = has_b ? *reinterpret_cast<const float4 *>(x2 + cb) : z;
+            const float g[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = v[i] / (1.0f + expf(-v[i])) * g[i];
+        }
+        if (args.fuse & kFuseNorm) {
+            // the rms factor of a row is linear: it multiplies the finished outputs, here only the squares are added up
+            float sq = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sq = fmaf(v[i], v[i], sq);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, off);
+            if (lane == 0 && norm_part != 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(norm_part), "f"(sq) : "memory");
+            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 wa = has_a ? *reinterpret_cast<const float4 *>(args.norm_w + col0 + ca) : z;
+            const float4 wb = has_b ? *reinterpret_cast<const float4 *>(args.norm_w + col0 + cb) : z;
+            const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= w[i];
+        }
+    }
+    if constexpr (tc_mins(TYPE) > 0) {
+        // sums of the columns that share a minimum, for the a and the b words: 8 lanes (32 columns) or 4 lanes (16)
+        float sa = (v[0] + v[1]) + (v[2] + v[3]), sb = (v[4] + v[5]) + (v[6] + v[7]);
+        constexpr bool k32 = TYPE != kQ2_K;
+#pragma unroll
+        for (int off = 4; off >= (k32 ? 1 : 2); off >>= 1) {
+            sa += __shfl_xor_sync(0xFFFFFFFFu, sa, off);
+            sb += __shfl_xor_sync(0xFFFFFFFFu, sb, off);
+        }
+        // group of a: sub-block 2 c (Q4_K, Q5_K), or 8 n + 2 j + half with j = 2 * core (Q2_K); b: the one after / two after
+        const bool writer = k32 ? (lane & 7) == 0 : (lane & 6) == 0;
+        const int ga = k32 ? 2 * (lane >> 3) : 8 * (lane >> 4) + 4 * (lane & 1) + ((lane >> 3) & 1), gb = ga + (k32 ? 1 : 2);
+        if (writer) {
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(MC) + ga * MC + t) * 4), "f"(sa) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(MC) + gb * MC + t) * 4), "f"(sb) : "memory");
+        }
+    }
+    // power of two that brings the largest magnitude below 2^10, and its inverse
+    uint32_t big = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t m = __float_as_uint(v[i]) & 0x7FFFFFFFu;
+        big = big > m ? big : m;
+    }
+    big = __reduce_max_sync(0xFFFFFFFFu, big);
+    const uint32_t want = 263u - (big >> 23), e = want < 253u ? want : 253u;
+    const float up = __uint_as_float(e << 23);
+    if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(__uint_as_float((254u - e) << 23)) : "memory");
+    constexpr int kOrder = tc_order(TYPE);
+    constexpr int order[3][8] = {{0, 2, 4, 6, 1, 3, 5, 7}, {0, 1, 4, 5, 2, 3, 6, 7}, {0, 2, 1, 3, 4, 6, 5, 7}};
+    uint32_t h[3][4];
+    const f32x2 up2 = pack2(up, up), k2048 = pack2(2048.0f, 2048.0f), neg = pack2(-2048.0f, -2048.0f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f32x2 r = mul2(pack2(v[order[kOrder][2 * i]], v[order[kOrder][2 * i + 1]]), up2);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            float lo, hi;
+            unpack2(r, lo, hi);
+            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h[p][i]) : "f"(hi), "f"(lo));
+            if (p < 2) {  // 2048 * (r - plane), exactly
+                const float flo = half_bits_to_float(h[p][i] & 0xFFFFu), fhi = half_bits_to_float(h[p][i] >> 16);
+                r = fma2(pack2(flo, fhi), neg, mul2(r, k2048));
+            }
+        }
+    }
+    const uint32_t at = b_stage + lane * kTcCore;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const int n = p * MC + t;
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (n >> 3) * kTcGroupB + (n & 7) * 16), "r"(h[p][0]), "r"(h[p][1]),
+                     "r"(h[p][2]), "r"(h[p][3])
+                     : "memory");
+    }
+}
+
+// A unit is what a group of warps takes of a step: one or two halves of 128 columns.  Its chunks go to the tensor cores in
+// batches; tensor memory holds one batch of a group (64 columns) and 64 columns of sums.  Types with a scale per 32 columns
+// have a sum per 32 columns: with N = 32 only one chunk's fit.
+__host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) ? 2 : 1; }
+template <int TYPE, int MC>
+__host__ __device__ constexpr int tc_batch_chunks() { return tc_block32(TYPE) && MC > 4 ? 1 : 2; }
+template <int TYPE, int MC>
+__host__ __device__ constexpr int tc_half_batches() { return 2 * tc_parts(TYPE) / tc_batch_chunks<TYPE, MC>(); }
+// sums per row that a batch leaves
+template <int TYPE, int MC>
+__host__ __device__ constexpr int tc_sums() { return tc_block32(TYPE) ? 2 * tc_batch_chunks<TYPE, MC>() : 1; }
+// whether a batch starts new sums (else only a unit's first one does)
+__host__ __device__ constexpr bool tc_fresh_batches(int type) { return tc_block32(type); }
+
+// What sums have to be multiplied with when they come back from tensor memory, one batch later.
+template <int TYPE, int MC>
+struct TcPending {
+    float s[tc_sums<TYPE, MC>()];        // super-scales of the sums
+    TcUnit<TYPE> unit[tc_halves(TYPE)];  // (only the minimums are used)
+    uint32_t info;                       // the step's activation scales and group sums
+    int kh;                              // the half, where a unit has one
+};
+
+// The sums of a row over the activation rows, in pairs for packed arithmetic (one activation row: the pair's upper half idles).
+template <int MC>
+struct TcAcc {
+    f32x2 v[(MC + 1) / 2];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < (MC + 1) / 2; ++i) v[i] = 0ull;
+    }
+    __device__ __forceinline__ void get(float (&f)[MC]) const {
+#pragma unroll
+        for (int i = 0; i < (MC + 1) / 2; ++i) {
+            float lo, hi;
+            unpack2(v[i], lo, hi);
+            f[2 * i] = lo;
+            if (2 * i + 1 < MC) f[2 * i + 1] = hi;
+        }
+    }
+};
+
+// acc[t] += scale * (h0 + 2^-11 h1 + 2^-22 h2 sums) * activation scale  -  minimums * group sums
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
+    constexpr int kSums = tc_sums<TYPE, MC>(), kMins = tc_mins(TYPE);
+    float v[kSums][3 * MC + 1];
+#pragma unroll
+    for (int g = 0; g < kSums; ++g) tc::ld_sums<MC>(d_at + g * TcShape<MC>::kN, v[g]);
+    f32x2 inv[(MC + 1) / 2];
+    if constexpr (MC == 1) {
+        inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
+    } else if constexpr (MC == 2) {
+        inv[0] = lds64(p.info);
+    } else {
+#pragma unroll
+        for (int t = 0; t < MC; t += 4) {
+            const ulonglong2 w = lds128(p.info + t * 4);
+            inv[t / 2] = w.x, inv[t / 2 + 1] = w.y;
+        }
+    }
+    tc::wait_ld();
+#pragma unroll
+    for (int g = 0; g < kSums; ++g) {
+        const float s = p.s[g];
+        if constexpr (MC == 1) {
+            float a, b, k, unused;
+            unpack2(acc.v[0], a, b);
+            unpack2(inv[0], k, unused);
+            a = fmaf(fmaf(v[g][2], 0x1p-22f, fmaf(v[g][1], 0x1p-11f, v[g][0])) * s, k, a);
+            acc.v[0] = pack2(a, b);
+        } else {
+            const f32x2 s2 = pack2(s, s), c1 = pack2(0x1p-11f, 0x1p-11f), c2 = pack2(0x1p-22f, 0x1p-22f);
+#pragma unroll
+            for (int t = 0; t < MC; t += 2) {
+                f32x2 u = fma2(pack2(v[g][MC + t], v[g][MC + t + 1]), c1, pack2(v[g][t], v[g][t + 1]));
+                u = fma2(pack2(v[g][2 * MC + t], v[g][2 * MC + t + 1]), c2, u);
+                acc.v[t / 2] = fma2(mul2(u, s2), inv[t / 2], acc.v[t / 2]);
+            }
+        }
+    }
+    if constexpr (kMins > 0) {
+#pragma unroll
+        for (int h = 0; h < tc_halves(TYPE); ++h) {
+            float sums[kMins * MC];
+#pragma unroll
+            for (int i = 0; i < kMins * MC; i += 4) {
+                const uint4 w = lds128u(p.info + (tc_info_scales(MC) + (tc_wide(TYPE) ? h : p.kh) * kMins * MC + i) * 4);
+                sums[i] = __uint_as_float(w.x), sums[i + 1] = __uint_as_float(w.y), sums[i + 2] = __uint_as_float(w.z), sums[i + 3] = __uint_as_float(w.w);
+            }
+            auto one = [&](auto tag) {
+                constexpr int G = decltype(tag)::value;
+                if constexpr (G < kMins) {
+                    const float m = -p.unit[h].template minimum<G>();
+                    if constexpr (MC == 1) {
+                        float a, b;
+                        unpack2(acc.v[0], a, b);
+                        acc.v[0] = pack2(fmaf(m, sums[G], a), b);
+                    } else {
+#pragma unroll
+                        for (int t = 0; t < MC; t += 2) acc.v[t / 2] = fma2(pack2(m, m), pack2(sums[G * MC + t], sums[G * MC + t + 1]), acc.v[t / 2]);
+                    }
+                }
+            };
+            one(TcInt<0>{}), one(TcInt<1>{}), one(TcInt<2>{}), one(TcInt<3>{});
+            one(TcInt<4>{}), one(TcInt<5>{}), one(TcInt<6>{}), one(TcInt<7>{});
+        }
+    }
+}
+
+__device__ __forceinline__ bool tc_better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
+
+// Fused argmax: block partials, then the last block to finish reduces them (ties to the lowest row, 0x7fffffff if nothing is
+// above -inf).  Warp w < 16 holds the best of activation row w % MC over its lanes' outputs.
+template <int MC>
+__device__ __forceinline__ void tc_finish_argmax(const MatvecArgs &a, int m, float bv, int bi, int warp, int lane, float *s_v, int *s_i, bool *s_last) {
+    auto warp_best = [&]() {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
+            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
+            if (tc_better(ov, oi, bv, bi)) bv = ov, bi = oi;
+        }
+    };
+    warp_best();
+    if (warp < 16 && lane == 0) s_v[warp] = bv, s_i[warp] = bi;
+    __syncthreads();
+    const int grid = static_cast<int>(gridDim.x);
+    if (threadIdx.x < static_cast<unsigned>(m)) {
+        const int t = static_cast<int>(threadIdx.x);
+        bv = s_v[t], bi = s_i[t];
+        for (int w = t + MC; w < 16; w += MC)
+            if (tc_better(s_v[w], s_i[w], bv, bi)) bv = s_v[w], bi = s_i[w];
+        a.part_val[t * grid + blockIdx.x] = bv;
+        a.part_idx[t * grid + blockIdx.x] = bi;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *s_last = atomicAdd(a.done_counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+    if (warp < m) {
+        bv = -INFINITY, bi = 0x7fffffff;
+        for (int b = lane; b < grid; b += 32) {
+            const float v = __ldcg(a.part_val + warp * grid + b);
+            const int i = __ldcg(a.part_idx + warp * grid + b);
+            if (tc_better(v, i, bv, bi)) bv = v, bi = i;
+        }
+        warp_best();
+        if (lane == 0) {
+            a.out_idx[warp] = bi == 0x7fffffff ? bi : bi + a.row_base;
+            if (a.out_val != nullptr) a.out_val[warp] = bv;
+        }
+    }
+    if (threadIdx.x == 0) *a.done_counter = 0;
+}
+
+template <int TYPE, int MC, typename MAPS>
+__global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_constant__ MatvecArgs a, const __grid_constant__ MAPS maps, const int m) {
+    using Shape = TcShape<MC>;
+    constexpr int kStages = tc_stages<TYPE, MC>(), kStageBytes = tc_stage_bytes<TYPE, MC>();
+    constexpr int kPitch = tc_pitch(TYPE), kStepBytes = tc_step_bytes(TYPE);
+    constexpr int kNB = tc_b_stages<TYPE, MC>();
+    constexpr bool kWide = tc_wide(TYPE);
+    constexpr uint32_t kTmD = 64;  // a group's sums start at this column of its 128
+    constexpr uint32_t kIdesc = (1u << 4) | (static_cast<uint32_t>(Shape::kN >> 3) << 17) | ((128u >> 4) << 24);  // fp32 += fp16 * fp16, M = 128
+    static_assert(kStages >= (kWide ? 3 : 2) && kStages + 2 <= kTcInfoSlots, "stage ring");
+    extern __shared__ uint8_t tc_raw[];
+    __shared__ __align__(8) uint64_t s_wfull[6], s_wempty[6], s_bfull[4], s_bempty[4], s_afull[4], s_done[4], s_cluster, s_read;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_failed;
+    __shared__ float s_norm[kMaxSplit][8];  // sums of squares of the activation rows, from every block of the cluster
+    __shared__ float s_best_v[16];
+    __shared__ int s_best_i[16];
+    __shared__ bool s_last;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // layout: stages (1024-byte aligned) | table | B ring | per-step info | sums of the tile | sums of squares
+    const uint32_t stages = (tc::s32(tc_raw) + 1023u) & ~1023u;
+    const uint32_t table = stages + kStages * kStageBytes;
+    const uint32_t b_ring = table + (grid_bytes(TYPE) + 127) / 128 * 128;
+    const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * kTcGroupB;
+    const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
+    const uint32_t norm_parts = red + 2 * 264 * MC * 4;
+    volatile int *failed = &s_failed;
+
+    const int k_split = a.k_split;
+    const int rank = static_cast<int>(blockIdx.x) % k_split, group = static_cast<int>(blockIdx.x) / k_split, n_groups = static_cast<int>(gridDim.x) / k_split;
+    const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
+    const int step0 = rank * n_steps / k_split, step1 = (rank + 1) * n_steps / k_split;
+    auto tiles_of = [&](int p) { return (a.part[p].rows + kTcRows - 1) / kTcRows; };
+    const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = end2 + tiles_of(3);
+    // the tensor a tile belongs to, and that tensor's first tile
+    auto part_of = [&](int tile) { return (tile >= end0) + (tile >= end1) + (tile >= end2); };
+    auto first_tile = [&](int p) { return p == 0 ? 0 : p == 1 ? end0 : p == 2 ? end1 : end2; };
+
+    // ---- copy side: stage s of a step holds, per row class, 32 rows of kPitch bytes, then the activation rows ----
+    auto class_mis = [&](const MatvecPart &p, int c) {
+        return static_cast<uint32_t>((reinterpret_cast<uintptr_t>(p.w) + static_cast<uintptr_t>(c) * static_cast<uintptr_t>(a.row_bytes)) & 15u);
+    };
+    auto copy_weights = [&](int tile, int step, int stage) {  // one thread
+        const int p = part_of(tile), y = (tile - first_tile(p)) * 32;
+        const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+        const uint32_t bar = tc::s32(&s_wfull[stage]), at = stages + stage * kStageBytes;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcRows * kPitch + m * cols_here * 4) : "memory");
+        const int n = tc_maps(a.part[p].rows, a.row_bytes);  // map c brings classes c, c + n, c + 2n, ...
+#pragma unroll 1
+        for (int c = 0; c < n; ++c) {
+            const uint32_t x = ((class_mis(a.part[p], c) + static_cast<uint32_t>(step) * kStepBytes) & ~15u) / kTcElemBytes;
+            asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                             at + c * (8 / n) * 32 * kPitch),
+                         "l"(&maps.m[p][c]), "r"(x), "r"(y), "r"(0), "r"(bar)
+                         : "memory");
+        }
+    };
+    auto copy_x = [&](int step, int stage) {  // one thread
+        const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+        for (int t = 0; t < m; ++t)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             stages + stage * kStageBytes + kTcRows * kPitch + t * (kTcStepCols * 4)),
+                         "l"(a.x + static_cast<size_t>(t) * a.cols + step * kTcStepCols), "r"(cols_here * 4), "r"(tc::s32(&s_wfull[stage]))
+                         : "memory");
+    };
+
+    if (warp == 16 && tc::elect_one()) {
+        for (int s = 0; s < kStages; ++s) {
+            tc::bar_init(tc::s32(&s_wfull[s]), 1);
+            tc::bar_init(tc::s32(&s_wempty[s]), kWide ? 8 : 16);
+        }
+        for (int s = 0; s < kNB; ++s) {
+            tc::bar_init(tc::s32(&s_bfull[s]), static_cast<uint32_t>(m));
+            tc::bar_init(tc::s32(&s_bempty[s]), kWide ? 2 : 4);
+        }
+        for (int g = 0; g < 4; ++g) {
+            tc::bar_init(tc::s32(&s_afull[g]), 4);
+            tc::bar_init(tc::s32(&s_done[g]), 1);
+        }
+        tc::bar_init(tc::s32(&s_cluster), 1);
+        tc::bar_init(tc::s32(&s_read), static_cast<uint32_t>(k_split));
+        s_failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // weights never depend on an earlier kernel: the first stages are requested before anything else
+        int t = group, k = step0;
+#pragma unroll 1
+        for (int s = 0; s < kStages && t < n_tiles; ++s) {
+            copy_weights(t, k, s);
+            if (++k == step1) k = step0, t += n_groups;
+        }
+    }
+    __syncwarp();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::s32(&s_tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc::fence_before();
+    __syncthreads();
+    // Announces this block's barriers to the cluster; whoever signals them waits for the announcements first.  (The barriers were
+    // published by the fence behind their initialisation; a releasing arrive would wait for the copies in flight, 3 us.)
+    if (k_split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    tc::fence_after();
+    const uint32_t tmem = s_tmem;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // activations are read and outputs written from here on
+    float best_v = -INFINITY;
+    int best_i = 0x7fffffff;
+
+    if (warp == 16) {
+        if (tc::elect_one()) {
+            int filled = 0, stage = 0;
+            uint32_t phase = 0;
+            for (int tile = group; tile < n_tiles && !*failed; tile += n_groups)
+                for (int step = step0; step < step1; ++step) {
+                    if (filled >= kStages) {
+                        tc::bar_wait_one(tc::s32(&s_wempty[stage]), phase ^ 1u, failed);
+                        if (*failed) break;
+                        copy_weights(tile, step, stage);
+                    }
+                    copy_x(step, stage);
+                    ++filled;
+                    if (++stage == kStages) stage = 0, phase ^= 1u;
+                }
+            // after a wait gave up: the copies already requested must land before the block may leave
+            if (*failed) {
+#pragma unroll 1
+                for (int s = 0; s < kStages; ++s)
+                    for (int i = 0; i < 4096 && !tc::bar_try(tc::s32(&s_wfull[s]), 0); ++i) __nanosleep(64);
+            }
+        }
+        __syncwarp();
+    } else if (warp > 16) {
+        // ---- MMA issue: warp 17 for groups 0 and 1, warp 18 for groups 2 and 3 ----
+        constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_halves(TYPE) * tc_half_batches<TYPE, MC>(), kMmas = 4 * kBC;
+        const int pair = warp - 17;
+        int bs = 0, st = 0;
+        uint32_t bphase = 0, aphase = 0;
+        for (int tile = group; tile < n_tiles; tile += n_groups)
+            for (int step = step0; step < step1; ++step) {
+                if (!kWide || (st & 1) == pair) {
+                    const uint64_t b_unit = tc::b_desc(b_ring + bs * (Shape::kGroupsB * kTcGroupB) + (kWide ? 0 : pair * (16 * kTcCore)));
+                    tc::bar_wait(tc::s32(&s_bfull[bs]), bphase, failed);
+#pragma unroll
+                    for (int b = 0; b < kBatches; ++b) {
+#pragma unroll
+                        for (int g = 0; g < 2; ++g) {
+                            const int wg = 2 * pair + g;
+                            tc::bar_wait(tc::s32(&s_afull[wg]), aphase, failed);
+                            tc::fence_after();
+                            if (tc::elect_one()) {
+                                const uint32_t tm = tmem + wg * 128;
+#pragma unroll
+                                for (int j = 0; j < kMmas; ++j) {
+                                    // the B tile of 16 columns behind the batch's j-th 16 A columns (two A tiles per B tile with two parts)
+                                    const int i = tc_parts(TYPE) == 2 ? ((b * kBC + (j >> 2)) * 2 + ((j & 3) >> 1)) : b * kMmas + j;
+                                    const int sum = tc_block32(TYPE) ? j >> 1 : 0;
+                                    const bool fresh = tc_block32(TYPE) ? (j & 1) == 0 : b == 0 && j == 0;
+                                    tc::mma(tm + kTmD + sum * Shape::kN, tm + j * 8, b_unit + static_cast<uint64_t>(i * (2 * kTcCore / 16)), kIdesc,
+                                            fresh ? 0u : 1u);
+                                }
+                                tc::commit(tc::s32(&s_done[wg]));
+                                if (b == kBatches - 1) tc::commit(tc::s32(&s_bempty[bs]));
+                            }
+                            __syncwarp();
+                        }
+                        aphase ^= 1u;
+                    }
+                }
+                ++st;
+                if (++bs == kNB) bs = 0, bphase ^= 1u;
+            }
+    } else {
+        const int wg = warp >> 2, quarter = warp & 3, rw = wg & 1, pair = wg >> 1, kh = kWide ? 0 : pair;
+        const int cls = rw * 4 + quarter;  // this warp's row class: rows cls, cls + 8, ... of the tile
+        const uint32_t tm_mine = tmem + wg * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t a_full = tc::s32(&s_afull[wg]), mma_done = tc::s32(&s_done[wg]);
+        int st = 0, stage = 0, bs = 0;  // step count, stage, B stage
+        uint32_t wphase = 0, bphase = 0, dphase = 0, rphase = 0, sphase = 0;
+        bool announced = false;                 // the cluster's barriers are known to exist
+        bool started = false, pending = false;  // MMAs are in flight; a unit's sums have not been read yet
+        TcPending<TYPE, MC> pend;
+        TcAcc<MC> acc;
+        acc.clear();
+
+        for (int tile = group; tile < n_tiles; tile += n_groups) {
+            const int p = part_of(tile), tile0 = first_tile(p);
+            const uint32_t mis0 = class_mis(a.part[p], cls);
+            const int n_maps = tc_maps(a.part[p].rows, a.row_bytes), slot = (cls % n_maps) * (8 / n_maps) + cls / n_maps;  // where the class lies
+            for (int step = step0; step < step1; ++step) {
+                if (!kWide || (st & 1) == pair) {
+                    tc::bar_wait(tc::s32(&s_wfull[stage]), wphase, failed);
+                    const uint32_t at = stages + stage * kStageBytes, info = info_ring + (st & (kTcInfoSlots - 1)) * tc_info_floats(TYPE, MC) * 4;
+                    {
+                        // the warps that share the step take turns at splitting activation rows
+                        const int t = kWide ? (warp - (st >> 1) * m) & 7 : (warp - st * m) & 15;
+                        if (t < m) {
+                            const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+                            tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
+                            const uint32_t part = tile == group ? norm_parts + ((step - step0) * MC + t) * 4 : 0u;
+                            tc_convert<TYPE, MC>(a, at + kTcRows * kPitch + t * (kTcStepCols * 4), t, step * kTcStepCols, cols_here,
+                                                 b_ring + bs * (Shape::kGroupsB * kTcGroupB), info, part, lane);
+                            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                            __syncwarp();
+                            if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[bs]));
+                        }
+                    }
+                    const uint32_t row = at + (slot * 32 + lane) * kPitch + ((mis0 + static_cast<uint32_t>(step) * kStepBytes) & 15u);
+                    const uint32_t wempty = tc::s32(&s_wempty[stage]);
+
+                    auto unit = [&](auto odd_tag) {
+                        constexpr bool O = decltype(odd_tag)::value != 0;
+                        constexpr bool kRowAddress = TYPE == kQ8_0 || TYPE == kIQ4_NL;
+                        const uint32_t line = kRowAddress ? row : row & ~7u, sh = (row & 2u) * 8u;
+                        TcUnit<TYPE> u[tc_halves(TYPE)];
+                        auto batch = [&](auto half_tag, auto batch_tag) {
+                            constexpr int H = decltype(half_tag)::value, B = decltype(batch_tag)::value, kBC = tc_batch_chunks<TYPE, MC>();
+                            constexpr bool kFirst = H == 0 && B == 0, kLast = H == tc_halves(TYPE) - 1 && B == tc_half_batches<TYPE, MC>() - 1;
+                            const int half = kWide ? H : kh;
+                            if constexpr (B == 0) u[H].template begin<O>(line, sh, half);
+                            uint32_t r[32];
+                            u[H].template chunk<O, B * kBC>(line, sh, half, r);
+                            if constexpr (kLast && kBC == 1) {  // everything of the stage has been read
+                                __syncwarp();
+                                if (lane == 0) tc::bar_arrive(wempty);
+                            }
+                            if (started) {  // the previous batch's MMAs: A may be overwritten, sums are complete
+                                tc::bar_wait(mma_done, dphase, failed);
+                                dphase ^= 1u;
+                                tc::fence_after();
+                            }
+                            tc::st32(tm_mine, r);
+                            if constexpr (kFirst || tc_fresh_batches(TYPE)) {
+                                if (pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
+                            }
+                            if constexpr (kBC == 2) {
+                                u[H].template chunk<O, B * kBC + 1>(line, sh, half, r);
+                                if constexpr (kLast) {
+                                    __syncwarp();
+                                    if (lane == 0) tc::bar_arrive(wempty);
+                                }
+                                tc::st32(tm_mine + 32, r);
+                            }
+                            tc::wait_st();
+                            tc::fence_before();
+                            __syncwarp();
+                            if (lane == 0) tc::bar_arrive(a_full);
+                            started = true;
+                            if constexpr (kLast || tc_fresh_batches(TYPE)) {
+#pragma unroll
+                                for (int h = 0; h < tc_halves(TYPE); ++h)
+                                    if (tc_mins(TYPE) > 0) pend.unit[h] = u[h];
+                                pend.info = info, pend.kh = kh;
+#pragma unroll
+                                for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = u[H].scale(tc_block32(TYPE) ? 2 * B * kBC + g : 0);
+                                pending = true;
+                            }
+                        };
+                        batch(TcInt<0>{}, TcInt<0>{});
+                        if constexpr (tc_half_batches<TYPE, MC>() > 1) batch(TcInt<0>{}, TcInt<1>{});
+                        if constexpr (kWide) {
+                            batch(TcInt<1>{}, TcInt<0>{});
+                            if constexpr (tc_half_batches<TYPE, MC>() > 1) batch(TcInt<1>{}, TcInt<1>{});
+                        }
+                    };
+                    if constexpr (block_align(TYPE) >= 8 || TYPE == kQ8_0 || TYPE == kIQ4_NL) {
+                        unit(TcInt<0>{});
+                    } else {
+                        if (row & 4u) unit(TcInt<1>{});
+                        else unit(TcInt<0>{});
+                    }
+                }
+                ++st;
+                if (++stage == kStages) stage = 0, wphase ^= 1u;
+                if (++bs == kNB) bs = 0, bphase ^= 1u;
+            }
+            // ---- the tile's last sums, then the outputs ----
+            if (started) {
+                tc::bar_wait(mma_done, dphase, failed);
+                dphase ^= 1u;
+                tc::fence_after();
+                tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
+            }
+            pending = started = false;
+            tc::fence_before();
+            // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
+            // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
+            const int red_rows = kTcRows / k_split + 1;
+            if ((a.fuse & kFuseNorm) && tile == group) {
+                tc::decoders_sync();  // (the last squares have been stored)
+                if (warp < m) {
+                    float sq = 0.0f;
+                    for (int i = lane; i < step1 - step0; i += 32) sq += __uint_as_float(lds32(norm_parts + (i * MC + warp) * 4));
+#pragma unroll
+                    for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, off);
+                    if (k_split == 1) {
+                        if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(tc::s32(&s_norm[0][warp])), "f"(sq) : "memory");
+                    } else {
+                        if (!announced) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+                        announced = true;
+                        if (lane < k_split) tc::st_async(tc::in_block(tc::s32(&s_norm[rank][warp]), lane), sq, tc::in_block(tc::s32(&s_cluster), lane));
+                    }
+                }
+            }
+            const int r0 = rank * kTcRows / k_split, r1 = (rank + 1) * kTcRows / k_split;
+            {
+                const int r = cls + 8 * lane, owner = (r * k_split + k_split - 1) / kTcRows;
+                float out[MC];
+                acc.get(out);
+                const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * kTcRows / k_split)) * (MC * 4);
+                if (k_split == 1) {
+#pragma unroll
+                    for (int t = 0; t < MC; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + t * 4), "f"(out[t]) : "memory");
+                } else {
+                    if (!announced) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+                    announced = true;
+                    if (threadIdx.x == 0) {
+                        const int bytes = (r1 - r0) * (2 * MC * 4) * k_split + ((a.fuse & kFuseNorm) && tile == group ? m * k_split * 4 : 0);
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::s32(&s_cluster)), "r"(bytes) : "memory");
+                    }
+                    tc::st_async_row<MC>(tc::in_block(to, owner), out, tc::in_block(tc::s32(&s_cluster), owner));
+                }
+                acc.clear();
+            }
+            if (k_split == 1) {
+                tc::decoders_sync();
+            } else {
+                tc::bar_wait_cluster(tc::s32(&s_cluster), rphase, failed);
+                rphase ^= 1u;
+            }
+            {
+                const int t = warp & (MC - 1);
+                const MatvecPart &part = a.part[p];
+                if (t < m) {
+                    float factor = 1.0f;
+                    if (a.fuse & kFuseNorm) {
+                        float sq = 0.0f;
+                        for (int k = 0; k < k_split; ++k) sq += s_norm[k][t];
+                        factor = 1.0f / sqrtf(sq / static_cast<float>(a.cols) + a.eps);
+                    }
+                    for (int r = r0 + (warp / MC) * 32 + lane; r < r1; r += 512 / MC) {
+                        const int row = (tile - tile0) * kTcRows + r;
+                        if (row >= part.rows) break;
+                        float sum = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kMaxSplit; ++k)
+                            if (k < k_split) {
+                                const uint32_t at = red + ((2 * k * red_rows + (r - r0)) * MC + t) * 4;
+                                sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + MC * red_rows * 4));
+                            }
+                        if (a.fuse & kFuseNorm) sum *= factor;
+                        if (part.y != nullptr) {
+                            float *y = part.y + static_cast<size_t>(t) * part.rows + row;
+                            if (a.fuse & kFuseAdd) sum += *y;
+                            *y = sum;
+                        }
+                        if (tc_better(sum, row, best_v, best_i)) best_v = sum, best_i = row;
+                    }
+                }
+            }
+            if (tile + n_groups < n_tiles) {  // the sums may be overwritten once everybody has read them
+                tc::decoders_sync();
+                if (k_split > 1) {
+                    if (threadIdx.x < static_cast<unsigned>(k_split))
+                        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tc::in_block(tc::s32(&s_read), threadIdx.x))
+                                     : "memory");
+                    tc::bar_wait_cluster(tc::s32(&s_read), sphase, failed);
+                    sphase ^= 1u;
+                }
+            }
+        }
+    }
+    tc::fence_before();
+    __syncthreads();
+    if (k_split > 1 && warp >= 16) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // (every thread takes part)
+    if (warp == 0) {
+        tc::fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        if (lane == 0 && s_failed) atomicCAS(a.status, 0u, kStatusWaitExpired);
+    }
+    if (a.out_idx != nullptr) tc_finish_argmax<MC>(a, m, best_v, best_i, warp, lane, s_best_v, s_best_i, &s_last);
+}
+
+}  // namespace vqm
