@@ -62,6 +62,10 @@ struct MatvecArgs {
     const float *x2;         // [M][cols], with kFuseSiluMul
     const float *norm_w;     // [cols], with kFuseNorm
     float eps;               // rmsnorm epsilon
+    // Filled in by the launcher of the tensor-core matvec (so that no block starts with integer divisions):
+    int tc_steps[9];         // block k of a cluster takes the 256-column steps [tc_steps[k], tc_steps[k + 1])
+    int tc_deal, tc_deal_recip;  // rows of a tile that each block of a cluster finishes, and 65536 / tc_deal rounded up
+    unsigned char tc_map_shift[kMaxParts];  // log2 of the number of tensor maps of each tensor
     PushInfo push;           // all zero when the tensor is not sharded
 };
 

@@ -18,7 +18,7 @@
 // A block: 16 decoder warps in four groups, one copy warp and two warps that issue the MMAs of two groups each.  Two groups
 // share the 256 rows of a step (a superblock column of 256); the two pairs take the steps in turn, or half of the columns of
 // each (tc_wide).
-//   copy warp    one to eight TMA tile copies (the row classes below, tc_maps) and one bulk copy per activation row into
+//   copy warp    one to eight TMA tile copies (the row classes below) and one bulk copy per activation row into
 //                the stage ring;
 //   converters   the decoder warps take turns to split one activation row's 256 columns into the B operand (shared memory);
 //   decoders     raw words -> 64 A columns at a time (a "chunk": 32 tensor-memory columns), two chunks to a batch of
@@ -58,6 +58,10 @@ __host__ __device__ constexpr int tc_pitch(int type) {
     const int lines = (tc_step_bytes(type) + (block_align(type) >= 16 ? 0 : 16 - block_align(type)) + 15) / 16;
     return (lines | 1) * 16;
 }
+// Rows that are not 8-byte aligned are read either in 8-byte loads, by one of two copies of the decoder (rows that start in the
+// lower and in the upper word), or in 4-byte loads, which have twice the bank conflicts.  Q3_K 75776 x 5120, 1 row: 74 us with
+// two copies (they do not fit into the instruction cache), 64 us with word loads; Q6_K, which loads twice as much: 84 and 88.
+__host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(type) < 8 && type != kQ6_K; }
 // A columns per weight: 2 where quant times sub-scale needs more than 11 bits and is split in two
 __host__ __device__ constexpr int tc_parts(int type) { return type == kQ6_K ? 2 : 1; }
 // types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit
@@ -68,9 +72,9 @@ enum : int { kOrderNibbles = 0, kOrderBytes = 1, kOrderGrid = 2 };
 __host__ __device__ constexpr int tc_order(int type) {
     return grid_is_codebook(type) ? kOrderGrid : (type == kIQ4_NL || type == kIQ4_XS) ? kOrderBytes : kOrderNibbles;
 }
-// tensor maps of a weight tensor (vqm_tcmv_maps.cu): its row classes share 1, 2, 4 or 8
-__host__ __device__ inline int tc_maps(int rows, long long row_bytes) {
-    return rows % 8 != 0 ? 8 : row_bytes % 16 == 0 ? 1 : row_bytes % 8 == 0 ? 2 : row_bytes % 4 == 0 ? 4 : 8;
+// log2 of the number of tensor maps of a weight tensor (vqm_tcmv_maps.cu): its row classes share 1, 2, 4 or 8
+inline int tc_map_shift(int rows, long long row_bytes) {
+    return rows % 8 != 0 ? 3 : row_bytes % 16 == 0 ? 0 : row_bytes % 8 == 0 ? 1 : row_bytes % 4 == 0 ? 2 : 3;
 }
 struct TcMaps1 {
     CUtensorMap m[1][8];
@@ -152,31 +156,16 @@ static __device__ __noinline__ bool give_up(unsigned long long *began, volatile 
     if (now - *began > 2000000000ull) *failed = 1;
     return *failed != 0;
 }
-// Up to `n` polls by a converged warp.  The vote makes the outcome uniform, so that a wait that is already over costs three
-// instructions (no reconvergence code).
-__device__ __forceinline__ bool bar_poll(uint32_t bar, uint32_t parity, uint32_t n) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 i;\n\t"
-        "mov.u32 i, %3;\n"
-        "AGAIN_%=:\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
-        "@q bra.uni DONE_%=;\n\t"
-        "sub.u32 i, i, 1;\n\t"
-        "setp.ne.u32 p, i, 0;\n\t"
-        "@p bra.uni AGAIN_%=;\n"
-        "DONE_%=:\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(n)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int *failed) {  // whole warp
+// (A form with a vote, so that the branches are uniform and need no reconvergence code, was measured: 8 % slower kernels.  It
+// polls faster, and polls of one warp delay the barriers of the others.)
+__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int *failed) {
+    if (bar_try(bar, parity)) return;
     unsigned long long began = 0;
-    while (!bar_poll(bar, parity, 256u))
-        if (give_up(&began, failed)) break;
+#pragma unroll 1
+    for (uint32_t i = 1;; ++i) {
+        if (bar_try(bar, parity)) return;
+        if ((i & 255u) == 0 && give_up(&began, failed)) return;
+    }
 }
 // acquire at cluster scope, for what other blocks of the cluster have stored
 __device__ __forceinline__ void bar_wait_cluster(uint32_t bar, uint32_t parity, volatile int *failed) {
@@ -187,13 +176,6 @@ __device__ __forceinline__ void bar_wait_cluster(uint32_t bar, uint32_t parity, 
         if (bar_try_cluster(bar, parity)) return;
         if ((i & 255u) == 0 && give_up(&began, failed)) return;
     }
-}
-// a wait of one thread
-__device__ __forceinline__ void bar_wait_one(uint32_t bar, uint32_t parity, volatile int *failed) {
-    unsigned long long began = 0;
-#pragma unroll 1
-    for (uint32_t i = 1; !bar_try(bar, parity); ++i)
-        if ((i & 255u) == 0 && give_up(&began, failed)) return;
 }
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
@@ -307,7 +289,8 @@ constexpr uint32_t kHi1024 = 0x64646464u, kHi64 = 0x54545454u;  // 1024 + b, 64 
 
 // ---- raw words of a row -------------------------------------------------------------------------------------------------
 // N consecutive 32-bit words at byte OFF (a multiple of 4) behind the row's first byte.  `line` is the row's address rounded
-// down to 8; O says whether the row starts in the upper word there, `sh` is 16 if it starts in the middle of a word.
+// down to 8 (4 with word loads); O says whether the row starts in the upper word there, `sh` is 16 if it starts in the middle of
+// a word.
 template <int TYPE, bool O, int OFF, int N>
 __device__ __forceinline__ void words(uint32_t line, uint32_t sh, uint32_t (&w)[N]) {
     constexpr int A = block_align(TYPE);
@@ -317,6 +300,13 @@ __device__ __forceinline__ void words(uint32_t line, uint32_t sh, uint32_t (&w)[
             const uint4 v = lds128u(line + OFF + 16 * i);
             w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
         }
+    } else if constexpr (tc_word_loads(TYPE)) {
+        constexpr bool kShift = A < 4;
+        uint32_t r[N + 1];
+#pragma unroll
+        for (int i = 0; i < N + (kShift ? 1 : 0); ++i) r[i] = lds32(line + OFF + 4 * i);
+#pragma unroll
+        for (int i = 0; i < N; ++i) w[i] = kShift ? __funnelshift_r(r[i], r[i + 1], sh) : r[i];
     } else {
         constexpr int first = (OFF / 4) % 2 + (O ? 1 : 0);  // word of the first 8-byte load that holds word 0
         constexpr int skip = first >= 2 ? 8 : 0, lead = first % 2;

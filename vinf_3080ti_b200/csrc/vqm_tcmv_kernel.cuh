@@ -27,21 +27,28 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
 }
 
 // Converts activation row t's 256 columns of a step into the B operand: called by a whole warp, lane = core row.
-//   xs: the row's columns in the stage; cols_here: how many exist; info: where the row's scale and group sums go (floats
+//   xs: the row's columns in the stage (not STAGED: they come straight from global memory); cols_here: how many exist; info: where the row's scale and group sums go (floats
 //   [MC] scales, padded to 4, then [groups][MC]); norm_part: where the row's sum of squares goes (0: nowhere)
-template <int TYPE, int MC>
+template <int TYPE, int MC, bool STAGED>
 __device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, int t, int col0, int cols_here, uint32_t b_stage, uint32_t info,
                                            uint32_t norm_part, int lane) {
     int ca, cb;
     tc_columns<TYPE>(lane, ca, cb);
     float v[8];
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(xs + ca * 4));
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(xs + cb * 4));
     const bool has_a = ca < cols_here, has_b = cb < cols_here;  // cols are multiples of 32: a word exists as a whole
+    if constexpr (STAGED) {
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(xs + ca * 4));
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(xs + cb * 4));
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        v[i] = has_a ? v[i] : 0.0f;
-        v[4 + i] = has_b ? v[4 + i] : 0.0f;
+        for (int i = 0; i < 4; ++i) {
+            v[i] = has_a ? v[i] : 0.0f;
+            v[4 + i] = has_b ? v[4 + i] : 0.0f;
+        }
+    } else {
+        const float *x = args.x + static_cast<size_t>(t) * args.cols + col0;
+        const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 xa = has_a ? __ldcg(reinterpret_cast<const float4 *>(x + ca)) : z, xb = has_b ? __ldcg(reinterpret_cast<const float4 *>(x + cb)) : z;
+        v[0] = xa.x, v[1] = xa.y, v[2] = xa.z, v[3] = xa.w, v[4] = xb.x, v[5] = xb.y, v[6] = xb.z, v[7] = xb.w;
     }
     if (args.fuse & (kFuseSiluMul | kFuseNorm)) {
         if (args.fuse & kFuseSiluMul) {
@@ -313,9 +320,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     volatile int *failed = &s_failed;
 
     const int k_split = a.k_split;
-    const int rank = static_cast<int>(blockIdx.x) % k_split, group = static_cast<int>(blockIdx.x) / k_split, n_groups = static_cast<int>(gridDim.x) / k_split;
-    const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
-    const int step0 = rank * n_steps / k_split, step1 = (rank + 1) * n_steps / k_split;
+    int rank, group, n_groups;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%clusterid.x;" : "=r"(group));
+    asm("mov.u32 %0, %%nclusterid.x;" : "=r"(n_groups));
+    const int step0 = a.tc_steps[rank], step1 = a.tc_steps[rank + 1];
     auto tiles_of = [&](int p) { return (a.part[p].rows + kTcRows - 1) / kTcRows; };
     const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = end2 + tiles_of(3);
     // the tensor a tile belongs to, and that tensor's first tile
@@ -326,17 +335,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     auto class_mis = [&](const MatvecPart &p, int c) {
         return static_cast<uint32_t>((reinterpret_cast<uintptr_t>(p.w) + static_cast<uintptr_t>(c) * static_cast<uintptr_t>(a.row_bytes)) & 15u);
     };
-    auto copy_weights = [&](int tile, int step, int stage) {  // one thread
+    auto copy_weights = [&](int tile, int step, int stage, bool with_x) {  // one thread
         const int p = part_of(tile), y = (tile - first_tile(p)) * 32;
         const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
         const uint32_t bar = tc::s32(&s_wfull[stage]), at = stages + stage * kStageBytes;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcRows * kPitch + m * cols_here * 4) : "memory");
-        const int n = tc_maps(a.part[p].rows, a.row_bytes);  // map c brings classes c, c + n, c + 2n, ...
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcRows * kPitch + (with_x ? m * cols_here * 4 : 0))
+                     : "memory");
+        const int shift = a.tc_map_shift[p];  // map c of n brings classes c, c + n, c + 2n, ...
 #pragma unroll 1
-        for (int c = 0; c < n; ++c) {
+        for (int c = 0; c < 1 << shift; ++c) {
             const uint32_t x = ((class_mis(a.part[p], c) + static_cast<uint32_t>(step) * kStepBytes) & ~15u) / kTcElemBytes;
             asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-                             at + c * (8 / n) * 32 * kPitch),
+                             at + ((c * 8) >> shift) * 32 * kPitch),
                          "l"(&maps.m[p][c]), "r"(x), "r"(y), "r"(0), "r"(bar)
                          : "memory");
         }
@@ -350,6 +360,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                          : "memory");
     };
 
+    if (warp == 17) {  // the first tile's maps, while the barriers are being set up
+        const int p = part_of(group);
+        if (lane < 1 << a.tc_map_shift[p]) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.m[p][lane]) : "memory");
+    }
     if (warp == 16 && tc::elect_one()) {
         for (int s = 0; s < kStages; ++s) {
             tc::bar_init(tc::s32(&s_wfull[s]), 1);
@@ -367,12 +381,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         tc::bar_init(tc::s32(&s_read), static_cast<uint32_t>(k_split));
         s_failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // weights never depend on an earlier kernel: the first stages are requested before anything else
         int t = group, k = step0;
 #pragma unroll 1
         for (int s = 0; s < kStages && t < n_tiles; ++s) {
-            copy_weights(t, k, s);
+            copy_weights(t, k, s, s >= kNB);
             if (++k == step1) k = step0, t += n_groups;
         }
     }
@@ -400,11 +413,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             for (int tile = group; tile < n_tiles && !*failed; tile += n_groups)
                 for (int step = step0; step < step1; ++step) {
                     if (filled >= kStages) {
-                        tc::bar_wait_one(tc::s32(&s_wempty[stage]), phase ^ 1u, failed);
+                        tc::bar_wait(tc::s32(&s_wempty[stage]), phase ^ 1u, failed);
                         if (*failed) break;
-                        copy_weights(tile, step, stage);
+                        copy_weights(tile, step, stage, filled >= kNB);
                     }
-                    copy_x(step, stage);
+                    if (filled >= kNB) copy_x(step, stage);
                     ++filled;
                     if (++stage == kStages) stage = 0, phase ^= 1u;
                 }
@@ -469,10 +482,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         TcAcc<MC> acc;
         acc.clear();
 
+        // The first kNB steps' activations are converted by all warps at once, straight from global memory: the way through the
+        // stages would put a copy and a turn of conversions (1 us) between the end of the previous kernel and the first MMAs.
+        for (int n = 0, t = warp;; t += 16) {
+            while (t >= m && n < kNB) t -= m, ++n;
+            if (n == kNB) break;
+            int local = n;
+            while (local >= step1 - step0) local -= step1 - step0;
+            const int step = step0 + local;
+            const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+            tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, b_ring + n * (Shape::kGroupsB * kTcGroupB),
+                                        info_ring + n * tc_info_floats(TYPE, MC) * 4, n == local ? norm_parts + (n * MC + t) * 4 : 0u, lane);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[n]));
+        }
+
         for (int tile = group; tile < n_tiles; tile += n_groups) {
             const int p = part_of(tile), tile0 = first_tile(p);
             const uint32_t mis0 = class_mis(a.part[p], cls);
-            const int n_maps = tc_maps(a.part[p].rows, a.row_bytes), slot = (cls % n_maps) * (8 / n_maps) + cls / n_maps;  // where the class lies
+            const int shift = a.tc_map_shift[p], slot = (((cls & ((1 << shift) - 1)) * 8) >> shift) + (cls >> shift);  // where the class lies
             for (int step = step0; step < step1; ++step) {
                 if (!kWide || (st & 1) == pair) {
                     tc::bar_wait(tc::s32(&s_wfull[stage]), wphase, failed);
@@ -480,11 +509,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     {
                         // the warps that share the step take turns at splitting activation rows
                         const int t = kWide ? (warp - (st >> 1) * m) & 7 : (warp - st * m) & 15;
-                        if (t < m) {
+                        if (t < m && st >= kNB) {
                             const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
                             tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
                             const uint32_t part = tile == group ? norm_parts + ((step - step0) * MC + t) * 4 : 0u;
-                            tc_convert<TYPE, MC>(a, at + kTcRows * kPitch + t * (kTcStepCols * 4), t, step * kTcStepCols, cols_here,
+                            tc_convert<TYPE, MC, true>(a, at + kTcRows * kPitch + t * (kTcStepCols * 4), t, step * kTcStepCols, cols_here,
                                                  b_ring + bs * (Shape::kGroupsB * kTcGroupB), info, part, lane);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                             __syncwarp();
@@ -497,16 +526,16 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     auto unit = [&](auto odd_tag) {
                         constexpr bool O = decltype(odd_tag)::value != 0;
                         constexpr bool kRowAddress = TYPE == kQ8_0 || TYPE == kIQ4_NL;
-                        const uint32_t line = kRowAddress ? row : row & ~7u, sh = (row & 2u) * 8u;
+                        const uint32_t line = kRowAddress ? row : row & (tc_word_loads(TYPE) ? ~3u : ~7u), sh = (row & 2u) * 8u;
+                        constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_half_batches<TYPE, MC>();
                         TcUnit<TYPE> u[tc_halves(TYPE)];
-                        auto batch = [&](auto half_tag, auto batch_tag) {
-                            constexpr int H = decltype(half_tag)::value, B = decltype(batch_tag)::value, kBC = tc_batch_chunks<TYPE, MC>();
-                            constexpr bool kFirst = H == 0 && B == 0, kLast = H == tc_halves(TYPE) - 1 && B == tc_half_batches<TYPE, MC>() - 1;
-                            const int half = kWide ? H : kh;
-                            if constexpr (B == 0) u[H].template begin<O>(line, sh, half);
+                        auto batch = [&](TcUnit<TYPE> &v, int half, auto batch_tag, bool first_half, bool last_half) {
+                            constexpr int B = decltype(batch_tag)::value;
+                            const bool first = first_half && B == 0, last = last_half && B == kBatches - 1;
+                            if constexpr (B == 0) v.template begin<O>(line, sh, half);
                             uint32_t r[32];
-                            u[H].template chunk<O, B * kBC>(line, sh, half, r);
-                            if constexpr (kLast && kBC == 1) {  // everything of the stage has been read
+                            v.template chunk<O, B * kBC>(line, sh, half, r);
+                            if (kBC == 1 && last) {  // everything of the stage has been read
                                 __syncwarp();
                                 if (lane == 0) tc::bar_arrive(wempty);
                             }
@@ -516,12 +545,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                 tc::fence_after();
                             }
                             tc::st32(tm_mine, r);
-                            if constexpr (kFirst || tc_fresh_batches(TYPE)) {
-                                if (pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
-                            }
+                            if ((first || tc_fresh_batches(TYPE)) && pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
                             if constexpr (kBC == 2) {
-                                u[H].template chunk<O, B * kBC + 1>(line, sh, half, r);
-                                if constexpr (kLast) {
+                                v.template chunk<O, B * kBC + 1>(line, sh, half, r);
+                                if (last) {
                                     __syncwarp();
                                     if (lane == 0) tc::bar_arrive(wempty);
                                 }
@@ -532,24 +559,29 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             __syncwarp();
                             if (lane == 0) tc::bar_arrive(a_full);
                             started = true;
-                            if constexpr (kLast || tc_fresh_batches(TYPE)) {
+                            if (last || tc_fresh_batches(TYPE)) {
+                                if constexpr (tc_mins(TYPE) > 0) {
 #pragma unroll
-                                for (int h = 0; h < tc_halves(TYPE); ++h)
-                                    if (tc_mins(TYPE) > 0) pend.unit[h] = u[h];
+                                    for (int h = 0; h < tc_halves(TYPE); ++h) pend.unit[h] = u[h];
+                                }
                                 pend.info = info, pend.kh = kh;
 #pragma unroll
-                                for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = u[H].scale(tc_block32(TYPE) ? 2 * B * kBC + g : 0);
+                                for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = v.scale(tc_block32(TYPE) ? 2 * B * kBC + g : 0);
                                 pending = true;
                             }
                         };
-                        batch(TcInt<0>{}, TcInt<0>{});
-                        if constexpr (tc_half_batches<TYPE, MC>() > 1) batch(TcInt<0>{}, TcInt<1>{});
-                        if constexpr (kWide) {
-                            batch(TcInt<1>{}, TcInt<0>{});
-                            if constexpr (tc_half_batches<TYPE, MC>() > 1) batch(TcInt<1>{}, TcInt<1>{});
+                        auto half_unit = [&](TcUnit<TYPE> &v, int half, bool first, bool last) {
+                            batch(v, half, TcInt<0>{}, first, last);
+                            if constexpr (kBatches > 1) batch(v, half, TcInt<1>{}, first, last);
+                        };
+                        if constexpr (!kWide) {
+                            half_unit(u[0], kh, true, true);
+                        } else {  // (a loop over the halves was measured: smaller code, but 7 % slower)
+                            half_unit(u[0], 0, true, false);
+                            half_unit(u[1], 1, false, true);
                         }
                     };
-                    if constexpr (block_align(TYPE) >= 8 || TYPE == kQ8_0 || TYPE == kIQ4_NL) {
+                    if constexpr (block_align(TYPE) >= 8 || tc_word_loads(TYPE)) {
                         unit(TcInt<0>{});
                     } else {
                         if (row & 4u) unit(TcInt<1>{});
@@ -571,7 +603,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             tc::fence_before();
             // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
             // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
-            const int red_rows = kTcRows / k_split + 1;
+            const int red_rows = a.tc_deal;
             if ((a.fuse & kFuseNorm) && tile == group) {
                 tc::decoders_sync();  // (the last squares have been stored)
                 if (warp < m) {
@@ -588,12 +620,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     }
                 }
             }
-            const int r0 = rank * kTcRows / k_split, r1 = (rank + 1) * kTcRows / k_split;
+            const int r0 = rank * red_rows, r1 = r0 + red_rows < kTcRows ? r0 + red_rows : kTcRows;
             {
-                const int r = cls + 8 * lane, owner = (r * k_split + k_split - 1) / kTcRows;
+                const int r = cls + 8 * lane, owner = (r * a.tc_deal_recip) >> 16;
                 float out[MC];
                 acc.get(out);
-                const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * kTcRows / k_split)) * (MC * 4);
+                const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * red_rows)) * (MC * 4);
                 if (k_split == 1) {
 #pragma unroll
                     for (int t = 0; t < MC; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + t * 4), "f"(out[t]) : "memory");

@@ -23,7 +23,7 @@ cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_b
         encode = reinterpret_cast<Encode>(fn);
     }
     const cuuint32_t elem = kTcElemBytes;
-    const int n = tc_maps(rows, row_bytes);
+    const int n = 1 << tc_map_shift(rows, row_bytes);
     const cuuint32_t box[3] = {static_cast<cuuint32_t>(tc_pitch(type)) / elem, 32, static_cast<cuuint32_t>(8 / n)}, step[3] = {1, 1, 1};
     const cuuint64_t stride[2] = {static_cast<cuuint64_t>(row_bytes) * 8, static_cast<cuuint64_t>(row_bytes) * (n == 8 ? 8 : n)};
     for (int c = 0; c < n; ++c) {

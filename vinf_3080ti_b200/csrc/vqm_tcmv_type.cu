@@ -103,6 +103,11 @@ cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const C
     int n_tiles = 0;
     for (int p = 0; p < kMaxParts; ++p) n_tiles += (a.part[p].rows + kTcRows - 1) / kTcRows;
     a.k_split = choose_tc_split(n_tiles, a.cols, a.allow_split, sm_count);
+    const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
+    for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
+    a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
+    a.tc_deal_recip = 65536 / a.tc_deal + 1;
+    for (int p = 0; p < n_parts; ++p) a.tc_map_shift[p] = static_cast<unsigned char>(tc_map_shift(a.part[p].rows, a.row_bytes));
 #define VQM_LAUNCH(MC)                                                                                           \
     (n_parts == 1 ? TcVariant<MC, TcMaps1>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream)                \
                   : TcVariant<MC, TcMaps4>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream))
