@@ -30,7 +30,7 @@ LIB = HERE / "libvinf_b200.so"
 TYPES = [(0, "F32"), (1, "F16"), (8, "Q8_0"), (10, "Q2_K"), (11, "Q3_K"), (12, "Q4_K"), (13, "Q5_K"), (14, "Q6_K"),
          (16, "IQ2_XXS"), (17, "IQ2_XS"), (18, "IQ3_XXS"), (20, "IQ4_NL"), (21, "IQ3_S"), (22, "IQ2_S"), (23, "IQ4_XS")]
 
-TC_TYPES = [t for t in TYPES if t[0] not in (0, 1, 16, 17, 18, 21, 22)]  # types of the tensor-core matvec
+TC_TYPES = [t for t in TYPES if t[0] not in (0, 1)]  # types of the tensor-core matvec
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

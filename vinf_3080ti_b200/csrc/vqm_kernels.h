@@ -86,9 +86,11 @@ enum : unsigned { kStatusOk = 0, kStatusWaitExpired = 1, kStatusPeerWaitExpired 
 VQM_FOR_EACH_TYPE(VQM_DECLARE_LAUNCHER)
 #undef VQM_DECLARE_LAUNCHER
 
+constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matvec: times 31 it has to fit into the 11 bits of fp16
 // The tensor-core matvec (vqm_tcmv_type.cu).  maps: per tensor of the launch its tensor maps (tc_encode_maps).
 #define VQM_FOR_EACH_TC_TYPE(X) \
-    X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(20, IQ4_NL) X(23, IQ4_XS)
+    X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(16, IQ2_XXS) X(17, IQ2_XS) X(18, IQ3_XXS) \
+    X(20, IQ4_NL) X(21, IQ3_S) X(22, IQ2_S) X(23, IQ4_XS)
 #define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
     cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, \
                                    cudaStream_t stream);

@@ -78,6 +78,7 @@ struct vqm_runtime {
     std::unordered_map<std::string, Tensor> tensors;
     std::unordered_map<std::string, Buffer> buffers;
     uint8_t *codebooks[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    bool codebook_small[5] = {};  // every magnitude is within kTcMaxMagnitude (those of the format are)
     // fixed device scratch: status word, argmax partials/results
     unsigned *status = nullptr;
     unsigned *done_counter = nullptr;
@@ -199,8 +200,9 @@ cudaError_t dispatch_qmv(int type, const vqm::MatvecArgs &a, int m, int sm_count
     }
 }
 
-// Whether a launch runs on the tensor-core matvec.
-bool use_tcmv(int type, const vqm::MatvecArgs &a) {
+// Whether a launch runs on the tensor-core matvec.  codebook_small: see vqm_runtime (a codebook nobody has looked at is not).
+bool use_tcmv(int type, const vqm::MatvecArgs &a, bool codebook_small) {
+    if (vqm::grid_is_codebook(type) && !codebook_small) return false;
     if (a.push.push_slot > 0 || a.push.wait_slot > 0) return false;
     if ((a.fuse & vqm::kFuseNorm) && a.cols > 128 * 256) return false;
     switch (type) {
@@ -223,7 +225,7 @@ cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap 
 
 // One tensor in device memory that has no Tensor record.
 cudaError_t dispatch_raw(int type, const vqm::MatvecArgs &a, int m, int sm_count, cudaStream_t stream) {
-    if (!use_tcmv(type, a)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
+    if (!use_tcmv(type, a, false)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
     CUtensorMap maps[8];
     const CUtensorMap *p[1] = {maps};
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, maps);
@@ -301,7 +303,10 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         a.row_base = t0.argmax_row_base;
     }
     cudaError_t err = cudaSuccess;
-    if (use_tcmv(t0.type, a)) {
+    bool codebook_small = false;
+    for (int i = 0; i < 5; ++i)
+        if (kCodebookTypes[i] == t0.type) codebook_small = rt->codebook_small[i];
+    if (use_tcmv(t0.type, a, codebook_small)) {
         const CUtensorMap *maps[vqm::kMaxParts];
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
             if (ts[i]->maps.empty()) {
@@ -438,6 +443,9 @@ int vqm_set_codebook(vqm_runtime *rt, const char *name, const void *data, size_t
         if (rt->codebooks[i] == nullptr) err = cudaMalloc(&rt->codebooks[i], want);
         if (err == cudaSuccess) err = cudaMemcpy(rt->codebooks[i], data, want, cudaMemcpyHostToDevice);
         if (err != cudaSuccess) return cuda_fail("codebook upload", err);
+        rt->codebook_small[i] = true;
+        for (size_t k = 0; k < want; ++k)
+            if (static_cast<const uint8_t *>(data)[k] > vqm::kTcMaxMagnitude) rt->codebook_small[i] = false;
         return VQM_OK;
     }
     return fail(VQM_ERR_KEY, "unknown codebook %s", name);

@@ -342,4 +342,180 @@ struct TcUnit<kIQ4_XS> {
     }
 };
 
+// ---- codebook types ------------------------------------------------------------------------------------------------------
+// Eight weights are magnitude bytes of a codebook in shared memory (one 8-byte or two 4-byte entries), eight sign bits and an
+// odd scale 2 s + 1 <= 31; magnitudes are at most 66 (the host checks the codebook), so magnitude * scale is exact in fp16.
+// The constant factor (1/8, 1/4 or 1) goes into d.  About 25 instructions per 8 weights: two or three for the index, two masks
+// per four magnitudes, one multiply, one shift and one LOP3 for the signs per two.
+struct TcGrid {
+    float d;
+    uint32_t table;  // the codebook
+    __device__ __forceinline__ float scale(int) const { return d; }
+
+    // fp16 2 s + 1, twice, from the byte 2 s + 1
+    static __device__ __forceinline__ uint32_t odd_scale(uint32_t b) { return tc::hadd2(tc::byte_h2<0>(b, tc::kHi1024), 0xE400E400u); }
+    // A core row from two words of magnitudes and the sign byte.  v = signs | signs << 14 puts the signs of weights (i, i + 2)
+    // 16 bits apart.  emit7: bit 31 of `eighth` flips weight 7 (types whose eighth sign is implied).
+    static __device__ __forceinline__ void emit(uint32_t m0, uint32_t m1, uint32_t signs, uint32_t k, uint32_t *r) {
+        const uint32_t v = signs * 0x4001u;
+        r[0] = tc::hmul2(m0 & 0x00FF00FFu, k) ^ ((v << 15) & 0x80008000u);
+        r[1] = tc::hmul2(__byte_perm(m0, 0u, 0x4341), k) ^ ((v << 14) & 0x80008000u);
+        r[2] = tc::hmul2(m1 & 0x00FF00FFu, k) ^ ((v << 11) & 0x80008000u);
+        r[3] = tc::hmul2(__byte_perm(m1, 0u, 0x4341), k) ^ ((v << 10) & 0x80008000u);
+    }
+    static __device__ __forceinline__ void emit7(uint32_t m0, uint32_t m1, uint32_t signs7, uint32_t eighth, uint32_t k, uint32_t *r) {
+        emit(m0, m1, signs7, k, r);
+        r[3] ^= eighth & 0x80000000u;
+    }
+    // bit 7 l: the parity of bits 7 l .. 7 l + 6
+    static __device__ __forceinline__ uint32_t parities(uint32_t x) {
+        const uint32_t x1 = x ^ (x >> 1), x2 = x1 ^ (x1 >> 2);
+        return x2 ^ (x1 >> 4) ^ (x >> 6);
+    }
+    __device__ __forceinline__ void entry8(uint32_t index, uint32_t &m0, uint32_t &m1) const {
+        const unsigned long long e = lds64(table + index * 8);
+        m0 = static_cast<uint32_t>(e), m1 = static_cast<uint32_t>(e >> 32);
+    }
+    __device__ __forceinline__ uint32_t entry4(uint32_t index) const { return lds32(table + index * 4); }
+};
+template <int K>
+__device__ __forceinline__ uint32_t tc_byte(uint32_t w) { return __byte_perm(w, 0u, 0x4440 | K); }
+// (everything behind the two bytes of d: the words() offsets of these types count from there)
+__device__ __forceinline__ uint32_t tc_line2(uint32_t row) { return (row + 2) & ~3u; }
+__device__ __forceinline__ uint32_t tc_shift2(uint32_t row) { return ((row + 2) & 2u) * 8u; }
+
+// IQ2_XXS: per 32 weights four index bytes and a word of 4 x 7 signs and a 4-bit scale.
+template <>
+struct TcUnit<kIQ2_XXS> : TcGrid {
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int) { d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f); }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[4];
+        tc::words<kIQ2_XXS, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t idx = w[2 * g], aux = w[2 * g + 1], par = parities(aux), k = odd_scale((aux >> 27) | 1u);
+            uint32_t m0, m1;
+            uint32_t *r = a + 16 * g;
+            entry8(tc_byte<0>(idx), m0, m1), emit7(m0, m1, aux & 127u, par << 31, k, r);
+            entry8(tc_byte<1>(idx), m0, m1), emit7(m0, m1, (aux >> 7) & 127u, par << 24, k, r + 4);
+            entry8(tc_byte<2>(idx), m0, m1), emit7(m0, m1, (aux >> 14) & 127u, par << 17, k, r + 8);
+            entry8(tc_byte<3>(idx), m0, m1), emit7(m0, m1, (aux >> 21) & 127u, par << 10, k, r + 12);
+        }
+    }
+};
+
+// IQ2_XS: 32 x (9-bit index, 7 signs) @2, 4-bit scale pairs @66.
+template <>
+struct TcUnit<kIQ2_XS> : TcGrid {
+    uint32_t sc;  // the half's four scale bytes: low nibble for the first 16 weights of 32, high for the others
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int kh) {
+        d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f);
+        uint32_t w[1];
+        tc::words<kIQ2_XS, false, 64, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        sc = w[0];
+    }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[4];
+        tc::words<kIQ2_XS, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // two entries, which share a scale
+            const uint32_t k = odd_scale(((sc >> (8 * (2 * CH + (i >> 1)) + 4 * (i & 1))) & 15u) * 2u + 1u);
+            uint32_t p = (w[i] >> 9) & 0x007F007Fu;
+            const uint32_t s = p;
+            p ^= p >> 4, p ^= p >> 2, p ^= p >> 1;  // bits 0 and 16: the parities
+            uint32_t m0, m1;
+            entry8(w[i] & 511u, m0, m1), emit7(m0, m1, s & 127u, p << 31, k, a + 8 * i);
+            entry8((w[i] >> 16) & 511u, m0, m1), emit7(m0, m1, s >> 16, p << 15, k, a + 8 * i + 4);
+        }
+    }
+};
+
+// IQ2_S: index low bytes @2, sign bytes @34, index high bits @66, scale pairs @74.
+template <>
+struct TcUnit<kIQ2_S> : TcGrid {
+    uint32_t sc, hi;
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int kh) {
+        d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f);
+        uint32_t w[1];
+        tc::words<kIQ2_S, false, 72, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        sc = w[0];
+        tc::words<kIQ2_S, false, 64, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        hi = w[0];
+    }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[2], s[2];
+        tc::words<kIQ2_S, false, 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), w);
+        tc::words<kIQ2_S, false, 32 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), s);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t b = sc >> (8 * (2 * CH + g)), q = hi >> (8 * (2 * CH + g));
+            const uint32_t k0 = odd_scale((b & 15u) * 2u + 1u), k1 = odd_scale(((b >> 4) & 15u) * 2u + 1u);
+            uint32_t m0, m1;
+            uint32_t *r = a + 16 * g;
+            entry8(tc_byte<0>(w[g]) | ((q << 8) & 0x300u), m0, m1), emit(m0, m1, tc_byte<0>(s[g]), k0, r);
+            entry8(tc_byte<1>(w[g]) | ((q << 6) & 0x300u), m0, m1), emit(m0, m1, tc_byte<1>(s[g]), k0, r + 4);
+            entry8(tc_byte<2>(w[g]) | ((q << 4) & 0x300u), m0, m1), emit(m0, m1, tc_byte<2>(s[g]), k1, r + 8);
+            entry8(tc_byte<3>(w[g]) | ((q << 2) & 0x300u), m0, m1), emit(m0, m1, tc_byte<3>(s[g]), k1, r + 12);
+        }
+    }
+};
+
+// IQ3_XXS: two index bytes per 8 weights @2, per 32 weights a word of 4 x 7 signs and a 4-bit scale @66.
+template <>
+struct TcUnit<kIQ3_XXS> : TcGrid {
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int) { d = half_bits_to_float(lds16(row)) * (kTc24 * 0.25f); }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[4], x[2];
+        tc::words<kIQ3_XXS, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
+        tc::words<kIQ3_XXS, false, 64 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), x);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t aux = x[g], par = parities(aux), k = odd_scale((aux >> 27) | 1u), i0 = w[2 * g], i1 = w[2 * g + 1];
+            uint32_t *r = a + 16 * g;
+            emit7(entry4(tc_byte<0>(i0)), entry4(tc_byte<1>(i0)), aux & 127u, par << 31, k, r);
+            emit7(entry4(tc_byte<2>(i0)), entry4(tc_byte<3>(i0)), (aux >> 7) & 127u, par << 24, k, r + 4);
+            emit7(entry4(tc_byte<0>(i1)), entry4(tc_byte<1>(i1)), (aux >> 14) & 127u, par << 17, k, r + 8);
+            emit7(entry4(tc_byte<2>(i1)), entry4(tc_byte<3>(i1)), (aux >> 21) & 127u, par << 10, k, r + 12);
+        }
+    }
+};
+
+// IQ3_S: index low bytes @2, index high bits @66, sign bytes @74, 4-bit scales @106.
+template <>
+struct TcUnit<kIQ3_S> : TcGrid {
+    uint32_t sc, hi;
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int kh) {
+        d = half_bits_to_float(lds16(row)) * kTc24;
+        uint32_t w[1];
+        tc::words<kIQ3_S, false, 104, 1>(tc_line2(row), tc_shift2(row), w);
+        sc = w[0] >> (16 * kh);
+        tc::words<kIQ3_S, false, 64, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        hi = w[0];
+    }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[4], s[2];
+        tc::words<kIQ3_S, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
+        tc::words<kIQ3_S, false, 72 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), s);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t k = odd_scale(((sc >> (4 * (2 * CH + g))) & 15u) * 2u + 1u), q = hi >> (8 * (2 * CH + g)), i0 = w[2 * g], i1 = w[2 * g + 1];
+            uint32_t *r = a + 16 * g;
+            emit(entry4(tc_byte<0>(i0) | ((q << 8) & 256u)), entry4(tc_byte<1>(i0) | ((q << 7) & 256u)), tc_byte<0>(s[g]), k, r);
+            emit(entry4(tc_byte<2>(i0) | ((q << 6) & 256u)), entry4(tc_byte<3>(i0) | ((q << 5) & 256u)), tc_byte<1>(s[g]), k, r + 4);
+            emit(entry4(tc_byte<0>(i1) | ((q << 4) & 256u)), entry4(tc_byte<1>(i1) | ((q << 3) & 256u)), tc_byte<2>(s[g]), k, r + 8);
+            emit(entry4(tc_byte<2>(i1) | ((q << 2) & 256u)), entry4(tc_byte<3>(i1) | ((q << 1) & 256u)), tc_byte<3>(s[g]), k, r + 12);
+        }
+    }
+};
+
 }  // namespace vqm

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // layout: stages (1024-byte aligned) | table | B ring | per-step info | sums of the tile | sums of squares
     const uint32_t stages = (tc::s32(tc_raw) + 1023u) & ~1023u;
-    const uint32_t table = stages + kStages * kStageBytes;
+    [[maybe_unused]] const uint32_t table = stages + kStages * kStageBytes;
     const uint32_t b_ring = table + (grid_bytes(TYPE) + 127) / 128 * 128;
     const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * kTcGroupB;
     const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
@@ -394,6 +394,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::s32(&s_tmem)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if constexpr (grid_is_codebook(TYPE)) {
+        for (int i = threadIdx.x; i < grid_bytes(TYPE) / 16; i += kTcThreads) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(a.codebook + i * 16);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(table + i * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+        }
     }
     tc::fence_before();
     __syncthreads();
@@ -525,13 +531,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
 
                     auto unit = [&](auto odd_tag) {
                         constexpr bool O = decltype(odd_tag)::value != 0;
-                        constexpr bool kRowAddress = TYPE == kQ8_0 || TYPE == kIQ4_NL;
+                        constexpr bool kRowAddress = TYPE == kQ8_0 || TYPE == kIQ4_NL || grid_is_codebook(TYPE);
                         const uint32_t line = kRowAddress ? row : row & (tc_word_loads(TYPE) ? ~3u : ~7u), sh = (row & 2u) * 8u;
                         constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_half_batches<TYPE, MC>();
                         TcUnit<TYPE> u[tc_halves(TYPE)];
                         auto batch = [&](TcUnit<TYPE> &v, int half, auto batch_tag, bool first_half, bool last_half) {
                             constexpr int B = decltype(batch_tag)::value;
                             const bool first = first_half && B == 0, last = last_half && B == kBatches - 1;
+                            if constexpr (grid_is_codebook(TYPE)) v.table = table;
                             if constexpr (B == 0) v.template begin<O>(line, sh, half);
                             uint32_t r[32];
                             v.template chunk<O, B * kBC>(line, sh, half, r);
