@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -65,10 +66,67 @@ struct Graph {
     bool uses_gemm_x = false;  // captured a prompt-pass GEMM, i.e. the address of the runtime's fp16 activation buffer
 };
 
+// Pinned staging that outlives a runtime: pinning a page costs more than a whole synchronous matvec.  Blocks are handed from a
+// destroyed runtime to the next one; at most kPinnedKeep bytes wait here, and none once the last runtime is gone.
+class PinnedPool {
+public:
+    void *take(size_t bytes, size_t *got) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        for (size_t i = 0; i < free_.size(); ++i)
+            if (free_[i].second >= bytes) {
+                void *p = free_[i].first;
+                *got = free_[i].second;
+                kept_ -= *got;
+                free_.erase(free_.begin() + static_cast<long>(i));
+                return p;
+            }
+        size_t size = 1u << 16;
+        while (size < bytes) size *= 2;
+        void *p = nullptr;
+        if (cudaMallocHost(&p, size) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        *got = size;
+        return p;
+    }
+    void give(void *p, size_t bytes) {
+        if (p == nullptr) return;
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (kept_ + bytes > kPinnedKeep) {
+            cudaFreeHost(p);
+            return;
+        }
+        free_.emplace_back(p, bytes);
+        kept_ += bytes;
+    }
+    void runtime_created() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        ++runtimes_;
+    }
+    void runtime_destroyed() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        if (--runtimes_ > 0) return;
+        for (auto &b : free_) cudaFreeHost(b.first);
+        free_.clear();
+        kept_ = 0;
+    }
+
+private:
+    static constexpr size_t kPinnedKeep = 8u << 20;
+    std::mutex mutex_;
+    std::vector<std::pair<void *, size_t>> free_;
+    size_t kept_ = 0;
+    int runtimes_ = 0;
+};
+PinnedPool g_pinned;
+
 const char *const kCodebookNames[5] = {"iq2xxs_grid", "iq2xs_grid", "iq2s_grid", "iq3xxs_grid", "iq3s_grid"};
 const int kCodebookTypes[5] = {vqm::kIQ2_XXS, vqm::kIQ2_XS, vqm::kIQ2_S, vqm::kIQ3_XXS, vqm::kIQ3_S};
 
 }  // namespace
+
+constexpr size_t kStatusWords = 4;  // status word of a synchronous matvec, padded to 16 bytes
 
 struct vqm_runtime {
     int device = 0;
@@ -88,8 +146,12 @@ struct vqm_runtime {
     float *argmax_vals = nullptr;  // [8]
     int allow_split = 1;  // short launches may be split by columns (VINF_B200_NO_SPLIT=1 turns it off)
     // scratch of the synchronous matvec entry
-    float *scratch_x = nullptr, *scratch_y = nullptr;
+    float *scratch_x = nullptr;
+    unsigned *scratch_y = nullptr;  // kStatusWords, then the outputs
     size_t scratch_x_n = 0, scratch_y_n = 0;
+    void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
+    size_t pinned_bytes = 0;
+    bool counted = false;    // by the pinned pool
     void *gemm_x = nullptr;  // fp16 copy of the activations of a prompt pass
     size_t gemm_x_len = 0;   // in elements
     // exchange of row-sharded outputs between ranks
@@ -200,17 +262,22 @@ cudaError_t dispatch_qmv(int type, const vqm::MatvecArgs &a, int m, int sm_count
     }
 }
 
-// Whether a launch runs on the tensor-core matvec.  codebook_small: see vqm_runtime (a codebook nobody has looked at is not).
-bool use_tcmv(int type, const vqm::MatvecArgs &a, bool codebook_small) {
-    if (vqm::grid_is_codebook(type) && !codebook_small) return false;
-    if (a.push.push_slot > 0 || a.push.wait_slot > 0) return false;
+// Whether a launch runs on the tensor-core matvec; sets a.k_split.  Launches that must not be split by columns stay on the
+// CUDA-core kernel, where an output does not depend on what else is in its launch.  codebook_small: see vqm_runtime (a codebook
+// nobody has looked at is not).
+bool use_tcmv(int type, vqm::MatvecArgs &a, int sm_count, bool codebook_small) {
+    if (a.push.push_slot > 0 || a.push.wait_slot > 0 || !a.allow_split) return false;
     if ((a.fuse & vqm::kFuseNorm) && a.cols > 128 * 256) return false;
+    if (vqm::grid_is_codebook(type) && !codebook_small) return false;
+    int split = 0;
     switch (type) {
-#define VQM_CASE(id, name) case id: return true;
+#define VQM_CASE(id, name) case id: split = vqm::split_tcmv_##name(a, sm_count); break;
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
-        default: return false;
+        default: break;
     }
+    if (split > 0) a.k_split = split;
+    return split > 0;
 }
 
 cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, cudaStream_t stream) {
@@ -224,8 +291,8 @@ cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap 
 }
 
 // One tensor in device memory that has no Tensor record.
-cudaError_t dispatch_raw(int type, const vqm::MatvecArgs &a, int m, int sm_count, cudaStream_t stream) {
-    if (!use_tcmv(type, a, false)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
+cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cudaStream_t stream) {
+    if (!use_tcmv(type, a, sm_count, false)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
     CUtensorMap maps[8];
     const CUtensorMap *p[1] = {maps};
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, maps);
@@ -306,7 +373,7 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
     bool codebook_small = false;
     for (int i = 0; i < 5; ++i)
         if (kCodebookTypes[i] == t0.type) codebook_small = rt->codebook_small[i];
-    if (use_tcmv(t0.type, a, codebook_small)) {
+    if (use_tcmv(t0.type, a, rt->sm_count, codebook_small)) {
         const CUtensorMap *maps[vqm::kMaxParts];
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
             if (ts[i]->maps.empty()) {
@@ -349,6 +416,11 @@ int resolve_group(vqm_runtime *rt, int n, const char *const *weights, const char
     return VQM_OK;
 }
 
+int status_failure(const char *ctx, unsigned status) {
+    return fail(VQM_ERR_CUDA, "%s failed: a kernel gave up a bounded wait (status %u: 1 = its own weight copies, 2 = another rank's push)", ctx,
+                status);
+}
+
 int check_status_word(vqm_runtime *rt, const char *ctx) {
     unsigned host = 0;
     cudaError_t err = cudaMemcpyAsync(&host, rt->status, sizeof(host), cudaMemcpyDeviceToHost, rt->stream);
@@ -356,8 +428,36 @@ int check_status_word(vqm_runtime *rt, const char *ctx) {
     if (err != cudaSuccess) return cuda_fail(ctx, err);
     if (host != 0) {
         cudaMemsetAsync(rt->status, 0, sizeof(unsigned), rt->stream);
-        return fail(VQM_ERR_CUDA, "%s failed: a kernel gave up a bounded wait (status %u: 1 = its own weight copies, 2 = another rank's push)",
-                    ctx, host);
+        return status_failure(ctx, host);
+    }
+    return VQM_OK;
+}
+
+// Device and pinned host scratch of the synchronous matvec, for vectors of at least this many columns and rows.
+int matvec_scratch(vqm_runtime *rt, size_t cols, size_t rows) {
+    cudaError_t err = cudaSuccess;
+    if (rt->scratch_x_n < cols) {
+        cudaFree(rt->scratch_x);
+        rt->scratch_x = nullptr;
+        rt->scratch_x_n = 0;
+        err = cudaMalloc(&rt->scratch_x, sizeof(float) * cols);
+        if (err == cudaSuccess) rt->scratch_x_n = cols;
+    }
+    if (err == cudaSuccess && rt->scratch_y_n < rows) {
+        cudaFree(rt->scratch_y);
+        rt->scratch_y = nullptr;
+        rt->scratch_y_n = 0;
+        err = cudaMalloc(&rt->scratch_y, sizeof(unsigned) * (kStatusWords + rows));
+        if (err == cudaSuccess) err = cudaMemsetAsync(rt->scratch_y, 0, sizeof(unsigned) * kStatusWords, rt->stream);
+        if (err == cudaSuccess) rt->scratch_y_n = rows;
+    }
+    if (err != cudaSuccess) return cuda_fail("scratch allocation", err);
+    const size_t bytes = sizeof(float) * (cols > rows + kStatusWords ? cols : rows + kStatusWords);
+    if (rt->pinned_bytes < bytes) {
+        g_pinned.give(rt->pinned, rt->pinned_bytes);
+        rt->pinned_bytes = 0;
+        rt->pinned = g_pinned.take(bytes, &rt->pinned_bytes);
+        if (rt->pinned == nullptr) return fail(VQM_ERR_MEMORY, "pinned staging of %zu bytes failed", bytes);
     }
     return VQM_OK;
 }
@@ -379,6 +479,8 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
         delete rt;
         return dev_rc;
     }
+    g_pinned.runtime_created();
+    rt->counted = true;
     cudaError_t err = cudaSuccess;
     if (err == cudaSuccess) err = cudaStreamCreate(&rt->own_stream);
     rt->stream = rt->own_stream;
@@ -424,6 +526,8 @@ void vqm_runtime_destroy(vqm_runtime *rt) {
     cudaFree(rt->argmax_vals);
     cudaFree(rt->scratch_x);
     cudaFree(rt->scratch_y);
+    g_pinned.give(rt->pinned, rt->pinned_bytes);
+    if (rt->counted) g_pinned.runtime_destroyed();
     cudaFree(rt->gemm_x);
     for (void *p : rt->exchange_opened) cudaIpcCloseMemHandle(p);
     cudaFree(rt->exchange_own);
@@ -993,29 +1097,28 @@ int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t 
     if (t.cols % 32 != 0) return fail(VQM_ERR_VALUE, "%s: matvec cols must be a multiple of 32", weight);
     int rc = no_capture(rt, "matvec");
     if (rc != VQM_OK) return rc;
-    cudaError_t err = cudaSuccess;
-    if (rt->scratch_x_n < static_cast<size_t>(t.cols)) {
-        cudaFree(rt->scratch_x);
-        rt->scratch_x = nullptr;
-        rt->scratch_x_n = 0;
-        err = cudaMalloc(&rt->scratch_x, sizeof(float) * t.cols);
-        if (err == cudaSuccess) rt->scratch_x_n = t.cols;
-    }
-    if (err == cudaSuccess && rt->scratch_y_n < static_cast<size_t>(t.rows)) {
-        cudaFree(rt->scratch_y);
-        rt->scratch_y = nullptr;
-        rt->scratch_y_n = 0;
-        err = cudaMalloc(&rt->scratch_y, sizeof(float) * t.rows);
-        if (err == cudaSuccess) rt->scratch_y_n = t.rows;
-    }
-    if (err != cudaSuccess) return cuda_fail("scratch allocation", err);
-    err = cudaMemcpyAsync(rt->scratch_x, x_host, x_bytes, cudaMemcpyHostToDevice, rt->stream);
+    // Host vectors go through pinned staging and come back, together with the status word, in one copy: with the caller's
+    // pageable memory every one of the three copies (x, y, status) is a synchronisation of its own.
+    if ((rc = matvec_scratch(rt, static_cast<size_t>(t.cols), static_cast<size_t>(t.rows))) != VQM_OK) return rc;
+    memcpy(rt->pinned, x_host, x_bytes);
+    cudaError_t err = cudaMemcpyAsync(rt->scratch_x, rt->pinned, x_bytes, cudaMemcpyHostToDevice, rt->stream);
     if (err != cudaSuccess) return cuda_fail("qmatvec H2D", err);
-    if ((rc = launch_group(rt, t, rt->scratch_x, rt->scratch_y, 1, false)) != VQM_OK) return rc;
-    err = cudaMemcpyAsync(y_host, rt->scratch_y, sizeof(float) * t.rows, cudaMemcpyDeviceToHost, rt->stream);
+    unsigned *const shared_status = rt->status;
+    rt->status = rt->scratch_y;  // the launch's own status word sits in front of its outputs
+    rc = launch_group(rt, t, rt->scratch_x, reinterpret_cast<float *>(rt->scratch_y + kStatusWords), 1, false);
+    rt->status = shared_status;
+    if (rc != VQM_OK) return rc;
+    const size_t back = sizeof(unsigned) * kStatusWords + sizeof(float) * t.rows;
+    err = cudaMemcpyAsync(rt->pinned, rt->scratch_y, back, cudaMemcpyDeviceToHost, rt->stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(rt->stream);
     if (err != cudaSuccess) return cuda_fail("qmatvec", err);
-    return check_status_word(rt, "qmatvec");
+    const unsigned *got = static_cast<const unsigned *>(rt->pinned);
+    if (got[0] != 0) {
+        cudaMemsetAsync(rt->scratch_y, 0, sizeof(unsigned), rt->stream);
+        return status_failure("qmatvec", got[0]);
+    }
+    memcpy(y_host, got + kStatusWords, sizeof(float) * t.rows);
+    return VQM_OK;
 }
 
 int vqm_argmax_rows(vqm_runtime *rt, const char *x, int n, int ntok, int *out) {

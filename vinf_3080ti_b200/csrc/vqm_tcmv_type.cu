@@ -75,21 +75,40 @@ struct TcVariant {
     }
 };
 
-// Into how many column ranges the rows' sums are split.  Time of a launch in steps of 256 columns: every group of blocks walks
-// `rounds` tiles of 256 rows, each block its share of the steps; a tile costs about one step more for its sums (and another
-// half for adding them up across a cluster).  Depends on rows and columns only.
-inline int choose_tc_split(int n_tiles, int cols, int allow_split, int sm_count) {
+inline int tc_tiles(const MatvecArgs &a) {
+    int n = 0;
+    for (int p = 0; p < kMaxParts; ++p) n += (a.part[p].rows + kTcRows - 1) / kTcRows;
+    return n;
+}
+
+// Into how many column ranges the rows' sums are split, 0 if the launch is too small for this kernel.  Depends on rows and
+// columns only.
+// Time of a launch in steps of 256 columns: every group of blocks walks `rounds` tiles of 256 rows, each block its share of the
+// steps (pairs of warp groups take whole steps in turn: an odd number costs as much as the next even one); a tile costs about
+// one step more for its sums, and another half for adding them up across a cluster.
+// A launch has a fixed cost of about 3.4 us here and of 2.6 us on the CUDA-core kernel, which reads all columns of a short
+// tensor at once while a block here walks its steps.  Measured with 1 / 4 / 8 rows, CUDA-core and this one (us):
+//   Q4_K 1024 x 5120:  5.0 / 7.0 / 10.0 and 6.1 / 6.8 / 8.1        Q4_K 2048 x 5120:  6.6 / 10.3 / 16.1 and 6.5 / 7.1 / 8.4
+//   Q4_K 4096 x 1024:  3.3 / 4.6 / 6.4  and 4.8 / 5.4 / 6.6        Q4_K 512 x 17408:  6.8 / 10.1 / 15.0 and 11.5 / 12.9 / 15.5
+//   Q6_K 2048 x 5120:  6.9 / 10.6 / 16.2 and 8.9 / 9.2 / 10.7      IQ3_S 2048 x 5120: 9.8 / 17.8 / 29.1 and 9.5 / 10.1 / 11.4
+// Launches in a row favour this kernel: its blocks wait on other SMs while the previous launch runs, but not beside blocks of the
+// other kernel.  A decoder layer (1 row / 4 rows fused) takes 81 / 90 us with its 1024 x 5120 projections here and 92 / 115 us with
+// them there, although each alone is faster there.  So it takes launches of 72 pieces of 256 x 256 weights or more of which no
+// block has to walk more than one in 20.
+inline int choose_tc_split(int n_tiles, int cols, int sm_count) {
     const int n_steps = (cols + kTcStepCols - 1) / kTcStepCols;
-    int best = 1;
+    if (static_cast<long long>(n_tiles) * n_steps < 72) return 0;
+    int best = 0, best_walk = 0;
     float best_cost = 0.0f;
-    for (int s = 1; s <= (allow_split ? kMaxSplit : 1) && s <= n_steps; ++s) {
+    for (int s = 1; s <= kMaxSplit && s <= n_steps; ++s) {
         const int fit = TcVariant<1, TcMaps1>::clusters(s, sm_count);
         if (fit == 0) continue;
-        const int groups = n_tiles < fit ? n_tiles : fit, rounds = (n_tiles + groups - 1) / groups;
-        const float cost = static_cast<float>(rounds) * (static_cast<float>((n_steps + s - 1) / s) + (s > 1 ? 1.5f : 1.0f));
-        if (s == 1 || cost < best_cost) best = s, best_cost = cost;
+        const int groups = n_tiles < fit ? n_tiles : fit, rounds = (n_tiles + groups - 1) / groups, steps = (n_steps + s - 1) / s;
+        const int walk = tc_wide(VQM_TYPE) ? (rounds * steps + 1) / 2 * 2 : rounds * steps;
+        const float cost = static_cast<float>(walk) + static_cast<float>(rounds) * (s > 1 ? 1.5f : 1.0f);
+        if (best == 0 || cost < best_cost) best = s, best_cost = cost, best_walk = rounds * steps;
     }
-    return best;
+    return static_cast<long long>(n_tiles) * n_steps >= 20ll * best_walk ? best : 0;
 }
 
 }  // namespace
@@ -97,12 +116,12 @@ inline int choose_tc_split(int n_tiles, int cols, int allow_split, int sm_count)
 #define VQM_CAT2(a, b) a##b
 #define VQM_CAT(a, b) VQM_CAT2(a, b)
 
+int VQM_CAT(split_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &a, int sm_count) { return choose_tc_split(tc_tiles(a), a.cols, sm_count); }
+
 cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, int m, int sm_count,
                                                  cudaStream_t stream) {
     MatvecArgs a = args;
-    int n_tiles = 0;
-    for (int p = 0; p < kMaxParts; ++p) n_tiles += (a.part[p].rows + kTcRows - 1) / kTcRows;
-    a.k_split = choose_tc_split(n_tiles, a.cols, a.allow_split, sm_count);
+    const int n_tiles = tc_tiles(a);
     const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
     for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
     a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;

@@ -208,12 +208,12 @@ class Runtime:
     def matvec(self, name: str, x) -> bytes:
         """matvec(name, x_f32_bytes) -> y_f32_bytes; synchronous single-row entry."""
         keep, addr, n = _ptr(x)
-        if not self.has(name):
+        key, info = _name(name), _capi.TensorInfo()
+        if self._lib.vqm_tensor_info(self._h, key, ctypes.byref(info)) != _capi.OK:
             raise KeyError(f"{name} is not resident on the GPU")
-        rows = self.tensor_info(name)[2]
-        out = np.empty(rows, dtype=np.float32)
-        _capi.check(self._lib.vqm_matvec(self._h, _name(name), addr, n, out.ctypes.data, out.nbytes))
-        return out.tobytes()
+        out = ctypes.create_string_buffer(4 * info.rows)
+        _capi.check(self._lib.vqm_matvec(self._h, key, addr, n, out, 4 * info.rows))
+        return out.raw
 
     def argmax(self, x: str, n: int) -> int:
         out = ctypes.c_int()
