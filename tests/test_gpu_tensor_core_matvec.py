@@ -1,0 +1,97 @@
+"""The tensor-core matvec at the sizes where it can go wrong: launches of 72 pieces of 256 x 256 weights and more.
+
+Bars as for the CUDA-core kernel: relative L2 error <= 1e-5 against dequantise + fp64 matvec, a pass of several rows
+equal bit for bit to its rows alone, one-hot activations give the dequantised weights.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from oracle import dequant_np as O
+from vinf_3080ti_b200.gguf_types import GGUFTensorType as T
+from vinf_3080ti_b200.synth import synthetic_activations, synthetic_blocks
+
+pytestmark = pytest.mark.gpu
+TYPES = [T.Q8_0, T.Q2_K, T.Q3_K, T.Q4_K, T.Q5_K, T.Q6_K, T.IQ2_XXS, T.IQ2_XS, T.IQ3_XXS, T.IQ4_NL, T.IQ3_S, T.IQ2_S, T.IQ4_XS]
+REL_L2 = 1e-5
+
+
+@pytest.fixture(scope="module")
+def rt(codebooks):
+    from vinf_3080ti_b200.runtime import Runtime
+
+    runtime = Runtime(codebooks["iq3s_grid"], codebooks)
+    yield runtime
+    runtime.close()
+
+
+def rel_l2(got, ref) -> float:
+    return float(np.linalg.norm(np.asarray(got, dtype=np.float64) - ref) / max(np.linalg.norm(ref), 1e-300))
+
+
+def _run(rt, names, outs, rows, x):
+    rt.alloc("x", x.size)
+    rt.write("x", np.ascontiguousarray(x))
+    for out, r in zip(outs, rows):
+        rt.alloc(out, x.shape[0] * r)
+    if len(names) == 1:
+        rt.qmv(names[0], "x", outs[0], x.shape[0])
+    else:
+        rt.qmv_group(names, "x", outs, x.shape[0])
+    rt.synchronize()
+    return [rt.read_array(out, x.shape[0] * r).reshape(x.shape[0], r).copy() for out, r in zip(outs, rows)]
+
+
+@pytest.mark.parametrize("shapes,cols", [
+    ((9473,), 512),           # 37 tiles and one row, one block per tile, two steps
+    ((2305,), 2304),          # columns split over a cluster, an odd number of steps per block
+    ((1024, 1000, 24, 8), 2560),  # four tensors, tiles that end inside a tensor, split columns
+    ((39000,), 256),          # more tiles than blocks, a single step
+], ids=str)
+@pytest.mark.parametrize("t", TYPES, ids=lambda t: t.name)
+def test_tiles_steps_and_splits_of_every_type(rt, codebooks, t, shapes, cols):
+    if t in (T.Q8_0, T.IQ4_NL) and cols > 512:
+        cols += 32 * 5  # ends inside a step
+    rng = np.random.default_rng(int(t) + sum(shapes) + cols)
+    names, outs = [f"w{i}" for i in range(len(shapes))], [f"y{i}" for i in range(len(shapes))]
+    raws = [synthetic_blocks(t, rows, cols, rng) for rows in shapes]
+    for name, raw, rows in zip(names, raws, shapes):
+        rt.upload(name, raw, int(t), cols, rows)
+    x = synthetic_activations(8, cols, rng)
+    x[1, : cols // 2] *= 1e-6  # a row whose chunks have very different ranges
+    x[2] = 0.0
+    x[2, [0, cols // 2 + 3, cols - 1][int(t) % 3]] = 1.0  # one-hot
+    refs = [O.matvec(raw, int(t), rows, cols, x, codebooks) for raw, rows in zip(raws, shapes)]
+    got = _run(rt, names, outs, shapes, x)
+    for g, ref in zip(got, refs):
+        assert max(rel_l2(g[k], ref[k]) for k in range(8)) <= REL_L2
+        if not t.name.endswith(("4_K", "5_K", "2_K")):  # (types with minimums subtract the group's sum in fp32)
+            assert np.array_equal(g[2], ref[2].astype(np.float32))
+    for m in (1, 2, 3, 5):  # each compiled row count, full and not
+        for g, part in zip(got, _run(rt, names, outs, shapes, x[:m])):
+            assert np.array_equal(part.view(np.uint32), g[:m].view(np.uint32)), m
+
+
+@pytest.mark.parametrize("t,rows,cols,ntok", [(T.Q6_K, 9473, 512, 1), (T.Q4_K, 2305, 2304, 4), (T.IQ4_XS, 2305, 2304, 8)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_prologues_residual_and_argmax(rt, codebooks, t, rows, cols, ntok):
+    rng = np.random.default_rng(rows + cols + ntok)
+    raw = synthetic_blocks(t, rows, cols, rng)
+    x, x2 = synthetic_activations(ntok, cols, rng), synthetic_activations(ntok, cols, rng)
+    nw = rng.uniform(0.5, 1.5, cols).astype(np.float32)
+    rt.upload("w", raw, int(t), cols, rows)
+    for name, v in (("x", x), ("x2", x2), ("nw", nw)):
+        rt.alloc(name, v.size)
+        rt.write(name, v)
+    rt.alloc("y", ntok * rows)
+    res = rng.standard_normal((ntok, rows)).astype(np.float32)
+    rt.write("y", res)
+    rt.qmv_fused("w", "x", "y", ntok, add=True, norm="nw", eps=1e-6, silu_mul="x2")
+    rt.synchronize()
+    ref = O.fused_matvec(raw, int(t), rows, cols, x, codebooks, x2=x2, norm_w=nw, eps=1e-6, residual=res)
+    assert rel_l2(rt.read_array("y", ntok * rows).reshape(ntok, rows), ref) <= 2e-5
+    ids = rt.qmv_argmax("w", "x", "y", ntok)
+    logits = rt.read_array("y", ntok * rows).reshape(ntok, rows)
+    assert rel_l2(logits, O.matvec(raw, int(t), rows, cols, x, codebooks)) <= REL_L2
+    assert ids == [int(v) for v in logits.argmax(axis=1)]
