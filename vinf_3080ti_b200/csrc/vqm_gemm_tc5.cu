@@ -2,35 +2,31 @@
 //
 // Same contract as the warp-level kernel in vqm_gemm.cu (replaces the reference's vinf_qgemm_kernel,
 // engine/csrc/megakernel/qwen_runtime.cu:655-769: fp16 operands, fp32 accumulation), built on tcgen05:
-//   * a block owns 128 weight rows per MMA M-half and 256 activation rows per accumulator, as one or two accumulators of
-//     128 x 256 fp32 in tensor memory (at most 512 columns, the whole TMEM of an SM: one block per SM); the shapes are
-//     listed at stage_bytes below;
-//   * two blocks of a cluster work as a pair (tcgen05.mma.cta_group::2, M = 256): each decodes its own 128 weight rows
-//     per accumulator and holds half of the accumulator's 256 activation rows in its shared memory, which halves what a
-//     block reads of the activations from L2; the first block issues the MMAs for both and commits to the barriers of
-//     both (multicast commit), the second block forwards its "full" slots to the first with one remote arrive per slot,
-//     each block drains its own 128 lanes of tensor memory;
-//   * the raw weight bytes come in by bulk copies (1-D TMA, no multicast), 256 columns of the block's rows at a time
-//     into a ring of two shared-memory buffers, one copy per row issued by the row's first decoder thread, so that the
-//     decoders never wait for global memory (F16 and F32, whose 256 columns are too wide for the ring, are decoded
-//     straight from global memory);
-//   * K is walked in stages of 64 (two to four stage buffers, as many as fit), each weight stage filled and consumed as
-//     two halves of 32 (the pipeline's slots): warps 0-15 dequantise the weight half-tiles - warps 0-7 the first half
-//     of every stage, warps 8-15 the second; four threads per row, one chunk of 8 weights each, two rows per thread -
-//     with the exact block decoders (Q4_K, Q5_K, Q6_K, Q3_K and Q8_0 with a per-block header and constant shifts, see
-//     FastHeader), store them as fp16 in the K-major 128-byte-swizzled layout the tensor core reads, make the writes
-//     visible to the async proxy and arrive, once per warp, on the slot's "full" mbarrier;
-//   * one thread of warp 16 feeds the activations: per stage one TMA tile copy (cp.async.bulk.tensor.2d, 64 columns x
-//     the block's activation rows of an accumulator, written by the hardware in the same 128-byte swizzle; no
-//     multicast) that completes on the stage's own mbarrier; a stage is refilled once the MMAs of its second half are done;
-//   * one thread of warp 17 issues, per slot, 2 K-steps x the accumulators of tcgen05.mma (kind::f16, N = 256, K = 16)
-//     from shared-memory descriptors and commits them to the slot's "empty" mbarrier, which hands the slot back to the
-//     producers, so tile production runs up to a ring's length ahead of the MMAs;
-//   * after the last commit, warps 0-15 read the accumulators with tcgen05.ld (warp w reads lanes 32 (w % 4) onwards, one
-//     weight row per thread; the four warps of a lane group share the columns) and store y; a warp stores 32
-//     consecutive rows of one activation row, 128 bytes.
-// Where the time goes: profiles/prompt_gemm_tc5_Q4_K_17408x5120x512.md has the step-by-step history, the ablation builds
-// (VQM_TC5_ABLATE) and the ncu figures.
+//   * two blocks of a cluster (two SMs) work as a pair on tcgen05.mma.cta_group::2: 256 weight rows (128 decoded by each
+//     block) by NH accumulators of up to 256 activation rows, half of which each block holds in its shared memory.  The
+//     first block issues the MMAs for both and commits to the barriers of both (multicast commit), the second forwards its
+//     "full" stages with one remote arrive each, each block drains its own 128 lanes of tensor memory;
+//   * K is walked in stages of 64 columns, as many stage buffers as fit;
+//   * one thread of warp 18 brings the raw weight bytes, 256 columns ("a run") of the block's rows at a time, into a ring of
+//     buffers by TMA tile copies (by row class, see vqm_tcmv_maps.cu; a bulk copy per row takes the copy unit 33 cycles, 98
+//     instead of 76 us for 64 activation rows x 17408 x 5120).  F16 and F32, whose runs are too wide for the ring, are
+//     decoded straight from global memory;
+//   * warps 0-15 dequantise: two or four groups of warps take the stages in turn, thread = weight row, so that scales
+//     are unpacked once per 32 weights and a warp does one wait, one fence and one arrive per 1024 or 2048 weights.  The weights are
+//     decoded into registers before the wait for the stage, which is then held for eight stores per thread only;
+//   * one thread of warp 16 feeds the activations, one TMA tile copy per stage and accumulator (no multicast);
+//   * one thread of warp 17 issues, per stage, 4 K-steps x NH tcgen05.mma (kind::f16) and commits them to "empty";
+//   * after the last commit, warps 0-15 read the accumulators with tcgen05.ld and store y, 32 consecutive rows per warp.
+//
+// What bounds it: with 512 activation rows the MMAs (0.60 us per stage alone, 0.75 on the whole GPU under the power cap), up
+// to 256 the decoders (0.39 us per stage).  Before, four threads shared a row and a stage was handed over as two halves with a
+// wait, fence, arrive and commit each, from a lane that the compiler could not tell to be alone (see elect_one): 0.36 us per
+// half before any weight was decoded.  64 / 256 / 512 rows: Q4_K 17408 x 5120 79 / 81 / 92 us before, 42 / 48 / 72 now; Q6_K
+// 6144 x 5120 77 / 77 / 89 and 27 / 31 / 44, Q4_K 5120 x 17408 236 / 237 / 271 and 49 / 57 / 84 (columns split).
+//
+// Split of the columns: tensors of few rows leave most SMs idle (6144 rows x 512: 24 pairs of 74), so up to four pairs form
+// a cluster that shares the columns of 256 weight rows.  Each pair sums its own range of columns; then every pair sends the
+// others their parts of its sums through distributed shared memory and adds what it receives in the order of the columns.
 // Every mbarrier wait is bounded: on expiry the block records a status code, everybody falls through to the end, and
 // the tensor memory is released before the block returns.
 #include <cuda.h>  // CUtensorMap and the driver entry point that encodes one (types only; nothing links against the driver)
@@ -38,65 +34,40 @@
 
 #include "vqm_formats.cuh"
 #include "vqm_kernels.h"
-#include "vqm_steps.cuh"
-
-#ifndef VQM_TC5_SHAPE
-#define VQM_TC5_SHAPE 0  // experiment builds: block shape for more than 256 activation rows, see launch_t
-#endif
-#ifndef VQM_TC5_ABLATE
-#define VQM_TC5_ABLATE 0  // experiment builds (wrong results): 1 = fast decoders store zeros, 2 = no activation copies,
-                         // 4 = no proxy fence by the producers, 8 = only the MMA issue loop runs, without waiting
-#endif
+#include "vqm_steps_iq4.cuh"
+#include "vqm_tcmv.cuh"
 
 namespace vqm {
 namespace {
 
-// A block computes kTM * MR weight rows by kTNH * NH activation rows: MR x NH accumulators of 128 x 256 in tensor memory
-// (MR * NH <= 2: 512 columns), alone or as a pair of blocks (see stage_bytes).  In use: 1 x 1 pairs up to 256 activation
-// rows, 1 x 2 pairs above; 2 x 1 (256 weight rows per block halve what the blocks together read of the activations from
-// L2, at the price of decoding every weight twice as often) and single blocks are kept for experiment builds, launch_t
-// has the measurements.
-constexpr int kTM = 128, kTNH = 256, kTK = 64;
-constexpr int kMaxStages = 4;  // stages of the tile ring: as many as fit into shared memory, see stages_for
-constexpr int kTA1 = kTM * kTK * 2, kTB1 = kTNH * kTK * 2;  // 16 KB per 128 weight rows, 32 KB per 256 activation rows
-// With PAIR two blocks of a cluster (two SMs) work as one: tcgen05.mma.cta_group::2 multiplies the 256 weight rows of the
-// two blocks (128 each, M = 256) by 256 activation rows of which each block holds one half in its shared memory, so a
-// block pulls only half of the activation tile out of L2 - the traffic that bounds this kernel.  Accumulator rows stay
-// with the block that decoded them (its 128 lanes of tensor memory).
-__host__ __device__ constexpr int stage_bytes(int mr, int nh, bool pair) { return mr * kTA1 + nh * (pair ? kTB1 / 2 : kTB1); }
-constexpr int kAThreads = 512;           // decoder warps 0-15
-constexpr int kTThreads = kAThreads + 64;  // warp 16: one thread feeds the activation tiles (TMA); warp 17: one thread issues the MMAs
-constexpr int kLoadWarp = kAThreads / 32;  // the MMA warp is the one after it
-// Raw-block ring: a "column" is 256 weight columns of the 128 rows; a row's bytes of one column are contiguous.
-constexpr int kRawCols = 256;
+// Activation rows of an accumulator: up to 256, a multiple of 64 (the MMA's N); NH accumulators: 1 or 2 (512 columns of
+// tensor memory, the whole of an SM's: one block per SM).
+constexpr int kTM = 128, kTNMax = 256, kTK = 64, kMaxPairs = 4;
+constexpr int kMaxStages = 6;
+constexpr int kTA = kTM * kTK * 2, kTB = kTNMax / 2 * kTK * 2;  // 16 KB of a block's weights, 16 KB of its half of the activations
+constexpr int kAThreads = 512;             // decoder warps 0-15
+constexpr int kTThreads = kAThreads + 96;  // warp 16: activation tiles; warp 17: MMAs; warp 18: raw weights
+// Raw-block ring: a "run" is 256 weight columns of the 128 rows; a row's bytes of one run are contiguous.
+constexpr int kRawCols = 256, kStagesPerRun = kRawCols / kTK;
+__host__ __device__ constexpr int raw_buffers(int nh) { return nh == 1 ? 3 : 2; }
 __host__ __device__ constexpr int raw_run_bytes(int type) { return kRawCols / chunk_block(type) * chunk_block_bytes(type); }
-// slot of one row: the run, up to 14 bytes in front (the copy starts at the 16-byte boundary below), the decoders' reads
-// of up to 8 bytes behind, rounded to 16
-__host__ __device__ constexpr int raw_slot_bytes(int type) { return (raw_run_bytes(type) + 14 + 8 + 15) / 16 * 16; }
+__host__ __device__ constexpr int raw_pitch(int type) { return tc_pitch(type); }  // bytes of a row in a buffer
 __host__ __device__ constexpr int table_bytes16(int type) { return grid_bytes(type) > 0 ? (grid_bytes(type) + 15) / 16 * 16 : 16; }
-// Staged where the ring fits beside two stages of tiles: every quantised type in the shapes in use (Q8_0 only beside a
-// pair's smaller stages); F16 and F32 never.
-__host__ __device__ constexpr size_t smem_without_ring(int type, int mr, int nh, bool pair, int stages) {
-    return table_bytes16(type) + 1024 + static_cast<size_t>(stages) * stage_bytes(mr, nh, pair);
+__host__ __device__ constexpr bool raw_staged(int type) { return raw_run_bytes(type) <= 288; }  // every quantised type
+__host__ __device__ constexpr int raw_ring_bytes(int type, int nh) { return raw_staged(type) ? raw_buffers(nh) * kTM * raw_pitch(type) + 16 : 0; }
+// Activation tiles in flight (32 KB each in blocks of two accumulators), and as many weight tiles as fit beside them.
+__host__ __device__ constexpr int x_stages(int nh) { return nh == 1 ? 4 : 3; }
+__host__ __device__ constexpr int tc5_smem_bytes(int type, int nh, int stages) {
+    return table_bytes16(type) + 1024 + x_stages(nh) * nh * kTB + stages * kTA + raw_ring_bytes(type, nh);
 }
-__host__ __device__ constexpr bool raw_staged(int type, int mr, int nh, bool pair) {
-    return raw_run_bytes(type) <= 272 && smem_without_ring(type, mr, nh, pair, 2) + 2 * mr * kTM * raw_slot_bytes(type) <= 227 * 1024;
-}
-__host__ __device__ constexpr int raw_ring_bytes(int type, int mr, int nh, bool pair) {
-    return raw_staged(type, mr, nh, pair) ? 2 * mr * kTM * raw_slot_bytes(type) : 0;
-}
-__host__ __device__ constexpr size_t tc5_smem_bytes(int type, int mr, int nh, bool pair, int stages) {
-    return smem_without_ring(type, mr, nh, pair, stages) + raw_ring_bytes(type, mr, nh, pair);
-}
-// The ring is what hides the refill round trip of a slot (MMAs done -> "empty" -> copies from L2 / decode -> "full"),
-// which is several times longer than a slot's MMAs: every stage that fits is used.
-__host__ __device__ constexpr int stages_for(int type, int mr, int nh, bool pair) {
+__host__ __device__ constexpr int stages_for(int type, int nh) {
     int s = kMaxStages;
-    while (s > 2 && tc5_smem_bytes(type, mr, nh, pair, s) > 227 * 1024) --s;
+    while (s > 2 && tc5_smem_bytes(type, nh, s) > 226 * 1024) --s;
     return s;
 }
-// 256 weight rows per block need the raw ring for 256 rows (reading them from global memory per chunk is too slow there)
-[[maybe_unused]] __host__ __device__ constexpr bool fits_two_row_halves(int type, bool pair) { return raw_staged(type, 2, 1, pair); }
+// Exchange between the pairs of a cluster: per accumulator, chunks of 16 activation rows go to pair (chunk % pairs), which
+// keeps the other pairs' sums of its chunks, 8 KB each, where the stages were.
+constexpr int kXChunk = 16, kXBytes = kXChunk * kTM * 4;
 
 __device__ __forceinline__ uint32_t s32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -171,32 +142,11 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
     return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) |
            (2ull << 61);
 }
-// Instruction descriptor, kind::f16: D fp32, A and B fp16, both K-major, N = 256, M = 128.
-constexpr uint32_t kIdesc = (1u << 4) | ((256u >> 3) << 17) | ((128u >> 4) << 24);
-
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// ---- fast chunk decoders of the producer warps --------------------------------------------------------------------------
-// The generic block decoder (deq8) unpacks the block header for every chunk of 8 weights.  A producer thread stays on one
-// row and walks a block's eight 32-column slots in order, so for the types below the header is unpacked once per block
-// and a chunk is a load of 8 bytes, one byte permute per weight and packed fp32 arithmetic - the same operations in the
-// same order as deq8, so the fp16 tiles are bit-identical to what the generic path stores.
-template <int N>
-struct Int {
-    static constexpr int value = N;
-};
-__host__ __device__ constexpr bool has_fast_chunk(int type) { return type == kQ4_K || type == kQ5_K || type == kQ6_K || type == kQ3_K || type == kQ8_0; }
-
+// ---- slot decoders ---------------------------------------------------------------------------------------------------
+// N * 32 weights of one row, columns 32 G .. of a 256-column run at `blk` (shared memory), as 16 N words `h` of two fp16
+// (N = 1, or N = 2 and G even: what two neighbouring slots share is read once).
+// Every value is the fp32 expression of deq8 rounded once to fp16, whichever decoder produces it.  G is a run-time value
+// (uniform over the warp): one copy of the code for all slots stays in the instruction cache.
 __device__ __forceinline__ uint32_t f16x2_of(f32x2 v) {  // (lo, hi) -> two fp16 in one word, round to nearest even
     float lo, hi;
     unpack2(v, lo, hi);
@@ -209,157 +159,141 @@ __device__ __forceinline__ void bytes_fma_f16(uint32_t w, f32x2 neg_magic, f32x2
     h0 = f16x2_of(fma2(bytes_to_pair<0, 1>(w, neg_magic), dl, nml));
     h1 = f16x2_of(fma2(bytes_to_pair<2, 3>(w, neg_magic), dl, nml));
 }
-
-template <int TYPE>
-struct FastHeader;
-
-// Q4_K / Q5_K (engine/csrc/common/qwen_quant.cuh:78-86, 171-196): d, dmin, 12 bytes of 6-bit scales and minimums; slot G of
-// the block is its sub-block G (32 weights with one scale and one minimum), weight = d * sc * q - dmin * mn.
-template <int TYPE>
-struct FastHeaderK45 {
-    uint32_t sc_lo, sc_hi, mn_lo, mn_hi;  // scales / minimums of sub-blocks 0..3 and 4..7, one per byte
-    float d, ndmin;
-    uint32_t qh0, qh1;  // Q5_K: the thread's 8 bytes of fifth bits (bit G belongs to slot G)
-    __device__ __forceinline__ void load(uint32_t blk, int quarter) {
-        const uint4 h = lds128u(blk);  // blocks of these types are 16-byte aligned
-        d = half_bits_to_float(h.x & 0xFFFFu);
-        ndmin = -half_bits_to_float(h.x >> 16);
-        sc_lo = h.y & 0x3F3F3F3Fu;
-        mn_lo = h.z & 0x3F3F3F3Fu;
-        sc_hi = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
-        mn_hi = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
-        if constexpr (TYPE == kQ5_K) {
-            const unsigned long long q = lds64(blk + 16 + 8 * quarter);
-            qh0 = static_cast<uint32_t>(q), qh1 = static_cast<uint32_t>(q >> 32);
-        }
-    }
-    template <int G>
-    __device__ __forceinline__ void chunk(uint32_t blk, int quarter, uint32_t (&h)[4]) const {
-        const float dl = d * byte_to_float<G & 3>(G < 4 ? sc_lo : sc_hi);
-        const float nml = ndmin * byte_to_float<G & 3>(G < 4 ? mn_lo : mn_hi);  // -(dmin * mn), exactly
-        const unsigned long long q = lds64(blk + (TYPE == kQ4_K ? 16 : 48) + 32 * (G >> 1) + 8 * quarter);
-        uint32_t w0 = static_cast<uint32_t>(q), w1 = static_cast<uint32_t>(q >> 32);
-        if constexpr (G & 1) w0 >>= 4, w1 >>= 4;
-        w0 &= 0x0F0F0F0Fu, w1 &= 0x0F0F0F0Fu;
-        if constexpr (TYPE == kQ5_K) {
-            w0 |= (G <= 4 ? qh0 << (4 - G) : qh0 >> (G - 4)) & 0x10101010u;
-            w1 |= (G <= 4 ? qh1 << (4 - G) : qh1 >> (G - 4)) & 0x10101010u;
-        }
-        const f32x2 neg_magic = pack2(-8388608.0f, -8388608.0f), dl2 = pack2(dl, dl), nml2 = pack2(nml, nml);
-        bytes_fma_f16(w0, neg_magic, dl2, nml2, h[0], h[1]);
-        bytes_fma_f16(w1, neg_magic, dl2, nml2, h[2], h[3]);
-    }
-};
-template <>
-struct FastHeader<kQ4_K> : FastHeaderK45<kQ4_K> {};
-template <>
-struct FastHeader<kQ5_K> : FastHeaderK45<kQ5_K> {};
 // the four bytes of `w` (minus the bias inside neg_magic) times dl (packed), as fp16
 __device__ __forceinline__ void bytes_mul_f16(uint32_t w, f32x2 neg_magic, f32x2 dl, uint32_t &h0, uint32_t &h1) {
     h0 = f16x2_of(mul2(bytes_to_pair<0, 1>(w, neg_magic), dl));
     h1 = f16x2_of(mul2(bytes_to_pair<2, 3>(w, neg_magic), dl));
 }
+// N words at a 2-byte aligned address
+template <int N>
+__device__ __forceinline__ void words_a2(uint32_t at, uint32_t (&w)[N]) {
+    const uint32_t base = at & ~3u, sh = (at & 2u) * 8u;
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i <= N; ++i) r[i] = lds32(base + 4 * i);
+#pragma unroll
+    for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(r[i], r[i + 1], sh);
+}
 
-// Q6_K (engine/csrc/common/qwen_quant.cuh:197-212): low nibbles @0 (128), high 2 bits @128 (64), int8 scales @192 (16),
-// d @208; weight = d * sc * (q - 32).  Chunk c = 4 G + quarter of the block: low nibbles at 64 (G / 4) + 32 (G % 2) +
-// 8 quarter, nibble (G % 4) / 2; high bits at 128 + 32 (G / 4) + 8 quarter, bit pair G % 4; scale c / 2.  The thread's six
-// 8-byte fields of the block are loaded once (the blocks are only 2-byte aligned).
-template <>
-struct FastHeader<kQ6_K> {
-    uint32_t ql[4][2], qh[2][2];  // [G / 4 * 2 + G % 2], [G / 4]
-    uint32_t sc[2];               // the thread's eight scales (slots 0..3, 4..7), one per byte, as int8 + 128
-    float d;
-    __device__ __forceinline__ void load(uint32_t blk, int quarter) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) lds64_a2(blk + (i >> 1) * 64 + (i & 1) * 32 + 8 * quarter, ql[i][0], ql[i][1]);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) lds64_a2(blk + 128 + 32 * i + 8 * quarter, qh[i][0], qh[i][1]);
-        uint32_t s0, s1, s2, s3;  // the 16 scales; the thread's are the even or the odd bytes
-        lds64_a2(blk + 192, s0, s1);
-        lds64_a2(blk + 200, s2, s3);
-        const uint32_t sel = (quarter >> 1) ? 0x7531u : 0x6420u;
-        sc[0] = __byte_perm(s0, s1, sel) ^ 0x80808080u;
-        sc[1] = __byte_perm(s2, s3, sel) ^ 0x80808080u;
-        d = half_bits_to_float(lds16(blk + 208));
-    }
-    template <int G>
-    __device__ __forceinline__ void chunk(uint32_t, int, uint32_t (&h)[4]) const {
-        const float dl = d * byte_to_float<G & 3>(sc[G >> 2], 128.0f);
-        constexpr int LS = ((G & 3) >> 1) * 4, HS = 2 * (G & 3);
-        uint32_t w[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const uint32_t lo = ql[(G >> 2) * 2 + (G & 1)][i], hi = qh[G >> 2][i];
-            w[i] = ((lo >> LS) & 0x0F0F0F0Fu) | ((HS <= 4 ? hi << (4 - HS) : hi >> (HS - 4)) & 0x30303030u);
+template <int TYPE, int N>
+__device__ __forceinline__ void decode_slots(uint32_t blk, int G, const uint8_t *table, uint32_t (&h)[16 * N]) {
+    if constexpr (TYPE == kQ4_K || TYPE == kQ5_K) {
+        // d, dmin, 12 bytes of 6-bit scales and minimums; slot G is sub-block G: d * sc * q - dmin * mn (16-byte aligned blocks)
+        const uint4 hd = lds128u(blk);
+        const uint32_t qa = blk + (TYPE == kQ4_K ? 16 : 48) + 32 * (G >> 1);
+        const uint4 q0 = lds128u(qa), q1 = lds128u(qa + 16);
+        const uint32_t q[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        uint32_t f[8];
+        if constexpr (TYPE == kQ5_K) {
+            const uint4 f0 = lds128u(blk + 16), f1 = lds128u(blk + 32);
+            f[0] = f0.x, f[1] = f0.y, f[2] = f0.z, f[3] = f0.w, f[4] = f1.x, f[5] = f1.y, f[6] = f1.z, f[7] = f1.w;
         }
-        const f32x2 neg_magic = pack2(-(8388608.0f + 32.0f), -(8388608.0f + 32.0f)), dl2 = pack2(dl, dl);
-        bytes_mul_f16(w[0], neg_magic, dl2, h[0], h[1]);
-        bytes_mul_f16(w[1], neg_magic, dl2, h[2], h[3]);
-    }
-};
-
-// Q3_K (engine/csrc/common/qwen_quant.cuh:225-246): high-bit mask @0 (32), 2-bit quants @32 (64), 12 bytes of 6-bit
-// scales @96, d @108; weight = d * (sc - 32) * ((q2 | hbit << 2) - 4).  Chunk c = 4 G + quarter: quants at 32 + 32 (G / 4) +
-// 8 quarter, bit pair G % 4; mask at 8 quarter, bit G; scale c / 2.
-template <>
-struct FastHeader<kQ3_K> {
-    uint32_t hm[2], qs[2][2];
-    uint32_t sc[4];  // sc[G / 2]: the scale of slot G in byte 2 (G % 2), as the 6-bit field (32 too large)
-    float d;
-    __device__ __forceinline__ void load(uint32_t blk, int quarter) {
-        lds64_a2(blk + 8 * quarter, hm[0], hm[1]);
+        const f32x2 neg_magic = pack2(-8388608.0f, -8388608.0f);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) lds64_a2(blk + 32 + 32 * i + 8 * quarter, qs[i][0], qs[i][1]);
-        uint32_t s0, s1;
-        lds64_a2(blk + 96, s0, s1);
-        const uint32_t s2 = lds32_a2(blk + 104);
-        d = half_bits_to_float(lds16(blk + 108));
-        // scales k = 0..15, four per word: low nibbles of bytes 0..7 (k < 8) or their high nibbles, two more bits from
-        // byte 8 + k % 4 at bit pair k / 4
-        const uint32_t k0 = (s0 & 0x0F0F0F0Fu) | ((s2 << 4) & 0x30303030u), k1 = (s1 & 0x0F0F0F0Fu) | ((s2 << 2) & 0x30303030u);
-        const uint32_t k2 = ((s0 >> 4) & 0x0F0F0F0Fu) | (s2 & 0x30303030u), k3 = ((s1 >> 4) & 0x0F0F0F0Fu) | ((s2 >> 2) & 0x30303030u);
-        // the thread's scale of slot G is k = 2 G + quarter / 2: byte 2 (G % 2) + quarter / 2 of word G / 2
-        const uint32_t sh = (quarter >> 1) * 8;
-        sc[0] = k0 >> sh, sc[1] = k1 >> sh, sc[2] = k2 >> sh, sc[3] = k3 >> sh;
-    }
-    template <int G>
-    __device__ __forceinline__ void chunk(uint32_t, int, uint32_t (&h)[4]) const {
-        const float dl = d * byte_to_float<2 * (G & 1)>(sc[G >> 1], 32.0f);
-        constexpr int QS = 2 * (G & 3);
-        uint32_t w[2];
+        for (int k = 0; k < N; ++k) {
+            const int g = G + k, s = 8 * (g & 3), sh = N == 2 ? 4 * k : 4 * (g & 1);
+            const uint32_t y = hd.y >> s, z = hd.z >> s, w3 = hd.w >> s;
+            const uint32_t sc = g < 4 ? y & 63u : (w3 & 15u) | ((y >> 2) & 48u), mn = g < 4 ? z & 63u : ((w3 >> 4) & 15u) | ((z >> 2) & 48u);
+            const float dl = half_bits_to_float(hd.x & 0xFFFFu) * static_cast<float>(sc);
+            const float nml = -half_bits_to_float(hd.x >> 16) * static_cast<float>(mn);
+            const f32x2 dl2 = pack2(dl, dl), nml2 = pack2(nml, nml);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            w[i] = ((qs[G >> 2][i] >> QS) & 0x03030303u) | ((G <= 2 ? hm[i] << (2 - G) : hm[i] >> (G - 2)) & 0x04040404u);
-        const f32x2 neg_magic = pack2(-(8388608.0f + 4.0f), -(8388608.0f + 4.0f)), dl2 = pack2(dl, dl);
-        bytes_mul_f16(w[0], neg_magic, dl2, h[0], h[1]);
-        bytes_mul_f16(w[1], neg_magic, dl2, h[2], h[3]);
+            for (int i = 0; i < 8; ++i) {
+                uint32_t w = (q[i] >> sh) & 0x0F0F0F0Fu;
+                if constexpr (TYPE == kQ5_K) w += ((f[i] >> g) & 0x01010101u) * 16u;
+                bytes_fma_f16(w, neg_magic, dl2, nml2, h[16 * k + 2 * i], h[16 * k + 2 * i + 1]);
+            }
+        }
+    } else if constexpr (TYPE == kQ6_K) {
+        // low nibbles @0, high bit pairs @128, int8 scales @192 (per 16 columns), d @208: d * sc * (q - 32)
+        const int n = G >> 2;
+        uint32_t hi[8];
+        words_a2<8>(blk + 128 + 32 * n, hi);
+        const float d = half_bits_to_float(lds16(blk + 208));
+        const f32x2 neg_magic = pack2(-(8388608.0f + 32.0f), -(8388608.0f + 32.0f));
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const int j = (G & 3) + k, ls = (j >> 1) * 4, hs = 2 * j;
+            uint32_t lo[8];
+            words_a2<8>(blk + 64 * n + 32 * (j & 1), lo);
+            const uint32_t sc = lds16(blk + 192 + 2 * (G + k));
+            const float dl[2] = {d * static_cast<float>(static_cast<int8_t>(sc & 0xFFu)), d * static_cast<float>(static_cast<int8_t>(sc >> 8))};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t q = ((lo[i] >> ls) & 0x0F0F0F0Fu) + ((hi[i] >> hs) & 0x03030303u) * 16u;
+                bytes_mul_f16(q, neg_magic, pack2(dl[i >> 2], dl[i >> 2]), h[16 * k + 2 * i], h[16 * k + 2 * i + 1]);
+            }
+        }
+    } else if constexpr (TYPE == kQ3_K) {
+        // high-bit mask @0, bit pairs @32, 6-bit scales @96 (per 16 columns), d @108: d * (sc - 32) * ((q2 | hbit << 2) - 4)
+        const int n = G >> 2;
+        uint32_t hm[8], qs[8];
+        words_a2<8>(blk, hm);
+        words_a2<8>(blk + 32 + 32 * n, qs);
+        const float d = half_bits_to_float(lds16(blk + 108));
+        const f32x2 neg_magic = pack2(-(8388608.0f + 4.0f), -(8388608.0f + 4.0f));
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            // scales 2 g and 2 g + 1: nibbles of bytes 0..7 (low ones first), two more bits from bytes 8..11, a pair per four scales
+            const int g = G + k, j = g & 3;
+            const uint32_t sc = ((lds16(blk + 96 + ((2 * g) & 7)) >> (4 * n)) & 0x0F0Fu) | (((lds16(blk + 104 + ((2 * g) & 3)) >> (g & 6)) & 0x0303u) << 4);
+            const float dl[2] = {d * static_cast<float>(static_cast<int>(sc & 0xFFu) - 32), d * static_cast<float>(static_cast<int>(sc >> 8) - 32)};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t q = ((qs[i] >> (2 * j)) & 0x03030303u) + ((hm[i] >> g) & 0x01010101u) * 4u;
+                bytes_mul_f16(q, neg_magic, pack2(dl[i >> 2], dl[i >> 2]), h[16 * k + 2 * i], h[16 * k + 2 * i + 1]);
+            }
+        }
+    } else if constexpr (TYPE == kQ8_0) {
+        // blocks of 32 weights: d @0, 32 int8 @2
+        const f32x2 neg_magic = pack2(-(8388608.0f + 128.0f), -(8388608.0f + 128.0f));
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const uint32_t at = blk + (G + k) * 34;
+            const float d = half_bits_to_float(lds16(at));
+            uint32_t w[8];
+            words_a2<8>(at + 2, w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)  // int8 + 128 is the unsigned byte
+                bytes_mul_f16(w[i] ^ 0x80808080u, neg_magic, pack2(d, d), h[16 * k + 2 * i], h[16 * k + 2 * i + 1]);
+        }
+    } else if constexpr (TYPE == kIQ4_XS || TYPE == kIQ4_NL) {
+        // byte i of a run of 16: weights i (low nibble) and 16 + i; levels + 128 are looked up four at a time (see iq4_levels4)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const int g = G + k;
+            uint32_t w[4];
+            float dl;
+            if constexpr (TYPE == kIQ4_NL) {
+                const uint32_t at = blk + g * 18;
+                dl = half_bits_to_float(lds16(at));
+                words_a2<4>(at + 2, w);
+            } else {
+                const uint32_t hb = lds16(blk + 2), lb = lds16(blk + 4 + 2 * (g >> 2));  // 6-bit scales: low nibbles @4, high pairs @2
+                const uint32_t sc = ((lb >> (4 * (g & 3))) & 15u) | (((hb >> (2 * g)) & 3u) << 4);
+                dl = half_bits_to_float(lds16(blk)) * static_cast<float>(static_cast<int>(sc) - 32);
+                words_a2<4>(blk + 8 + 16 * g, w);
+            }
+            const f32x2 neg_magic = pack2(-(8388608.0f + 128.0f), -(8388608.0f + 128.0f)), d2 = pack2(dl, dl);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t a = iq4_levels4(w[i] & 0xFFFFu), b = iq4_levels4(w[i] >> 16);  // nibbles of bytes 0, 1 and 2, 3
+                bytes_mul_f16(__byte_perm(a, b, 0x6420), neg_magic, d2, h[16 * k + 2 * i], h[16 * k + 2 * i + 1]);
+                bytes_mul_f16(__byte_perm(a, b, 0x7531), neg_magic, d2, h[16 * k + 8 + 2 * i], h[16 * k + 8 + 2 * i + 1]);
+            }
+        }
+    } else {
+        constexpr int CPB = chunk_block(TYPE) / 8, BB = chunk_block_bytes(TYPE);
+#pragma unroll
+        for (int k = 0; k < 4 * N; ++k) {
+            const int c = 4 * G + k;
+            float v[8];
+            deq8<TYPE>(static_cast<const uint8_t *>(__cvta_shared_to_generic(blk + (c / CPB) * BB)), c % CPB, v, table);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) h[4 * k + e] = f16x2_of(pack2(v[2 * e], v[2 * e + 1]));
+        }
     }
-};
-
-// Q8_0 (engine/csrc/common/qwen_quant.cuh:163-170): blocks of 32 weights, d @0 and 32 int8 @2; slot G of a 256-column run is
-// its block G, the thread's chunk the 8 bytes at 2 + 8 * quarter of it.  Nothing to unpack per run.
-template <>
-struct FastHeader<kQ8_0> {
-    __device__ __forceinline__ void load(uint32_t, int) {}
-    template <int G>
-    __device__ __forceinline__ void chunk(uint32_t blk, int quarter, uint32_t (&h)[4]) const {
-        const uint32_t at = blk + G * 34;
-        const float d = half_bits_to_float(lds16(at));
-        uint32_t w0, w1;
-        lds64_a2(at + 2 + 8 * quarter, w0, w1);
-        const f32x2 neg_magic = pack2(-(8388608.0f + 128.0f), -(8388608.0f + 128.0f)), d2 = pack2(d, d);
-        bytes_mul_f16(w0 ^ 0x80808080u, neg_magic, d2, h[0], h[1]);  // int8 + 128 is the unsigned byte
-        bytes_mul_f16(w1 ^ 0x80808080u, neg_magic, d2, h[2], h[3]);
-    }
-};
-
-// (types without a fast decoder never instantiate this)
-template <int TYPE>
-struct FastHeader {
-    __device__ __forceinline__ void load(uint32_t, int) {}
-    template <int G>
-    __device__ __forceinline__ void chunk(uint32_t, int, uint32_t (&)[4]) const {}
-};
+}
 
 // ---- the two blocks of a pair ----------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -380,63 +314,74 @@ __device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_addr) {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Instruction descriptor of the pair MMA: M = 256 (128 rows from each block), N = 256.
-constexpr uint32_t kIdescPair = (1u << 4) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
-__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(kIdescPair), "r"(accumulate)
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// arrives on the barrier at this address in both blocks of the pair once the MMAs issued so far are done
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-    const uint16_t both = 3;
+// arrives on the barrier at this address in both blocks of pair `pair` once the MMAs issued so far are done
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t pair) {
+    const uint16_t both = static_cast<uint16_t>(3u << (2 * pair));
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(both)
                  : "memory");
 }
 
-template <int TYPE, int MR, int NH, bool PAIR>
-__global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_constant__ CUtensorMap x_map, const uint8_t *w, float *y, int rows,
-                                                                 int cols, long long row_bytes, int ntok, const uint8_t *codebook,
+struct Tc5Maps {
+    CUtensorMap x;     // activations
+    CUtensorMap w[8];  // weights, by row class
+};
+
+template <int TYPE, int NH>
+__global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_constant__ Tc5Maps maps, const uint8_t *w, float *y, int rows,
+                                                                 int cols, long long row_bytes, int ntok, int n_acc, int map_shift, const uint8_t *codebook,
                                                                  unsigned *status) {
     constexpr int CPB = chunk_block(TYPE) / 8, BB = chunk_block_bytes(TYPE);
     constexpr int TABLE = table_bytes16(TYPE);
-    constexpr int kTStage = stage_bytes(MR, NH, PAIR), kTA = MR * kTA1, kTN = NH * kTNH;
-    constexpr int kBN = PAIR ? kTNH / 2 : kTNH;       // activation rows of an accumulator's tile that this block holds
-    constexpr int kRowsPerAcc = PAIR ? 2 * kTM : kTM;  // weight rows of an accumulator (both blocks of a pair)
-    constexpr int kTStages = stages_for(TYPE, MR, NH, PAIR), kTSlots = 2 * kTStages;  // slots: half stages
-    constexpr uint32_t kTmemCols = 256 * MR * NH;
-    static_assert(MR * NH <= 2, "512 columns of tensor memory");
+    constexpr int kTStages = stages_for(TYPE, NH), kXStages = x_stages(NH), kRaw = raw_buffers(NH);
+    constexpr bool kStaged = raw_staged(TYPE);
+    // Decoder warps of a stage, and groups that take turns: a group must not run two uses of a stage ahead of another, the
+    // parity of the barriers would not tell them apart, so there are no more groups than stages.
+    constexpr int kGroupWarps = kStaged && kTStages >= 4 ? 4 : 8, kGroups = 16 / kGroupWarps;
+    static_assert(kGroups <= kTStages, "barrier phases");
+    constexpr uint32_t kTmemCols = 256 * NH;
     extern __shared__ uint8_t tc5_raw[];
-    __shared__ __align__(8) uint64_t s_full[2 * kMaxStages], s_empty[2 * kMaxStages], s_xfull[kMaxStages], s_done, s_raw_full[2], s_raw_empty[2];
+    __shared__ __align__(8) uint64_t s_full[kMaxStages], s_empty[kMaxStages], s_xfull[4], s_xempty[4], s_done, s_raw_full[3], s_raw_empty[3];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
     // table first, then the stages on a 1024-byte boundary (the swizzle works on absolute shared-memory address bits)
     uint8_t *table = tc5_raw;
     const uint32_t tiles = (s32(tc5_raw) + TABLE + 1023u) & ~1023u;
-    constexpr bool kStaged = raw_staged(TYPE, MR, NH, PAIR);
-    constexpr int RSLOT = raw_slot_bytes(TYPE), RUN = raw_run_bytes(TYPE);
-    const uint32_t raw_ring = tiles + kTStages * kTStage;  // two buffers of MR * kTM row slots
+    constexpr int PITCH = raw_pitch(TYPE), RUN = raw_run_bytes(TYPE);
+    const uint32_t x_tiles = tiles + kTStages * kTA, raw_ring = x_tiles + kXStages * (NH * kTB);  // buffers of kTM rows
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // a pair is two consecutive blocks of the grid's x; block `rank` of it owns rows rank * 128 .. + 127 of each accumulator
-    const uint32_t rank = PAIR ? cluster_rank() : 0u;
-    const int row0 = static_cast<int>(PAIR ? blockIdx.x >> 1 : blockIdx.x) * (kRowsPerAcc * MR) + static_cast<int>(rank) * kTM;
-    const int tok0 = blockIdx.y * kTN;
-    const int n_k = cols / kTK;
+    // a cluster: `pairs` pairs of blocks that share the columns of 256 weight rows; block `rank` of a pair owns rows rank * 128 ..
+    uint32_t cluster_blocks;
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(cluster_blocks));
+    const uint32_t in_cluster = cluster_rank(), rank = in_cluster & 1u;
+    const int pairs = static_cast<int>(cluster_blocks >> 1), pair = static_cast<int>(in_cluster >> 1);
+    const int row0 = static_cast<int>(blockIdx.x / cluster_blocks) * (2 * kTM) + static_cast<int>(rank) * kTM;
+    const int tok0 = blockIdx.y * (NH * n_acc);
+    const int n_runs = (cols + kRawCols - 1) / kRawCols;
+    const int run0 = pair * n_runs / pairs, run1 = (pair + 1) * n_runs / pairs;  // this pair's columns, in runs of 256
+    const int n_k = (run1 * kStagesPerRun < cols / kTK ? run1 * kStagesPerRun : cols / kTK) - run0 * kStagesPerRun;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kTSlots; ++s) {
-            // one arrive per decoder warp of the group that owns the slot, and in the first block of a pair one more for the
-            // second block's slot
-            bar_init(s32(&s_full[s]), kAThreads / 64 + ((PAIR && rank == 0) ? 1 : 0));
+        for (int s = 0; s < kTStages; ++s) {
+            // one arrive per decoder warp of the group that fills the stage, and in the first block of a pair one more for the
+            // second block's stage
+            bar_init(s32(&s_full[s]), kGroupWarps + (rank == 0 ? 1 : 0));
             bar_init(s32(&s_empty[s]), 1);
         }
-        for (int s = 0; s < kTStages; ++s) bar_init(s32(&s_xfull[s]), 1);  // the feeding thread's arrive with the stage's byte count
+        for (int s = 0; s < kXStages; ++s) {
+            bar_init(s32(&s_xfull[s]), 1);  // the feeding thread's arrive with the tile's byte count
+            bar_init(s32(&s_xempty[s]), 1);
+        }
         bar_init(s32(&s_done), 1);
-        for (int b = 0; b < 2; ++b) {
-            bar_init(s32(&s_raw_full[b]), kTM / 2);     // one arrive (with its byte count) per copy-issuing thread
+        for (int b = 0; b < kRaw; ++b) {
+            bar_init(s32(&s_raw_full[b]), 1);
             bar_init(s32(&s_raw_empty[b]), kAThreads / 32);  // every decoder warp is done with the buffer
         }
         s_failed = 0;
@@ -451,300 +396,248 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
         }
     }
     if (warp == 0) {  // tensor memory: 256 columns per accumulator (one block per SM)
-        if constexpr (PAIR) {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&s_tmem)), "r"(kTmemCols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&s_tmem)), "r"(kTmemCols) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        }
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(&s_tmem)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if constexpr (PAIR) cluster_sync_all();  // the other block's barriers and tensor memory exist before anybody signals or multiplies
+    cluster_sync_all();  // the other blocks' barriers and tensor memory exist before anybody signals or multiplies
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
     volatile int *failed = &s_failed;
-    // "full" is counted per block; the second block of a pair forwards each completed slot to the first block, which
-    // issues the MMAs, with one arrive of cluster scope (such an arrive per producer warp made every slot take a
-    // microsecond)
-    auto full_arrive = [&](int slot) { warp_arrive(s32(&s_full[slot])); };
 
-    const int n_slots = 2 * n_k;  // slot q of the pipeline: stage (q / 2) % 2, K half q % 2
-#if VQM_TC5_ABLATE & 8
-    if (warp <= kLoadWarp) {
-    } else
-#endif
     if (warp < 16) {
-        // ---- weight half-tile: four threads per row, one chunk each; chunk c of the stage (8 weights, 16 bytes of fp16)
-        //      goes to 16-byte slot c ^ (row % 8) of the row.
-        // What a warp does for a slot is one chain of dependent steps (wait for "empty", load, decode, store, proxy fence,
-        // arrive), so the warps are split into two groups that take the slots in turn - warps 0-7 the first K half of
-        // every stage, warps 8-15 the second - and a thread decodes two rows (r and r + 64) of each row half instead of
-        // one: twice the independent work per chain, half as many chains per warp (measured on one GPU with the TMA-fed
-        // activation tiles, 17408 x 5120 x 512: IQ4_XS with the generic decoder 103-105 instead of 108-113 us, the types
-        // with a fast decoder unchanged within the spread between runs).
-        // The rows of a warp go 0, 4, 1, 5, ...: the 8 lanes the store unit serves together then hit 8 different 16-byte
-        // columns of the swizzle (rows r and r + 4 use opposite halves).
-        constexpr int NR = 2 * MR;  // rows per thread: i -> row half i / 2, row r + 64 * (i % 2) of it
-        const int grp = warp >> 3;
-        const int quarter = threadIdx.x & 3, r8 = (threadIdx.x >> 2) & 7;
-        const int r = (warp & 7) * 8 + ((r8 >> 1) | ((r8 & 1) << 2));
-        bool valid[NR];
-        const uint8_t *w_row[NR];
-#pragma unroll
-        for (int i = 0; i < NR; ++i) {
-            const int row = row0 + (i >> 1) * kRowsPerAcc + r + 64 * (i & 1);
-            valid[i] = row < rows;
-            w_row[i] = w + static_cast<size_t>(valid[i] ? row : 0) * row_bytes;
-        }
-        // One slot of this thread: wait until the MMAs that read the slot's previous contents are done, store the 8 fp16
-        // weights of chunk `quarter` of the half stage for each of its rows (swizzled), make them visible to the tensor
-        // core, arrive.
-        auto slot_wait = [&](int q) -> bool { return warp_wait(s32(&s_empty[q % kTSlots]), ((q / kTSlots) & 1) ^ 1, failed); };
-        auto slot_put = [&](int q, int i, const uint32_t (&h)[4]) {
-            const int slot = q % kTSlots, c = (slot & 1) * 4 + quarter;  // chunk within the stage
-            const int row = (i >> 1) * kTM + r + 64 * (i & 1);          // row of the block's weight tile
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tiles + (slot >> 1) * kTStage + row * 128 + ((c ^ (r & 7)) << 4)),
-                         "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
+        // ---- weight tile: chunk c of the stage (8 weights, 16 bytes of fp16) goes to 16-byte slot c ^ (row % 8) of the row.
+        //      "full" is counted per block; the second block of a pair forwards each completed stage to the first block, which
+        //      issues the MMAs (such an arrive per producer warp made every half stage take a microsecond).
+        const int group = warp / kGroupWarps;
+        auto stage_wait = [&](int q) -> bool { return warp_wait(s32(&s_empty[q % kTStages]), ((q / kTStages) & 1) ^ 1, failed); };
+        auto stage_done = [&](int q) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            warp_arrive(s32(&s_full[q % kTStages]));
+        };
+        auto put = [&](int q, int row, int c, uint32_t h0, uint32_t h1, uint32_t h2, uint32_t h3) {
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(tiles + (q % kTStages) * kTA + row * 128 + ((c ^ (row & 7)) << 4)),
+                         "r"(h0), "r"(h1), "r"(h2), "r"(h3)
                          : "memory");
         };
-        auto slot_done = [&](int q) {
-#if !(VQM_TC5_ABLATE & 4)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#endif
-            full_arrive(q % kTSlots);
-        };
-        auto to_f16 = [](const float (&v)[8], uint32_t (&h)[4]) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const __half2 p = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-                h[e] = *reinterpret_cast<const uint32_t *>(&p);
-            }
-        };
         if constexpr (!kStaged) {
-            static_assert(kStaged || MR == 1, "two row halves only with the raw ring");
-            for (int q = grp; q < n_slots; q += 2) {
-                if (!slot_wait(q)) break;
-                const int kc = (q >> 1) * (kTK / 8) + (q & 1) * 4 + quarter;  // chunk within the row
+            // four threads per row, one chunk each, two rows per thread; rows go 0, 4, 1, 5, ... over a warp's lanes: the 8
+            // lanes that the store unit serves together then hit 8 different 16-byte columns of the swizzle
+            const int quarter = threadIdx.x & 3, r8 = (threadIdx.x >> 2) & 7;
+            const int r = (warp & 7) * 8 + ((r8 >> 1) | ((r8 & 1) << 2));
+            const uint8_t *w_row[2];
 #pragma unroll
-                for (int i = 0; i < NR; ++i) {
-                    uint32_t h[4] = {0u, 0u, 0u, 0u};
-                    if (valid[i]) {
-                        float v[8];
-                        deq8<TYPE>(w_row[i] + static_cast<size_t>(kc / CPB) * BB, kc % CPB, v, table);
-                        to_f16(v, h);
-                    }
-                    slot_put(q, i, h);
+            for (int i = 0; i < 2; ++i) w_row[i] = w + static_cast<size_t>(row0 + r + 64 * i < rows ? row0 + r + 64 * i : 0) * row_bytes;
+            for (int q = group; q < n_k; q += kGroups) {
+                if (!stage_wait(q)) break;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int c = quarter + 4 * (i >> 1), kc = (run0 * kStagesPerRun + q) * (kTK / 8) + c;  // chunk within the stage, the row
+                    float v[8];
+                    deq8<TYPE>(w_row[i & 1] + static_cast<size_t>(kc / CPB) * BB, kc % CPB, v, table);
+                    put(q, r + 64 * (i & 1), c, f16x2_of(pack2(v[0], v[1])), f16x2_of(pack2(v[2], v[3])), f16x2_of(pack2(v[4], v[5])),
+                        f16x2_of(pack2(v[6], v[7])));
                 }
-                slot_done(q);
+                stage_done(q);
             }
         } else {
-            // Raw ring: column `col` (256 weight columns) of the block's rows goes to buffer col % 2.  The first thread of a
-            // row in the first group issues the copies of its rows; the bytes keep their position inside their 16-byte line.
-            constexpr int kSlotsPerCol = 2 * kRawCols / kTK;  // 8
-            const int n_raw = (cols + kRawCols - 1) / kRawCols;
-            int raw_issued = 0;  // columns this thread has queued copies for
-            int raw_taken = 0;   // columns whose bytes this thread has waited for
-            auto issue_raw = [&](int col) -> bool {  // the whole warp calls it (first group only); true unless a wait gave up
-                const int b = col & 1;
-                if (col >= 2 && !warp_wait(s32(&s_raw_empty[b]), ((col >> 1) - 1) & 1, failed)) return false;
-                if (quarter == 0) {
-                    raw_issued = col + 1;
-                    const long long at = static_cast<long long>(col) * RUN;
-                    const uint32_t run = row_bytes - at < RUN ? static_cast<uint32_t>(row_bytes - at) : static_cast<uint32_t>(RUN);
-                    const uint32_t bar = s32(&s_raw_full[b]);
-                    uintptr_t p[NR];
-                    uint32_t bytes[NR], total = 0;
-#pragma unroll
-                    for (int i = 0; i < NR; ++i) {
-                        p[i] = reinterpret_cast<uintptr_t>(w_row[i]) + static_cast<uintptr_t>(at);
-                        bytes[i] = valid[i] ? ((static_cast<uint32_t>(p[i]) & 15u) + run + 15u) & ~15u : 0u;
-                        total += bytes[i];
-                    }
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(total) : "memory");
-#pragma unroll
-                    for (int i = 0; i < NR; ++i)
-                        if (bytes[i])
-                            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                             raw_ring + ((b * MR + (i >> 1)) * kTM + r + 64 * (i & 1)) * RSLOT),
-                                         "l"(p[i] & ~static_cast<uintptr_t>(15)), "r"(bytes[i]), "r"(bar)
-                                         : "memory");
+            const int r = (warp & 3) * 32 + lane;
+            // position of the row's bytes inside their 16-byte line, and of its class (row % 8) in a buffer
+            const uint32_t mis = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(w) + static_cast<size_t>(r & 7) * static_cast<size_t>(row_bytes)) & 15u);
+            const int cls = r & 7, slot = (((cls & ((1 << map_shift) - 1)) * 8) >> map_shift) + (cls >> map_shift);
+            const uint32_t row_at = raw_ring + (slot * (kTM / 8) + (r >> 3)) * PITCH;
+            const int part = kGroups == 4 ? 0 : (warp >> 2) & 1;  // two groups: which 32 columns of a stage
+            for (int q = group, run = 0, b = 0, use = 0; q < n_k; q += kGroups) {
+                const int in_run = q % kStagesPerRun;
+                if (in_run < kGroups && !warp_wait(s32(&s_raw_full[b]), use & 1, failed)) break;  // every lane: it reads the bytes
+                const uint32_t blk = row_at + b * (kTM * PITCH) + ((mis + static_cast<uint32_t>(run0 + run) * RUN) & 15u);
+                uint32_t h[kGroups == 4 ? 32 : 16];
+                decode_slots<TYPE, kGroups == 4 ? 2 : 1>(blk, 2 * in_run + part, table, h);
+                if (in_run + kGroups >= kStagesPerRun) {  // the group's last read of the buffer
+                    warp_arrive(s32(&s_raw_empty[b]));
+                    ++run;
+                    if (++b == kRaw) b = 0, ++use;
                 }
-                return true;
-            };
-            // Before slot g of column col.  Column col + 1 goes into the buffer column col - 1 left a little earlier: by the
-            // first group's second slot every decoder warp has normally handed it back, so the wait inside holds nobody up.
-            auto slot_begin = [&](int col, int g) -> bool {
-                if (g == 2 && col >= 1 && col + 1 < n_raw && !issue_raw(col + 1)) return false;
-                return slot_wait(col * kSlotsPerCol + g);
-            };
-            bool alive = grp != 0 || (issue_raw(0) && (n_raw < 2 || issue_raw(1)));
-            for (int col = 0; alive && col < n_raw; ++col) {
-                if (!warp_wait(s32(&s_raw_full[col & 1]), (col >> 1) & 1, failed)) break;  // every lane: it reads the bytes
-                raw_taken = col + 1;
-                uint32_t blk[NR];  // the rows' blocks of this column
+                if (!stage_wait(q)) break;
 #pragma unroll
-                for (int i = 0; i < NR; ++i)
-                    blk[i] = raw_ring + (((col & 1) * MR + (i >> 1)) * kTM + r + 64 * (i & 1)) * RSLOT +
-                             (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(w_row[i]) + static_cast<uintptr_t>(col) * RUN) & 15u);
-                if constexpr (has_fast_chunk(TYPE)) {
-                    // one block per column; the block header is unpacked once, the group's four slots are unrolled so that
-                    // every shift and byte position is a constant
-                    FastHeader<TYPE> hdr[NR];
-#pragma unroll
-                    for (int i = 0; i < NR; ++i) hdr[i].load(blk[i], quarter);
-                    auto one = [&](auto g_tag) -> bool {
-                        constexpr int G = decltype(g_tag)::value;
-                        if (col * kSlotsPerCol + G >= n_slots) return true;  // the last run of a 32-weight-block type may be short
-                        if (!slot_begin(col, G)) return false;
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) {
-                            uint32_t h[4] = {0u, 0u, 0u, 0u};
-#if !(VQM_TC5_ABLATE & 1)
-                            if (valid[i]) hdr[i].template chunk<G>(blk[i], quarter, h);
-#endif
-                            slot_put(col * kSlotsPerCol + G, i, h);
-                        }
-                        slot_done(col * kSlotsPerCol + G);
-                        return true;
-                    };
-                    if (grp == 0) alive = one(Int<0>{}) && one(Int<2>{}) && one(Int<4>{}) && one(Int<6>{});
-                    else alive = one(Int<1>{}) && one(Int<3>{}) && one(Int<5>{}) && one(Int<7>{});
-                } else {
-                    const int slots_here = n_slots - col * kSlotsPerCol < kSlotsPerCol ? n_slots - col * kSlotsPerCol : kSlotsPerCol;
-#pragma unroll 1
-                    for (int g = grp; g < slots_here; g += 2) {
-                        if (!slot_begin(col, g)) {
-                            alive = false;
-                            break;
-                        }
-                        const int in_col = g * 4 + quarter;  // chunk within the column
-#pragma unroll
-                        for (int i = 0; i < NR; ++i) {
-                            uint32_t h[4] = {0u, 0u, 0u, 0u};
-                            if (valid[i]) {
-                                float v[8];
-                                deq8<TYPE>(static_cast<const uint8_t *>(__cvta_shared_to_generic(blk[i] + (in_col / CPB) * BB)), in_col % CPB, v, table);
-                                to_f16(v, h);
-                            }
-                            slot_put(col * kSlotsPerCol + g, i, h);
-                        }
-                        slot_done(col * kSlotsPerCol + g);
-                    }
-                }
-                if (alive) warp_arrive(s32(&s_raw_empty[col & 1]));  // hand the buffer back
-            }
-            // Only after a wait gave up: copies this thread queued and nobody waited for must land before the block may
-            // leave (bounded; the columns complete in order).
-            for (int col = raw_taken; col < raw_issued; ++col) {
-#pragma unroll 1
-                for (int i = 0; i < (1 << 16) && !bar_try(s32(&s_raw_full[col & 1]), (col >> 1) & 1); ++i) __nanosleep(64);
+                for (int c = 0; c < 32 / kGroupWarps; ++c) put(q, r, 4 * part + c, h[4 * c], h[4 * c + 1], h[4 * c + 2], h[4 * c + 3]);
+                stage_done(q);
             }
         }
-    } else if (warp == kLoadWarp) {
-        // ---- activation tiles: one thread, one TMA tile copy per accumulator column block and stage (64 columns x kBN rows,
-        //      written in the same 128-byte swizzle; no multicast; rows beyond ntok exist in the buffer and are zero).  A stage
-        //      is refilled once the MMAs of its second half are done (MMAs complete in order).
+    } else if (warp == 16) {
+        // ---- activation tiles: one thread, one TMA tile copy per accumulator and stage (64 columns x half of the
+        //      accumulator's activation rows, in the same 128-byte swizzle; no multicast; rows beyond ntok arrive as zeros).
+        //      A buffer is refilled once its MMAs are done.
         if (lane == 0) {
             // The kernel is launched while the conversion of the activations may still run (programmatic stream
             // serialization); this thread is the only reader of its output.
             asm volatile("griddepcontrol.wait;" ::: "memory");
+            const int half = n_acc / 2;
             for (int k = 0; k < n_k; ++k) {
-                const int stage = k % kTStages, use = k / kTStages;
-                if (!bar_wait(s32(&s_empty[2 * stage + 1]), (use & 1) ^ 1, failed)) break;
+                const int stage = k % kXStages, use = k / kXStages;
+                if (!bar_wait(s32(&s_xempty[stage]), (use & 1) ^ 1, failed)) break;
                 const uint32_t bar = s32(&s_xfull[stage]);
-#if VQM_TC5_ABLATE & 2
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-#else
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(NH * kBN * 128) : "memory");
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(NH * half * 128) : "memory");
 #pragma unroll
                 for (int nh = 0; nh < NH; ++nh)
                     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                                     tiles + stage * kTStage + kTA + nh * kBN * 128),
-                                 "l"(&x_map), "r"(k * kTK), "r"(tok0 + nh * kTNH + static_cast<int>(rank) * kBN), "r"(bar)
+                                     x_tiles + stage * (NH * kTB) + nh * kTB),
+                                 "l"(&maps.x), "r"(run0 * kRawCols + k * kTK), "r"(tok0 + nh * n_acc + static_cast<int>(rank) * half), "r"(bar)
                                  : "memory");
-#endif
             }
         }
-    } else if (lane == 0 && rank != 0) {
-        // ---- second block of a pair: tell the first block about every slot that is full here
-        for (int q = 0; q < n_slots; ++q) {
-            const int slot = q % kTSlots;
-            if (!bar_wait(s32(&s_full[slot]), (q / kTSlots) & 1, failed)) break;
-            if ((q & 1) == 0 && !bar_wait(s32(&s_xfull[slot >> 1]), (q / kTSlots) & 1, failed)) break;  // this block's activation tile too
-            bar_arrive_cluster(in_block(s32(&s_full[slot]), 0));
-        }
-    } else if (lane == 0) {
-        // ---- MMA issue (the first block of a pair issues for both): accumulator (mr, nh) at column (mr * NH + nh) * 256
-        for (int q = 0; q < n_slots; ++q) {
-            const int slot = q % kTSlots;
-#if !(VQM_TC5_ABLATE & 8)
-            if (!(PAIR ? bar_wait_cluster(s32(&s_full[slot]), (q / kTSlots) & 1, failed) : bar_wait(s32(&s_full[slot]), (q / kTSlots) & 1, failed))) break;
-            if ((q & 1) == 0 && !bar_wait(s32(&s_xfull[slot >> 1]), (q / kTSlots) & 1, failed)) break;  // the stage's activation tile
-#endif
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t a_desc = sw128_desc(tiles + (slot >> 1) * kTStage), b_desc = sw128_desc(tiles + (slot >> 1) * kTStage + kTA);
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj) {  // 32 bytes further along K inside the swizzled rows per step
-                const int j = (slot & 1) * 2 + jj;
-                const uint32_t acc = (q | jj) != 0;
-#pragma unroll
-                for (int mr = 0; mr < MR; ++mr)
-#pragma unroll
-                    for (int nh = 0; nh < NH; ++nh) {  // accumulator (mr, nh): 128 weight rows (per block) x 256 activation rows
-                        const uint64_t a = a_desc + 2 * j + ((mr * kTM * 128) >> 4), bd = b_desc + 2 * j + ((nh * kBN * 128) >> 4);
-                        if constexpr (PAIR) mma_f16_pair(tmem + (mr * NH + nh) * 256, a, bd, acc);
-                        else mma_f16(tmem + (mr * NH + nh) * 256, a, bd, acc);
-                    }
+        __syncwarp();
+    } else if (warp == 17) {
+        if (rank != 0) {
+            // ---- second block of a pair: tell the first block about every stage that is full here
+            for (int q = 0; q < n_k; ++q) {
+                const int stage = q % kTStages;
+                // (and the activation tile that goes with it)
+                if (!warp_wait(s32(&s_xfull[q % kXStages]), (q / kXStages) & 1, failed)) break;
+                if (!warp_wait(s32(&s_full[stage]), (q / kTStages) & 1, failed)) break;
+                if (lane == 0) bar_arrive_cluster(in_block(s32(&s_full[stage]), in_cluster & ~1u));
             }
-            // the slot is free again, in both blocks of a pair, once these MMAs have read it
-            if constexpr (PAIR) mma_commit_pair(s32(&s_empty[slot]));
-            else mma_commit(s32(&s_empty[slot]));
+        } else {
+            // ---- MMA issue for both blocks: accumulator nh at column nh * 256.  D fp32, A and B fp16, both K-major, M = 256
+            const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(n_acc >> 3) << 17) | ((256u >> 4) << 24);
+            for (int q = 0; q < n_k; ++q) {
+                const int stage = q % kTStages, xs = q % kXStages;
+                if (!warp_wait(s32(&s_xfull[xs]), (q / kXStages) & 1, failed)) break;  // the stage's activation tile
+                if (!__all_sync(0xFFFFFFFFu, bar_wait_cluster(s32(&s_full[stage]), (q / kTStages) & 1, failed) ? 1 : 0)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (tc::elect_one()) {
+                    const uint64_t a_desc = sw128_desc(tiles + stage * kTA), b_desc = sw128_desc(x_tiles + xs * (NH * kTB));
+#pragma unroll
+                    for (int j = 0; j < kTK / 16; ++j)  // 32 bytes further along K inside the swizzled rows per step
+#pragma unroll
+                        for (int nh = 0; nh < NH; ++nh)
+                            mma_f16_pair(tmem + nh * 256, a_desc + 2 * j, b_desc + 2 * j + ((nh * kTB) >> 4), idesc, (q | j) != 0);
+                    // the buffers are free again, in both blocks of the pair, once these MMAs have read them
+                    mma_commit_pair(s32(&s_empty[stage]), static_cast<uint32_t>(pair));
+                    mma_commit_pair(s32(&s_xempty[xs]), static_cast<uint32_t>(pair));
+                }
+                __syncwarp();
+            }
+            if (tc::elect_one()) mma_commit_pair(s32(&s_done), static_cast<uint32_t>(pair));
         }
-        if constexpr (PAIR) mma_commit_pair(s32(&s_done));
-        else mma_commit(s32(&s_done));
+        __syncwarp();
+    } else if constexpr (kStaged) {
+        // ---- raw weights: one thread, map c of n brings the rows of classes c, c + n, ... (rows beyond the tensor arrive as zeros)
+        if (lane == 0) {
+            const int n_maps = 1 << map_shift;
+            int issued = 0;
+            for (int b = 0, use = 0; issued < run1 - run0; ++issued) {
+                if (use > 0 && !bar_wait(s32(&s_raw_empty[b]), (use - 1) & 1, failed)) break;
+                const uint32_t bar = s32(&s_raw_full[b]);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTM * PITCH) : "memory");
+#pragma unroll 1
+                for (int c = 0; c < n_maps; ++c) {
+                    const uint32_t mis = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(w) + static_cast<size_t>(c) * static_cast<size_t>(row_bytes)) & 15u);
+                    const uint32_t x = ((mis + static_cast<uint32_t>(run0 + issued) * RUN) & ~15u) / kTcElemBytes;
+                    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                                     raw_ring + b * (kTM * PITCH) + ((c * 8) >> map_shift) * (kTM / 8) * PITCH),
+                                 "l"(&maps.w[c]), "r"(x), "r"(row0 / 8), "r"(0), "r"(bar)
+                                 : "memory");
+                }
+                if (++b == kRaw) b = 0, ++use;
+            }
+            // the last copies land before the block may leave, also when the decoders gave up (bounded)
+            for (int run = issued > kRaw ? issued - kRaw : 0; run < issued; ++run)
+                for (int i = 0; i < (1 << 16) && !bar_try(s32(&s_raw_full[run % kRaw]), (run / kRaw) & 1); ++i) __nanosleep(64);
+        }
+        __syncwarp();
     }
 
+    const int lane_group = warp & 3, col_group = warp >> 2;  // a warp may read the 32 lanes (warp % 4) * 32 onwards
+    const uint32_t tm_mine = tmem + (static_cast<uint32_t>(lane_group * 32) << 16);
+    const int row = row0 + lane_group * 32 + lane;  // thread = weight row, the warps of a lane group share the column chunks
+    bool ok = true;
     if (warp < 16) {
-        // ---- epilogue: thread = weight row (TMEM lane) of each row half, loads of 32 columns.  A warp may read the 32 lanes
-        //      (warp % 4) * 32 onwards, so the sixteen decoder warps work as four groups that share the column chunks.
-        const bool ok = bar_wait(s32(&s_done), 0, failed);
+        ok = warp_wait(s32(&s_done), 0, failed);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int lane_group = warp & 3, col_group = warp >> 2;
-        if (ok) {
-#pragma unroll 1
-            for (int cc = col_group; cc < MR * (kTN / 32); cc += 4) {
-                const int mr = cc / (kTN / 32), c = cc % (kTN / 32);
-                const int row = row0 + mr * kRowsPerAcc + lane_group * 32 + lane;
-                uint32_t v[32];
-                const uint32_t at = tmem + (static_cast<uint32_t>(lane_group * 32) << 16) + mr * kTN + c * 32;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, "
-                    "%18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                      "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                      "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(at)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row < rows) {
+    }
+    auto read16 = [&](uint32_t at, float (&v)[16]) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+              "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+            : "r"(at)
+            : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    };
+    auto store16 = [&](int tok, const float (&v)[16]) {
+        if (row >= rows) return;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const int tok = tok0 + c * 32 + j;
-                        if (tok < ntok) y[static_cast<size_t>(tok) * rows + row] = __uint_as_float(v[j]);
+        for (int j = 0; j < 16; ++j)
+            if (tok + j < ntok) y[static_cast<size_t>(tok + j) * rows + row] = v[j];
+    };
+    const int chunks = n_acc / kXChunk;  // of an accumulator
+    if (pairs == 1) {
+        if (warp < 16 && ok) {
+#pragma unroll 1
+            for (int c = col_group; c < NH * chunks; c += 4) {
+                const int nh = c >= chunks ? 1 : 0, local = c - nh * chunks;
+                float v[16];
+                read16(tm_mine + nh * 256 + local * kXChunk, v);
+                store16(tok0 + nh * n_acc + local * kXChunk, v);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int nh = 0; nh < NH; ++nh) {
+            cluster_sync_all();  // everybody's MMAs are done with the stages (and the sums of the round before have been read)
+            if (warp < 16) {
+#pragma unroll 1
+                for (int c = col_group; c < chunks; c += 4) {
+                    const int owner = c % pairs;
+                    if (owner == pair) continue;
+                    float v[16];
+                    read16(tm_mine + nh * 256 + c * kXChunk, v);
+                    const uint32_t to = in_block(tiles + ((c / pairs) * (pairs - 1) + (pair < owner ? pair : pair - 1)) * kXBytes +
+                                                     (lane_group * 32 + lane) * 16,
+                                                 static_cast<uint32_t>(owner) * 2 + rank);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + j * (kTM * 16)), "f"(v[4 * j]), "f"(v[4 * j + 1]),
+                                     "f"(v[4 * j + 2]), "f"(v[4 * j + 3])
+                                     : "memory");
+                }
+            }
+            cluster_sync_all();
+            if (warp < 16) {
+#pragma unroll 1
+                for (int c = pair + pairs * col_group; c < chunks; c += 4 * pairs) {
+                    float own[16], v[16];
+                    read16(tm_mine + nh * 256 + c * kXChunk, own);
+#pragma unroll 1
+                    for (int p = 0; p < pairs; ++p) {  // in the order of the columns
+                        float from[16];
+                        if (p == pair) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) from[j] = own[j];
+                        } else {
+                            const uint32_t at = tiles + ((c / pairs) * (pairs - 1) + (p < pair ? p : p - 1)) * kXBytes + (lane_group * 32 + lane) * 16;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const uint4 q = lds128u(at + j * (kTM * 16));
+                                from[4 * j] = __uint_as_float(q.x), from[4 * j + 1] = __uint_as_float(q.y);
+                                from[4 * j + 2] = __uint_as_float(q.z), from[4 * j + 3] = __uint_as_float(q.w);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] = p == 0 ? from[j] : v[j] + from[j];
                     }
+                    store16(tok0 + nh * n_acc + c * kXChunk, v);
                 }
             }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if constexpr (PAIR) cluster_sync_all();  // neither block's shared or tensor memory goes away under the other
+    cluster_sync_all();  // no block's shared or tensor memory goes away under another
     if (warp == 0) {
-        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
         if (lane == 0 && s_failed) atomicExch(status, kStatusWaitExpired);
     }
 }
@@ -752,93 +645,121 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
 using PFN_encodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                      const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-template <int TYPE, int MR, int NH, bool PAIR>
-cudaError_t launch_shape(const uint8_t *w, const __half *xh, float *y, int rows, int cols, long long row_bytes, int ntok, const uint8_t *codebook,
-                         unsigned *status, cudaStream_t stream) {
-    constexpr size_t smem = tc5_smem_bytes(TYPE, MR, NH, PAIR, stages_for(TYPE, MR, NH, PAIR));
-    static_assert(smem <= 227 * 1024, "shared memory of the tcgen05 GEMM");
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t err =
-            cudaFuncSetAttribute(qgemm_tc5_kernel<TYPE, MR, NH, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+// The activations as a 2-D tensor [activation rows][cols] of fp16; a tile is 64 columns (one 128-byte swizzled row each) of
+// `box_rows` activation rows, rows beyond the last are zeros.
+cudaError_t encode_x_map(CUtensorMap *map, const __half *xh, int cols, int ntok, int box_rows) {
+    static PFN_encodeTiled encode = nullptr;
+    if (encode == nullptr) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
         if (err != cudaSuccess) return err;
-        configured = true;
+        if (fn == nullptr || found != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
+        encode = reinterpret_cast<PFN_encodeTiled>(fn);
     }
-    constexpr int kRowsPerUnit = kTM * MR * (PAIR ? 2 : 1);  // weight rows of a block, or of a pair of blocks
-    // The activations as a 2-D tensor [padded activation rows][cols] of fp16; a tile is 64 columns (one 128-byte swizzled
-    // row each) of the activation rows one block holds of an accumulator.
-    CUtensorMap x_map;
-    {
-        static PFN_encodeTiled encode = nullptr;
-        if (encode == nullptr) {
-            void *fn = nullptr;
-            cudaDriverEntryPointQueryResult found;
-            const cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
-            if (err != cudaSuccess) return err;
-            if (fn == nullptr || found != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
-            encode = reinterpret_cast<PFN_encodeTiled>(fn);
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(ntok)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
+    const cuuint32_t box[2] = {kTK, static_cast<cuuint32_t>(box_rows)}, elem[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+               ? cudaSuccess
+               : cudaErrorInvalidValue;
+}
+
+template <int TYPE, int NH>
+struct Tc5Variant {
+    static constexpr int kSmem = tc5_smem_bytes(TYPE, NH, stages_for(TYPE, NH));
+    static_assert(kSmem <= 227 * 1024, "shared memory of the tcgen05 GEMM");
+    static_assert(kSmem - table_bytes16(TYPE) - 1024 >= (kMaxPairs - 1) * (kTNMax / kXChunk / kMaxPairs) * kXBytes, "room for the exchange");
+    static constexpr auto kKernel = qgemm_tc5_kernel<TYPE, NH>;
+
+    static void configure(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int row_tiles, int tok_tiles, int pairs, cudaStream_t stream) {
+        cfg.gridDim = dim3(static_cast<unsigned>(row_tiles * pairs * 2), static_cast<unsigned>(tok_tiles));
+        cfg.blockDim = dim3(kTThreads);
+        cfg.dynamicSmemBytes = kSmem;
+        cfg.stream = stream;
+        // May start while the kernel before it in the stream (the fp32 -> fp16 conversion of the activations) still runs: the
+        // set-up, the first weight copies and the first decoded tiles overlap it; the thread that feeds the activations waits.
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = static_cast<unsigned>(pairs * 2);
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+    }
+    // clusters of `pairs` pairs that fit on the GPU at once (cached; one device per process), 0 if the kernel cannot run
+    static int clusters(int pairs) {
+        static int cached[kMaxPairs + 1] = {};
+        if (cached[pairs] == 0) {
+            int n = 0;
+            cudaLaunchConfig_t cfg{};
+            cudaLaunchAttribute attr[2];
+            configure(cfg, attr, 1024, 1, pairs, nullptr);
+            if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
+                cudaOccupancyMaxActiveClusters(&n, kKernel, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                n = 0;
+            }
+            cached[pairs] = n > 0 ? n : -1;
         }
-        const int tile = 2 * kTNH, padded = (ntok + tile - 1) / tile * tile;  // the runtime pads the buffer to gemm_tc5_token_tile()
-        const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(padded)};
-        const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-        const cuuint32_t box[2] = {kTK, PAIR ? kTNH / 2 : kTNH}, elem[2] = {1, 1};
-        if (encode(&x_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(xh), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorInvalidValue;
+        return cached[pairs] < 0 ? 0 : cached[pairs];
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((rows + kRowsPerUnit - 1) / kRowsPerUnit * (PAIR ? 2 : 1), (ntok + kTNH * NH - 1) / (kTNH * NH));
-    cfg.blockDim = dim3(kTThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    // May start while the kernel before it in the stream (the fp32 -> fp16 conversion of the activations) still runs: the
-    // set-up, the first weight copies and the first decoded tiles overlap it; the thread that feeds the activations waits for it.
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    int n_attr = 1;
-    if constexpr (PAIR) {  // the two blocks of a pair form a cluster
-        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-        attr[n_attr].val.clusterDim.x = 2;
-        attr[n_attr].val.clusterDim.y = 1;
-        attr[n_attr].val.clusterDim.z = 1;
-        ++n_attr;
+};
+
+// Shape of a launch: accumulators per block (NH), activation rows of each, tiles of activation rows, and how many pairs share
+// the columns.  Estimated time in us, fitted to Q6_K 1024 x 5120 and Q4_K 5120 x 17408 with 64 to 512 activation rows, which
+// took, alone and in every shape, what this says within 2 us: a wave of clusters walks its share of the stages, pays for start and
+// end, and for the sums that the pairs of a cluster send each other.
+struct Tc5Plan {
+    int nh, n_acc, tok_tiles, pairs;
+};
+template <int TYPE>
+Tc5Plan plan_t(int rows, int cols, int ntok) {
+    const int row_tiles = (rows + 2 * kTM - 1) / (2 * kTM), n_runs = (cols + kRawCols - 1) / kRawCols;
+    Tc5Plan best{};
+    float best_cost = 0.0f;
+    for (int nh = 1; nh <= 2; ++nh) {
+        const int tok_tiles = (ntok + nh * kTNMax - 1) / (nh * kTNMax);
+        const int n_acc = ((ntok + tok_tiles * nh - 1) / (tok_tiles * nh) + 63) / 64 * 64;
+        for (int pairs = 1; pairs <= kMaxPairs && pairs <= n_runs; ++pairs) {
+            const int fit = nh == 1 ? Tc5Variant<TYPE, 1>::clusters(pairs) : Tc5Variant<TYPE, 2>::clusters(pairs);
+            if (fit == 0) continue;
+            const int waves = (row_tiles * tok_tiles + fit - 1) / fit, stages = (n_runs + pairs - 1) / pairs * kStagesPerRun;
+            const float f = static_cast<float>(n_acc) / 256.0f, both = static_cast<float>(nh) * f;
+            const float stage = nh == 1 ? 0.385f + 0.045f * f : 0.44f + 0.16f * f * f;  // decoding bounds one accumulator, the MMAs two
+            const float cost = static_cast<float>(waves) * (static_cast<float>(stages) * stage + 9.0f + both +
+                                                            (pairs > 1 ? 1.0f + both * (1.6f * static_cast<float>(pairs) - 0.7f) : 0.0f));
+            if (best.nh == 0 || cost < best_cost) best = {nh, n_acc, tok_tiles, pairs}, best_cost = cost;
+        }
     }
-    cfg.attrs = attr;
-    cfg.numAttrs = n_attr;
-    return cudaLaunchKernelEx(&cfg, qgemm_tc5_kernel<TYPE, MR, NH, PAIR>, x_map, w, y, rows, cols, row_bytes, ntok, codebook, status);
+    return best;
 }
 
 template <int TYPE>
 cudaError_t launch_t(const uint8_t *w, const __half *xh, float *y, int rows, int cols, long long row_bytes, int ntok, const uint8_t *codebook,
                      unsigned *status, cudaStream_t stream) {
-    // Which shape for which case was measured on 17408 x 5120 weights with 512 activation rows (times with the conversion
-    // of the activations; VQM_TC5_SHAPE selects the alternatives in an experiment build):
-    //   0  pairs of 1 x 2 blocks: 99-101 us for the four K-quants with a fast decoder, IQ4_XS 106, Q8_0 133 - the default
-    //   1  single 1 x 2 blocks: the same for the K-quants, IQ4_XS 123, Q8_0 137
-    //   2  2 x 1 (256 weight rows per block; pairs where the raw ring only fits beside a pair's smaller stages): 114-122;
-    //      every weight is decoded once per 256 instead of once per 512 activation rows, which costs more than the halved
-    //      activation traffic saves now that TMA feeds the activation tiles
-    // Up to 256 activation rows: a pair of 1 x 1 blocks (90 us).
-    if (ntok <= kTNH) return launch_shape<TYPE, 1, 1, true>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
-#if VQM_TC5_SHAPE == 1
-    return launch_shape<TYPE, 1, 2, false>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
-#elif VQM_TC5_SHAPE == 2
-    if constexpr (has_fast_chunk(TYPE) && fits_two_row_halves(TYPE, false)) {
-        return launch_shape<TYPE, 2, 1, false>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
-    } else if constexpr (has_fast_chunk(TYPE) && fits_two_row_halves(TYPE, true)) {
-        return launch_shape<TYPE, 2, 1, true>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
-    } else {
-        return launch_shape<TYPE, 1, 2, true>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
+    const Tc5Plan plan = plan_t<TYPE>(rows, cols, ntok);
+    if (plan.nh == 0) return cudaErrorInvalidConfiguration;
+    Tc5Maps maps{};
+    cudaError_t err = encode_x_map(&maps.x, xh, cols, ntok, plan.n_acc / 2);
+    if (err == cudaSuccess && raw_staged(TYPE)) err = tc_encode_maps(TYPE, w, rows, row_bytes, kTM / 8, maps.w);
+    if (err != cudaSuccess) return err;
+    const int shift = tc_map_shift(rows, row_bytes);
+    const int row_tiles = (rows + 2 * kTM - 1) / (2 * kTM);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[2];
+    if (plan.nh == 1) {
+        Tc5Variant<TYPE, 1>::configure(cfg, attr, row_tiles, plan.tok_tiles, plan.pairs, stream);
+        return cudaLaunchKernelEx(&cfg, Tc5Variant<TYPE, 1>::kKernel, maps, w, y, rows, cols, row_bytes, ntok, plan.n_acc, shift, codebook, status);
     }
-#else
-    return launch_shape<TYPE, 1, 2, true>(w, xh, y, rows, cols, row_bytes, ntok, codebook, status, stream);
-#endif
+    Tc5Variant<TYPE, 2>::configure(cfg, attr, row_tiles, plan.tok_tiles, plan.pairs, stream);
+    return cudaLaunchKernelEx(&cfg, Tc5Variant<TYPE, 2>::kKernel, maps, w, y, rows, cols, row_bytes, ntok, plan.n_acc, shift, codebook, status);
 }
 
 }  // namespace
 
-int gemm_tc5_token_tile() { return 2 * kTNH; }  // the activation buffer is padded to the largest tile
+int gemm_tc5_token_tile() { return 2 * kTNMax; }
 bool gemm_tc5_supports(int cols) { return cols % kTK == 0; }
 
 cudaError_t launch_qgemm_tc5(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,

@@ -86,6 +86,7 @@ enum : unsigned { kStatusOk = 0, kStatusWaitExpired = 1, kStatusPeerWaitExpired 
 VQM_FOR_EACH_TYPE(VQM_DECLARE_LAUNCHER)
 #undef VQM_DECLARE_LAUNCHER
 
+constexpr int kTcTileRows = 256;   // rows of a tile of the tensor-core matvec
 constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matvec: times 31 it has to fit into the 11 bits of fp16
 // The tensor-core matvec (vqm_tcmv_type.cu).  maps: per tensor of the launch its tensor maps (tc_encode_maps).
 #define VQM_FOR_EACH_TC_TYPE(X) \
@@ -98,7 +99,8 @@ constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matve
                                    cudaStream_t stream);
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_TC_LAUNCHER)
 #undef VQM_DECLARE_TC_LAUNCHER
-cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, CUtensorMap *out);
+// box_rows: rows of a class that one copy brings (32: a tile of 256 rows in all)
+cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, int box_rows, CUtensorMap *out);
 
 constexpr int kMaxGrid = 4096;  // upper bound on the matvec grid (sizes the argmax partial arrays)
 

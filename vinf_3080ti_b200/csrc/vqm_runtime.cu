@@ -295,7 +295,7 @@ cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cuda
     if (!use_tcmv(type, a, sm_count, false)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
     CUtensorMap maps[8];
     const CUtensorMap *p[1] = {maps};
-    const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, maps);
+    const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, vqm::kTcTileRows / 8, maps);
     if (err != cudaSuccess) return err;
     return dispatch_tcmv(type, a, p, 1, m, sm_count, stream);
 }
@@ -378,7 +378,8 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
             if (ts[i]->maps.empty()) {
                 ts[i]->maps.resize(8);
-                err = vqm::tc_encode_maps(ts[i]->type, ts[i]->data, ts[i]->rows, static_cast<long long>(ts[i]->row_bytes), ts[i]->maps.data());
+                err = vqm::tc_encode_maps(ts[i]->type, ts[i]->data, ts[i]->rows, static_cast<long long>(ts[i]->row_bytes), vqm::kTcTileRows / 8,
+                                          ts[i]->maps.data());
                 if (err != cudaSuccess) ts[i]->maps.clear();
             }
             maps[i] = ts[i]->maps.data();
@@ -961,7 +962,9 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
             if (err != cudaSuccess) return cuda_fail("prompt-pass activation buffer", err);
             rt->gemm_x_len = need;
         }
-        err = vqm::launch_f32_to_f16_rows(xp, rt->gemm_x, static_cast<long long>(ntok) * t->cols, static_cast<long long>(need), rt->stream);
+        // (the tcgen05 kernel's tile copies fill in the rows beyond the last themselves)
+        err = vqm::launch_f32_to_f16_rows(xp, rt->gemm_x, static_cast<long long>(ntok) * t->cols,
+                                          tc5 ? static_cast<long long>(ntok) * t->cols : static_cast<long long>(need), rt->stream);
         if (err == cudaSuccess) {
             if (tc5)
                 err = vqm::launch_qgemm_tc5(t->type, t->data, rt->gemm_x, yp, t->rows, t->cols, static_cast<long long>(t->row_bytes), ntok, cb,

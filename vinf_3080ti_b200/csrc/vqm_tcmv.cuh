@@ -44,7 +44,7 @@
 
 namespace vqm {
 
-constexpr int kTcRows = 256, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
+constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcGroupB = 32 * kTcCore;           // bytes of 8 B rows over a step
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums

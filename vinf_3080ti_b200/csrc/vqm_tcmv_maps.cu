@@ -10,7 +10,7 @@ namespace vqm {
 // remainder.  A copy never reads past the tensor: with a number of rows that is no multiple of 8 every class has a map of its
 // own, with its own number of rows.
 // (Eight copies per stage instead of one cost 1.2 us at a launch's start: each map is fetched on its own.)
-cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, CUtensorMap *out) {
+cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, int box_rows, CUtensorMap *out) {
     using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static Encode encode = nullptr;
@@ -24,7 +24,7 @@ cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_b
     }
     const cuuint32_t elem = kTcElemBytes;
     const int n = 1 << tc_map_shift(rows, row_bytes);
-    const cuuint32_t box[3] = {static_cast<cuuint32_t>(tc_pitch(type)) / elem, 32, static_cast<cuuint32_t>(8 / n)}, step[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {static_cast<cuuint32_t>(tc_pitch(type)) / elem, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(8 / n)}, step[3] = {1, 1, 1};
     const cuuint64_t stride[2] = {static_cast<cuuint64_t>(row_bytes) * 8, static_cast<cuuint64_t>(row_bytes) * (n == 8 ? 8 : n)};
     for (int c = 0; c < n; ++c) {
         const int first = c < rows ? c : 0;  // (a class without rows is copied from somewhere valid and never used)
