@@ -79,7 +79,20 @@ cudaError_t launch_dequant_t(const uint8_t *w, float *out, long long numel, cons
     return cudaGetLastError();
 }
 
+// Copies from pinned host memory (16-byte words), one word in flight per thread: what follows it in the stream may be launched
+// with programmatic stream serialization and sets itself up meanwhile.
+__global__ void __launch_bounds__(256) fetch_kernel(const uint4 *from, uint4 *to, int n) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) to[i] = from[i];
+}
+
 }  // namespace
+
+cudaError_t launch_fetch(const void *from, void *to, int n16, cudaStream_t stream) {
+    fetch_kernel<<<(n16 + 255) / 256, 256, 0, stream>>>(static_cast<const uint4 *>(from), static_cast<uint4 *>(to), n16);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_argmax_rows(const float *x, int n, int ntok, int *out, cudaStream_t stream) {
     argmax_rows_kernel<<<ntok, 1024, 0, stream>>>(x, n, out);

@@ -118,6 +118,8 @@ bool gemm_tc5_supports(int cols);
 cudaError_t launch_qgemm_tc5(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,
                              const uint8_t *codebook, unsigned *status, cudaStream_t stream);
 
+// n16 16-byte words from pinned host memory
+cudaError_t launch_fetch(const void *from, void *to, int n16, cudaStream_t stream);
 cudaError_t launch_argmax_rows(const float *x, int n, int ntok, int *out, cudaStream_t stream);
 cudaError_t launch_dequant(int type, const uint8_t *w, float *out, long long numel, const uint8_t *codebook,
                            cudaStream_t stream);

@@ -126,6 +126,9 @@ const int kCodebookTypes[5] = {vqm::kIQ2_XXS, vqm::kIQ2_XS, vqm::kIQ2_S, vqm::kI
 
 }  // namespace
 
+// A synchronous matvec stores up to this many outputs straight into host memory; more are faster through device memory and one
+// copy (F32 32768 x 64: 58 us, 62 straight; Q4_K 17408 x 5120: the same either way; Q6_K 1024 x 5120: 34 us, 32 straight).
+constexpr int kDirectRows = 16384;
 constexpr size_t kStatusWords = 4;  // status word of a synchronous matvec, padded to 16 bytes
 
 struct vqm_runtime {
@@ -147,7 +150,7 @@ struct vqm_runtime {
     int allow_split = 1;  // short launches may be split by columns (VINF_B200_NO_SPLIT=1 turns it off)
     // scratch of the synchronous matvec entry
     float *scratch_x = nullptr;
-    unsigned *scratch_y = nullptr;  // kStatusWords, then the outputs
+    unsigned *scratch_y = nullptr;  // kStatusWords, then the outputs, of more than kDirectRows rows
     size_t scratch_x_n = 0, scratch_y_n = 0;
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
@@ -444,7 +447,7 @@ int matvec_scratch(vqm_runtime *rt, size_t cols, size_t rows) {
         err = cudaMalloc(&rt->scratch_x, sizeof(float) * cols);
         if (err == cudaSuccess) rt->scratch_x_n = cols;
     }
-    if (err == cudaSuccess && rt->scratch_y_n < rows) {
+    if (err == cudaSuccess && rows > kDirectRows && rt->scratch_y_n < rows) {
         cudaFree(rt->scratch_y);
         rt->scratch_y = nullptr;
         rt->scratch_y_n = 0;
@@ -453,7 +456,7 @@ int matvec_scratch(vqm_runtime *rt, size_t cols, size_t rows) {
         if (err == cudaSuccess) rt->scratch_y_n = rows;
     }
     if (err != cudaSuccess) return cuda_fail("scratch allocation", err);
-    const size_t bytes = sizeof(float) * (cols > rows + kStatusWords ? cols : rows + kStatusWords);
+    const size_t bytes = sizeof(float) * (kStatusWords + (rows + 3) / 4 * 4 + cols);
     if (rt->pinned_bytes < bytes) {
         g_pinned.give(rt->pinned, rt->pinned_bytes);
         rt->pinned_bytes = 0;
@@ -1100,27 +1103,28 @@ int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t 
     if (t.cols % 32 != 0) return fail(VQM_ERR_VALUE, "%s: matvec cols must be a multiple of 32", weight);
     int rc = no_capture(rt, "matvec");
     if (rc != VQM_OK) return rc;
-    // Host vectors go through pinned staging and come back, together with the status word, in one copy: with the caller's
-    // pageable memory every one of the three copies (x, y, status) is a synchronisation of its own.
+    // Pinned staging holds the status word, y and x.  A kernel fetches x, and few outputs go straight into the staging: a copy on
+    // a copy engine costs the stream a hand-over each way.
     if ((rc = matvec_scratch(rt, static_cast<size_t>(t.cols), static_cast<size_t>(t.rows))) != VQM_OK) return rc;
-    memcpy(rt->pinned, x_host, x_bytes);
-    cudaError_t err = cudaMemcpyAsync(rt->scratch_x, rt->pinned, x_bytes, cudaMemcpyHostToDevice, rt->stream);
+    unsigned *const got = static_cast<unsigned *>(rt->pinned), *const out = t.rows > kDirectRows ? rt->scratch_y : got;
+    float *const y_at = reinterpret_cast<float *>(got + kStatusWords), *const x_at = y_at + (t.rows + 3) / 4 * 4;
+    memcpy(x_at, x_host, x_bytes);
+    got[0] = 0;
+    cudaError_t err = vqm::launch_fetch(x_at, rt->scratch_x, t.cols / 4, rt->stream);
     if (err != cudaSuccess) return cuda_fail("qmatvec H2D", err);
     unsigned *const shared_status = rt->status;
-    rt->status = rt->scratch_y;  // the launch's own status word sits in front of its outputs
-    rc = launch_group(rt, t, rt->scratch_x, reinterpret_cast<float *>(rt->scratch_y + kStatusWords), 1, false);
+    rt->status = out;  // the launch's own status word sits in front of its outputs
+    rc = launch_group(rt, t, rt->scratch_x, reinterpret_cast<float *>(out + kStatusWords), 1, false);
     rt->status = shared_status;
     if (rc != VQM_OK) return rc;
-    const size_t back = sizeof(unsigned) * kStatusWords + sizeof(float) * t.rows;
-    err = cudaMemcpyAsync(rt->pinned, rt->scratch_y, back, cudaMemcpyDeviceToHost, rt->stream);
+    if (out != got) err = cudaMemcpyAsync(got, out, sizeof(unsigned) * (kStatusWords + static_cast<size_t>(t.rows)), cudaMemcpyDeviceToHost, rt->stream);
     if (err == cudaSuccess) err = cudaStreamSynchronize(rt->stream);
     if (err != cudaSuccess) return cuda_fail("qmatvec", err);
-    const unsigned *got = static_cast<const unsigned *>(rt->pinned);
     if (got[0] != 0) {
-        cudaMemsetAsync(rt->scratch_y, 0, sizeof(unsigned), rt->stream);
+        if (out != got) cudaMemsetAsync(out, 0, sizeof(unsigned), rt->stream);
         return status_failure("qmatvec", got[0]);
     }
-    memcpy(y_host, got + kStatusWords, sizeof(float) * t.rows);
+    memcpy(y_host, y_at, sizeof(float) * t.rows);
     return VQM_OK;
 }
 
