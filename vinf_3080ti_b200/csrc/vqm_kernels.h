@@ -37,6 +37,7 @@ struct MatvecPart {
 struct MatvecArgs {
     MatvecPart part[kMaxParts];
     const float *x;          // [M][cols] fp32, 16-byte aligned
+    const uint8_t *x_split;  // ready-made B operands of more than 8 activation rows (tensor-core matvec)
     const uint8_t *codebook;  // device copy of the type's GGUF codebook (IQ2/IQ3 types), else null
     unsigned *status;        // device error word (0 = fine)
     // fused argmax (all null / 0 when unused; single-tensor launches only)
@@ -97,6 +98,13 @@ constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matve
     int split_tcmv_##name(const MatvecArgs &a, int sm_count);                                                                    \
     cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, \
                                    cudaStream_t stream);
+// split_bytes_*: size of a.x_split for a launch of 9..16 rows over a.cols columns, 0 if the type takes 8 at most;
+// launch_split_*: fills a.x_split (writable there) from a.x.
+#define VQM_DECLARE_SPLIT(id, name)                   \
+    size_t split_bytes_##name(int cols);               \
+    cudaError_t launch_split_##name(const MatvecArgs &a, int m, cudaStream_t stream);
+VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_SPLIT)
+#undef VQM_DECLARE_SPLIT
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_TC_LAUNCHER)
 #undef VQM_DECLARE_TC_LAUNCHER
 // box_rows: rows of a class that one copy brings (32: a tile of 256 rows in all)

@@ -152,6 +152,9 @@ struct vqm_runtime {
     float *scratch_x = nullptr;
     unsigned *scratch_y = nullptr;  // kStatusWords, then the outputs, of more than kDirectRows rows
     size_t scratch_x_n = 0, scratch_y_n = 0;
+    uint8_t *x_split = nullptr;     // ready-made B operands of 9..16 activation rows
+    size_t x_split_bytes = 0;
+    std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
     bool counted = false;    // by the pinned pool
@@ -181,6 +184,13 @@ const uint8_t *codebook_for(vqm_runtime *rt, int type) {
     for (int i = 0; i < 5; ++i)
         if (kCodebookTypes[i] == type) return rt->codebooks[i];
     return nullptr;
+}
+
+// Whether the type's codebook, if it has one, is small enough for the tensor-core matvec.
+bool codebook_fits(const vqm_runtime *rt, int type) {
+    for (int i = 0; i < 5; ++i)
+        if (kCodebookTypes[i] == type) return rt->codebook_small[i];
+    return false;
 }
 
 Tensor *find_tensor(vqm_runtime *rt, const char *name, int *status) {
@@ -293,6 +303,24 @@ cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap 
     }
 }
 
+// Ready-made B operands of 9..16 activation rows: their size (0: the type takes 8 rows at most), and the kernel that makes them.
+size_t split_bytes(int type, int cols) {
+    switch (type) {
+#define VQM_CASE(id, name) case id: return vqm::split_bytes_##name(cols);
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+        default: return 0;
+    }
+}
+cudaError_t dispatch_split(int type, const vqm::MatvecArgs &a, int m, cudaStream_t stream) {
+    switch (type) {
+#define VQM_CASE(id, name) case id: return vqm::launch_split_##name(a, m, stream);
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 // One tensor in device memory that has no Tensor record.
 cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cudaStream_t stream) {
     if (!use_tcmv(type, a, sm_count, false)) return dispatch_qmv(type, a, m, sm_count, stream, nullptr);
@@ -373,10 +401,7 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         a.row_base = t0.argmax_row_base;
     }
     cudaError_t err = cudaSuccess;
-    bool codebook_small = false;
-    for (int i = 0; i < 5; ++i)
-        if (kCodebookTypes[i] == t0.type) codebook_small = rt->codebook_small[i];
-    if (use_tcmv(t0.type, a, rt->sm_count, codebook_small)) {
+    if (use_tcmv(t0.type, a, rt->sm_count, codebook_fits(rt, t0.type))) {
         const CUtensorMap *maps[vqm::kMaxParts];
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
             if (ts[i]->maps.empty()) {
@@ -386,6 +411,11 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
                 if (err != cudaSuccess) ts[i]->maps.clear();
             }
             maps[i] = ts[i]->maps.data();
+        }
+        if (err == cudaSuccess && m > 8) {
+            a.x_split = rt->x_split;
+            err = dispatch_split(t0.type, a, m, rt->stream);
+            count_launch(rt);
         }
         if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, m, rt->sm_count, rt->stream);
     } else {
@@ -400,6 +430,27 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
     Tensor *ts[1] = {&t};
     float *ys[1] = {y};
     return launch_parts(rt, 1, ts, x, ys, m, with_argmax, push);
+}
+
+// Whether the tensor takes 9..16 activation rows in one launch; makes room for their B operands.
+bool takes_sixteen(vqm_runtime *rt, const Tensor &t) {
+    const size_t need = split_bytes(t.type, t.cols);
+    if (need == 0) return false;
+    vqm::MatvecArgs a{};
+    set_single_part(a, t.data, nullptr, t.rows);
+    a.rows = t.rows, a.cols = t.cols, a.allow_split = rt->allow_split;
+    if (!use_tcmv(t.type, a, rt->sm_count, codebook_fits(rt, t.type))) return false;
+    if (need <= rt->x_split_bytes) return true;
+    if (rt->capturing) return false;
+    uint8_t *p = nullptr;
+    if (cudaMalloc(&p, need) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    if (rt->x_split != nullptr) rt->retired.push_back(rt->x_split);  // a captured graph may hold its address
+    rt->x_split = p;
+    rt->x_split_bytes = need;
+    return true;
 }
 
 // The tensors and output buffers of a group call, checked: same type and columns, every y large enough.
@@ -530,6 +581,8 @@ void vqm_runtime_destroy(vqm_runtime *rt) {
     cudaFree(rt->argmax_vals);
     cudaFree(rt->scratch_x);
     cudaFree(rt->scratch_y);
+    cudaFree(rt->x_split);
+    for (uint8_t *p : rt->retired) cudaFree(p);
     g_pinned.give(rt->pinned, rt->pinned_bytes);
     if (rt->counted) g_pinned.runtime_destroyed();
     cudaFree(rt->gemm_x);
@@ -980,9 +1033,10 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
         count_launch(rt, 2);
         return VQM_OK;
     }
-    // every group of 8 activation rows re-reads the weight (from L2 when it fits)
-    for (int c = 0; c < ntok; c += 8) {
-        const int m = ntok - c < 8 ? ntok - c : 8;
+    // every group of 8 or 16 activation rows re-reads the weight (from L2 when it fits)
+    const int widest = ntok > 8 && takes_sixteen(rt, *t) ? 16 : 8;
+    for (int c = 0, m = 0; c < ntok; c += m) {
+        m = ntok - c < widest ? ntok - c : widest;
         rc = launch_group(rt, *t, xp + static_cast<size_t>(c) * t->cols, yp + static_cast<size_t>(c) * t->rows, m, false);
         if (rc != VQM_OK) return rc;
     }

@@ -91,18 +91,22 @@ __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 
 template <int MC>
 struct TcShape {
     static constexpr int kGroupsB = (3 * MC + 7) / 8;
-    static constexpr int kN = kGroupsB <= 2 ? 16 : 32;
+    static constexpr int kN = kGroupsB <= 2 ? 16 : kGroupsB <= 4 ? 32 : 48;
 };
 // per step: the activation rows' scales, then the sums of the column groups that share a minimum
 __host__ __device__ constexpr int tc_info_scales(int mc) { return mc < 4 ? 4 : mc; }
 __host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(mc) + 2 * tc_mins(type) * mc; }
+// More than 8 activation rows: their B operand and infos come ready-made (tc_split_kernel), by bulk copies, because the stages
+// have no room for 16 KB of activations; the tile's sums go out 8 activation rows at a time.
+__host__ __device__ constexpr bool tc_presplit(int mc) { return mc > 8; }
+__host__ __device__ constexpr int tc_out_rows(int mc) { return mc > 8 ? 8 : mc; }
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(TYPE) + MC * kTcStepCols * 4; }
+__host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(TYPE) + (tc_presplit(MC) ? 0 : MC * kTcStepCols * 4); }
 // Shared memory beside the weight stages, with `b` B stages (an MMA may read one group of rows further).
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_fixed_bytes(int b) {
     return (grid_bytes(TYPE) + 127) / 128 * 128 + (b * TcShape<MC>::kGroupsB + 1) * kTcGroupB + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
-           2 * 264 * MC * 4 + (kTcMaxNormSteps + 2) * MC * 4 + 256;
+           2 * 264 * tc_out_rows(MC) * 4 + (tc_presplit(MC) ? 0 : (kTcMaxNormSteps + 2) * MC * 4) + 256;
 }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_stages_beside(int b) {
@@ -117,6 +121,12 @@ template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_smem_bytes() {
     return 1024 + tc_fixed_bytes<TYPE, MC>(tc_b_stages<TYPE, MC>()) + tc_stages<TYPE, MC>() * tc_stage_bytes<TYPE, MC>();
 }
+
+// bytes of a step in the buffer of ready-made B operands: the operand, then the infos
+template <int TYPE, int MC>
+__host__ __device__ constexpr int tc_split_bytes() { return TcShape<MC>::kGroupsB * kTcGroupB + tc_info_floats(TYPE, MC) * 4; }
+// 16 activation rows at a time: not the types with a sum per 32 columns (96 columns of sums do not fit beside A in tensor memory)
+__host__ __device__ constexpr bool tc_sixteen(int type) { return !tc_block32(type); }
 
 // ---- primitives --------------------------------------------------------------------------------------------------------
 namespace tc {

@@ -177,6 +177,47 @@ struct TcAcc {
 template <int TYPE, int MC>
 __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
     constexpr int kSums = tc_sums<TYPE, MC>(), kMins = tc_mins(TYPE);
+    if constexpr (MC > 8) {  // eight activation rows at a time, for the registers' sake
+        static_assert(kSums == 1, "one sum per unit");
+        const f32x2 s2 = pack2(p.s[0], p.s[0]), c1 = pack2(0x1p-11f, 0x1p-11f), c2 = pack2(0x1p-22f, 0x1p-22f);
+#pragma unroll
+        for (int t0 = 0; t0 < MC; t0 += 8) {
+            float v0[8], v1[8], v2[8];
+            tc::ld8(d_at + t0, v0);
+            tc::ld8(d_at + MC + t0, v1);
+            tc::ld8(d_at + 2 * MC + t0, v2);
+            const ulonglong2 ia = lds128(p.info + t0 * 4), ib = lds128(p.info + t0 * 4 + 16);
+            const f32x2 inv[4] = {ia.x, ia.y, ib.x, ib.y};
+            tc::wait_ld();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                f32x2 u = fma2(pack2(v1[2 * i], v1[2 * i + 1]), c1, pack2(v0[2 * i], v0[2 * i + 1]));
+                u = fma2(pack2(v2[2 * i], v2[2 * i + 1]), c2, u);
+                acc.v[t0 / 2 + i] = fma2(mul2(u, s2), inv[i], acc.v[t0 / 2 + i]);
+            }
+        }
+        if constexpr (kMins > 0) {
+#pragma unroll
+            for (int h = 0; h < tc_halves(TYPE); ++h) {
+                auto one = [&](auto tag) {
+                    constexpr int G = decltype(tag)::value;
+                    if constexpr (G < kMins) {
+                        const float m = -p.unit[h].template minimum<G>();
+                        const uint32_t at = p.info + (tc_info_scales(MC) + ((tc_wide(TYPE) ? h : p.kh) * kMins + G) * MC) * 4;
+#pragma unroll
+                        for (int t = 0; t < MC; t += 4) {
+                            const ulonglong2 w = lds128(at + t * 4);
+                            acc.v[t / 2] = fma2(pack2(m, m), w.x, acc.v[t / 2]);
+                            acc.v[t / 2 + 1] = fma2(pack2(m, m), w.y, acc.v[t / 2 + 1]);
+                        }
+                    }
+                };
+                one(TcInt<0>{}), one(TcInt<1>{}), one(TcInt<2>{}), one(TcInt<3>{});
+                one(TcInt<4>{}), one(TcInt<5>{}), one(TcInt<6>{}), one(TcInt<7>{});
+            }
+        }
+        return;
+    }
     float v[kSums][3 * MC + 1];
 #pragma unroll
     for (int g = 0; g < kSums; ++g) tc::ld_sums<MC>(d_at + g * TcShape<MC>::kN, v[g]);
@@ -291,13 +332,29 @@ __device__ __forceinline__ void tc_finish_argmax(const MatvecArgs &a, int m, flo
     if (threadIdx.x == 0) *a.done_counter = 0;
 }
 
+// B operands and infos of up to MC activation rows, one block per step: what every block of the matvec would work out for itself.
+template <int TYPE, int MC>
+__global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant__ MatvecArgs a, uint8_t *out, const int m) {
+    constexpr int kOperand = TcShape<MC>::kGroupsB * kTcGroupB, kBytes = tc_split_bytes<TYPE, MC>();
+    __shared__ __align__(16) uint8_t image[kBytes];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int step = blockIdx.x, t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+    if (t < m) tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, tc::s32(image), tc::s32(image) + kOperand, 0u, lane);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kBytes / 16; i += MC * 32)
+        reinterpret_cast<uint4 *>(out + static_cast<size_t>(step) * kBytes)[i] = reinterpret_cast<const uint4 *>(image)[i];
+}
+
 template <int TYPE, int MC, typename MAPS>
 __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_constant__ MatvecArgs a, const __grid_constant__ MAPS maps, const int m) {
     using Shape = TcShape<MC>;
     constexpr int kStages = tc_stages<TYPE, MC>(), kStageBytes = tc_stage_bytes<TYPE, MC>();
     constexpr int kPitch = tc_pitch(TYPE), kStepBytes = tc_step_bytes(TYPE);
     constexpr int kNB = tc_b_stages<TYPE, MC>();
-    constexpr bool kWide = tc_wide(TYPE);
+    constexpr bool kWide = tc_wide(TYPE), kPresplit = tc_presplit(MC);
+    constexpr int kOut = tc_out_rows(MC);  // activation rows whose sums go out together
     constexpr uint32_t kTmD = 64;  // a group's sums start at this column of its 128
     constexpr uint32_t kIdesc = (1u << 4) | (static_cast<uint32_t>(Shape::kN >> 3) << 17) | ((128u >> 4) << 24);  // fp32 += fp16 * fp16, M = 128
     static_assert(kStages >= (kWide ? 3 : 2) && kStages + 2 <= kTcInfoSlots, "stage ring");
@@ -316,7 +373,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     const uint32_t b_ring = table + (grid_bytes(TYPE) + 127) / 128 * 128;
     const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * kTcGroupB;
     const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
-    const uint32_t norm_parts = red + 2 * 264 * MC * 4;
+    const uint32_t norm_parts = red + 2 * 264 * kOut * 4;
     volatile int *failed = &s_failed;
 
     const int k_split = a.k_split;
@@ -339,7 +396,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         const int p = part_of(tile), y = (tile - first_tile(p)) * 32;
         const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
         const uint32_t bar = tc::s32(&s_wfull[stage]), at = stages + stage * kStageBytes;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcRows * kPitch + (with_x ? m * cols_here * 4 : 0))
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTcRows * kPitch + (with_x && !kPresplit ? m * cols_here * 4 : 0))
                      : "memory");
         const int shift = a.tc_map_shift[p];  // map c of n brings classes c, c + n, c + 2n, ...
 #pragma unroll 1
@@ -353,6 +410,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     };
     auto copy_x = [&](int step, int stage) {  // one thread
         const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+        if constexpr (kPresplit) return;
         for (int t = 0; t < m; ++t)
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                              stages + stage * kStageBytes + kTcRows * kPitch + t * (kTcStepCols * 4)),
@@ -370,7 +428,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             tc::bar_init(tc::s32(&s_wempty[s]), kWide ? 8 : 16);
         }
         for (int s = 0; s < kNB; ++s) {
-            tc::bar_init(tc::s32(&s_bfull[s]), static_cast<uint32_t>(m));
+            tc::bar_init(tc::s32(&s_bfull[s]), kPresplit ? 1u : static_cast<uint32_t>(m));
             tc::bar_init(tc::s32(&s_bempty[s]), kWide ? 2 : 4);
         }
         for (int g = 0; g < 4; ++g) {
@@ -416,6 +474,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         if (tc::elect_one()) {
             int filled = 0, stage = 0;
             uint32_t phase = 0;
+            [[maybe_unused]] int bs = 0;
+            [[maybe_unused]] uint32_t bphase = 0;
             for (int tile = group; tile < n_tiles && !*failed; tile += n_groups)
                 for (int step = step0; step < step1; ++step) {
                     if (filled >= kStages) {
@@ -424,6 +484,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         copy_weights(tile, step, stage, filled >= kNB);
                     }
                     if (filled >= kNB) copy_x(step, stage);
+                    if constexpr (kPresplit) {  // the step's B operand and infos
+                        constexpr int kOperand = Shape::kGroupsB * kTcGroupB, kInfo = tc_info_floats(TYPE, MC) * 4;
+                        if (filled >= kNB) {
+                            tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
+                            if (*failed) break;
+                        }
+                        const uint8_t *from = a.x_split + static_cast<size_t>(step) * tc_split_bytes<TYPE, MC>();
+                        const uint32_t bar = tc::s32(&s_bfull[bs]);
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kOperand + kInfo) : "memory");
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                         b_ring + bs * kOperand),
+                                     "l"(from), "r"(kOperand), "r"(bar)
+                                     : "memory");
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                         info_ring + (filled & (kTcInfoSlots - 1)) * kInfo),
+                                     "l"(from + kOperand), "r"(kInfo), "r"(bar)
+                                     : "memory");
+                        if (++bs == kNB) bs = 0, bphase ^= 1u;
+                    }
                     ++filled;
                     if (++stage == kStages) stage = 0, phase ^= 1u;
                 }
@@ -490,7 +569,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
 
         // The first kNB steps' activations are converted by all warps at once, straight from global memory: the way through the
         // stages would put a copy and a turn of conversions (1 us) between the end of the previous kernel and the first MMAs.
-        for (int n = 0, t = warp;; t += 16) {
+        for (int n = kPresplit ? kNB : 0, t = warp; n < kNB; t += 16) {
             while (t >= m && n < kNB) t -= m, ++n;
             if (n == kNB) break;
             int local = n;
@@ -512,7 +591,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 if (!kWide || (st & 1) == pair) {
                     tc::bar_wait(tc::s32(&s_wfull[stage]), wphase, failed);
                     const uint32_t at = stages + stage * kStageBytes, info = info_ring + (st & (kTcInfoSlots - 1)) * tc_info_floats(TYPE, MC) * 4;
-                    {
+                    if constexpr (!kPresplit) {
                         // the warps that share the step take turns at splitting activation rows
                         const int t = kWide ? (warp - (st >> 1) * m) & 7 : (warp - st * m) & 15;
                         if (t < m && st >= kNB) {
@@ -628,24 +707,29 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 }
             }
             const int r0 = rank * red_rows, r1 = r0 + red_rows < kTcRows ? r0 + red_rows : kTcRows;
+            float sums[MC];
+            acc.get(sums);
+            acc.clear();
+#pragma unroll
+            for (int round = 0; round < MC / kOut; ++round) {
             {
                 const int r = cls + 8 * lane, owner = (r * a.tc_deal_recip) >> 16;
-                float out[MC];
-                acc.get(out);
-                const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * red_rows)) * (MC * 4);
+                float out[kOut];
+#pragma unroll
+                for (int t = 0; t < kOut; ++t) out[t] = sums[round * kOut + t];
+                const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * red_rows)) * (kOut * 4);
                 if (k_split == 1) {
 #pragma unroll
-                    for (int t = 0; t < MC; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + t * 4), "f"(out[t]) : "memory");
+                    for (int t = 0; t < kOut; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + t * 4), "f"(out[t]) : "memory");
                 } else {
                     if (!announced) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
                     announced = true;
                     if (threadIdx.x == 0) {
-                        const int bytes = (r1 - r0) * (2 * MC * 4) * k_split + ((a.fuse & kFuseNorm) && tile == group ? m * k_split * 4 : 0);
+                        const int bytes = (r1 - r0) * (2 * kOut * 4) * k_split + ((a.fuse & kFuseNorm) && tile == group ? m * k_split * 4 : 0);
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::s32(&s_cluster)), "r"(bytes) : "memory");
                     }
-                    tc::st_async_row<MC>(tc::in_block(to, owner), out, tc::in_block(tc::s32(&s_cluster), owner));
+                    tc::st_async_row<kOut>(tc::in_block(to, owner), out, tc::in_block(tc::s32(&s_cluster), owner));
                 }
-                acc.clear();
             }
             if (k_split == 1) {
                 tc::decoders_sync();
@@ -654,7 +738,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 rphase ^= 1u;
             }
             {
-                const int t = warp & (MC - 1);
+                const int t = round * kOut + (warp & (kOut - 1));
                 const MatvecPart &part = a.part[p];
                 if (t < m) {
                     float factor = 1.0f;
@@ -663,15 +747,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         for (int k = 0; k < k_split; ++k) sq += s_norm[k][t];
                         factor = 1.0f / sqrtf(sq / static_cast<float>(a.cols) + a.eps);
                     }
-                    for (int r = r0 + (warp / MC) * 32 + lane; r < r1; r += 512 / MC) {
+                    for (int r = r0 + (warp / kOut) * 32 + lane; r < r1; r += 512 / kOut) {
                         const int row = (tile - tile0) * kTcRows + r;
                         if (row >= part.rows) break;
                         float sum = 0.0f;
 #pragma unroll
                         for (int k = 0; k < kMaxSplit; ++k)
                             if (k < k_split) {
-                                const uint32_t at = red + ((2 * k * red_rows + (r - r0)) * MC + t) * 4;
-                                sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + MC * red_rows * 4));
+                                const uint32_t at = red + ((2 * k * red_rows + (r - r0)) * kOut + (warp & (kOut - 1))) * 4;
+                                sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + kOut * red_rows * 4));
                             }
                         if (a.fuse & kFuseNorm) sum *= factor;
                         if (part.y != nullptr) {
@@ -683,7 +767,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     }
                 }
             }
-            if (tile + n_groups < n_tiles) {  // the sums may be overwritten once everybody has read them
+            if (round + 1 < MC / kOut || tile + n_groups < n_tiles) {  // the sums may be overwritten once everybody has read them
                 tc::decoders_sync();
                 if (k_split > 1) {
                     if (threadIdx.x < static_cast<unsigned>(k_split))
@@ -692,6 +776,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     tc::bar_wait_cluster(tc::s32(&s_read), sphase, failed);
                     sphase ^= 1u;
                 }
+            }
             }
         }
     }

@@ -111,12 +111,46 @@ inline int choose_tc_split(int n_tiles, int cols, int sm_count) {
     return static_cast<long long>(n_tiles) * n_steps >= 20ll * best_walk ? best : 0;
 }
 
+// More than 8 activation rows (templates, so that types without the variant do not compile it)
+template <int TYPE>
+cudaError_t launch_sixteen(const MatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+    if constexpr (tc_sixteen(TYPE)) {
+        if (a.x_split == nullptr || a.fuse != 0 || a.out_idx != nullptr) return cudaErrorInvalidValue;
+        return TcVariant<(TYPE >= 0 ? 16 : 0), TcMaps1>::launch(a, maps, 1, n_tiles, m, sm_count, stream);
+    } else {
+        return cudaErrorInvalidValue;
+    }
+}
+template <int TYPE>
+cudaError_t split_sixteen(const MatvecArgs &a, int m, cudaStream_t stream) {
+    if constexpr (tc_sixteen(TYPE)) {
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = dim3(static_cast<unsigned>((a.cols + kTcStepCols - 1) / kTcStepCols));
+        cfg.blockDim = dim3(16 * 32);
+        cfg.stream = stream;
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = a.overlap_launch ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, tc_split_kernel<TYPE, 16>, a, const_cast<uint8_t *>(a.x_split), m);
+    } else {
+        return cudaErrorInvalidValue;
+    }
+}
+
 }  // namespace
 
 #define VQM_CAT2(a, b) a##b
 #define VQM_CAT(a, b) VQM_CAT2(a, b)
 
 int VQM_CAT(split_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &a, int sm_count) { return choose_tc_split(tc_tiles(a), a.cols, sm_count); }
+
+size_t VQM_CAT(split_bytes_, VQM_TYPE_NAME)(int cols) {
+    return tc_sixteen(VQM_TYPE) ? static_cast<size_t>((cols + kTcStepCols - 1) / kTcStepCols) * tc_split_bytes<VQM_TYPE, 16>() : 0;
+}
+
+cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, int m, cudaStream_t stream) { return split_sixteen<VQM_TYPE>(a, m, stream); }
 
 cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, int m, int sm_count,
                                                  cudaStream_t stream) {
@@ -134,6 +168,7 @@ cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const C
     if (m == 2) return VQM_LAUNCH(2);
     if (m <= 4) return VQM_LAUNCH(4);
     if (m <= 8) return VQM_LAUNCH(8);
+    if (m <= 16 && n_parts == 1) return launch_sixteen<VQM_TYPE>(a, maps, n_tiles, m, sm_count, stream);
     return cudaErrorInvalidValue;
 #undef VQM_LAUNCH
 }
