@@ -24,15 +24,18 @@ constexpr int kBM = 64, kBN = 256, kBK = 32, kLd = kBK + 8;  // +8 halves: confl
 constexpr int kGemmThreads = 256;
 
 // The GEMM that follows is launched with programmatic stream serialization: its blocks may set themselves up while this
-// kernel still runs (they wait for its completion before they read xh), so the trigger comes first.
+// kernel still runs (they wait for its completion before they read xh), so the trigger comes first.  This kernel is launched
+// the same way and waits for what comes before it (which may produce x, or still read xh).
 __global__ void __launch_bounds__(256) f32_to_f16_rows_kernel(const float *x, __half *xh, long long n_valid, long long n_total) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n_total) xh[i] = __float2half_rn(i < n_valid ? x[i] : 0.0f);
 }
 // Eight elements per thread: two 16-byte loads, one 16-byte store (x 16-byte aligned, both counts multiples of 8).
 __global__ void __launch_bounds__(256) f32_to_f16_rows8_kernel(const float4 *x, uint4 *xh, long long n_valid8, long long n_total8) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n_total8) return;
     uint4 out = make_uint4(0u, 0u, 0u, 0u);
@@ -183,15 +186,19 @@ cudaError_t launch_t(const uint8_t *w, const __half *xh, float *y, int rows, int
 int gemm_token_tile() { return kBN; }
 
 cudaError_t launch_f32_to_f16_rows(const float *x, void *xh, long long n_valid, long long n_total, cudaStream_t stream) {
-    if (n_valid % 8 == 0 && n_total % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(xh) % 16 == 0) {
-        const long long blocks = (n_total / 8 + 255) / 256;
-        f32_to_f16_rows8_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(reinterpret_cast<const float4 *>(x), static_cast<uint4 *>(xh),
-                                                                                   n_valid / 8, n_total / 8);
-    } else {
-        const long long blocks = (n_total + 255) / 256;
-        f32_to_f16_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(x, static_cast<__half *>(xh), n_valid, n_total);
-    }
-    return cudaGetLastError();
+    const bool wide = n_valid % 8 == 0 && n_total % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(xh) % 16 == 0;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(static_cast<unsigned>((n_total / (wide ? 8 : 1) + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (wide)
+        return cudaLaunchKernelEx(&cfg, f32_to_f16_rows8_kernel, reinterpret_cast<const float4 *>(x), static_cast<uint4 *>(xh), n_valid / 8, n_total / 8);
+    return cudaLaunchKernelEx(&cfg, f32_to_f16_rows_kernel, x, static_cast<__half *>(xh), n_valid, n_total);
 }
 
 cudaError_t launch_qgemm(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,

@@ -403,6 +403,8 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     __syncthreads();
     cluster_sync_all();  // the other blocks' barriers and tensor memory exist before anybody signals or multiplies
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // (the next conversion of activations may be launched; it waits for this kernel's end before it touches anything)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem = s_tmem;
     volatile int *failed = &s_failed;
 
