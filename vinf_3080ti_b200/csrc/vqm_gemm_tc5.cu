@@ -761,7 +761,6 @@ cudaError_t launch_t(const uint8_t *w, const __half *xh, float *y, int rows, int
 
 }  // namespace
 
-int gemm_tc5_token_tile() { return 2 * kTNMax; }
 bool gemm_tc5_supports(int cols) { return cols % kTK == 0; }
 
 cudaError_t launch_qgemm_tc5(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,

@@ -66,6 +66,7 @@ struct MatvecArgs {
     // Filled in by the launcher of the tensor-core matvec (so that no block starts with integer divisions):
     int tc_steps[9];         // block k of a cluster takes the 256-column steps [tc_steps[k], tc_steps[k + 1])
     int tc_deal, tc_deal_recip;  // rows of a tile that each block of a cluster finishes, and 65536 / tc_deal rounded up
+    int tc_first, tc_end;        // tiles of this launch (a launch may take the last round of another, see choose_tc_tail)
     unsigned char tc_map_shift[kMaxParts];  // log2 of the number of tensor maps of each tensor
     PushInfo push;           // all zero when the tensor is not sharded
 };
@@ -118,10 +119,9 @@ cudaError_t launch_f32_to_f16_rows(const float *x, void *xh, long long n_valid, 
 cudaError_t launch_qgemm(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,
                          const uint8_t *codebook, cudaStream_t stream);
 
-// Prompt-pass GEMM on tcgen05 tensor cores with the accumulators in tensor memory (vqm_gemm_tc5.cu): xh padded to
-// gemm_tc5_token_tile() rows; needs cols to be a multiple of 64.  status: device word that receives a code if a bounded
+// Prompt-pass GEMM on tcgen05 tensor cores with the accumulators in tensor memory (vqm_gemm_tc5.cu); xh: ntok rows, needs
+// cols to be a multiple of 64.  status: device word that receives a code if a bounded
 // wait expires.
-int gemm_tc5_token_tile();
 bool gemm_tc5_supports(int cols);
 cudaError_t launch_qgemm_tc5(int type, const uint8_t *w, const void *xh, float *y, int rows, int cols, long long row_bytes, int ntok,
                              const uint8_t *codebook, unsigned *status, cudaStream_t stream);

@@ -998,9 +998,9 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
         const uint8_t *cb = codebook_for(rt, t->type);
         if (vqm::grid_is_codebook(t->type) && cb == nullptr)
             return fail(VQM_ERR_VALUE, "the codebook for GGUF type %d has not been set (vqm_set_codebook)", t->type);
-        // tcgen05 kernel (activation buffer padded to 512 rows) from 64 rows on, the warp-level MMA kernel below that
+        // tcgen05 kernel (its tile copies fill in rows beyond the last) from 64 rows on, the warp-level MMA kernel below that
         const bool tc5 = rt->gemm_tcgen05 && ntok >= 64 && vqm::gemm_tc5_supports(t->cols);
-        const int tile = tc5 ? vqm::gemm_tc5_token_tile() : vqm::gemm_token_tile();
+        const int tile = tc5 ? 1 : vqm::gemm_token_tile();
         const size_t need = static_cast<size_t>((ntok + tile - 1) / tile * tile) * t->cols;
         cudaError_t err = cudaSuccess;
         if (need > rt->gemm_x_len) {
@@ -1018,9 +1018,7 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
             if (err != cudaSuccess) return cuda_fail("prompt-pass activation buffer", err);
             rt->gemm_x_len = need;
         }
-        // (the tcgen05 kernel's tile copies fill in the rows beyond the last themselves)
-        err = vqm::launch_f32_to_f16_rows(xp, rt->gemm_x, static_cast<long long>(ntok) * t->cols,
-                                          tc5 ? static_cast<long long>(ntok) * t->cols : static_cast<long long>(need), rt->stream);
+        err = vqm::launch_f32_to_f16_rows(xp, rt->gemm_x, static_cast<long long>(ntok) * t->cols, static_cast<long long>(need), rt->stream);
         if (err == cudaSuccess) {
             if (tc5)
                 err = vqm::launch_qgemm_tc5(t->type, t->data, rt->gemm_x, yp, t->rows, t->cols, static_cast<long long>(t->row_bytes), ntok, cb,

@@ -325,8 +325,12 @@ __device__ __forceinline__ void tc_finish_argmax(const MatvecArgs &a, int m, flo
         }
         warp_best();
         if (lane == 0) {
-            a.out_idx[warp] = bi == 0x7fffffff ? bi : bi + a.row_base;
-            if (a.out_val != nullptr) a.out_val[warp] = bv;
+            bi = bi == 0x7fffffff ? bi : bi + a.row_base;
+            // a launch that takes the last tiles of a tensor: the launch before it has left the best of the others, all lower rows
+            if (a.tc_first == 0 || bv > a.out_val[warp]) {
+                a.out_idx[warp] = bi;
+                if (a.out_val != nullptr) a.out_val[warp] = bv;
+            }
         }
     }
     if (threadIdx.x == 0) *a.done_counter = 0;
@@ -383,7 +387,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     asm("mov.u32 %0, %%nclusterid.x;" : "=r"(n_groups));
     const int step0 = a.tc_steps[rank], step1 = a.tc_steps[rank + 1];
     auto tiles_of = [&](int p) { return (a.part[p].rows + kTcRows - 1) / kTcRows; };
-    const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = end2 + tiles_of(3);
+    const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = a.tc_end;
+    group += a.tc_first;
     // the tensor a tile belongs to, and that tensor's first tile
     auto part_of = [&](int tile) { return (tile >= end0) + (tile >= end1) + (tile >= end2); };
     auto first_tile = [&](int p) { return p == 0 ? 0 : p == 1 ? end0 : p == 2 ? end1 : end2; };

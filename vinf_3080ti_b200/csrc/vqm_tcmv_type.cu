@@ -81,6 +81,26 @@ inline int tc_tiles(const MatvecArgs &a) {
     return n;
 }
 
+// Tall tensors, whose blocks walk whole rows: the last round of tiles may occupy a few SMs only (LM head, 151936 rows: 594 tiles
+// on 148 SMs, 2 of them in a fifth round).  Its tiles then go to a second launch that splits their columns, if that saves more
+// than a launch costs (3.4 us, two to three steps).  first: its first tile, 0 if there is none.
+struct TcTail {
+    int first = 0, k_split = 0;
+};
+inline TcTail choose_tc_tail(int n_tiles, int cols, int sm_count, int k_split) {
+    const int n_steps = (cols + kTcStepCols - 1) / kTcStepCols, fit1 = TcVariant<1, TcMaps1>::clusters(1, sm_count);
+    if (k_split != 1 || fit1 == 0 || n_tiles <= fit1 || n_tiles % fit1 == 0) return {};
+    const int rest = n_tiles % fit1;
+    int best = 0, best_steps = n_steps;
+    for (int s = 2; s <= kMaxSplit && s <= n_steps; ++s)
+        if (rest <= TcVariant<1, TcMaps1>::clusters(s, sm_count) && (n_steps + s - 1) / s < best_steps) best = s, best_steps = (n_steps + s - 1) / s;
+    if (best == 0 || best_steps + 4 > n_steps) return {};
+    return {n_tiles - rest, best};
+}
+
+// (one tensor; an argmax is merged through its values)
+inline bool takes_tail(const MatvecArgs &a) { return a.part[1].rows == 0 && (a.out_idx == nullptr || a.out_val != nullptr); }
+
 // Into how many column ranges the rows' sums are split, 0 if the launch is too small for this kernel.  Depends on rows and
 // columns only.
 // Time of a launch in steps of 256 columns: every group of blocks walks `rounds` tiles of 256 rows, each block its share of the
@@ -95,7 +115,7 @@ inline int tc_tiles(const MatvecArgs &a) {
 // other kernel.  A decoder layer (1 row / 4 rows fused) takes 81 / 90 us with its 1024 x 5120 projections here and 92 / 115 us with
 // them there, although each alone is faster there.  So it takes launches of 72 pieces of 256 x 256 weights or more of which no
 // block has to walk more than one in 20.
-inline int choose_tc_split(int n_tiles, int cols, int sm_count) {
+inline int choose_tc_split(int n_tiles, int cols, int sm_count, bool single) {
     const int n_steps = (cols + kTcStepCols - 1) / kTcStepCols;
     if (static_cast<long long>(n_tiles) * n_steps < 72) return 0;
     int best = 0, best_walk = 0;
@@ -105,8 +125,13 @@ inline int choose_tc_split(int n_tiles, int cols, int sm_count) {
         if (fit == 0) continue;
         const int groups = n_tiles < fit ? n_tiles : fit, rounds = (n_tiles + groups - 1) / groups, steps = (n_steps + s - 1) / s;
         const int walk = tc_wide(VQM_TYPE) ? (rounds * steps + 1) / 2 * 2 : rounds * steps;
-        const float cost = static_cast<float>(walk) + static_cast<float>(rounds) * (s > 1 ? 1.5f : 1.0f);
-        if (best == 0 || cost < best_cost) best = s, best_cost = cost, best_walk = rounds * steps;
+        float cost = static_cast<float>(walk) + static_cast<float>(rounds) * (s > 1 ? 1.5f : 1.0f);
+        int walked = rounds * steps;
+        if (const TcTail tail = s == 1 ? choose_tc_tail(n_tiles, cols, sm_count, s) : TcTail{}; single && tail.first > 0) {
+            walked = (rounds - 1) * steps + (steps + tail.k_split - 1) / tail.k_split;
+            cost = static_cast<float>(walked + rounds) + 3.0f;
+        }
+        if (best == 0 || cost < best_cost) best = s, best_cost = cost, best_walk = walked;
     }
     return static_cast<long long>(n_tiles) * n_steps >= 20ll * best_walk ? best : 0;
 }
@@ -144,7 +169,9 @@ cudaError_t split_sixteen(const MatvecArgs &a, int m, cudaStream_t stream) {
 #define VQM_CAT2(a, b) a##b
 #define VQM_CAT(a, b) VQM_CAT2(a, b)
 
-int VQM_CAT(split_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &a, int sm_count) { return choose_tc_split(tc_tiles(a), a.cols, sm_count); }
+int VQM_CAT(split_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &a, int sm_count) {
+    return choose_tc_split(tc_tiles(a), a.cols, sm_count, takes_tail(a));
+}
 
 size_t VQM_CAT(split_bytes_, VQM_TYPE_NAME)(int cols) {
     return tc_sixteen(VQM_TYPE) ? static_cast<size_t>((cols + kTcStepCols - 1) / kTcStepCols) * tc_split_bytes<VQM_TYPE, 16>() : 0;
@@ -155,7 +182,18 @@ cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, int m, cu
 cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, int m, int sm_count,
                                                  cudaStream_t stream) {
     MatvecArgs a = args;
-    const int n_tiles = tc_tiles(a);
+    int n_tiles = tc_tiles(a);
+    if (const TcTail tail = takes_tail(a) ? choose_tc_tail(n_tiles, a.cols, sm_count, a.k_split) : TcTail{};
+        tail.first > 0) {
+        if (a.tc_end == 0) {  // the whole rounds first, then (below) the rest
+            a.tc_end = tail.first;
+            if (const cudaError_t err = VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(a, maps, n_parts, m, sm_count, stream); err != cudaSuccess) return err;
+            a.k_split = tail.k_split, a.tc_first = tail.first, a.tc_end = n_tiles;
+        }
+        n_tiles = a.tc_end - a.tc_first;
+    } else if (a.tc_end == 0) {
+        a.tc_end = n_tiles;
+    }
     const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
     for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
     a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
