@@ -354,8 +354,8 @@ def prefill_gemm(rt, torch, stream, dev, peaks: dict) -> dict:
             "TFLOPs": round(flops / ms / 1e9, 1), "frac_of_bf16_burst": round(flops / ms / 1e9 / peaks["bf16_tflops"], 4),
             "frac_of_bf16_sustained": round(flops / ms / 1e9 / peaks["bf16_tflops_sustained"], 4) if peaks.get("bf16_tflops_sustained") else None,
             "note": "fp32 activations -> fp16; pairs of blocks on tcgen05.mma.cta_group::2, each 128 weight rows x 512 activation rows with fp32 "
-                    "accumulators in tensor memory; weights: raw blocks staged in shared memory by bulk copies, per-block decoders to fp16 "
-                    "tiles; activations: TMA tile copies; "
+                    "accumulators in tensor memory; weights: raw blocks staged in shared memory by TMA tile copies, decoded to fp16 tiles; "
+                    "activations: TMA tile copies; "
                     "time includes the fp32 -> fp16 conversion of the activations"}
 
 
@@ -699,7 +699,7 @@ def run_gpu(args) -> None:
                     "tokens_per_s": m / (e2e_ms * 1e-3)},
             "gpu_launches": int(launches),
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
-                         "traffic": NCU_TRAFFIC_BYTES_PER_LAUNCH if (m == 4 and world == 1) else None, "kernel": f"qmv_kernel<Q3_K, M={m}> {d_rows}x{dom[0][3]}",
+                         "traffic": NCU_TRAFFIC_BYTES_PER_LAUNCH if (m == 4 and world == 1) else None, "kernel": f"tcmv_kernel<Q3_K, M={m}> {d_rows}x{dom[0][3]}",
                          "algorithmic_bytes_per_launch": alg_bytes, "us_per_launch": dom_ms * 1e3, "peak_source": f"of {peaks['source']}",
                          "fp32_fma_ceiling": {"weight_GBs": fma_ceiling, "frac": achieved / min(peaks["hbm_gbs"], fma_ceiling),
                                               "note": "achieved / min(HBM peak, rate at which one FMA per weight per activation row saturates the fp32 pipe)"}},
