@@ -565,9 +565,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         const uint32_t tm_mine = tmem + wg * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
         const uint32_t a_full = tc::s32(&s_afull[wg]), mma_done = tc::s32(&s_done[wg]);
         int st = 0, stage = 0, bs = 0;  // step count, stage, B stage
-        uint32_t wphase = 0, bphase = 0, dphase = 0, rphase = 0, sphase = 0;
+        uint32_t wphase = 0, bphase = 0, dphase = 1, rphase = 0, sphase = 0;  // (dphase: of the batch before the next one)
         bool announced = false;                 // the cluster's barriers are known to exist
-        bool started = false, pending = false;  // MMAs are in flight; a unit's sums have not been read yet
+        bool pending = false;    // a unit's sums have not been read yet
         TcPending<TYPE, MC> pend;
         TcAcc<MC> acc;
         acc.clear();
@@ -630,11 +630,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                 __syncwarp();
                                 if (lane == 0) tc::bar_arrive(wempty);
                             }
-                            if (started) {  // the previous batch's MMAs: A may be overwritten, sums are complete
-                                tc::bar_wait(mma_done, dphase, failed);
-                                dphase ^= 1u;
-                                tc::fence_after();
-                            }
+                            // the previous batch's MMAs: A may be overwritten, sums are complete
+                            tc::bar_wait(mma_done, dphase, failed);
+                            dphase ^= 1u;
+                            tc::fence_after();
                             tc::st32(tm_mine, r);
                             if ((first || tc_fresh_batches(TYPE)) && pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
                             if constexpr (kBC == 2) {
@@ -649,7 +648,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             tc::fence_before();
                             __syncwarp();
                             if (lane == 0) tc::bar_arrive(a_full);
-                            started = true;
                             if (last || tc_fresh_batches(TYPE)) {
                                 if constexpr (tc_mins(TYPE) > 0) {
 #pragma unroll
@@ -684,13 +682,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 if (++bs == kNB) bs = 0, bphase ^= 1u;
             }
             // ---- the tile's last sums, then the outputs ----
-            if (started) {
+            if (pending) {
                 tc::bar_wait(mma_done, dphase, failed);
-                dphase ^= 1u;
                 tc::fence_after();
                 tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
             }
-            pending = started = false;
+            pending = false;
             tc::fence_before();
             // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
             // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
