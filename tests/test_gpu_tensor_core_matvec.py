@@ -109,3 +109,20 @@ def test_sixteen_rows_at_a_time_equal_eight_bit_for_bit(rt, t, rows, cols, ntok)
     for c in range(0, ntok, 8):
         (part,) = _run(rt, ["w"], ["y"], (rows,), x[c:c + 8])
         assert np.array_equal(part.view(np.uint32), got[c:c + 8].view(np.uint32)), c
+
+
+@pytest.mark.parametrize("ntok", [1, 33, 63])
+@pytest.mark.parametrize("t,rows,cols", [(T.Q4_K, 257, 512), (T.Q6_K, 70, 2304), (T.Q8_0, 300, 1088), (T.F16, 129, 320)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_prompt_gemm_of_few_rows(rt, codebooks, t, rows, cols, ntok):
+    rng = np.random.default_rng(rows + cols + ntok)
+    raw = synthetic_blocks(t, rows, cols, rng)
+    rt.upload("w", raw, int(t), cols, rows)
+    x = synthetic_activations(ntok, cols, rng)
+    ref = O.matvec(raw, int(t), rows, cols, x, codebooks)
+    rt.set_gemm_min_rows(1)
+    try:
+        (got,) = _run(rt, ["w"], ["y"], (rows,), x)
+    finally:
+        rt.set_gemm_min_rows(0)
+    assert np.all(np.abs(got - ref) <= 3e-3 * np.abs(ref).max())  # fp16 operands

@@ -166,7 +166,7 @@ struct vqm_runtime {
     vqm::PushInfo push{};                   // regions, rank, counters
     int exchange_slots = 0;
     int gemm_min_rows = 0;
-    int gemm_tcgen05 = 1;    // prompt passes of 128+ rows run on the tcgen05 kernel (VINF_B200_GEMM=mma: warp-level MMA only)
+    int gemm_tcgen05 = 1;    // prompt passes run on the tcgen05 kernel (VINF_B200_GEMM=mma: warp-level MMA only)
     int overlap_launch = 1;  // programmatic dependent launch of consecutive matvecs (VINF_B200_NO_PDL=1 turns it off)
     bool capturing = false;
     uint64_t launches = 0, capture_launches = 0;
@@ -998,8 +998,9 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
         const uint8_t *cb = codebook_for(rt, t->type);
         if (vqm::grid_is_codebook(t->type) && cb == nullptr)
             return fail(VQM_ERR_VALUE, "the codebook for GGUF type %d has not been set (vqm_set_codebook)", t->type);
-        // tcgen05 kernel (its tile copies fill in rows beyond the last) from 64 rows on, the warp-level MMA kernel below that
-        const bool tc5 = rt->gemm_tcgen05 && ntok >= 64 && vqm::gemm_tc5_supports(t->cols);
+        // tcgen05 kernel (its tile copies fill in rows beyond the last), the warp-level MMA kernel for other column counts: 16 rows of
+        // Q4_K 5120 x 17408 take 45 us on the one and 568 on the other, Q8_0 1024 x 1024 7 and 32
+        const bool tc5 = rt->gemm_tcgen05 && vqm::gemm_tc5_supports(t->cols);
         const int tile = tc5 ? 1 : vqm::gemm_token_tile();
         const size_t need = static_cast<size_t>((ntok + tile - 1) / tile * tile) * t->cols;
         cudaError_t err = cudaSuccess;
