@@ -126,3 +126,54 @@ def test_prompt_gemm_of_few_rows(rt, codebooks, t, rows, cols, ntok):
     finally:
         rt.set_gemm_min_rows(0)
     assert np.all(np.abs(got - ref) <= 3e-3 * np.abs(ref).max())  # fp16 operands
+
+
+def _captured_kernels(rt, work) -> list[str]:
+    """Names of the kernels that `work` launches when another library (torch) captures the stream."""
+    import torch
+    from cuda.bindings import driver
+
+    def call(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result[0]
+        return result[1:] if len(result) > 2 else result[1] if len(result) == 2 else None
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    stream = torch.cuda.Stream()
+    try:
+        with torch.cuda.graph(graph, stream=stream):
+            rt.set_stream(torch.cuda.current_stream().cuda_stream)
+            work()
+    finally:
+        rt.set_stream(None)
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    names = []
+    for node in call(driver.cuGraphGetNodes(raw, call(driver.cuGraphGetNodes(raw, 0))[1]))[0]:
+        if call(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = call(driver.cuGraphKernelNodeGetParams(node))
+            name = call(driver.cuKernelGetName(params.kern)) if int(params.kern) else call(driver.cuFuncGetName(params.func))
+            names.append(name.decode())
+    return names
+
+
+@pytest.mark.parametrize("extra", [0, 4])  # floats behind 16 rows of x: with some, only the pass shows how many rows there are
+def test_the_first_pass_of_sixteen_rows_may_be_captured(codebooks, extra):
+    import torch
+    from vinf_3080ti_b200.runtime import Runtime
+
+    rng = np.random.default_rng(16)
+    shapes = [(T.Q4_K, 2305, 2304), (T.Q6_K, 1025, 17408)]  # the second one wider than the first
+    raws = [synthetic_blocks(t, rows, cols, rng) for t, rows, cols in shapes]
+    for attempt in range(2):  # (the first runtime of a process loads the kernels, which takes memory)
+        runtime = Runtime(codebooks["iq3s_grid"], codebooks)
+        try:
+            for i, (t, rows, cols) in enumerate(shapes):
+                runtime.upload(f"w{i}", raws[i], int(t), cols, rows)
+                runtime.alloc(f"x{i}", 16 * cols + extra)
+                runtime.alloc(f"y{i}", 16 * rows)
+            free = torch.cuda.mem_get_info()[0]
+            kernels = _captured_kernels(runtime, lambda: [runtime.qmv(f"w{i}", f"x{i}", f"y{i}", 16) for i in range(2)])
+            assert attempt == 0 or extra or torch.cuda.mem_get_info()[0] == free  # allocates nothing
+            assert len(kernels) == 4  # per tensor: the B operands, then all 16 rows at once
+            assert all("tc_split_kernel" in k or "Li16E" in k for k in kernels), kernels
+        finally:
+            runtime.close()

@@ -18,6 +18,7 @@
 #include <string>
 #include <thread>
 #include <unordered_map>
+#include <unordered_set>
 #include <vector>
 
 #include "../../include/vinf_b200.h"
@@ -49,7 +50,8 @@ struct Tensor {
     size_t row_bytes = 0, nbytes = 0;
     int argmax_row_base = 0;
     bool owned = true;
-    std::vector<CUtensorMap> maps;  // of the tensor-core matvec, encoded on first use
+    bool mapped = false;
+    CUtensorMap maps[8];  // of the tensor-core matvec, if `mapped`
 };
 
 struct Buffer {
@@ -154,7 +156,10 @@ struct vqm_runtime {
     size_t scratch_x_n = 0, scratch_y_n = 0;
     uint8_t *x_split = nullptr;     // ready-made B operands of 9..16 activation rows
     size_t x_split_bytes = 0;
-    std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use
+    size_t split_need = 0;                      // what the widest tensor so far needs of it
+    std::unordered_set<size_t> split_cols;      // columns of the tensors that use it
+    bool wide_seen = false;                     // a buffer holds more than 8 rows of so many columns
+    std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use (together at most twice the present one)
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
     bool counted = false;    // by the pinned pool
@@ -275,6 +280,16 @@ cudaError_t dispatch_qmv(int type, const vqm::MatvecArgs &a, int m, int sm_count
     }
 }
 
+// Into how many column ranges the tensor-core matvec would split the launch, 0 = the CUDA-core kernel is better (or the only one).
+int tc_column_split(int type, const vqm::MatvecArgs &a, int sm_count) {
+    switch (type) {
+#define VQM_CASE(id, name) case id: return vqm::split_tcmv_##name(a, sm_count);
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+        default: return 0;
+    }
+}
+
 // Whether a launch runs on the tensor-core matvec; sets a.k_split.  Launches that must not be split by columns stay on the
 // CUDA-core kernel, where an output does not depend on what else is in its launch.  codebook_small: see vqm_runtime (a codebook
 // nobody has looked at is not).
@@ -282,13 +297,7 @@ bool use_tcmv(int type, vqm::MatvecArgs &a, int sm_count, bool codebook_small) {
     if (a.push.push_slot > 0 || a.push.wait_slot > 0 || !a.allow_split) return false;
     if ((a.fuse & vqm::kFuseNorm) && a.cols > 128 * 256) return false;
     if (vqm::grid_is_codebook(type) && !codebook_small) return false;
-    int split = 0;
-    switch (type) {
-#define VQM_CASE(id, name) case id: split = vqm::split_tcmv_##name(a, sm_count); break;
-        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
-#undef VQM_CASE
-        default: break;
-    }
+    const int split = tc_column_split(type, a, sm_count);
     if (split > 0) a.k_split = split;
     return split > 0;
 }
@@ -329,6 +338,13 @@ cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cuda
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, vqm::kTcTileRows / 8, maps);
     if (err != cudaSuccess) return err;
     return dispatch_tcmv(type, a, p, 1, m, sm_count, stream);
+}
+
+cudaError_t encode_maps(Tensor &t) {
+    if (t.mapped) return cudaSuccess;
+    const cudaError_t err = vqm::tc_encode_maps(t.type, t.data, t.rows, static_cast<long long>(t.row_bytes), vqm::kTcTileRows / 8, t.maps);
+    t.mapped = err == cudaSuccess;
+    return err;
 }
 
 int check_shape(const char *name, int type, int cols, int rows, size_t *row_bytes) {
@@ -404,13 +420,8 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
     if (use_tcmv(t0.type, a, rt->sm_count, codebook_fits(rt, t0.type))) {
         const CUtensorMap *maps[vqm::kMaxParts];
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
-            if (ts[i]->maps.empty()) {
-                ts[i]->maps.resize(8);
-                err = vqm::tc_encode_maps(ts[i]->type, ts[i]->data, ts[i]->rows, static_cast<long long>(ts[i]->row_bytes), vqm::kTcTileRows / 8,
-                                          ts[i]->maps.data());
-                if (err != cudaSuccess) ts[i]->maps.clear();
-            }
-            maps[i] = ts[i]->maps.data();
+            err = encode_maps(*ts[i]);
+            maps[i] = ts[i]->maps;
         }
         if (err == cudaSuccess && m > 8) {
             a.x_split = rt->x_split;
@@ -432,25 +443,63 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
     return launch_parts(rt, 1, ts, x, ys, m, with_argmax, push);
 }
 
-// Whether the tensor takes 9..16 activation rows in one launch; makes room for their B operands.
-bool takes_sixteen(vqm_runtime *rt, const Tensor &t) {
-    const size_t need = split_bytes(t.type, t.cols);
-    if (need == 0) return false;
-    vqm::MatvecArgs a{};
-    set_single_part(a, t.data, nullptr, t.rows);
-    a.rows = t.rows, a.cols = t.cols, a.allow_split = rt->allow_split;
-    if (!use_tcmv(t.type, a, rt->sm_count, codebook_fits(rt, t.type))) return false;
-    if (need <= rt->x_split_bytes) return true;
-    if (rt->capturing) return false;
+// Room for the B operands of 9..16 activation rows of every tensor so far.  The allocator is entered in relaxed capture mode: the
+// pass that finds the room missing may be one that is being captured, by this runtime or by another library.
+bool make_split_room(vqm_runtime *rt) {
+    if (rt->split_need <= rt->x_split_bytes) return true;
+    // 28 KB per 256 columns; 2 MB hold up to 17920 columns of any type, so that a runtime allocates once
+    size_t bytes = rt->split_need < (2u << 20) ? 2u << 20 : rt->split_need;
+    if (bytes < rt->x_split_bytes + rt->x_split_bytes / 2) bytes = rt->x_split_bytes + rt->x_split_bytes / 2;
     uint8_t *p = nullptr;
-    if (cudaMalloc(&p, need) != cudaSuccess) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t err = cudaMalloc(&p, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (err != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
-    if (rt->x_split != nullptr) rt->retired.push_back(rt->x_split);  // a captured graph may hold its address
+    if (rt->x_split != nullptr) rt->retired.push_back(rt->x_split);
     rt->x_split = p;
-    rt->x_split_bytes = need;
+    rt->x_split_bytes = bytes;
     return true;
+}
+
+// Whether the tensor takes 9..16 activation rows in one launch.
+bool takes_sixteen(vqm_runtime *rt, const Tensor &t) {
+    if (split_bytes(t.type, t.cols) == 0) return false;
+    vqm::MatvecArgs a{};
+    set_single_part(a, t.data, nullptr, t.rows);
+    a.cols = t.cols, a.allow_split = rt->allow_split;
+    return use_tcmv(t.type, a, rt->sm_count, codebook_fits(rt, t.type)) && make_split_room(rt);
+}
+
+void see_buffer(vqm_runtime *rt, const Buffer &b) {
+    if (b.elem == 4)
+        for (const size_t cols : rt->split_cols) rt->wide_seen |= b.n % cols == 0 && b.n / cols > 8;
+}
+
+// What the passes of a new tensor or buffer will need is made here, so that the first of them does not pay for it: the maps of a
+// tensor of the tensor-core matvec, and, once there is a buffer that holds more than 8 rows of some such tensor's activations, the
+// room for their B operands.  (An allocation of 2 MB takes 0.4 ms, which programs without such passes need not pay.)  Where
+// something fails the launches make up for it, and passes of more than 8 rows run 8 at a time.
+// First pass of 24 rows over three tensors in a new runtime: 530 us without this, 155 with it (later ones alone: 154).
+void prepare_tensor(vqm_runtime *rt, Tensor &t) {
+    vqm::MatvecArgs a{};
+    set_single_part(a, t.data, nullptr, t.rows);
+    a.cols = t.cols;
+    if (t.cols % 32 != 0 || tc_column_split(t.type, a, rt->sm_count) == 0) return;
+    (void)encode_maps(t);
+    const size_t need = split_bytes(t.type, t.cols);
+    if (need == 0) return;
+    if (need > rt->split_need) rt->split_need = need;
+    if (rt->split_cols.insert(t.cols).second)
+        for (const auto &kv : rt->buffers) see_buffer(rt, kv.second);
+    if (rt->wide_seen) (void)make_split_room(rt);
+}
+void prepare_buffer(vqm_runtime *rt, const Buffer &b) {
+    see_buffer(rt, b);
+    if (rt->wide_seen) (void)make_split_room(rt);
 }
 
 // The tensors and output buffers of a group call, checked: same type and columns, every y large enough.
@@ -640,6 +689,7 @@ int vqm_upload(vqm_runtime *rt, const char *name, const void *data, size_t nbyte
     t.cols = cols;
     t.row_bytes = row_bytes;
     t.nbytes = want;
+    prepare_tensor(rt, t);
     rt->tensors[name] = t;
     return VQM_OK;
 }
@@ -775,6 +825,7 @@ int vqm_upload_file(vqm_runtime *rt, const char *name, const char *path, uint64_
     t.cols = cols;
     t.row_bytes = row_bytes;
     t.nbytes = want;
+    prepare_tensor(rt, t);
     rt->tensors[name] = t;
     return VQM_OK;
 }
@@ -799,6 +850,7 @@ int vqm_bind_tensor(vqm_runtime *rt, const char *name, const void *device_ptr, i
     t.cols = cols;
     t.row_bytes = row_bytes;
     t.nbytes = row_bytes * static_cast<size_t>(rows);
+    prepare_tensor(rt, t);
     rt->tensors[name] = t;
     return VQM_OK;
 }
@@ -858,6 +910,7 @@ int vqm_alloc(vqm_runtime *rt, const char *name, size_t n, int elem) {
         release(b);
         return cuda_fail("cudaMalloc buffer", err);
     }
+    prepare_buffer(rt, b);
     rt->buffers[name] = b;
     return VQM_OK;
 }
@@ -878,6 +931,7 @@ int vqm_bind(vqm_runtime *rt, const char *name, void *device_ptr, size_t n, int 
     b.n = n;
     b.elem = elem;
     b.owned = false;
+    prepare_buffer(rt, b);
     rt->buffers[name] = b;
     return VQM_OK;
 }
