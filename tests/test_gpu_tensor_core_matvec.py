@@ -177,3 +177,46 @@ def test_the_first_pass_of_sixteen_rows_may_be_captured(codebooks, extra):
             assert all("tc_split_kernel" in k or "Li16E" in k for k in kernels), kernels
         finally:
             runtime.close()
+
+
+@pytest.mark.parametrize("t", TYPES, ids=lambda t: t.name)
+def test_infinite_and_undefined_activations(rt, codebooks, t):
+    """An output is infinite or undefined exactly where weight times activation makes it so, as on the CUDA cores; the other
+    activation rows of the pass do not notice."""
+    rng = np.random.default_rng(int(t))
+    rows, cols = 2305, 2304
+    raw = synthetic_blocks(t, rows, cols, rng)
+    w = O.dequantize(raw, int(t), rows * cols, codebooks).reshape(rows, cols).astype(np.float64)
+    x = synthetic_activations(12, cols, rng)
+    x[0, 700] = np.inf
+    x[1, [3, 2303]] = np.inf, -np.inf
+    x[2, 1111] = np.nan
+    x[3, 600] = -np.inf
+    with np.errstate(invalid="ignore"):
+        want = x[:4].astype(np.float64)[:, None, :] * w[None]
+        want = want.sum(axis=2)
+    rt.upload("w", raw, int(t), cols, rows)
+    (plain,) = _run(rt, ["w"], ["y"], (rows,), np.where(np.isfinite(x), x, np.float32(0)))
+    for m in (12, 8, 4, 1):
+        (got,) = _run(rt, ["w"], ["y"], (rows,), x[:m])
+        for k in range(min(m, 4)):
+            assert np.array_equal(np.isnan(got[k]), np.isnan(want[k])) and not np.isfinite(got[k]).any(), (m, k)
+            assert np.array_equal(np.sign(got[k][~np.isnan(got[k])]), np.sign(want[k][~np.isnan(want[k])])), (m, k)
+        assert np.array_equal(got[4:].view(np.uint32), plain[4:m].view(np.uint32)), m
+    nw, x2 = rng.uniform(0.5, 1.5, cols).astype(np.float32), synthetic_activations(4, cols, rng)
+    for name, v in (("x", x[:4]), ("x2", x2), ("nw", nw)):
+        rt.alloc(name, v.size)
+        rt.write(name, np.ascontiguousarray(v))
+    rt.alloc("y", 4 * rows)
+    outs = []
+    for split in (True, False):  # the tensor cores and the CUDA cores
+        rt.set_column_split(split)
+        try:
+            for fuse in ({"silu_mul": "x2"}, {"norm": "nw"}):
+                rt.qmv_fused("w", "x", "y", 4, **fuse)
+                rt.synchronize()
+                outs.append(rt.read_array("y", 4 * rows).copy())
+        finally:
+            rt.set_column_split(True)
+    for a, b in zip(outs[:2], outs[2:]):
+        assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))

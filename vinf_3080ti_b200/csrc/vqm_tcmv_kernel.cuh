@@ -282,6 +282,31 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
     }
 }
 
+// One output weight by weight, for sums that came out as no number: an infinite or undefined activation has no exact planes, and
+// a weight in two parts, or with a minimum beside it, turns an infinity into the difference of two.  What is returned is
+// infinite or undefined where the weights and the activations themselves make it so.
+template <int TYPE>
+__device__ __noinline__ float tc_plain_sum(const MatvecArgs &a, const uint8_t *row, int t, float factor) {
+    constexpr int kChunks = chunk_block(TYPE) / 8;
+    const uint8_t *table = grid_is_codebook(TYPE) ? a.codebook : reinterpret_cast<const uint8_t *>(kIq4Levels);
+    const size_t x0 = static_cast<size_t>(t) * a.cols;
+    float sum = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < a.cols / 8; ++c) {
+        float w[8];
+        deq8<TYPE>(row + static_cast<size_t>(c / kChunks) * chunk_block_bytes(TYPE), c % kChunks, w, table);
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+            const int col = 8 * c + i;
+            float x = a.x[x0 + col];
+            if (a.fuse & kFuseSiluMul) x = x / (1.0f + expf(-x)) * a.x2[x0 + col];
+            if (a.fuse & kFuseNorm) x *= factor * a.norm_w[col];
+            sum = fmaf(w[i], x, sum);
+        }
+    }
+    return sum;
+}
+
 __device__ __forceinline__ bool tc_better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
 
 // Fused argmax: block partials, then the last block to finish reduces them (ties to the lowest row, 0x7fffffff if nothing is
@@ -760,6 +785,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                 sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + kOut * red_rows * 4));
                             }
                         if (a.fuse & kFuseNorm) sum *= factor;
+                        if (sum != sum) sum = tc_plain_sum<TYPE>(a, part.w + static_cast<size_t>(row) * a.row_bytes, t, factor);
                         if (part.y != nullptr) {
                             float *y = part.y + static_cast<size_t>(t) * part.rows + row;
                             if (a.fuse & kFuseAdd) sum += *y;
