@@ -99,6 +99,27 @@ def test_matvec_entry_on_the_reference_test_shape(rt, codebooks, t):
     assert rt.device_bytes() == 0
 
 
+def test_matvec_staging_belongs_to_its_runtime(codebooks):
+    """The pinned staging of the synchronous matvec grows with the vectors and goes with its runtime, whichever is closed first."""
+    from vinf_3080ti_b200.runtime import Runtime
+
+    rng = np.random.default_rng(7)
+    first, second = Runtime(codebooks["iq3s_grid"], codebooks), Runtime(codebooks["iq3s_grid"], codebooks)
+    try:
+        for runtimes, rows, cols in (((first, second), 40, 256), ((second, first), 16400, 64), ((second,), 600, 17408), ((second,), 40, 256)):
+            raw = synthetic_blocks(T.Q8_0, rows, cols, rng)
+            x = synthetic_activations(1, cols, rng)
+            ref = O.matvec(raw, int(T.Q8_0), rows, cols, x, codebooks)[0]
+            for runtime in runtimes:
+                runtime.upload("w", raw, int(T.Q8_0), cols, rows)
+                assert rel_l2(np.frombuffer(runtime.matvec("w", x[0]), dtype=np.float32), ref) <= REL_L2
+            if first in runtimes and rows == 16400:
+                first.close()
+    finally:
+        first.close()
+        second.close()
+
+
 @pytest.mark.parametrize("t", ALL_TYPES, ids=lambda t: t.name)
 @pytest.mark.parametrize("ntok", [1, 2, 3, 4, 5, 6, 7, 8])
 def test_qmv_every_type_and_row_count(rt, codebooks, t, ntok):

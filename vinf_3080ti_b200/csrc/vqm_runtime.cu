@@ -14,7 +14,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -68,61 +67,6 @@ struct Graph {
     bool uses_gemm_x = false;  // captured a prompt-pass GEMM, i.e. the address of the runtime's fp16 activation buffer
 };
 
-// Pinned staging that outlives a runtime: pinning a page costs more than a whole synchronous matvec.  Blocks are handed from a
-// destroyed runtime to the next one; at most kPinnedKeep bytes wait here, and none once the last runtime is gone.
-class PinnedPool {
-public:
-    void *take(size_t bytes, size_t *got) {
-        std::lock_guard<std::mutex> lock(mutex_);
-        for (size_t i = 0; i < free_.size(); ++i)
-            if (free_[i].second >= bytes) {
-                void *p = free_[i].first;
-                *got = free_[i].second;
-                kept_ -= *got;
-                free_.erase(free_.begin() + static_cast<long>(i));
-                return p;
-            }
-        size_t size = 1u << 16;
-        while (size < bytes) size *= 2;
-        void *p = nullptr;
-        if (cudaMallocHost(&p, size) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return nullptr;
-        }
-        *got = size;
-        return p;
-    }
-    void give(void *p, size_t bytes) {
-        if (p == nullptr) return;
-        std::lock_guard<std::mutex> lock(mutex_);
-        if (kept_ + bytes > kPinnedKeep) {
-            cudaFreeHost(p);
-            return;
-        }
-        free_.emplace_back(p, bytes);
-        kept_ += bytes;
-    }
-    void runtime_created() {
-        std::lock_guard<std::mutex> lock(mutex_);
-        ++runtimes_;
-    }
-    void runtime_destroyed() {
-        std::lock_guard<std::mutex> lock(mutex_);
-        if (--runtimes_ > 0) return;
-        for (auto &b : free_) cudaFreeHost(b.first);
-        free_.clear();
-        kept_ = 0;
-    }
-
-private:
-    static constexpr size_t kPinnedKeep = 8u << 20;
-    std::mutex mutex_;
-    std::vector<std::pair<void *, size_t>> free_;
-    size_t kept_ = 0;
-    int runtimes_ = 0;
-};
-PinnedPool g_pinned;
-
 const char *const kCodebookNames[5] = {"iq2xxs_grid", "iq2xs_grid", "iq2s_grid", "iq3xxs_grid", "iq3s_grid"};
 const int kCodebookTypes[5] = {vqm::kIQ2_XXS, vqm::kIQ2_XS, vqm::kIQ2_S, vqm::kIQ3_XXS, vqm::kIQ3_S};
 
@@ -162,7 +106,6 @@ struct vqm_runtime {
     std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use (together at most twice the present one)
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
-    bool counted = false;    // by the pinned pool
     void *gemm_x = nullptr;  // fp16 copy of the activations of a prompt pass
     size_t gemm_x_len = 0;   // in elements
     // exchange of row-sharded outputs between ranks
@@ -558,10 +501,17 @@ int matvec_scratch(vqm_runtime *rt, size_t cols, size_t rows) {
     if (err != cudaSuccess) return cuda_fail("scratch allocation", err);
     const size_t bytes = sizeof(float) * (kStatusWords + (rows + 3) / 4 * 4 + cols);
     if (rt->pinned_bytes < bytes) {
-        g_pinned.give(rt->pinned, rt->pinned_bytes);
+        size_t size = 1u << 16;
+        while (size < bytes) size *= 2;
+        cudaFreeHost(rt->pinned);
+        rt->pinned = nullptr;
         rt->pinned_bytes = 0;
-        rt->pinned = g_pinned.take(bytes, &rt->pinned_bytes);
-        if (rt->pinned == nullptr) return fail(VQM_ERR_MEMORY, "pinned staging of %zu bytes failed", bytes);
+        if (cudaMallocHost(&rt->pinned, size) != cudaSuccess) {
+            (void)cudaGetLastError();
+            rt->pinned = nullptr;
+            return fail(VQM_ERR_MEMORY, "pinned staging of %zu bytes failed", size);
+        }
+        rt->pinned_bytes = size;
     }
     return VQM_OK;
 }
@@ -583,8 +533,6 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
         delete rt;
         return dev_rc;
     }
-    g_pinned.runtime_created();
-    rt->counted = true;
     cudaError_t err = cudaSuccess;
     if (err == cudaSuccess) err = cudaStreamCreate(&rt->own_stream);
     rt->stream = rt->own_stream;
@@ -632,8 +580,7 @@ void vqm_runtime_destroy(vqm_runtime *rt) {
     cudaFree(rt->scratch_y);
     cudaFree(rt->x_split);
     for (uint8_t *p : rt->retired) cudaFree(p);
-    g_pinned.give(rt->pinned, rt->pinned_bytes);
-    if (rt->counted) g_pinned.runtime_destroyed();
+    cudaFreeHost(rt->pinned);
     cudaFree(rt->gemm_x);
     for (void *p : rt->exchange_opened) cudaIpcCloseMemHandle(p);
     cudaFree(rt->exchange_own);
