@@ -220,3 +220,33 @@ def test_infinite_and_undefined_activations(rt, codebooks, t):
             rt.set_column_split(True)
     for a, b in zip(outs[:2], outs[2:]):
         assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))
+
+
+@pytest.mark.parametrize("what", ["tall", "tall argmax", "24 rows", "short", "prompt"])
+def test_launch_count_is_the_number_of_kernels(rt, what):
+    import torch
+
+    t, rows, cols, m = T.Q4_K, 2305, 2304, 4
+    if "tall" in what:  # one tile more than SMs: the last one's columns are split, in a launch of its own
+        rows, cols = 256 * torch.cuda.get_device_properties(0).multi_processor_count + 256, 2560
+    elif what == "24 rows":
+        m = 24
+    elif what == "short":
+        rows = 48
+    rt.upload("w", synthetic_blocks(t, rows, cols, np.random.default_rng(3)), int(t), cols, rows)
+    rt.alloc("x", m * cols)
+    rt.alloc("y", m * rows)
+    if what == "tall argmax":
+        work = lambda: rt.qmv_argmax("w", "x", "y", m, blocking=False)  # noqa: E731
+    else:
+        work = lambda: rt.qmv("w", "x", "y", m)  # noqa: E731
+    if what == "prompt":
+        rt.set_gemm_min_rows(1)
+    try:
+        work()
+        rt.synchronize()
+        before = rt.launch_count()
+        kernels = _captured_kernels(rt, work)
+    finally:
+        rt.set_gemm_min_rows(0)
+    assert rt.launch_count() - before == len(kernels) == {"24 rows": 3, "short": 1}.get(what, 2)

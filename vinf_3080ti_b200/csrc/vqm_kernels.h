@@ -95,10 +95,11 @@ constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matve
     X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(16, IQ2_XXS) X(17, IQ2_XS) X(18, IQ3_XXS) \
     X(20, IQ4_NL) X(21, IQ3_S) X(22, IQ2_S) X(23, IQ4_XS)
 // split_tcmv_*: into how many column ranges the launch would be split (to go into a.k_split), 0 = the CUDA-core kernel is better.
+// launch_tcmv_*: n_launched (may be null) is counted up by the kernels launched, one or two.
 #define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
     int split_tcmv_##name(const MatvecArgs &a, int sm_count);                                                                    \
     cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, \
-                                   cudaStream_t stream);
+                                   cudaStream_t stream, int *n_launched);
 // split_bytes_*: size of a.x_split for a launch of 9..16 rows over a.cols columns, 0 if the type takes 8 at most;
 // launch_split_*: fills a.x_split (writable there) from a.x.
 #define VQM_DECLARE_SPLIT(id, name)                   \

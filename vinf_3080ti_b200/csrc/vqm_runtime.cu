@@ -245,10 +245,11 @@ bool use_tcmv(int type, vqm::MatvecArgs &a, int sm_count, bool codebook_small) {
     return split > 0;
 }
 
-cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, cudaStream_t stream) {
+cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, cudaStream_t stream,
+                          int *n_launched) {
     switch (type) {
 #define VQM_CASE(id, name) \
-    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, m, sm_count, stream);
+    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, m, sm_count, stream, n_launched);
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
         default: return cudaErrorInvalidValue;
@@ -280,7 +281,7 @@ cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cuda
     const CUtensorMap *p[1] = {maps};
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, vqm::kTcTileRows / 8, maps);
     if (err != cudaSuccess) return err;
-    return dispatch_tcmv(type, a, p, 1, m, sm_count, stream);
+    return dispatch_tcmv(type, a, p, 1, m, sm_count, stream, nullptr);
 }
 
 cudaError_t encode_maps(Tensor &t) {
@@ -360,6 +361,7 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         a.row_base = t0.argmax_row_base;
     }
     cudaError_t err = cudaSuccess;
+    int launched = 0;
     if (use_tcmv(t0.type, a, rt->sm_count, codebook_fits(rt, t0.type))) {
         const CUtensorMap *maps[vqm::kMaxParts];
         for (int i = 0; i < n && err == cudaSuccess; ++i) {
@@ -369,14 +371,15 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         if (err == cudaSuccess && m > 8) {
             a.x_split = rt->x_split;
             err = dispatch_split(t0.type, a, m, rt->stream);
-            count_launch(rt);
+            ++launched;
         }
-        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, m, rt->sm_count, rt->stream);
+        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, m, rt->sm_count, rt->stream, &launched);
     } else {
         err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
+        ++launched;
     }
     if (err != cudaSuccess) return cuda_fail("qmv launch", err);
-    count_launch(rt);
+    count_launch(rt, static_cast<uint64_t>(launched));
     return VQM_OK;
 }
 
@@ -1166,6 +1169,7 @@ int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t 
     got[0] = 0;
     cudaError_t err = vqm::launch_fetch(x_at, rt->scratch_x, t.cols / 4, rt->stream);
     if (err != cudaSuccess) return cuda_fail("qmatvec H2D", err);
+    count_launch(rt);
     unsigned *const shared_status = rt->status;
     rt->status = out;  // the launch's own status word sits in front of its outputs
     rc = launch_group(rt, t, rt->scratch_x, reinterpret_cast<float *>(out + kStatusWords), 1, false);

@@ -180,14 +180,14 @@ size_t VQM_CAT(split_bytes_, VQM_TYPE_NAME)(int cols) {
 cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, int m, cudaStream_t stream) { return split_sixteen<VQM_TYPE>(a, m, stream); }
 
 cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, int m, int sm_count,
-                                                 cudaStream_t stream) {
+                                                 cudaStream_t stream, int *n_launched) {
     MatvecArgs a = args;
     int n_tiles = tc_tiles(a);
     if (const TcTail tail = takes_tail(a) ? choose_tc_tail(n_tiles, a.cols, sm_count, a.k_split) : TcTail{};
         tail.first > 0) {
         if (a.tc_end == 0) {  // the whole rounds first, then (below) the rest
             a.tc_end = tail.first;
-            if (const cudaError_t err = VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(a, maps, n_parts, m, sm_count, stream); err != cudaSuccess) return err;
+            if (const cudaError_t err = VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(a, maps, n_parts, m, sm_count, stream, n_launched); err != cudaSuccess) return err;
             a.k_split = tail.k_split, a.tc_first = tail.first, a.tc_end = n_tiles;
         }
         n_tiles = a.tc_end - a.tc_first;
@@ -199,6 +199,7 @@ cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const C
     a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
     a.tc_deal_recip = 65536 / a.tc_deal + 1;
     for (int p = 0; p < n_parts; ++p) a.tc_map_shift[p] = static_cast<unsigned char>(tc_map_shift(a.part[p].rows, a.row_bytes));
+    if (n_launched != nullptr) ++*n_launched;
 #define VQM_LAUNCH(MC)                                                                                           \
     (n_parts == 1 ? TcVariant<MC, TcMaps1>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream)                \
                   : TcVariant<MC, TcMaps4>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream))
