@@ -37,7 +37,6 @@ struct MatvecPart {
 struct MatvecArgs {
     MatvecPart part[kMaxParts];
     const float *x;          // [M][cols] fp32, 16-byte aligned
-    const uint8_t *x_split;  // ready-made B operands of more than 8 activation rows (tensor-core matvec)
     const uint8_t *codebook;  // device copy of the type's GGUF codebook (IQ2/IQ3 types), else null
     unsigned *status;        // device error word (0 = fine)
     // fused argmax (all null / 0 when unused; single-tensor launches only)
@@ -63,12 +62,18 @@ struct MatvecArgs {
     const float *x2;         // [M][cols], with kFuseSiluMul
     const float *norm_w;     // [cols], with kFuseNorm
     float eps;               // rmsnorm epsilon
-    // Filled in by the launcher of the tensor-core matvec (so that no block starts with integer divisions):
+    PushInfo push;           // all zero when the tensor is not sharded
+};
+
+// What the tensor-core matvec needs beside that; filled in by its launcher, so that no block starts with integer divisions.  (Not
+// in MatvecArgs: with these 64 bytes the CUDA-core kernel's small launches take 1 to 3 % longer, 3.07 instead of 2.98 us.)
+static_assert(sizeof(MatvecArgs) <= 384, "parameters of the CUDA-core kernel");
+struct TcMatvecArgs : MatvecArgs {
+    const uint8_t *x_split;  // ready-made B operands of more than 8 activation rows
     int tc_steps[9];         // block k of a cluster takes the 256-column steps [tc_steps[k], tc_steps[k + 1])
     int tc_deal, tc_deal_recip;  // rows of a tile that each block of a cluster finishes, and 65536 / tc_deal rounded up
     int tc_first, tc_end;        // tiles of this launch (a launch may take the last round of another, see choose_tc_tail)
     unsigned char tc_map_shift[kMaxParts];  // log2 of the number of tensor maps of each tensor
-    PushInfo push;           // all zero when the tensor is not sharded
 };
 
 enum : int { kFuseAdd = 1, kFuseNorm = 2, kFuseSiluMul = 8 };  // (4 is the fused argmax, which has its own fields)
@@ -95,16 +100,17 @@ constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matve
     X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(16, IQ2_XXS) X(17, IQ2_XS) X(18, IQ3_XXS) \
     X(20, IQ4_NL) X(21, IQ3_S) X(22, IQ2_S) X(23, IQ4_XS)
 // split_tcmv_*: into how many column ranges the launch would be split (to go into a.k_split), 0 = the CUDA-core kernel is better.
-// launch_tcmv_*: n_launched (may be null) is counted up by the kernels launched, one or two.
+// launch_tcmv_*: x_split holds the B operands of more than 8 activation rows; n_launched (may be null) is counted up by the
+// kernels launched, one or two.
 #define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
     int split_tcmv_##name(const MatvecArgs &a, int sm_count);                                                                    \
-    cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, \
-                                   cudaStream_t stream, int *n_launched);
-// split_bytes_*: size of a.x_split for a launch of 9..16 rows over a.cols columns, 0 if the type takes 8 at most;
-// launch_split_*: fills a.x_split (writable there) from a.x.
+    cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m, \
+                                   int sm_count, cudaStream_t stream, int *n_launched);
+// split_bytes_*: size of x_split for a launch of 9..16 rows over so many columns, 0 if the type takes 8 at most;
+// launch_split_*: makes it from a.x.
 #define VQM_DECLARE_SPLIT(id, name)                   \
     size_t split_bytes_##name(int cols);               \
-    cudaError_t launch_split_##name(const MatvecArgs &a, int m, cudaStream_t stream);
+    cudaError_t launch_split_##name(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream);
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_SPLIT)
 #undef VQM_DECLARE_SPLIT
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_TC_LAUNCHER)

@@ -245,11 +245,11 @@ bool use_tcmv(int type, vqm::MatvecArgs &a, int sm_count, bool codebook_small) {
     return split > 0;
 }
 
-cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int m, int sm_count, cudaStream_t stream,
-                          int *n_launched) {
+cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m, int sm_count,
+                          cudaStream_t stream, int *n_launched) {
     switch (type) {
 #define VQM_CASE(id, name) \
-    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, m, sm_count, stream, n_launched);
+    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, x_split, m, sm_count, stream, n_launched);
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
         default: return cudaErrorInvalidValue;
@@ -265,9 +265,9 @@ size_t split_bytes(int type, int cols) {
         default: return 0;
     }
 }
-cudaError_t dispatch_split(int type, const vqm::MatvecArgs &a, int m, cudaStream_t stream) {
+cudaError_t dispatch_split(int type, const vqm::MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
     switch (type) {
-#define VQM_CASE(id, name) case id: return vqm::launch_split_##name(a, m, stream);
+#define VQM_CASE(id, name) case id: return vqm::launch_split_##name(a, x_split, m, stream);
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
         default: return cudaErrorInvalidValue;
@@ -281,7 +281,7 @@ cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cuda
     const CUtensorMap *p[1] = {maps};
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, vqm::kTcTileRows / 8, maps);
     if (err != cudaSuccess) return err;
-    return dispatch_tcmv(type, a, p, 1, m, sm_count, stream, nullptr);
+    return dispatch_tcmv(type, a, p, 1, nullptr, m, sm_count, stream, nullptr);
 }
 
 cudaError_t encode_maps(Tensor &t) {
@@ -369,11 +369,10 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
             maps[i] = ts[i]->maps;
         }
         if (err == cudaSuccess && m > 8) {
-            a.x_split = rt->x_split;
-            err = dispatch_split(t0.type, a, m, rt->stream);
+            err = dispatch_split(t0.type, a, rt->x_split, m, rt->stream);
             ++launched;
         }
-        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, m, rt->sm_count, rt->stream, &launched);
+        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, rt->x_split, m, rt->sm_count, rt->stream, &launched);
     } else {
         err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
         ++launched;

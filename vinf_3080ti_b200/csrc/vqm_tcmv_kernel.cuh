@@ -312,7 +312,7 @@ __device__ __forceinline__ bool tc_better(float v, int i, float bv, int bi) { re
 // Fused argmax: block partials, then the last block to finish reduces them (ties to the lowest row, 0x7fffffff if nothing is
 // above -inf).  Warp w < 16 holds the best of activation row w % MC over its lanes' outputs.
 template <int MC>
-__device__ __forceinline__ void tc_finish_argmax(const MatvecArgs &a, int m, float bv, int bi, int warp, int lane, float *s_v, int *s_i, bool *s_last) {
+__device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, float bv, int bi, int warp, int lane, float *s_v, int *s_i, bool *s_last) {
     auto warp_best = [&]() {
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant
 }
 
 template <int TYPE, int MC, typename MAPS>
-__global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_constant__ MatvecArgs a, const __grid_constant__ MAPS maps, const int m) {
+__global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_constant__ TcMatvecArgs a, const __grid_constant__ MAPS maps, const int m) {
     using Shape = TcShape<MC>;
     constexpr int kStages = tc_stages<TYPE, MC>(), kStageBytes = tc_stage_bytes<TYPE, MC>();
     constexpr int kPitch = tc_pitch(TYPE), kStepBytes = tc_step_bytes(TYPE);

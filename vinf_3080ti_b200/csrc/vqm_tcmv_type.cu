@@ -61,7 +61,7 @@ struct TcVariant {
         cfg.numAttrs = n;
     }
 
-    static cudaError_t launch(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+    static cudaError_t launch(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int n_tiles, int m, int sm_count, cudaStream_t stream) {
         const int fit = clusters(a.k_split, sm_count);
         if (fit == 0) return cudaErrorInvalidConfiguration;
         const int grid = (n_tiles < fit ? n_tiles : fit) * a.k_split;
@@ -138,7 +138,7 @@ inline int choose_tc_split(int n_tiles, int cols, int sm_count, bool single) {
 
 // More than 8 activation rows (templates, so that types without the variant do not compile it)
 template <int TYPE>
-cudaError_t launch_sixteen(const MatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+cudaError_t launch_sixteen(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
     if constexpr (tc_sixteen(TYPE)) {
         if (a.x_split == nullptr || a.fuse != 0 || a.out_idx != nullptr) return cudaErrorInvalidValue;
         return TcVariant<(TYPE >= 0 ? 16 : 0), TcMaps1>::launch(a, maps, 1, n_tiles, m, sm_count, stream);
@@ -147,7 +147,7 @@ cudaError_t launch_sixteen(const MatvecArgs &a, const CUtensorMap *const *maps, 
     }
 }
 template <int TYPE>
-cudaError_t split_sixteen(const MatvecArgs &a, int m, cudaStream_t stream) {
+cudaError_t split_sixteen(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
     if constexpr (tc_sixteen(TYPE)) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
@@ -158,10 +158,34 @@ cudaError_t split_sixteen(const MatvecArgs &a, int m, cudaStream_t stream) {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = a.overlap_launch ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, tc_split_kernel<TYPE, 16>, a, const_cast<uint8_t *>(a.x_split), m);
+        return cudaLaunchKernelEx(&cfg, tc_split_kernel<TYPE, 16>, a, x_split, m);
     } else {
         return cudaErrorInvalidValue;
     }
+}
+
+// Tiles [first, end) of a launch.
+inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int first, int end, int m,
+                                int sm_count, cudaStream_t stream, int *n_launched) {
+    TcMatvecArgs a{args};
+    a.x_split = x_split;
+    const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
+    for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
+    a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
+    a.tc_deal_recip = 65536 / a.tc_deal + 1;
+    a.tc_first = first, a.tc_end = end;
+    for (int p = 0; p < n_parts; ++p) a.tc_map_shift[p] = static_cast<unsigned char>(tc_map_shift(a.part[p].rows, a.row_bytes));
+    if (n_launched != nullptr) ++*n_launched;
+#define VQM_LAUNCH(MC)                                                                                                  \
+    (n_parts == 1 ? TcVariant<MC, TcMaps1>::launch(a, maps, n_parts, end - first, m, sm_count, stream)                \
+                  : TcVariant<MC, TcMaps4>::launch(a, maps, n_parts, end - first, m, sm_count, stream))
+    if (m == 1) return VQM_LAUNCH(1);
+    if (m == 2) return VQM_LAUNCH(2);
+    if (m <= 4) return VQM_LAUNCH(4);
+    if (m <= 8) return VQM_LAUNCH(8);
+    if (m <= 16 && n_parts == 1) return launch_sixteen<VQM_TYPE>(a, maps, end - first, m, sm_count, stream);
+    return cudaErrorInvalidValue;
+#undef VQM_LAUNCH
 }
 
 }  // namespace
@@ -177,39 +201,21 @@ size_t VQM_CAT(split_bytes_, VQM_TYPE_NAME)(int cols) {
     return tc_sixteen(VQM_TYPE) ? static_cast<size_t>((cols + kTcStepCols - 1) / kTcStepCols) * tc_split_bytes<VQM_TYPE, 16>() : 0;
 }
 
-cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, int m, cudaStream_t stream) { return split_sixteen<VQM_TYPE>(a, m, stream); }
+cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
+    return split_sixteen<VQM_TYPE>(a, x_split, m, stream);
+}
 
-cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, int m, int sm_count,
-                                                 cudaStream_t stream, int *n_launched) {
+cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m,
+                                                 int sm_count, cudaStream_t stream, int *n_launched) {
+    const int n_tiles = tc_tiles(args);
+    const TcTail tail = takes_tail(args) ? choose_tc_tail(n_tiles, args.cols, sm_count, args.k_split) : TcTail{};
+    if (tail.first == 0) return launch_tiles(args, maps, n_parts, x_split, 0, n_tiles, m, sm_count, stream, n_launched);
+    // the whole rounds, then the rest
+    const cudaError_t err = launch_tiles(args, maps, n_parts, x_split, 0, tail.first, m, sm_count, stream, n_launched);
+    if (err != cudaSuccess) return err;
     MatvecArgs a = args;
-    int n_tiles = tc_tiles(a);
-    if (const TcTail tail = takes_tail(a) ? choose_tc_tail(n_tiles, a.cols, sm_count, a.k_split) : TcTail{};
-        tail.first > 0) {
-        if (a.tc_end == 0) {  // the whole rounds first, then (below) the rest
-            a.tc_end = tail.first;
-            if (const cudaError_t err = VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(a, maps, n_parts, m, sm_count, stream, n_launched); err != cudaSuccess) return err;
-            a.k_split = tail.k_split, a.tc_first = tail.first, a.tc_end = n_tiles;
-        }
-        n_tiles = a.tc_end - a.tc_first;
-    } else if (a.tc_end == 0) {
-        a.tc_end = n_tiles;
-    }
-    const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
-    for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
-    a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
-    a.tc_deal_recip = 65536 / a.tc_deal + 1;
-    for (int p = 0; p < n_parts; ++p) a.tc_map_shift[p] = static_cast<unsigned char>(tc_map_shift(a.part[p].rows, a.row_bytes));
-    if (n_launched != nullptr) ++*n_launched;
-#define VQM_LAUNCH(MC)                                                                                           \
-    (n_parts == 1 ? TcVariant<MC, TcMaps1>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream)                \
-                  : TcVariant<MC, TcMaps4>::launch(a, maps, n_parts, n_tiles, m, sm_count, stream))
-    if (m == 1) return VQM_LAUNCH(1);
-    if (m == 2) return VQM_LAUNCH(2);
-    if (m <= 4) return VQM_LAUNCH(4);
-    if (m <= 8) return VQM_LAUNCH(8);
-    if (m <= 16 && n_parts == 1) return launch_sixteen<VQM_TYPE>(a, maps, n_tiles, m, sm_count, stream);
-    return cudaErrorInvalidValue;
-#undef VQM_LAUNCH
+    a.k_split = tail.k_split;
+    return launch_tiles(a, maps, n_parts, x_split, tail.first, n_tiles, m, sm_count, stream, n_launched);
 }
 
 }  // namespace vqm
