@@ -156,7 +156,11 @@ int vqm_mem_info(size_t *free_bytes, size_t *total_bytes);
 /* The runtime's stream (a cudaStream_t), so that a caller can record events on it or order other work. */
 void *vqm_stream(vqm_runtime *rt);
 /* Makes the runtime launch on a stream the caller owns (for instance the stream another library is
- * capturing into a graph, or one that also carries NCCL collectives); NULL restores the runtime's own. */
+ * capturing into a graph, or one that also carries NCCL collectives); NULL restores the runtime's own.  Work on the new
+ * stream is not ordered behind work on the old one, with one exception: passes of more than 8 activation rows outside of
+ * prompt mode share scratch memory of the runtime, so the first such pass on the new stream waits for the last one on the
+ * old.  (The old stream must still exist if there was one.)  Other shared scratch - the argmax results, the activations of
+ * prompt passes, what a graph uses that another library captured - is the caller's to order. */
 int vqm_set_stream(vqm_runtime *rt, void *stream);
 /* Records the launches made between begin and end into a CUDA graph instead of running them (a whole
  * decoder pass of qmv calls becomes one launch).  Blocking entry points are not allowed in between. */

@@ -250,3 +250,52 @@ def test_launch_count_is_the_number_of_kernels(rt, what):
     finally:
         rt.set_gemm_min_rows(0)
     assert rt.launch_count() - before == len(kernels) == {"24 rows": 3, "short": 1}.get(what, 2)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_wide_passes_on_two_streams_take_turns(rt, graph):
+    """The B operands of a pass of more than 8 rows lie in scratch of the runtime: on another stream the next such pass waits."""
+    import time
+
+    import torch
+
+    t, rows, cols, m = T.Q4_K, 2305, 2304, 24
+    rng = np.random.default_rng(24)
+    rt.upload("w", synthetic_blocks(t, rows, cols, rng), int(t), cols, rows)
+    xs = [synthetic_activations(m, cols, rng) for _ in range(2)]
+    for i in range(2):
+        rt.alloc(f"x{i}", m * cols)
+        rt.alloc(f"y{i}", m * rows)
+        rt.write(f"x{i}", xs[i])
+        rt.qmv("w", f"x{i}", f"y{i}", m)
+    rt.synchronize()
+    want = [rt.read_array(f"y{i}", m * rows).copy() for i in range(2)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    ids = []
+    for i in range(2):
+        rt.zero(f"y{i}")
+        rt.capture_begin()
+        rt.qmv("w", f"x{i}", f"y{i}", m)
+        ids.append(rt.capture_end())
+    rt.synchronize()
+    done = torch.cuda.Event()
+    try:
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(600_000_000)  # some 0.3 s
+        for i in range(2):
+            rt.set_stream(streams[i].cuda_stream)
+            if graph:
+                rt.graph_launch(ids[i])
+            else:
+                rt.qmv("w", f"x{i}", f"y{i}", m)
+        done.record(streams[1])
+        time.sleep(0.05)
+        waited = not done.query()
+    finally:
+        rt.set_stream(None)
+        torch.cuda.synchronize()
+        for g in ids:
+            rt.graph_destroy(g)
+    assert waited
+    for i in range(2):
+        assert np.array_equal(rt.read_array(f"y{i}", m * rows).view(np.uint32), want[i].view(np.uint32)), i

@@ -64,6 +64,7 @@ struct Buffer {
 struct Graph {
     cudaGraphExec_t exec = nullptr;
     uint64_t kernels = 0;
+    bool uses_split = false;   // captured a pass of more than 8 rows, which reads x_split
     bool uses_gemm_x = false;  // captured a prompt-pass GEMM, i.e. the address of the runtime's fp16 activation buffer
 };
 
@@ -103,6 +104,10 @@ struct vqm_runtime {
     size_t split_need = 0;                      // what the widest tensor so far needs of it
     std::unordered_set<size_t> split_cols;      // columns of the tensors that use it
     bool wide_seen = false;                     // a buffer holds more than 8 rows of so many columns
+    // x_split serves one stream at a time: split_event follows its last use on the stream before (see claim_split)
+    bool split_used = false, split_wait = false;
+    cudaStream_t split_stream = nullptr;
+    cudaEvent_t split_event = nullptr;
     std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use (together at most twice the present one)
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
@@ -118,7 +123,7 @@ struct vqm_runtime {
     int overlap_launch = 1;  // programmatic dependent launch of consecutive matvecs (VINF_B200_NO_PDL=1 turns it off)
     bool capturing = false;
     uint64_t launches = 0, capture_launches = 0;
-    bool capture_uses_gemm_x = false;
+    bool capture_uses_gemm_x = false, capture_uses_split = false;
     std::vector<Graph> graphs;
     // file loader: per reader thread two pinned staging slots, a copy stream and an event per slot (created on first use)
     std::vector<uint8_t *> load_slots;
@@ -291,6 +296,36 @@ cudaError_t encode_maps(Tensor &t) {
     return err;
 }
 
+// Before x_split is used on the present stream: what used it on another one comes first.  (A capture must not wait for what is
+// outside of it: vqm_graph_launch claims for its graphs.)
+cudaError_t claim_split(vqm_runtime *rt) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaError_t err = cudaStreamIsCapturing(rt->stream, &status);
+    if (err != cudaSuccess) return err;
+    if (status != cudaStreamCaptureStatusNone) {
+        rt->capture_uses_split = true;
+        return cudaSuccess;
+    }
+    if (rt->split_wait) err = cudaStreamWaitEvent(rt->stream, rt->split_event, 0);
+    if (err == cudaSuccess) rt->split_wait = false, rt->split_used = true;
+    return err;
+}
+// Before the present stream is replaced.
+cudaError_t leave_stream(vqm_runtime *rt, cudaStream_t next) {
+    if (next == rt->stream) return cudaSuccess;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaError_t err = rt->split_used ? cudaStreamIsCapturing(rt->stream, &status) : cudaSuccess;
+    if (err == cudaSuccess && rt->split_used && status == cudaStreamCaptureStatusNone) {
+        if (rt->split_event == nullptr) err = cudaEventCreateWithFlags(&rt->split_event, cudaEventDisableTiming);
+        if (err == cudaSuccess) err = cudaEventRecord(rt->split_event, rt->stream);
+        if (err == cudaSuccess) rt->split_stream = rt->stream;
+    }
+    if (err != cudaSuccess) return err;
+    rt->split_used = false;
+    rt->split_wait = rt->split_event != nullptr && rt->split_stream != next;
+    return cudaSuccess;
+}
+
 int check_shape(const char *name, int type, int cols, int rows, size_t *row_bytes) {
     const vqm::Traits t = vqm::traits_of(type);
     if (t.block == 0) return fail(VQM_ERR_VALUE, "unsupported GGUF tensor type id %d for CUDA matvec", type);
@@ -368,6 +403,7 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
             err = encode_maps(*ts[i]);
             maps[i] = ts[i]->maps;
         }
+        if (err == cudaSuccess && m > 8) err = claim_split(rt);
         if (err == cudaSuccess && m > 8) {
             err = dispatch_split(t0.type, a, rt->x_split, m, rt->stream);
             ++launched;
@@ -582,6 +618,7 @@ void vqm_runtime_destroy(vqm_runtime *rt) {
     cudaFree(rt->scratch_y);
     cudaFree(rt->x_split);
     for (uint8_t *p : rt->retired) cudaFree(p);
+    if (rt->split_event != nullptr) cudaEventDestroy(rt->split_event);
     cudaFreeHost(rt->pinned);
     cudaFree(rt->gemm_x);
     for (void *p : rt->exchange_opened) cudaIpcCloseMemHandle(p);
@@ -1246,7 +1283,10 @@ void *vqm_stream(vqm_runtime *rt) { return rt->stream; }
 int vqm_set_stream(vqm_runtime *rt, void *stream) {
     const int rc = no_capture(rt, "set_stream");
     if (rc != VQM_OK) return rc;
-    rt->stream = stream != nullptr ? static_cast<cudaStream_t>(stream) : rt->own_stream;
+    const cudaStream_t next = stream != nullptr ? static_cast<cudaStream_t>(stream) : rt->own_stream;
+    const cudaError_t err = leave_stream(rt, next);
+    if (err != cudaSuccess) return cuda_fail("set_stream", err);
+    rt->stream = next;
     return VQM_OK;
 }
 
@@ -1256,7 +1296,7 @@ int vqm_capture_begin(vqm_runtime *rt) {
     if (err != cudaSuccess) return cuda_fail("cudaStreamBeginCapture", err);
     rt->capturing = true;
     rt->capture_launches = 0;
-    rt->capture_uses_gemm_x = false;
+    rt->capture_uses_gemm_x = rt->capture_uses_split = false;
     return VQM_OK;
 }
 
@@ -1272,6 +1312,7 @@ int vqm_capture_end(vqm_runtime *rt, int *graph_id) {
     if (err != cudaSuccess) return cuda_fail("cudaGraphInstantiate", err);
     g.kernels = rt->capture_launches;
     g.uses_gemm_x = rt->capture_uses_gemm_x;
+    g.uses_split = rt->capture_uses_split;
     rt->graphs.push_back(g);
     *graph_id = static_cast<int>(rt->graphs.size()) - 1;
     return VQM_OK;
@@ -1280,7 +1321,8 @@ int vqm_capture_end(vqm_runtime *rt, int *graph_id) {
 int vqm_graph_launch(vqm_runtime *rt, int graph_id) {
     if (graph_id < 0 || graph_id >= static_cast<int>(rt->graphs.size()) || rt->graphs[graph_id].exec == nullptr)
         return fail(VQM_ERR_KEY, "unknown graph %d", graph_id);
-    const cudaError_t err = cudaGraphLaunch(rt->graphs[graph_id].exec, rt->stream);
+    cudaError_t err = rt->graphs[graph_id].uses_split ? claim_split(rt) : cudaSuccess;
+    if (err == cudaSuccess) err = cudaGraphLaunch(rt->graphs[graph_id].exec, rt->stream);
     if (err != cudaSuccess) return cuda_fail("cudaGraphLaunch", err);
     count_launch(rt, rt->graphs[graph_id].kernels);
     return VQM_OK;
