@@ -476,7 +476,8 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
             // serialization); this thread is the only reader of its output.
             asm volatile("griddepcontrol.wait;" ::: "memory");
             const int half = n_acc / 2;
-            for (int k = 0; k < n_k; ++k) {
+            int k = 0;
+            for (; k < n_k; ++k) {
                 const int stage = k % kXStages, use = k / kXStages;
                 if (!bar_wait(s32(&s_xempty[stage]), (use & 1) ^ 1, failed)) break;
                 const uint32_t bar = s32(&s_xfull[stage]);
@@ -488,6 +489,9 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
                                  "l"(&maps.x), "r"(run0 * kRawCols + k * kTK), "r"(tok0 + nh * n_acc + static_cast<int>(rank) * half), "r"(bar)
                                  : "memory");
             }
+            // the last tiles land before the block may leave, also when a wait gave up (bounded)
+            for (int last = k > kXStages ? k - kXStages : 0; last < k; ++last)
+                for (int i = 0; i < (1 << 16) && !bar_try(s32(&s_xfull[last % kXStages]), (last / kXStages) & 1); ++i) __nanosleep(64);
         }
         __syncwarp();
     } else if (warp == 17) {

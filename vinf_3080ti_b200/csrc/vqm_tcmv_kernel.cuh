@@ -536,11 +536,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     ++filled;
                     if (++stage == kStages) stage = 0, phase ^= 1u;
                 }
-            // after a wait gave up: the copies already requested must land before the block may leave
+            // After a wait gave up: the copies already requested must land before the block may leave.  The next fill would go to
+            // `stage` in phase `phase`; stages behind it have been filled in that phase, the others in the one before.
             if (*failed) {
 #pragma unroll 1
                 for (int s = 0; s < kStages; ++s)
-                    for (int i = 0; i < 4096 && !tc::bar_try(tc::s32(&s_wfull[s]), 0); ++i) __nanosleep(64);
+                    for (int i = 0; i < 4096 && !tc::bar_try(tc::s32(&s_wfull[s]), s < stage || filled < kStages ? phase : phase ^ 1u); ++i) __nanosleep(64);
+                if constexpr (kPresplit) {
+#pragma unroll 1
+                    for (int s = 0; s < kNB && s < filled; ++s)
+                        for (int i = 0; i < 4096 && !tc::bar_try(tc::s32(&s_bfull[s]), s < bs ? bphase : bphase ^ 1u); ++i) __nanosleep(64);
+                }
             }
         }
         __syncwarp();
