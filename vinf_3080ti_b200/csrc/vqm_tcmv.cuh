@@ -1,4 +1,4 @@
-// Quantized matvec for 1..8 activation rows on the 5th-generation tensor cores:  y[t][r] = sum_k W[r][k] x[t][k].
+// Quantized matvec for 1..16 activation rows on the 5th-generation tensor cores:  y[t][r] = sum_k W[r][k] x[t][k].
 //
 // Same contract as the CUDA-core kernel (vqm_matvec.cuh): raw GGUF blocks read once for all activation rows, inputs and
 // sums of fp32 precision.  What bounds that kernel is instruction issue - a permute, half a packed FMA and half a packed
@@ -44,6 +44,8 @@
 
 namespace vqm {
 
+// (608 threads cap every thread at 96 registers.  Q8_0 and IQ4_XS with 8 rows, IQ4_XS with 2, IQ4_NL with 2 and 8, and the
+// 16-row kernels of Q2_K, Q4_K, Q5_K, Q6_K and IQ2_XS spill 20 to 150 bytes of sums and scales in the batch loop.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcGroupB = 32 * kTcCore;           // bytes of 8 B rows over a step
