@@ -2,8 +2,8 @@
 
 Workload: one decode pass over the synthetic 27B matvec set at M activation rows (default 4, the MTP k=3 verify
 pass): 64 layers x {Q6_K q/k/v/o, Q3_K gate/up, Q4_K down} with hidden 5120 / FFN 17408, then the Q6_K LM head
-151936 x 5120 with the fused on-device argmax - 257 launches (q/k/v and gate/up of a layer go out as one launch each)
-over 12.6 GB of raw GGUF blocks, all resident in HBM.  Weights are seeded synthetic blocks (uniform-random bytes,
+151936 x 5120 with the fused on-device argmax - 257 calls (q/k/v and gate/up of a layer go out as one launch each, the LM head
+as two) over 12.6 GB of raw GGUF blocks, all resident in HBM.  Weights are seeded synthetic blocks (uniform-random bytes,
 fp16 super-scales uniform in [1e-3, 1e-2)), activations fp32 N(0,1).  The pass is 100x larger than L2, so no flush is
 needed between steps.
 
@@ -47,8 +47,8 @@ from vinf_3080ti_b200.sharding import pick_best, shard_rows  # noqa: E402
 from vinf_3080ti_b200.synth import IQ_SWEEP, LAYER_SET, LM_HEAD, N_LAYERS, synthetic_activations, synthetic_blocks, tensor_bytes  # noqa: E402
 
 METRIC = "quant-matvec weight GB/s, synthetic-27B decode pass"
-# DRAM bytes (read + write) of one launch of the dominant kernel (Q3_K 17408 x 5120, M = 4) from an ncu capture
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 38447616
+# DRAM bytes (read + write) of one launch of the dominant kernel (tcmv_kernel, Q3_K 17408 x 5120, M = 4) from an ncu capture
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 38455040
 SM_COUNT, SM_LANES, SM_MAX_HZ = 148, 128, 1.965e9
 
 
@@ -469,7 +469,7 @@ def run_gpu(args) -> None:
     ids_addr, vals_addr = rt.argmax_result()
     torch.cuda.synchronize()
 
-    # The launches of a pass.  Tensors that read the same activations and share type and columns go out as ONE launch
+    # The calls of a pass.  Tensors that read the same activations and share type and columns go out as ONE launch
     # (q/k/v, gate/up) unless --launches per-tensor asks for the reference's one kernel per tensor.
     GROUPS = {"attn_q": 0, "attn_k": 0, "attn_v": 0, "attn_o": 1, "ffn_gate": 2, "ffn_up": 2, "ffn_down": 3, "output": 4}
     launches_of_pass: list[list[tuple[str, T, int, int]]] = []
@@ -690,7 +690,7 @@ def run_gpu(args) -> None:
             "ms_per_step": ms, "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": f"synthetic-27B decode pass, M={m}: 64 x (Q6_K q/k/v/o, Q3_K gate/up, Q4_K down) + Q6_K LM head 151936x5120 "
                                    f"with fused argmax; {weight_bytes_total} weight bytes resident in HBM", "activation_rows": m,
-                       "launches_per_pass": len(launches_of_pass), "launches": args.launches, "l2": "pass is ~100x larger than L2 (no flush needed)",
+                       "launches_per_pass": launches // args.steps, "launches": args.launches, "l2": "pass is ~100x larger than L2 (no flush needed)",
                        "parallelism": "single GPU, one CUDA graph per pass" if world == 1 else (f"output rows sharded over {world} GPUs; every matvec pushes its slice into all ranks' gathered vector over NVLink from its epilogue "
                                         "and waits for the flags of the launch that produced its input (decoder dependency chain); one CUDA graph per rank, no collective" if use_push else
                                         f"output rows sharded over {world} GPUs, NCCL all-gather after every matvec, eager launches")},
