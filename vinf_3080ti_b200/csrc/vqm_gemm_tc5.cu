@@ -29,7 +29,7 @@
 // others their parts of its sums through distributed shared memory and adds what it receives in the order of the columns.
 // Every mbarrier wait is bounded: on expiry the block records a status code, everybody falls through to the end, and
 // the tensor memory is released before the block returns.
-#include <cuda.h>  // CUtensorMap and the driver entry point that encodes one (types only; nothing links against the driver)
+#include <cuda.h>  // CUtensorMap (types only; nothing links against the driver)
 #include <cuda_fp16.h>
 
 #include "vqm_formats.cuh"
@@ -69,37 +69,7 @@ __host__ __device__ constexpr int stages_for(int type, int nh) {
 // keeps the other pairs' sums of its chunks, 8 KB each, where the stages were.
 constexpr int kXChunk = 16, kXBytes = kXChunk * kTM * 4;
 
-__device__ __forceinline__ uint32_t s32(const void *p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// try_wait that acquires at cluster scope: pairs with the other block's arrive of cluster scope
-__device__ __forceinline__ bool bar_try_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
+using tc::bar_arrive, tc::bar_init, tc::bar_try, tc::bar_try_cluster, tc::in_block, tc::s32;
 // Bounded wait; also gives up as soon as another thread of the block has (`failed` is a shared flag).
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int *failed) {
 #pragma unroll 1
@@ -301,12 +271,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-// the address, in the cluster's shared window, of the same variable in block `rank`
-__device__ __forceinline__ uint32_t in_block(uint32_t local, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void bar_arrive_cluster(uint32_t cluster_addr) {
     // default semantics, as for a consumer's release of a remote slot; with .release.cluster every slot took 0.2 us longer
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -502,7 +466,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
                 // (and the activation tile that goes with it)
                 if (!warp_wait(s32(&s_xfull[q % kXStages]), (q / kXStages) & 1, failed)) break;
                 if (!warp_wait(s32(&s_full[stage]), (q / kTStages) & 1, failed)) break;
-                if (lane == 0) bar_arrive_cluster(in_block(s32(&s_full[stage]), in_cluster & ~1u));
+                if (lane == 0) bar_arrive_cluster(in_block(s32(&s_full[stage]), static_cast<int>(in_cluster & ~1u)));
             }
         } else {
             // ---- MMA issue for both blocks: accumulator nh at column nh * 256.  D fp32, A and B fp16, both K-major, M = 256
@@ -602,7 +566,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
                     read16(tm_mine + nh * 256 + c * kXChunk, v);
                     const uint32_t to = in_block(tiles + ((c / pairs) * (pairs - 1) + (pair < owner ? pair : pair - 1)) * kXBytes +
                                                      (lane_group * 32 + lane) * 16,
-                                                 static_cast<uint32_t>(owner) * 2 + rank);
+                                                 owner * 2 + static_cast<int>(rank));
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to + j * (kTM * 16)), "f"(v[4 * j]), "f"(v[4 * j + 1]),
@@ -648,21 +612,11 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     }
 }
 
-using PFN_encodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                     const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // The activations as a 2-D tensor [activation rows][cols] of fp16; a tile is 64 columns (one 128-byte swizzled row each) of
 // `box_rows` activation rows, rows beyond the last are zeros.
 cudaError_t encode_x_map(CUtensorMap *map, const __half *xh, int cols, int ntok, int box_rows) {
-    static PFN_encodeTiled encode = nullptr;
-    if (encode == nullptr) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        const cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
-        if (err != cudaSuccess) return err;
-        if (fn == nullptr || found != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
-        encode = reinterpret_cast<PFN_encodeTiled>(fn);
-    }
+    TcEncode encode = nullptr;
+    if (const cudaError_t err = tc_encoder(&encode); err != cudaSuccess) return err;
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(ntok)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
     const cuuint32_t box[2] = {kTK, static_cast<cuuint32_t>(box_rows)}, elem[2] = {1, 1};

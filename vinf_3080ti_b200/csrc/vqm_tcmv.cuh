@@ -85,6 +85,11 @@ struct TcMaps4 {
     CUtensorMap m[kMaxParts][8];
 };
 
+// cuTensorMapEncodeTiled of the driver (vqm_tcmv_maps.cu)
+using TcEncode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                              const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+cudaError_t tc_encoder(TcEncode *out);
+
 // Which part of a step a warp group takes: whole steps, every other one (wide types), or half of the columns of every step
 // where two steps of weights in use and one in flight do not fit into shared memory.
 __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 176; }

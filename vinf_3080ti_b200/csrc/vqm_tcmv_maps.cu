@@ -1,7 +1,21 @@
-// Host side of the tensor-core matvec's weight copies: the tensor maps of a weight tensor.
+// Host side of the TMA tile copies: the driver's encoder, and the tensor maps of a weight tensor.
 #include "vqm_tcmv.cuh"
 
 namespace vqm {
+
+cudaError_t tc_encoder(TcEncode *out) {
+    static TcEncode encode = nullptr;
+    if (encode == nullptr) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
+        if (err != cudaSuccess) return err;
+        if (fn == nullptr || found != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
+        encode = reinterpret_cast<TcEncode>(fn);
+    }
+    *out = encode;
+    return cudaSuccess;
+}
 
 // The rows as a three-dimensional array: bytes of a row, row / 8 (stride 8 * row_bytes), row % 8 - the row class - (stride
 // row_bytes).  A map's base and strides have to be multiples of 16 bytes, so classes share a map where the row stride allows
@@ -11,17 +25,8 @@ namespace vqm {
 // own, with its own number of rows.
 // (Eight copies per stage instead of one cost 1.2 us at a launch's start: each map is fetched on its own.)
 cudaError_t tc_encode_maps(int type, const uint8_t *w, int rows, long long row_bytes, int box_rows, CUtensorMap *out) {
-    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Encode encode = nullptr;
-    if (encode == nullptr) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        const cudaError_t err = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found);
-        if (err != cudaSuccess) return err;
-        if (fn == nullptr) return cudaErrorNotSupported;
-        encode = reinterpret_cast<Encode>(fn);
-    }
+    TcEncode encode = nullptr;
+    if (const cudaError_t err = tc_encoder(&encode); err != cudaSuccess) return err;
     const cuuint32_t elem = kTcElemBytes;
     const int n = 1 << tc_map_shift(rows, row_bytes);
     const cuuint32_t box[3] = {static_cast<cuuint32_t>(tc_pitch(type)) / elem, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(8 / n)}, step[3] = {1, 1, 1};
