@@ -31,7 +31,7 @@ CASES = [  # type, rows, cols, ntok, silu_mul, norm, add
     (T.Q4_K, 300, 2048, 1, False, True, False),   # the q/k/v and gate/up projections: rmsnorm on the way in
     (T.Q6_K, 129, 5120, 4, False, True, True),
     (T.Q4_K, 96, 1536, 3, True, False, True),     # the down projection: silu(gate) * up on the way in, residual on the way out
-    (T.Q3_K, 5000, 1024, 2, True, True, False),   # both prologues; tall enough for several rows per warp
+    (T.Q3_K, 5000, 1024, 2, True, True, False),   # both prologues; tall enough for the tensor cores
     (T.IQ4_XS, 70, 768, 8, False, False, True),   # the residual add alone
     (T.Q6_K, 9, 5120, 1, True, True, True),       # a short launch, split by columns over a cluster
     (T.Q8_0, 40, 1056, 5, True, True, True),      # columns not a multiple of 256: a ragged last segment
@@ -65,6 +65,16 @@ def test_fused_prologues_and_residual_match_the_formulas(rt, codebooks, t, rows,
     own, own_ref = (got.astype(np.float64) - res, ref - res) if add else (got, ref)
     assert rel_l2(np.asarray(own), own_ref) <= (2e-5 if add else REL_L2)  # (the fp32 add of a large residual rounds the sum)
     assert np.array_equal(rt.read_array("x").reshape(ntok, cols), x)  # the inputs are left as they were
+
+
+@pytest.mark.parametrize("t,rows,cols,ntok,silu,norm,add", CASES + [(T.Q6_K, 3000, 1280, 4, True, True, True)], ids=lambda v: getattr(v, "name", str(v)))
+def test_fused_prologues_on_the_cuda_cores(rt, codebooks, t, rows, cols, ntok, silu, norm, add):
+    """The column split off: no launch runs on the tensor cores, tall ones have several rows per warp."""
+    rt.set_column_split(False)
+    try:
+        test_fused_prologues_and_residual_match_the_formulas(rt, codebooks, t, rows, cols, ntok, silu, norm, add)
+    finally:
+        rt.set_column_split(True)
 
 
 def test_fused_flags_leave_the_plain_matvec_bit_identical(rt):

@@ -132,6 +132,30 @@ def test_qmv_every_type_and_row_count(rt, codebooks, t, ntok):
     assert rel_l2(got, ref) <= REL_L2
 
 
+@pytest.mark.parametrize("rows", [2001, 4501, 9600])  # one, two and four rows in a warp's chunk (up to 4 activation rows)
+@pytest.mark.parametrize("t", ALL_TYPES, ids=lambda t: t.name)
+def test_cuda_core_kernel_at_every_chunk_height(rt, codebooks, t, rows):
+    """With the column split off every launch runs on the CUDA-core kernel, as row-sharded launches do: every type, chunk height
+    and number of activation rows against the oracle, one of the rows one-hot and therefore exact."""
+    rng = np.random.default_rng(900 + int(t) + rows)
+    cols = 1280  # a full segment and a quarter
+    raw = synthetic_blocks(t, rows, cols, rng)
+    x = synthetic_activations(8, cols, rng)
+    x[0] = 0.0
+    x[0, (37 * int(t) + rows) % cols] = 1.0
+    ref = O.matvec(raw, int(t), rows, cols, x, codebooks)
+    rt.set_column_split(False)
+    try:
+        full = run_qmv(rt, raw, t, rows, cols, x)
+        for m in range(1, 8):
+            part = run_qmv(rt, raw, t, rows, cols, x[:m])
+            assert np.array_equal(part.view(np.uint32), full[:m].view(np.uint32)), m
+    finally:
+        rt.set_column_split(True)
+    assert max(rel_l2(full[k], ref[k]) for k in range(1, 8)) <= REL_L2
+    assert np.array_equal(full[0], ref[0].astype(np.float32))
+
+
 @pytest.mark.parametrize("t,rows,cols", [
     (T.Q8_0, 3, 32), (T.IQ4_NL, 1, 32), (T.F32, 9, 32), (T.F16, 2, 64), (T.Q4_K, 1, 256), (T.Q6_K, 7, 256),
     (T.Q3_K, 1025, 768), (T.IQ2_XXS, 33, 2304), (T.Q5_K, 300, 1024), (T.Q2_K, 5, 4352), (T.IQ4_XS, 129, 5120),
@@ -501,11 +525,9 @@ def test_group_launch_error_contract(rt):
 @pytest.mark.parametrize("rows,ntok", [(200, 130), (300, 300), (200, 700)], ids=lambda v: str(v))
 @pytest.mark.parametrize("t", ALL_TYPES, ids=lambda t: t.name)
 def test_prompt_gemm_tcgen05_matches_the_matvec_path_for_every_type(rt, codebooks, t, rows, ntok):
-    """Passes of 64+ activation rows take the tcgen05 kernel (accumulators in tensor memory), in each of its block shapes:
-    up to 256 activation rows (one accumulator per block); more than that (two accumulators: 256 weight rows per block,
-    or 512 activation rows for the types whose raw blocks for 256 rows do not fit in shared memory); several tiles of
-    activation rows.  The weight rows end inside a tile, and inside its first half.  Same tolerance as the warp-level
-    kernel."""
+    """Prompt passes take the tcgen05 kernel (accumulators in tensor memory), in each of its block shapes: up to 256 activation
+    rows (one accumulator per block), more than that (two), several tiles of activation rows.  The weight rows end inside a
+    tile, and inside its first half.  Same tolerance as the warp-level kernel."""
     rng = np.random.default_rng(5100 + int(t) + ntok)
     cols = 1024
     raw = synthetic_blocks(t, rows, cols, rng)
