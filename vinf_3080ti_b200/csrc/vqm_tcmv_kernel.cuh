@@ -284,7 +284,9 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
 
 // One output weight by weight, for sums that came out as no number: an infinite or undefined activation has no exact planes, and
 // a weight in two parts, or with a minimum beside it, turns an infinity into the difference of two.  What is returned is
-// infinite or undefined where the weights and the activations themselves make it so.
+// infinite or undefined where the weights and the activations themselves make it so.  One thread per output, uncoalesced: an LM
+// head of 151936 x 5120 whose 8 rows are all undefined takes 17 ms instead of 0.2; the check alone costs up to 0.6 % (a layer of
+// 4 rows with prologues 88.7 -> 89.2 us).
 template <int TYPE>
 __device__ __noinline__ float tc_plain_sum(const MatvecArgs &a, const uint8_t *row, int t, float factor) {
     constexpr int kChunks = chunk_block(TYPE) / 8;
