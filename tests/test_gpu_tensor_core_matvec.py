@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from oracle import dequant_np as O
-from vinf_3080ti_b200.gguf_types import GGUFTensorType as T
+from vinf_3080ti_b200.gguf_types import F16_FIELDS, TRAITS, GGUFTensorType as T
 from vinf_3080ti_b200.synth import synthetic_activations, synthetic_blocks
 
 pytestmark = pytest.mark.gpu
@@ -71,6 +71,36 @@ def test_tiles_steps_and_splits_of_every_type(rt, codebooks, t, shapes, cols):
     for m in (1, 2, 3, 5):  # each compiled row count, full and not
         for g, part in zip(got, _run(rt, names, outs, shapes, x[:m])):
             assert np.array_equal(part.view(np.uint32), g[:m].view(np.uint32)), m
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("t", [T.Q3_K, T.Q2_K], ids=lambda t: t.name)
+def test_integer_sums_at_the_ends_of_their_range(rt, codebooks, t, m):
+    """Types whose products are summed as integers: the largest and smallest weights times activations at both ends of the
+    32-bit range they are rounded to, all of one sign, and activations at both ends of fp32's range."""
+    rows, cols = 2305, 2304
+    block, size = TRAITS[t]
+    raw = np.zeros((rows, cols // block, size), dtype=np.uint8)
+    raw[1::3] = 0xFF
+    raw[2::3] = np.random.default_rng(0).integers(0, 256, raw[2::3].shape, dtype=np.uint8)
+    for off in F16_FIELDS[t]:
+        raw[:, :, off:off + 2] = np.frombuffer(np.float16(1.0).tobytes(), dtype=np.uint8)
+    raw = raw.tobytes()
+    x = np.empty((16, cols), dtype=np.float32)
+    top = np.float32(2.0) - np.float32(2.0**-23)
+    x[0], x[1] = top, -top
+    x[2] = np.where(np.arange(cols) % 2, top, -top)
+    x[3], x[4] = top * np.float32(2.0**-126), 3 * np.float32(2.0**-149)  # the least normal numbers, subnormal ones
+    x[5], x[6] = np.float32(2.0**100), np.float32(2.0**-95)
+    x[7] = np.float32(2.0**-97) * np.arange(cols)
+    x[8:] = x[:8][::-1]
+    rt.upload("w", raw, int(t), cols, rows)
+    for first in range(0, 16, m):
+        (got,) = _run(rt, ["w"], ["y"], (rows,), x[first:first + m])
+        ref = O.matvec(raw, int(t), rows, cols, x[first:first + m], codebooks)
+        for k in range(m):
+            bound = 1e-6 * np.linalg.norm(ref[k]) + 2.0**-149 * np.sqrt(rows)  # fp32 sums over 9 steps; the last place of subnormals
+            assert np.linalg.norm(got[k] - ref[k]) <= bound, (first + k, np.linalg.norm(got[k] - ref[k]) / np.linalg.norm(ref[k]))
 
 
 @pytest.mark.parametrize("t,rows,cols,ntok", [(T.Q6_K, 9473, 512, 1), (T.Q4_K, 2305, 2304, 4), (T.IQ4_XS, 2305, 2304, 8)],

@@ -11,6 +11,8 @@
 //     per 256 columns (33 bits for a 24-bit number; values far below the chunk's largest lose nothing either until they
 //     are 2^-39 of it).  The planes are separate columns of the B operand, so M rows make 3M columns.  Products are exact,
 //     the tensor core adds in fp32.
+//     Q3_K and Q2_K: quant times sub-scale fits into 8 bits, and everything is a byte and an integer: a quarter of the multiplies
+//     that scale, half the stores to tensor memory, exact sums (see TcUnit<kQ3_K>, tc_convert_bytes).
 //   * A block owns 256 rows.  Thread = weight row (lane of tensor memory): scales are decoded once per row, by the one
 //     thread that needs them, and the A operand is written from registers to tensor memory with tcgen05.st (measured: an
 //     MMA of 128 x 16 with A in tensor memory takes 9.4 cycles at N = 16 and 16.4 at N = 32; with A in shared memory 40).
@@ -48,7 +50,6 @@ namespace vqm {
 // 16-row kernels of Q2_K, Q4_K, Q5_K, Q6_K and IQ2_XS spill 20 to 150 bytes of sums and scales in the batch loop.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
-constexpr int kTcGroupB = 32 * kTcCore;           // bytes of 8 B rows over a step
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums
 constexpr int kTcMaxNormSteps = 128;
 constexpr int kTcElemBytes = 2;                   // element of the tensor maps (rows are even numbers of bytes)
@@ -68,7 +69,12 @@ __host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(
 __host__ __device__ constexpr int tc_parts(int type) { return type == kQ6_K ? 2 : 1; }
 // types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit
 __host__ __device__ constexpr bool tc_block32(int type) { return type == kQ8_0 || type == kIQ4_NL || type == kIQ4_XS; }
-__host__ __device__ constexpr int tc_mins(int type) { return type == kQ4_K || type == kQ5_K ? 4 : type == kQ2_K ? 8 : 0; }  // per half step
+__host__ __device__ constexpr int tc_groups(int type) { return type == kQ4_K || type == kQ5_K ? 8 : type == kQ2_K ? 16 : 0; }  // minimums per step
+// Types whose weights times sub-scale fit into 8 bits: the operands are bytes (kind::i8), see TcUnit<kQ3_K>.
+__host__ __device__ constexpr bool tc_bytes(int type) { return type == kQ3_K || type == kQ2_K; }
+__host__ __device__ constexpr int tc_byte_offset(int type) { return type == kQ3_K ? 127 : 0; }  // what an A byte is above the weight
+__host__ __device__ constexpr int tc_mins(int type) { return tc_bytes(type) ? tc_groups(type) : tc_groups(type) / 2; }  // per half (bytes: whole) step
+__host__ __device__ constexpr int tc_group_b(int type) { return (tc_bytes(type) ? 16 : 32) * kTcCore; }  // bytes of 8 B rows over a step
 // order of a B core row's 8 columns, made of the column words a and b (4 columns each), see tc_columns
 enum : int { kOrderNibbles = 0, kOrderBytes = 1, kOrderGrid = 2 };
 __host__ __device__ constexpr int tc_order(int type) {
@@ -94,15 +100,17 @@ cudaError_t tc_encoder(TcEncode *out);
 // where two steps of weights in use and one in flight do not fit into shared memory.
 __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 176; }
 
-// activation rows a kernel is compiled for, their B rows (3 planes) in groups of 8, and the MMA's N
-template <int MC>
+// activation rows a kernel is compiled for, their B rows (3 planes; bytes: 4 planes and a row of ones) in groups of 8, and the MMA's N
+template <int TYPE, int MC>
 struct TcShape {
-    static constexpr int kGroupsB = (3 * MC + 7) / 8;
-    static constexpr int kN = kGroupsB <= 2 ? 16 : kGroupsB <= 4 ? 32 : 48;
+    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + 1 : 3 * MC;
+    static constexpr int kGroupsB = (kRowsB + 7) / 8;
+    static constexpr int kN = (kGroupsB + 1) / 2 * 16;
 };
-// per step: the activation rows' scales, then the sums of the column groups that share a minimum
-__host__ __device__ constexpr int tc_info_scales(int mc) { return mc < 4 ? 4 : mc; }
-__host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(mc) + 2 * tc_mins(type) * mc; }
+// per step: the activation rows' scales (bytes: and two integer sums each), then the sums of the column groups that share a minimum
+__host__ __device__ constexpr int tc_info_rows(int mc) { return mc < 4 ? 4 : mc; }
+__host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_bytes(type) ? 3 : 1) * tc_info_rows(mc); }
+__host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(type, mc) + tc_groups(type) * mc; }
 // More than 8 activation rows: their B operand and infos come ready-made (tc_split_kernel), by bulk copies, because the stages
 // have no room for 16 KB of activations; the tile's sums go out 8 activation rows at a time.
 __host__ __device__ constexpr bool tc_presplit(int mc) { return mc > 8; }
@@ -112,7 +120,7 @@ __host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(T
 // Shared memory beside the weight stages, with `b` B stages (an MMA may read one group of rows further).
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_fixed_bytes(int b) {
-    return (grid_bytes(TYPE) + 127) / 128 * 128 + (b * TcShape<MC>::kGroupsB + 1) * kTcGroupB + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
+    return (grid_bytes(TYPE) + 127) / 128 * 128 + (b * TcShape<TYPE, MC>::kGroupsB + 1) * tc_group_b(TYPE) + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
            2 * 264 * tc_out_rows(MC) * 4 + (tc_presplit(MC) ? 0 : (kTcMaxNormSteps + 2) * MC * 4) + 256;
 }
 template <int TYPE, int MC>
@@ -131,7 +139,7 @@ __host__ __device__ constexpr int tc_smem_bytes() {
 
 // bytes of a step in the buffer of ready-made B operands: the operand, then the infos
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_split_bytes() { return TcShape<MC>::kGroupsB * kTcGroupB + tc_info_floats(TYPE, MC) * 4; }
+__host__ __device__ constexpr int tc_split_bytes() { return TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE) + tc_info_floats(TYPE, MC) * 4; }
 // 16 activation rows at a time: not the types with a sum per 32 columns (96 columns of sums do not fit beside A in tensor memory)
 __host__ __device__ constexpr bool tc_sixteen(int type) { return !tc_block32(type); }
 
@@ -202,19 +210,35 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// D (tensor memory) (+)= A (tensor memory, 128 x 16 fp16) * B (shared memory, N x 16 fp16, K-major core matrices)
+// D (tensor memory) (+)= A (tensor memory, 128 x 32 bytes) * B (shared memory, N x 32 bytes, K-major core matrices); 16 fp16 or
+// 32 unsigned bytes along K, sums in fp32 or 32-bit integers
+template <int TYPE>
 __device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if constexpr (tc_bytes(TYPE)) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+            ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+            : "memory");
+    }
 }
-// Shared-memory descriptor without swizzle: 8 x 16-byte core matrices, kTcCore bytes apart along K, kTcGroupB bytes along N.
+// Instruction descriptor: 128 rows, N columns; fp32 += fp16 * fp16, or s32 += u8 * u8.
+__host__ __device__ constexpr uint32_t instruction(int type, int n) {
+    return ((tc_bytes(type) ? 2u : 1u) << 4) | (static_cast<uint32_t>(n >> 3) << 17) | ((128u >> 4) << 24);
+}
+// Shared-memory descriptor without swizzle: 8 x 16-byte core matrices, kTcCore bytes apart along K, tc_group_b bytes along N.
+template <int TYPE>
 __device__ __forceinline__ uint64_t b_desc(uint32_t addr) {
     return static_cast<uint64_t>((addr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(kTcCore >> 4) << 16) |
-           (static_cast<uint64_t>(kTcGroupB >> 4) << 32) | (1ull << 46);
+           (static_cast<uint64_t>(tc_group_b(TYPE) >> 4) << 32) | (1ull << 46);
 }
 __device__ __forceinline__ void st32(uint32_t at, const uint32_t (&r)[32]) {
     asm volatile(
@@ -227,6 +251,18 @@ __device__ __forceinline__ void st32(uint32_t at, const uint32_t (&r)[32]) {
 }
 __device__ __forceinline__ void ld4(uint32_t at, float *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ld1(uint32_t at, uint32_t &v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ld4(uint32_t at, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void ld8(uint32_t at, uint32_t *v) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(at)
+                 : "memory");
 }
 __device__ __forceinline__ void ld8(uint32_t at, float *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

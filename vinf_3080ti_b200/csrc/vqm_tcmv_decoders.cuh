@@ -138,97 +138,117 @@ struct TcUnit<kQ6_K> {
     }
 };
 
-// Q3_K: high-bit mask @0, bit pairs @32, 12 bytes of 6-bit scales @96, d @108; weight = d * (sc - 32) * (q2 + 4 h - 4).
-// Chunk CH: byte columns 16 CH .. 16 CH + 15 of each of the half's four 32-column groups.  10 + 8 per 8 weights.
+// ---- bytes ---------------------------------------------------------------------------------------------------------------
+// Q3_K and Q2_K: quant times sub-scale fits into 8 bits, so an A column is a byte and ONE 32-bit multiply scales four weights: no
+// byte of the product carries into the next.  Half the registers and stores of fp16 and one integer instruction per four weights
+// less; a step is one batch.  Bound by unpacking as the others (warp instructions per 8 weights of Q3_K, 1 row: 31.5 as fp16, 21.2 so).
+// 17408 x 5120, 1 / 4 / 8 / 16 rows, fp16 and bytes, us: Q3_K 19.8 / 20.9 / 23.0 / 26.6 and 15.7 / 17.5 / 20.4 / 24.8, Q2_K 15.2 / 16.8 /
+// 20.6 / 26.6 and 12.7 / 14.8 / 18.5 / 26.0.  Error against 64 bits, Q3_K: 1.5e-7 and 7e-8; with outliers of 1000 times the rest 1e-6 and 7e-8.
+// (Q4_K's products need 10 bits, Q6_K's 14: two and three bytes a weight.)
+// Chunk CH: byte columns 16 CH .. 16 CH + 15 of each of the eight 32-column groups (half * 4 + j);
+// register (half * 4 + i) * 4 + j holds columns 128 half + 32 j + 16 CH + 4 i .. + 3.
+
+// Byte K of `w`, sign-extended.
+template <int K>
+__device__ __forceinline__ uint32_t tc_signed_byte(uint32_t w) {  // (__byte_perm has no sign replication)
+    uint32_t d;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(d) : "r"(w), "n"(0x8880 | (K * 0x1111)));
+    return d;
+}
+
+// Q3_K: high-bit mask @0, bit pairs @32, 12 bytes of 6-bit scales @96, d @108; weight = d * (sc - 32) * (q2 + 4 h - 4).  A byte is
+// (sc - 32) * (q2 + 4 h - 4) + 127, 3 .. 255.  6 integer instructions + 3 multiplies per 8 weights.
 template <>
 struct TcUnit<kQ3_K> {
     float d;
-    uint32_t sc[2];  // the half's eight 6-bit scales: byte 2 (j % 2) + CH of sc[j / 2] belongs to group j
+    uint32_t sc[4];  // scales - 32, one per byte: byte 2 (j % 2) + CH of sc[2 half + j / 2]
     template <bool O>
-    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int kh) {
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int) {
         uint32_t s[4];
         tc::words<kQ3_K, O, 96, 4>(line, sh, s);
-        d = half_bits_to_float(s[3] & 0xFFFFu) * kTc24;
-        if (kh == 0) {
-            sc[0] = (s[0] & 0x0F0F0F0Fu) | ((s[2] << 4) & 0x30303030u);
-            sc[1] = (s[1] & 0x0F0F0F0Fu) | ((s[2] << 2) & 0x30303030u);
-        } else {
-            sc[0] = ((s[0] >> 4) & 0x0F0F0F0Fu) | (s[2] & 0x30303030u);
-            sc[1] = ((s[1] >> 4) & 0x0F0F0F0Fu) | ((s[2] >> 2) & 0x30303030u);
-        }
+        d = half_bits_to_float(s[3] & 0xFFFFu) * (1.0f / kTc24);
+        sc[0] = (s[0] & 0x0F0F0F0Fu) | ((s[2] << 4) & 0x30303030u);
+        sc[1] = (s[1] & 0x0F0F0F0Fu) | ((s[2] << 2) & 0x30303030u);
+        sc[2] = ((s[0] >> 4) & 0x0F0F0F0Fu) | (s[2] & 0x30303030u);
+        sc[3] = ((s[1] >> 4) & 0x0F0F0F0Fu) | ((s[2] >> 2) & 0x30303030u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sc[i] = (sc[i] + 0x60606060u) ^ 0x80808080u;  // (no carries: at most 63 + 96)
     }
     __device__ __forceinline__ float scale(int) const { return d; }
+    // Bits 0 and 2 of every byte of `x` at bits 2 and 6 (beside them copies that the caller masks out; a byte stays below 101).
+    static __device__ __forceinline__ uint32_t spread(uint32_t x) { return x * 20u; }
     template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
-        uint32_t k[4], f[4], b[4];  // multipliers of the bit pair and of the high bit, bias
-        {
-            const uint32_t n1056 = 0xE420E420u;  // -(1024 + 32)
-            const uint32_t s0 = tc::hadd2(tc::byte_h2<CH>(sc[0], tc::kHi1024), n1056), s1 = tc::hadd2(tc::byte_h2<2 + CH>(sc[0], tc::kHi1024), n1056);
-            const uint32_t s2 = tc::hadd2(tc::byte_h2<CH>(sc[1], tc::kHi1024), n1056), s3 = tc::hadd2(tc::byte_h2<2 + CH>(sc[1], tc::kHi1024), n1056);
-            b[0] = tc::hmul2(s0, 0x80048004u), b[1] = tc::hmul2(s1, 0x80048004u);  // * -4 * 2^-24
-            b[2] = tc::hmul2(s2, 0x80048004u), b[3] = tc::hmul2(s3, 0x80048004u);
-            f[0] = tc::hmul2(s0, 0x44004400u), f[1] = tc::hmul2(s1, 0x40004000u), f[2] = s2, f[3] = tc::hmul2(s3, 0x38003800u);  // 4 / 2^j
-            k[0] = s0, k[1] = tc::hmul2(s1, 0x34003400u), k[2] = tc::hmul2(s2, 0x2C002C00u), k[3] = tc::hmul2(s3, 0x24002400u);  // 1 / 4^j
-        }
-        uint32_t h[4], q[4];
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int, uint32_t (&a)[32]) const {
+        uint32_t h[4];
         tc::words<kQ3_K, O, 16 * CH, 4>(line, sh, h);
-        tc::words<kQ3_K, O, 32 + 16 * CH, 4>(line + 32 * kh, sh, q);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t w = q[i], v = w >> 8, m = h[i] >> (4 * kh), n = h[i] >> (4 * kh + 8);
-            uint32_t *r = a + 8 * i;
-            r[0] = tc::hfma2(w & 0x00030003u, k[0], tc::hfma2(m & 0x00010001u, f[0], b[0]));
-            r[1] = tc::hfma2(w & 0x000C000Cu, k[1], tc::hfma2(m & 0x00020002u, f[1], b[1]));
-            r[2] = tc::hfma2(v & 0x00030003u, k[0], tc::hfma2(n & 0x00010001u, f[0], b[0]));
-            r[3] = tc::hfma2(v & 0x000C000Cu, k[1], tc::hfma2(n & 0x00020002u, f[1], b[1]));
-            r[4] = tc::hfma2(w & 0x00300030u, k[2], tc::hfma2(m & 0x00040004u, f[2], b[2]));
-            r[5] = tc::hfma2(w & 0x00C000C0u, k[3], tc::hfma2(m & 0x00080008u, f[3], b[3]));
-            r[6] = tc::hfma2(v & 0x00300030u, k[2], tc::hfma2(n & 0x00040004u, f[2], b[2]));
-            r[7] = tc::hfma2(v & 0x00C000C0u, k[3], tc::hfma2(n & 0x00080008u, f[3], b[3]));
+        for (int half = 0; half < 2; ++half) {
+            uint32_t k[4], b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t w = sc[2 * half + (j >> 1)];
+                k[j] = (j & 1) ? tc_signed_byte<2 + CH>(w) : tc_signed_byte<CH>(w);
+                b[j] = 0x7F7F7F7Fu - 0x04040404u * k[j];
+            }
+            uint32_t q[4];
+            if (half == 0) tc::words<kQ3_K, O, 32 + 16 * CH, 4>(line, sh, q);
+            else tc::words<kQ3_K, O, 64 + 16 * CH, 4>(line, sh, q);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t m = half == 0 ? h[i] : h[i] >> 4;
+                // three-bit quants, one per nibble: groups 0 and 2, groups 1 and 3
+                const uint32_t he = spread(m & 0x05050505u), ho = (m & 0x0A0A0A0Au) * 10u;
+                const uint32_t e = (q[i] & 0x33333333u) | (he & 0xCCCCCCCCu), o = ((q[i] >> 2) & 0x33333333u) | (ho & 0xCCCCCCCCu);
+                uint32_t *r = a + (half * 4 + i) * 4;
+                r[0] = (e & 0x07070707u) * k[0] + b[0];
+                r[1] = (o & 0x07070707u) * k[1] + b[1];
+                r[2] = ((e >> 4) & 0x07070707u) * k[2] + b[2];
+                r[3] = ((o >> 4) & 0x07070707u) * k[3] + b[3];
+            }
         }
     }
 };
 
-// Q2_K: 16 bytes of 4-bit scales and minimums @0, bit pairs @16, d @80, dmin @82.  5 + 4 per 8 weights.
+// Q2_K: 16 bytes of 4-bit scales and minimums @0, bit pairs @16, d @80, dmin @82.  A byte is 4 * scale * quant, at most 180: the
+// upper of two neighbouring bit pairs already has the factor 4.  2.5 integer instructions + 2 multiplies per 8 weights.
 template <>
 struct TcUnit<kQ2_K> {
     float d, dm;
-    uint32_t sc[2], mn[2];  // the half's eight scales and minimums, one per byte: 2 j + half of the 32-column group j
+    uint32_t sc[4], mn[4];  // scales (of even groups times 4) and minimums, one per byte: byte 2 (j % 2) + CH of word 2 half + j / 2
     template <bool O>
-    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int kh) {
-        uint32_t s[2], w[1];
-        tc::words<kQ2_K, O, 0, 2>(line + 8 * kh, sh, s);
+    __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int) {
+        uint32_t s[4], w[1];
+        tc::words<kQ2_K, O, 0, 4>(line, sh, s);
         tc::words<kQ2_K, O, 80, 1>(line, sh, w);
-        sc[0] = s[0] & 0x0F0F0F0Fu, sc[1] = s[1] & 0x0F0F0F0Fu;
-        mn[0] = (s[0] >> 4) & 0x0F0F0F0Fu, mn[1] = (s[1] >> 4) & 0x0F0F0F0Fu;
-        d = half_bits_to_float(w[0] & 0xFFFFu) * kTc24;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            sc[i] = (s[i] & 0x0F0F0000u) | ((s[i] << 2) & 0x00003C3Cu);
+            mn[i] = (s[i] >> 4) & 0x0F0F0F0Fu;
+        }
+        d = half_bits_to_float(w[0] & 0xFFFFu) * (0.25f / kTc24);
         dm = half_bits_to_float(w[0] >> 16);
     }
     __device__ __forceinline__ float scale(int) const { return d; }
     template <int G>
     __device__ __forceinline__ float minimum() const { return dm * byte_to_float<G & 3>(mn[G >> 2]); }
     template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) const {
-        const uint32_t n1024 = 0xE400E400u;
-        uint32_t k[4];
-        k[0] = tc::hadd2(tc::byte_h2<CH>(sc[0], tc::kHi1024), n1024);
-        k[1] = tc::hmul2(tc::hadd2(tc::byte_h2<2 + CH>(sc[0], tc::kHi1024), n1024), 0x34003400u);
-        k[2] = tc::hadd2(tc::byte_h2<CH>(sc[1], tc::kHi64), 0xD400D400u);
-        k[3] = tc::hmul2(tc::hadd2(tc::byte_h2<2 + CH>(sc[1], tc::kHi64), 0xD400D400u), 0x34003400u);
-        uint32_t q[4];
-        tc::words<kQ2_K, O, 16 + 16 * CH, 4>(line + 32 * kh, sh, q);
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int, uint32_t (&a)[32]) const {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t w = q[i], v = w >> 8;
-            uint32_t *r = a + 8 * i;
-            r[0] = tc::hmul2(w & 0x00030003u, k[0]);
-            r[1] = tc::hmul2(w & 0x000C000Cu, k[1]);
-            r[2] = tc::hmul2(v & 0x00030003u, k[0]);
-            r[3] = tc::hmul2(v & 0x000C000Cu, k[1]);
-            r[4] = tc::hmul2(w & 0x00300030u, k[2]);
-            r[5] = tc::hmul2(w & 0x00C000C0u, k[3]);
-            r[6] = tc::hmul2(v & 0x00300030u, k[2]);
-            r[7] = tc::hmul2(v & 0x00C000C0u, k[3]);
+        for (int half = 0; half < 2; ++half) {
+            uint32_t q[4];
+            if (half == 0) tc::words<kQ2_K, O, 16 + 16 * CH, 4>(line, sh, q);
+            else tc::words<kQ2_K, O, 48 + 16 * CH, 4>(line, sh, q);
+            const uint32_t k0 = __byte_perm(sc[2 * half], 0u, 0x4440 | CH), k1 = __byte_perm(sc[2 * half], 0u, 0x4442 | CH);
+            const uint32_t k2 = __byte_perm(sc[2 * half + 1], 0u, 0x4440 | CH), k3 = __byte_perm(sc[2 * half + 1], 0u, 0x4442 | CH);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t w = q[i], v = w >> 4;
+                uint32_t *r = a + (half * 4 + i) * 4;
+                r[0] = (w & 0x03030303u) * k0;
+                r[1] = (w & 0x0C0C0C0Cu) * k1;
+                r[2] = (v & 0x03030303u) * k2;
+                r[3] = (v & 0x0C0C0C0Cu) * k3;
+            }
         }
     }
 };

@@ -17,12 +17,97 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
         a = 64 * (l >> 3) + 4 * (l & 7), b = a + 32;
     } else if constexpr (TYPE == kQ6_K) {            // half, word, pair of quarters
         a = 128 * (l >> 4) + 32 * (l & 1) + 4 * ((l >> 1) & 7), b = a + 64;
-    } else if constexpr (TYPE == kQ3_K || TYPE == kQ2_K) {
-        a = 128 * (l >> 4) + 64 * (l & 1) + 4 * ((l >> 1) & 7), b = a + 32;
+    } else if constexpr (tc_bytes(TYPE)) {           // (half a row of 16 columns) chunk, half, word, pair of 32-column groups
+        a = 128 * ((l >> 3) & 1) + 16 * (l >> 4) + 4 * ((l >> 1) & 3) + 64 * (l & 1), b = a + 32;
     } else if constexpr (TYPE == kIQ4_NL || TYPE == kIQ4_XS) {
         a = 32 * (l >> 2) + 4 * (l & 3), b = a + 16;
     } else {
         a = 8 * l, b = a + 4;
+    }
+}
+
+// The B operand of bytes.  x = X * 2^-k exactly rounded to 32-bit integers, k from the chunk's largest magnitude (biased exponent
+// `big`): what is lost is below 2^-32 of it, 2^-28.8 of the chunk's 2-norm at most, where fp32 sums lose 2^-24.  The planes are the
+// four bytes of X + 2^31, most significant first; one row of ones behind them gives the sums of A that the 2^31 (and A's own offset)
+// are taken out with.  Sums of products are integers and exact.
+//   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(24 - k), then the integers -offset * sum of X's
+//   upper 16 bits (signed), and of its lower ones.
+template <int TYPE, int MC, bool ONES>
+__device__ __forceinline__ void tc_convert_bytes(const float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
+    const uint32_t e = big > 7u ? big : 7u;  // (2^-151 is the unit of X then: below every fp32 number's)
+    // X = v * 2^(157 - e), in two factors where the power is beyond fp32
+    const float up = __uint_as_float((e < 30u ? 254u : 284u - e) << 23), up2 = __uint_as_float((e < 30u ? 157u - e : 127u) << 23);
+    uint32_t x[8];
+    int hi = 0, lo = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int n = __float2int_rn(v[i] * up * up2);
+        hi += n >> 16, lo += n & 0xFFFF;
+        x[i] = static_cast<uint32_t>(n) ^ 0x80000000u;
+    }
+    constexpr int kOffset = tc_byte_offset(TYPE);
+    if constexpr (kOffset != 0) hi = __reduce_add_sync(0xFFFFFFFFu, hi), lo = __reduce_add_sync(0xFFFFFFFFu, lo);
+    if (lane == 0) {
+        // 2^(e - 133); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
+        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 6u) << 23);
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (tc_info_rows(MC) + t) * 4), "r"(-kOffset * hi) : "memory");
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (2 * tc_info_rows(MC) + t) * 4), "r"(-kOffset * lo) : "memory");
+    }
+    uint32_t plane[4][2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const uint32_t *c = x + 4 * w;
+        const uint32_t l01 = __byte_perm(c[0], c[1], 0x5140), l23 = __byte_perm(c[2], c[3], 0x5140);
+        const uint32_t h01 = __byte_perm(c[0], c[1], 0x7362), h23 = __byte_perm(c[2], c[3], 0x7362);
+        plane[0][w] = __byte_perm(h01, h23, 0x7632), plane[1][w] = __byte_perm(h01, h23, 0x5410);
+        plane[2][w] = __byte_perm(l01, l23, 0x7632), plane[3][w] = __byte_perm(l01, l23, 0x5410);
+    }
+    const uint32_t at = b_stage + (lane >> 1) * kTcCore + (lane & 1) * 8;
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        const int n = p * MC + t;
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(plane[p][0]), "r"(plane[p][1]) : "memory");
+    }
+    if (ONES && t == 0) {
+        constexpr int n = 4 * MC;
+        asm volatile("st.shared.v2.u32 [%0], {%1, %1};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(0x01010101u) : "memory");
+    }
+}
+
+// The B operand of fp16: three planes, x = s * (h0 + 2^-11 h1 + 2^-22 h2), s a power of two that brings the largest magnitude below 2^10
+// (`big`: its biased exponent).
+//   v: the lane's 2 x 4 columns, a core row; info: [rows] factors
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_convert_halves(const float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
+    const uint32_t want = 263u - big, e = want < 253u ? want : 253u;
+    const float up = __uint_as_float(e << 23);
+    if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(__uint_as_float((254u - e) << 23)) : "memory");
+    constexpr int kOrder = tc_order(TYPE);
+    constexpr int order[3][8] = {{0, 2, 4, 6, 1, 3, 5, 7}, {0, 1, 4, 5, 2, 3, 6, 7}, {0, 2, 1, 3, 4, 6, 5, 7}};
+    uint32_t h[3][4];
+    const f32x2 up2 = pack2(up, up), k2048 = pack2(2048.0f, 2048.0f), neg = pack2(-2048.0f, -2048.0f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f32x2 r = mul2(pack2(v[order[kOrder][2 * i]], v[order[kOrder][2 * i + 1]]), up2);
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            float lo, hi;
+            unpack2(r, lo, hi);
+            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h[p][i]) : "f"(hi), "f"(lo));
+            if (p < 2) {  // 2048 * (r - plane), exactly
+                const float flo = half_bits_to_float(h[p][i] & 0xFFFFu), fhi = half_bits_to_float(h[p][i] >> 16);
+                r = fma2(pack2(flo, fhi), neg, mul2(r, k2048));
+            }
+        }
+    }
+    const uint32_t at = b_stage + lane * kTcCore;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const int n = p * MC + t;
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(h[p][0]), "r"(h[p][1]),
+                     "r"(h[p][2]), "r"(h[p][3])
+                     : "memory");
     }
 }
 
@@ -84,15 +169,14 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, 
             sa += __shfl_xor_sync(0xFFFFFFFFu, sa, off);
             sb += __shfl_xor_sync(0xFFFFFFFFu, sb, off);
         }
-        // group of a: sub-block 2 c (Q4_K, Q5_K), or 8 n + 2 j + half with j = 2 * core (Q2_K); b: the one after / two after
+        // group of a: sub-block 2 c (Q4_K, Q5_K), or 8 half + 2 j + chunk with j = 2 * (lane & 1) (Q2_K); b: the one after / two after
         const bool writer = k32 ? (lane & 7) == 0 : (lane & 6) == 0;
-        const int ga = k32 ? 2 * (lane >> 3) : 8 * (lane >> 4) + 4 * (lane & 1) + ((lane >> 3) & 1), gb = ga + (k32 ? 1 : 2);
+        const int ga = k32 ? 2 * (lane >> 3) : 8 * ((lane >> 3) & 1) + 4 * (lane & 1) + (lane >> 4), gb = ga + (k32 ? 1 : 2);
         if (writer) {
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(MC) + ga * MC + t) * 4), "f"(sa) : "memory");
-            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(MC) + gb * MC + t) * 4), "f"(sb) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(TYPE, MC) + ga * MC + t) * 4), "f"(sa) : "memory");
+            asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(TYPE, MC) + gb * MC + t) * 4), "f"(sb) : "memory");
         }
     }
-    // power of two that brings the largest magnitude below 2^10, and its inverse
     uint32_t big = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -100,43 +184,17 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, 
         big = big > m ? big : m;
     }
     big = __reduce_max_sync(0xFFFFFFFFu, big);
-    const uint32_t want = 263u - (big >> 23), e = want < 253u ? want : 253u;
-    const float up = __uint_as_float(e << 23);
-    if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(__uint_as_float((254u - e) << 23)) : "memory");
-    constexpr int kOrder = tc_order(TYPE);
-    constexpr int order[3][8] = {{0, 2, 4, 6, 1, 3, 5, 7}, {0, 1, 4, 5, 2, 3, 6, 7}, {0, 2, 1, 3, 4, 6, 5, 7}};
-    uint32_t h[3][4];
-    const f32x2 up2 = pack2(up, up), k2048 = pack2(2048.0f, 2048.0f), neg = pack2(-2048.0f, -2048.0f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f32x2 r = mul2(pack2(v[order[kOrder][2 * i]], v[order[kOrder][2 * i + 1]]), up2);
-#pragma unroll
-        for (int p = 0; p < 3; ++p) {
-            float lo, hi;
-            unpack2(r, lo, hi);
-            asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h[p][i]) : "f"(hi), "f"(lo));
-            if (p < 2) {  // 2048 * (r - plane), exactly
-                const float flo = half_bits_to_float(h[p][i] & 0xFFFFu), fhi = half_bits_to_float(h[p][i] >> 16);
-                r = fma2(pack2(flo, fhi), neg, mul2(r, k2048));
-            }
-        }
-    }
-    const uint32_t at = b_stage + lane * kTcCore;
-#pragma unroll
-    for (int p = 0; p < 3; ++p) {
-        const int n = p * MC + t;
-        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + (n >> 3) * kTcGroupB + (n & 7) * 16), "r"(h[p][0]), "r"(h[p][1]),
-                     "r"(h[p][2]), "r"(h[p][3])
-                     : "memory");
-    }
+    if constexpr (tc_bytes(TYPE)) tc_convert_bytes<TYPE, MC, !STAGED>(v, big >> 23, t, b_stage, info, lane);
+    else tc_convert_halves<TYPE, MC>(v, big >> 23, t, b_stage, info, lane);
 }
 
 // A unit is what a group of warps takes of a step: one or two halves of 128 columns.  Its chunks go to the tensor cores in
 // batches; tensor memory holds one batch of a group (64 columns) and 64 columns of sums.  Types with a scale per 32 columns
 // have a sum per 32 columns: with N = 32 only one chunk's fit.
-__host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) ? 2 : 1; }
+// Bytes: a unit is a whole step, of two chunks.
+__host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) && !tc_bytes(type) ? 2 : 1; }
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_batch_chunks() { return tc_block32(TYPE) && MC > 4 ? 1 : 2; }
+__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_bytes(TYPE) && MC > 8) ? 1 : 2; }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_half_batches() { return 2 * tc_parts(TYPE) / tc_batch_chunks<TYPE, MC>(); }
 // sums per row that a batch leaves
@@ -173,9 +231,101 @@ struct TcAcc {
     }
 };
 
+// The sums of bytes: with D_p the sums over plane p and S the sum of A,
+//   sum of weight * X = 2^16 (2^8 D_0 + D_1 - 2^15 S - offset * upper halves of X) + (2^8 D_2 + D_3 - offset * lower halves of X),
+// both brackets exact in 32 bits (modulo 2^32 on the way): |weight| <= 128 or 0 <= weight <= 180 over 256 columns.
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_accumulate_bytes(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
+    static_assert(tc_sums<TYPE, MC>() == 1, "one sum per unit");
+    constexpr int kStep = MC > 8 ? 8 : MC, kMins = tc_mins(TYPE);  // activation rows at a time, for the registers' sake
+    uint32_t ones;
+    tc::ld1(d_at + 4 * MC, ones);
+#pragma unroll
+    for (int t0 = 0; t0 < MC; t0 += kStep) {
+        uint32_t v[4][kStep < 4 ? 4 : kStep];
+        if constexpr (MC == 1) {
+            uint32_t w[4];
+            tc::ld4(d_at, w);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i][0] = w[i];
+        } else if constexpr (MC == 2) {
+            uint32_t w[8];
+            tc::ld8(d_at, w);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i >> 1][i & 1] = w[i];
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if constexpr (MC == 4) tc::ld4(d_at + i * MC, v[i]);
+                else tc::ld8(d_at + i * MC + t0, v[i]);
+            }
+        }
+        uint32_t c[3][kStep < 4 ? 4 : kStep];  // factors, sums of the upper and of the lower halves
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            if (i > 0 && tc_byte_offset(TYPE) == 0) {
+#pragma unroll
+                for (int t = 0; t < kStep; ++t) c[i][t] = 0u;
+            } else if constexpr (MC == 1) {
+                c[i][0] = lds32(p.info + i * tc_info_rows(MC) * 4);
+            } else if constexpr (MC == 2) {
+                const unsigned long long w = lds64(p.info + i * tc_info_rows(MC) * 4);
+                c[i][0] = static_cast<uint32_t>(w), c[i][1] = static_cast<uint32_t>(w >> 32);
+            } else {
+#pragma unroll
+                for (int t = 0; t < kStep; t += 4) {
+                    const uint4 w = lds128u(p.info + (i * tc_info_rows(MC) + t0 + t) * 4);
+                    c[i][t] = w.x, c[i][t + 1] = w.y, c[i][t + 2] = w.z, c[i][t + 3] = w.w;
+                }
+            }
+        }
+        tc::wait_ld();
+        auto value = [&](int t) {
+            const uint32_t hi = v[0][t] * 256u + v[1][t] + (c[1][t] - 32768u * ones), lo = v[2][t] * 256u + v[3][t] + c[2][t];
+            // (with an offset the lower sums are signed)
+            return fmaf(static_cast<float>(static_cast<int>(hi)), 65536.0f, tc_byte_offset(TYPE) != 0 ? static_cast<float>(static_cast<int>(lo)) : static_cast<float>(lo));
+        };
+        if constexpr (MC == 1) {
+            float a, b;
+            unpack2(acc.v[0], a, b);
+            acc.v[0] = pack2(fmaf(value(0) * p.s[0], __uint_as_float(c[0][0]), a), b);
+        } else {
+            const f32x2 s2 = pack2(p.s[0], p.s[0]);
+#pragma unroll
+            for (int t = 0; t < kStep; t += 2)
+                acc.v[(t0 + t) / 2] = fma2(mul2(pack2(value(t), value(t + 1)), s2), pack2(__uint_as_float(c[0][t]), __uint_as_float(c[0][t + 1])), acc.v[(t0 + t) / 2]);
+        }
+    }
+    if constexpr (kMins > 0) {
+        auto one = [&](auto tag) {
+            constexpr int G = decltype(tag)::value;
+            if constexpr (G < kMins) {
+                const float m = -p.unit[0].template minimum<G>();
+                const uint32_t at = p.info + (tc_info_scales(TYPE, MC) + G * MC) * 4;
+                if constexpr (MC == 1) {
+                    float a, b;
+                    unpack2(acc.v[0], a, b);
+                    acc.v[0] = pack2(fmaf(m, __uint_as_float(lds32(at)), a), b);
+                } else if constexpr (MC == 2) {
+                    acc.v[0] = fma2(pack2(m, m), lds64(at), acc.v[0]);
+                } else {
+#pragma unroll
+                    for (int t = 0; t < MC; t += 4) {
+                        const ulonglong2 w = lds128(at + t * 4);
+                        acc.v[t / 2] = fma2(pack2(m, m), w.x, acc.v[t / 2]);
+                        acc.v[t / 2 + 1] = fma2(pack2(m, m), w.y, acc.v[t / 2 + 1]);
+                    }
+                }
+            }
+        };
+        one(TcInt<0>{}), one(TcInt<1>{}), one(TcInt<2>{}), one(TcInt<3>{}), one(TcInt<4>{}), one(TcInt<5>{}), one(TcInt<6>{}), one(TcInt<7>{});
+        one(TcInt<8>{}), one(TcInt<9>{}), one(TcInt<10>{}), one(TcInt<11>{}), one(TcInt<12>{}), one(TcInt<13>{}), one(TcInt<14>{}), one(TcInt<15>{});
+    }
+}
+
 // acc[t] += scale * (h0 + 2^-11 h1 + 2^-22 h2 sums) * activation scale  -  minimums * group sums
 template <int TYPE, int MC>
-__device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
+__device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
     constexpr int kSums = tc_sums<TYPE, MC>(), kMins = tc_mins(TYPE);
     if constexpr (MC > 8) {  // eight activation rows at a time, for the registers' sake
         static_assert(kSums == 1, "one sum per unit");
@@ -203,7 +353,7 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
                     constexpr int G = decltype(tag)::value;
                     if constexpr (G < kMins) {
                         const float m = -p.unit[h].template minimum<G>();
-                        const uint32_t at = p.info + (tc_info_scales(MC) + ((tc_wide(TYPE) ? h : p.kh) * kMins + G) * MC) * 4;
+                        const uint32_t at = p.info + (tc_info_scales(TYPE, MC) + ((tc_wide(TYPE) ? h : p.kh) * kMins + G) * MC) * 4;
 #pragma unroll
                         for (int t = 0; t < MC; t += 4) {
                             const ulonglong2 w = lds128(at + t * 4);
@@ -220,7 +370,7 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
     }
     float v[kSums][3 * MC + 1];
 #pragma unroll
-    for (int g = 0; g < kSums; ++g) tc::ld_sums<MC>(d_at + g * TcShape<MC>::kN, v[g]);
+    for (int g = 0; g < kSums; ++g) tc::ld_sums<MC>(d_at + g * TcShape<TYPE, MC>::kN, v[g]);
     f32x2 inv[(MC + 1) / 2];
     if constexpr (MC == 1) {
         inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
@@ -259,7 +409,7 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
             float sums[kMins * MC];
 #pragma unroll
             for (int i = 0; i < kMins * MC; i += 4) {
-                const uint4 w = lds128u(p.info + (tc_info_scales(MC) + (tc_wide(TYPE) ? h : p.kh) * kMins * MC + i) * 4);
+                const uint4 w = lds128u(p.info + (tc_info_scales(TYPE, MC) + (tc_wide(TYPE) ? h : p.kh) * kMins * MC + i) * 4);
                 sums[i] = __uint_as_float(w.x), sums[i + 1] = __uint_as_float(w.y), sums[i + 2] = __uint_as_float(w.z), sums[i + 3] = __uint_as_float(w.w);
             }
             auto one = [&](auto tag) {
@@ -280,6 +430,12 @@ __device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint
             one(TcInt<4>{}), one(TcInt<5>{}), one(TcInt<6>{}), one(TcInt<7>{});
         }
     }
+}
+
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
+    if constexpr (tc_bytes(TYPE)) tc_accumulate_bytes<TYPE, MC>(p, d_at, acc);
+    else tc_accumulate_halves<TYPE, MC>(p, d_at, acc);
 }
 
 // One output weight by weight, for sums that came out as no number: an infinite or undefined activation has no exact planes, and
@@ -366,7 +522,7 @@ __device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, f
 // B operands and infos of up to MC activation rows, one block per step: what every block of the matvec would work out for itself.
 template <int TYPE, int MC>
 __global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant__ MatvecArgs a, uint8_t *out, const int m) {
-    constexpr int kOperand = TcShape<MC>::kGroupsB * kTcGroupB, kBytes = tc_split_bytes<TYPE, MC>();
+    constexpr int kOperand = TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE), kBytes = tc_split_bytes<TYPE, MC>();
     __shared__ __align__(16) uint8_t image[kBytes];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -380,14 +536,15 @@ __global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant
 
 template <int TYPE, int MC, typename MAPS>
 __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_constant__ TcMatvecArgs a, const __grid_constant__ MAPS maps, const int m) {
-    using Shape = TcShape<MC>;
+    using Shape = TcShape<TYPE, MC>;
     constexpr int kStages = tc_stages<TYPE, MC>(), kStageBytes = tc_stage_bytes<TYPE, MC>();
     constexpr int kPitch = tc_pitch(TYPE), kStepBytes = tc_step_bytes(TYPE);
     constexpr int kNB = tc_b_stages<TYPE, MC>();
     constexpr bool kWide = tc_wide(TYPE), kPresplit = tc_presplit(MC);
     constexpr int kOut = tc_out_rows(MC);  // activation rows whose sums go out together
-    constexpr uint32_t kTmD = 64;  // a group's sums start at this column of its 128
-    constexpr uint32_t kIdesc = (1u << 4) | (static_cast<uint32_t>(Shape::kN >> 3) << 17) | ((128u >> 4) << 24);  // fp32 += fp16 * fp16, M = 128
+    constexpr uint32_t kTmD = 32 * tc_batch_chunks<TYPE, MC>();  // a group's sums start at this column of its 128
+    constexpr uint32_t kIdesc = tc::instruction(TYPE, Shape::kN);
+    static_assert(kTmD + tc_sums<TYPE, MC>() * Shape::kN <= 128, "tensor memory of a group");
     static_assert(kStages >= (kWide ? 3 : 2) && kStages + 2 <= kTcInfoSlots, "stage ring");
     extern __shared__ uint8_t tc_raw[];
     __shared__ __align__(8) uint64_t s_wfull[6], s_wempty[6], s_bfull[4], s_bempty[4], s_afull[4], s_done[4], s_cluster, s_read;
@@ -402,7 +559,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     const uint32_t stages = (tc::s32(tc_raw) + 1023u) & ~1023u;
     [[maybe_unused]] const uint32_t table = stages + kStages * kStageBytes;
     const uint32_t b_ring = table + (grid_bytes(TYPE) + 127) / 128 * 128;
-    const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * kTcGroupB;
+    const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * tc_group_b(TYPE);
     const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
     const uint32_t norm_parts = red + 2 * 264 * kOut * 4;
     volatile int *failed = &s_failed;
@@ -517,7 +674,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     }
                     if (filled >= kNB) copy_x(step, stage);
                     if constexpr (kPresplit) {  // the step's B operand and infos
-                        constexpr int kOperand = Shape::kGroupsB * kTcGroupB, kInfo = tc_info_floats(TYPE, MC) * 4;
+                        constexpr int kOperand = Shape::kGroupsB * tc_group_b(TYPE), kInfo = tc_info_floats(TYPE, MC) * 4;
                         if (filled >= kNB) {
                             tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
                             if (*failed) break;
@@ -561,7 +718,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         for (int tile = group; tile < n_tiles; tile += n_groups)
             for (int step = step0; step < step1; ++step) {
                 if (!kWide || (st & 1) == pair) {
-                    const uint64_t b_unit = tc::b_desc(b_ring + bs * (Shape::kGroupsB * kTcGroupB) + (kWide ? 0 : pair * (16 * kTcCore)));
+                    const uint64_t b_unit = tc::b_desc<TYPE>(b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)) + (kWide ? 0 : pair * (16 * kTcCore)));
                     tc::bar_wait(tc::s32(&s_bfull[bs]), bphase, failed);
 #pragma unroll
                     for (int b = 0; b < kBatches; ++b) {
@@ -578,7 +735,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                     const int i = tc_parts(TYPE) == 2 ? ((b * kBC + (j >> 2)) * 2 + ((j & 3) >> 1)) : b * kMmas + j;
                                     const int sum = tc_block32(TYPE) ? j >> 1 : 0;
                                     const bool fresh = tc_block32(TYPE) ? (j & 1) == 0 : b == 0 && j == 0;
-                                    tc::mma(tm + kTmD + sum * Shape::kN, tm + j * 8, b_unit + static_cast<uint64_t>(i * (2 * kTcCore / 16)), kIdesc,
+                                    tc::mma<TYPE>(tm + kTmD + sum * Shape::kN, tm + j * 8, b_unit + static_cast<uint64_t>(i * (2 * kTcCore / 16)), kIdesc,
                                             fresh ? 0u : 1u);
                                 }
                                 tc::commit(tc::s32(&s_done[wg]));
@@ -614,7 +771,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             while (local >= step1 - step0) local -= step1 - step0;
             const int step = step0 + local;
             const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
-            tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, b_ring + n * (Shape::kGroupsB * kTcGroupB),
+            tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, b_ring + n * (Shape::kGroupsB * tc_group_b(TYPE)),
                                         info_ring + n * tc_info_floats(TYPE, MC) * 4, n == local ? norm_parts + (n * MC + t) * 4 : 0u, lane);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -637,7 +794,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
                             const uint32_t part = tile == group ? norm_parts + ((step - step0) * MC + t) * 4 : 0u;
                             tc_convert<TYPE, MC, true>(a, at + kTcRows * kPitch + t * (kTcStepCols * 4), t, step * kTcStepCols, cols_here,
-                                                 b_ring + bs * (Shape::kGroupsB * kTcGroupB), info, part, lane);
+                                                 b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)), info, part, lane);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                             __syncwarp();
                             if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[bs]));
@@ -696,7 +853,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             batch(v, half, TcInt<0>{}, first, last);
                             if constexpr (kBatches > 1) batch(v, half, TcInt<1>{}, first, last);
                         };
-                        if constexpr (!kWide) {
+                        if constexpr (tc_halves(TYPE) == 1) {
                             half_unit(u[0], kh, true, true);
                         } else {  // (a loop over the halves was measured: smaller code, but 7 % slower)
                             half_unit(u[0], 0, true, false);
