@@ -33,35 +33,42 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
 //   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(24 - k), then the integers -offset * sum of X's
 //   upper 16 bits (signed), and of its lower ones.
 template <int TYPE, int MC, bool ONES>
-__device__ __forceinline__ void tc_convert_bytes(const float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
+__device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
     const uint32_t e = big > 7u ? big : 7u;  // (2^-151 is the unit of X then: below every fp32 number's)
     // X = v * 2^(157 - e), in two factors where the power is beyond fp32
     const float up = __uint_as_float((e < 30u ? 254u : 284u - e) << 23), up2 = __uint_as_float((e < 30u ? 157u - e : 127u) << 23);
-    uint32_t x[8];
-    int hi = 0, lo = 0;
+    if (e < 30u) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int n = __float2int_rn(v[i] * up * up2);
-        hi += n >> 16, lo += n & 0xFFFF;
-        x[i] = static_cast<uint32_t>(n) ^ 0x80000000u;
+        for (int i = 0; i < 8; ++i) v[i] *= up2;
     }
-    constexpr int kOffset = tc_byte_offset(TYPE);
-    if constexpr (kOffset != 0) hi = __reduce_add_sync(0xFFFFFFFFu, hi), lo = __reduce_add_sync(0xFFFFFFFFu, lo);
-    if (lane == 0) {
-        // 2^(e - 133); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
-        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 6u) << 23);
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (tc_info_rows(MC) + t) * 4), "r"(-kOffset * hi) : "memory");
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (2 * tc_info_rows(MC) + t) * 4), "r"(-kOffset * lo) : "memory");
-    }
+    uint32_t x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = static_cast<uint32_t>(__float2int_rn(v[i] * up));
     uint32_t plane[4][2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
         const uint32_t *c = x + 4 * w;
         const uint32_t l01 = __byte_perm(c[0], c[1], 0x5140), l23 = __byte_perm(c[2], c[3], 0x5140);
         const uint32_t h01 = __byte_perm(c[0], c[1], 0x7362), h23 = __byte_perm(c[2], c[3], 0x7362);
-        plane[0][w] = __byte_perm(h01, h23, 0x7632), plane[1][w] = __byte_perm(h01, h23, 0x5410);
+        plane[0][w] = __byte_perm(h01, h23, 0x7632) ^ 0x80808080u, plane[1][w] = __byte_perm(h01, h23, 0x5410);
         plane[2][w] = __byte_perm(l01, l23, 0x7632), plane[3][w] = __byte_perm(l01, l23, 0x5410);
+    }
+    constexpr unsigned kOffset = tc_byte_offset(TYPE);
+    unsigned hi = 0, lo = 0;  // sums of the upper halves of X + 2^31, and of the lower ones
+    if constexpr (kOffset != 0) {
+        unsigned sum[4];
+#pragma unroll
+        for (int p = 0; p < 4; ++p) sum[p] = __dp4a(plane[p][0], 0x01010101u, __dp4a(plane[p][1], 0x01010101u, 0u));
+        hi = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[0] + sum[1]), lo = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[2] + sum[3]);
+    }
+    if (lane == 0) {
+        // 2^(e - 133); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
+        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 6u) << 23);
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
+        if constexpr (kOffset != 0) {
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (tc_info_rows(MC) + t) * 4), "r"(kOffset * (32768u * kTcStepCols - hi)) : "memory");
+            asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (2 * tc_info_rows(MC) + t) * 4), "r"(0u - kOffset * lo) : "memory");
+        }
     }
     const uint32_t at = b_stage + (lane >> 1) * kTcCore + (lane & 1) * 8;
 #pragma unroll
@@ -111,38 +118,51 @@ __device__ __forceinline__ void tc_convert_halves(const float (&v)[8], uint32_t 
     }
 }
 
-// Converts activation row t's 256 columns of a step into the B operand: called by a whole warp, lane = core row.
-//   xs: the row's columns in the stage (not STAGED: they come straight from global memory); cols_here: how many exist; info: where the row's scale and group sums go (floats
-//   [MC] scales, padded to 4, then [groups][MC]); norm_part: where the row's sum of squares goes (0: nowhere)
-template <int TYPE, int MC, bool STAGED>
-__device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, int t, int col0, int cols_here, uint32_t b_stage, uint32_t info,
-                                           uint32_t norm_part, int lane) {
-    int ca, cb;
-    tc_columns<TYPE>(lane, ca, cb);
+// A lane's 2 x 4 columns (tc_columns) of a row of activations (or of what the fused prologues need beside them): v[0..3] and v[4..7].
+struct TcColumns {
     float v[8];
-    const bool has_a = ca < cols_here, has_b = cb < cols_here;  // cols are multiples of 32: a word exists as a whole
-    if constexpr (STAGED) {
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(xs + ca * 4));
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "r"(xs + cb * 4));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            v[i] = has_a ? v[i] : 0.0f;
-            v[4 + i] = has_b ? v[4 + i] : 0.0f;
-        }
-    } else {
-        const float *x = args.x + static_cast<size_t>(t) * args.cols + col0;
+    template <bool CG>
+    __device__ __forceinline__ void load(const float *from, int ca, int cb, bool has_a, bool has_b) {
         const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        const float4 xa = has_a ? __ldcg(reinterpret_cast<const float4 *>(x + ca)) : z, xb = has_b ? __ldcg(reinterpret_cast<const float4 *>(x + cb)) : z;
+        const float4 *pa = reinterpret_cast<const float4 *>(from + ca), *pb = reinterpret_cast<const float4 *>(from + cb);
+        const float4 xa = has_a ? (CG ? __ldcg(pa) : *pa) : z, xb = has_b ? (CG ? __ldcg(pb) : *pb) : z;
         v[0] = xa.x, v[1] = xa.y, v[2] = xa.z, v[3] = xa.w, v[4] = xb.x, v[5] = xb.y, v[6] = xb.z, v[7] = xb.w;
     }
+};
+// Activation row t in the step at col0, before the loop.  cols_here: how many columns exist (a multiple of 32: a word exists as a whole)
+template <int TYPE>
+__device__ __forceinline__ void tc_fetch(const MatvecArgs &args, int t, int col0, int cols_here, int lane, TcColumns &c) {
+    int ca, cb;
+    tc_columns<TYPE>(lane, ca, cb);
+    const bool has_a = ca < cols_here, has_b = cb < cols_here;
+    const size_t at = static_cast<size_t>(t) * args.cols + col0;
+    c.load<true>(args.x + at, ca, cb, has_a, has_b);
+    if (args.fuse & (kFuseSiluMul | kFuseNorm)) {  // requested now, used by tc_convert
+        auto prefetch = [&](const float *from) {
+            if (has_a) asm volatile("prefetch.global.L1 [%0];" ::"l"(from + ca));
+            if (has_b) asm volatile("prefetch.global.L1 [%0];" ::"l"(from + cb));
+        };
+        if (args.fuse & kFuseSiluMul) prefetch(args.x2 + at);
+        if (args.fuse & kFuseNorm) prefetch(args.norm_w + col0);
+    }
+}
+
+// Converts activation row t's 256 columns of a step into the B operand: called by a whole warp, lane = core row (bytes: half of one).
+//   c: the lane's columns; info: where the row's scale and group sums go (floats [MC] scales, padded to 4, then [groups][MC]); norm_part:
+//   where the row's sum of squares goes (0: nowhere); ONES: before the loop, when bytes want their row of ones
+template <int TYPE, int MC, bool ONES>
+__device__ __forceinline__ void tc_convert(const MatvecArgs &args, TcColumns &c, int t, int col0, int cols_here, uint32_t b_stage, uint32_t info,
+                                           uint32_t norm_part, int lane) {
+    float (&v)[8] = c.v;
     if (args.fuse & (kFuseSiluMul | kFuseNorm)) {
+        int ca, cb;
+        tc_columns<TYPE>(lane, ca, cb);
+        const bool has_a = ca < cols_here, has_b = cb < cols_here;
         if (args.fuse & kFuseSiluMul) {
-            const float *x2 = args.x2 + static_cast<size_t>(t) * args.cols + col0;
-            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float4 ga = has_a ? *reinterpret_cast<const float4 *>(x2 + ca) : z, gb = has_b ? *reinterpret_cast<const float4 *>(x2 + cb) : z;
-            const float g[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+            TcColumns g;
+            g.load<false>(args.x2 + static_cast<size_t>(t) * args.cols + col0, ca, cb, has_a, has_b);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = v[i] / (1.0f + expf(-v[i])) * g[i];
+            for (int i = 0; i < 8; ++i) v[i] = v[i] / (1.0f + expf(-v[i])) * g.v[i];
         }
         if (args.fuse & kFuseNorm) {
             // the rms factor of a row is linear: it multiplies the finished outputs, here only the squares are added up
@@ -152,12 +172,10 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, 
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, off);
             if (lane == 0 && norm_part != 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(norm_part), "f"(sq) : "memory");
-            const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float4 wa = has_a ? *reinterpret_cast<const float4 *>(args.norm_w + col0 + ca) : z;
-            const float4 wb = has_b ? *reinterpret_cast<const float4 *>(args.norm_w + col0 + cb) : z;
-            const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+            TcColumns w;
+            w.load<false>(args.norm_w + col0, ca, cb, has_a, has_b);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] *= w[i];
+            for (int i = 0; i < 8; ++i) v[i] *= w.v[i];
         }
     }
     if constexpr (tc_mins(TYPE) > 0) {
@@ -177,15 +195,15 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, uint32_t xs, 
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + (tc_info_scales(TYPE, MC) + gb * MC + t) * 4), "f"(sb) : "memory");
         }
     }
-    uint32_t big = 0;
+    uint32_t big = 0;  // the largest magnitude's bits, shifted left by the sign
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t m = __float_as_uint(v[i]) & 0x7FFFFFFFu;
-        big = big > m ? big : m;
+    for (int i = 0; i < 8; i += 2) {
+        const uint32_t m0 = __float_as_uint(v[i]) * 2u, m1 = __float_as_uint(v[i + 1]) * 2u;
+        big = max(big, max(m0, m1));
     }
-    big = __reduce_max_sync(0xFFFFFFFFu, big);
-    if constexpr (tc_bytes(TYPE)) tc_convert_bytes<TYPE, MC, !STAGED>(v, big >> 23, t, b_stage, info, lane);
-    else tc_convert_halves<TYPE, MC>(v, big >> 23, t, b_stage, info, lane);
+    big = __reduce_max_sync(0xFFFFFFFFu, big) >> 24;
+    if constexpr (tc_bytes(TYPE)) tc_convert_bytes<TYPE, MC, ONES>(v, big, t, b_stage, info, lane);
+    else tc_convert_halves<TYPE, MC>(v, big, t, b_stage, info, lane);
 }
 
 // A unit is what a group of warps takes of a step: one or two halves of 128 columns.  Its chunks go to the tensor cores in
@@ -528,7 +546,11 @@ __global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int step = blockIdx.x, t = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
-    if (t < m) tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, tc::s32(image), tc::s32(image) + kOperand, 0u, lane);
+    if (t < m) {
+        TcColumns c;
+        tc_fetch<TYPE>(a, t, step * kTcStepCols, cols_here, lane, c);
+        tc_convert<TYPE, MC, true>(a, c, t, step * kTcStepCols, cols_here, tc::s32(image), tc::s32(image) + kOperand, 0u, lane);
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < kBytes / 16; i += MC * 32)
         reinterpret_cast<uint4 *>(out + static_cast<size_t>(step) * kBytes)[i] = reinterpret_cast<const uint4 *>(image)[i];
@@ -607,60 +629,82 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                          : "memory");
     };
 
-    if (warp == 17) {  // the first tile's maps, while the barriers are being set up
-        const int p = part_of(group);
-        if (lane < 1 << a.tc_map_shift[p]) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.m[p][lane]) : "memory");
-    }
-    if (warp == 16 && tc::elect_one()) {
-        for (int s = 0; s < kStages; ++s) {
-            tc::bar_init(tc::s32(&s_wfull[s]), 1);
-            tc::bar_init(tc::s32(&s_wempty[s]), kWide ? 8 : 16);
-        }
-        for (int s = 0; s < kNB; ++s) {
-            tc::bar_init(tc::s32(&s_bfull[s]), kPresplit ? 1u : static_cast<uint32_t>(m));
-            tc::bar_init(tc::s32(&s_bempty[s]), kWide ? 2 : 4);
-        }
-        for (int g = 0; g < 4; ++g) {
-            tc::bar_init(tc::s32(&s_afull[g]), 4);
-            tc::bar_init(tc::s32(&s_done[g]), 1);
-        }
-        tc::bar_init(tc::s32(&s_cluster), 1);
-        tc::bar_init(tc::s32(&s_read), static_cast<uint32_t>(k_split));
-        s_failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        // weights never depend on an earlier kernel: the first stages are requested before anything else
-        int t = group, k = step0;
+    // Set-up: the copy warp requests the first stages and does not wait for anybody; the other warps meanwhile load the first steps'
+    // activations.  (A block's first MMAs came 7800 cycles after its start, of which weights take 4700: everybody waited 1300 cycles for
+    // the requests to be issued, and activations requested behind 150 KB of weights came 2500 cycles later.  Now 5400.  17408 x 5120,
+    // 1 row: Q3_K 15.7 -> 15.3 us, Q4_K 15.7 -> 15.0.)
+    constexpr int kFirst = kPresplit ? 0 : (kNB * MC + 15) / 16;  // conversions of a warp before the loop
+    [[maybe_unused]] TcColumns first[kFirst == 0 ? 1 : kFirst];
+    int copy_tile = group, copy_step = step0, copied = 0;  // copy warp: the next stage's tile and step
+    auto copy_next = [&](int n) {                          // weights never depend on an earlier kernel
 #pragma unroll 1
-        for (int s = 0; s < kStages && t < n_tiles; ++s) {
-            copy_weights(t, k, s, s >= kNB);
-            if (++k == step1) k = step0, t += n_groups;
+        for (; copied < n && copy_tile < n_tiles; ++copied) {
+            copy_weights(copy_tile, copy_step, copied, copied >= kNB);
+            if (++copy_step == step1) copy_step = step0, copy_tile += n_groups;
         }
+    };
+    if (warp == 16) {
+        if (tc::elect_one()) {
+            for (int s = 0; s < kStages; ++s) tc::bar_init(tc::s32(&s_wfull[s]), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            copy_next(kWide ? 2 : 1);
+            for (int s = 0; s < kStages; ++s) tc::bar_init(tc::s32(&s_wempty[s]), kWide ? 8 : 16);
+            for (int s = 0; s < kNB; ++s) {
+                tc::bar_init(tc::s32(&s_bfull[s]), kPresplit ? 1u : static_cast<uint32_t>(m));
+                tc::bar_init(tc::s32(&s_bempty[s]), kWide ? 2 : 4);
+            }
+            for (int g = 0; g < 4; ++g) {
+                tc::bar_init(tc::s32(&s_afull[g]), 4);
+                tc::bar_init(tc::s32(&s_done[g]), 1);
+            }
+            tc::bar_init(tc::s32(&s_cluster), 1);
+            tc::bar_init(tc::s32(&s_read), static_cast<uint32_t>(k_split));
+            s_failed = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("bar.arrive 6, %0;" ::"n"(kTcThreads) : "memory");
+    } else {
+        if (warp == 17) {  // the first tile's maps
+            const int p = part_of(group);
+            if (lane < 1 << a.tc_map_shift[p]) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.m[p][lane]) : "memory");
+        } else if (warp == 18) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::s32(&s_tmem)), "r"(512u) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+            tc::fence_before();
+        } else {
+            if constexpr (grid_is_codebook(TYPE)) {
+                for (int i = threadIdx.x; i < grid_bytes(TYPE) / 16; i += kTcDecoders) {
+                    const uint4 w = *reinterpret_cast<const uint4 *>(a.codebook + i * 16);
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(table + i * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
+                }
+            }
+            asm volatile("griddepcontrol.wait;" ::: "memory");  // activations are read and outputs written from here on
+#pragma unroll
+            for (int i = 0; i < kFirst; ++i) {
+                const int n = (warp + 16 * i) / MC, t = (warp + 16 * i) % MC;
+                if (n < kNB && t < m) {
+                    int step = step0 + n;
+                    while (step >= step1) step -= step1 - step0;
+                    const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+                    tc_fetch<TYPE>(a, t, step * kTcStepCols, cols_here, lane, first[i]);
+                }
+            }
+        }
+        asm volatile("bar.sync 6, %0;" ::"n"(kTcThreads) : "memory");
     }
-    __syncwarp();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::s32(&s_tmem)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if constexpr (grid_is_codebook(TYPE)) {
-        for (int i = threadIdx.x; i < grid_bytes(TYPE) / 16; i += kTcThreads) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(a.codebook + i * 16);
-            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(table + i * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
-        }
-    }
-    tc::fence_before();
-    __syncthreads();
     // Announces this block's barriers to the cluster; whoever signals them waits for the announcements first.  (The barriers were
     // published by the fence behind their initialisation; a releasing arrive would wait for the copies in flight, 3 us.)
     if (k_split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     tc::fence_after();
-    const uint32_t tmem = s_tmem;
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // activations are read and outputs written from here on
     float best_v = -INFINITY;
     int best_i = 0x7fffffff;
 
     if (warp == 16) {
         if (tc::elect_one()) {
+            copy_next(kStages);
+            asm volatile("griddepcontrol.wait;" ::: "memory");
             int filled = 0, stage = 0;
             uint32_t phase = 0;
             [[maybe_unused]] int bs = 0;
@@ -713,6 +757,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         // ---- MMA issue: warp 17 for groups 0 and 1, warp 18 for groups 2 and 3 ----
         constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_halves(TYPE) * tc_half_batches<TYPE, MC>(), kMmas = 4 * kBC;
         const int pair = warp - 17;
+        const uint32_t tmem = s_tmem;
         int bs = 0, st = 0;
         uint32_t bphase = 0, aphase = 0;
         for (int tile = group; tile < n_tiles; tile += n_groups)
@@ -749,10 +794,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 ++st;
                 if (++bs == kNB) bs = 0, bphase ^= 1u;
             }
+        if (warp == 18) {  // once the decoders have read the last sums, beside the outputs
+            asm volatile("bar.sync 7, %0;" ::"n"(kTcDecoders + 32) : "memory");
+            tc::fence_after();
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        }
     } else {
         const int wg = warp >> 2, quarter = warp & 3, rw = wg & 1, pair = wg >> 1, kh = kWide ? 0 : pair;
         const int cls = rw * 4 + quarter;  // this warp's row class: rows cls, cls + 8, ... of the tile
-        const uint32_t tm_mine = tmem + wg * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
+        const uint32_t tm_mine = s_tmem + wg * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
         const uint32_t a_full = tc::s32(&s_afull[wg]), mma_done = tc::s32(&s_done[wg]);
         int st = 0, stage = 0, bs = 0;  // step count, stage, B stage
         uint32_t wphase = 0, bphase = 0, dphase = 1, rphase = 0, sphase = 0;  // (dphase: of the batch before the next one)
@@ -764,18 +814,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
 
         // The first kNB steps' activations are converted by all warps at once, straight from global memory: the way through the
         // stages would put a copy and a turn of conversions (1 us) between the end of the previous kernel and the first MMAs.
-        for (int n = kPresplit ? kNB : 0, t = warp; n < kNB; t += 16) {
-            while (t >= m && n < kNB) t -= m, ++n;
-            if (n == kNB) break;
-            int local = n;
-            while (local >= step1 - step0) local -= step1 - step0;
-            const int step = step0 + local;
-            const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
-            tc_convert<TYPE, MC, false>(a, 0u, t, step * kTcStepCols, cols_here, b_ring + n * (Shape::kGroupsB * tc_group_b(TYPE)),
-                                        info_ring + n * tc_info_floats(TYPE, MC) * 4, n == local ? norm_parts + (n * MC + t) * 4 : 0u, lane);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[n]));
+#pragma unroll
+        for (int i = 0; i < kFirst; ++i) {
+            const int n = (warp + 16 * i) / MC, t = (warp + 16 * i) % MC;
+            if (n < kNB && t < m) {
+                int step = step0 + n;
+                while (step >= step1) step -= step1 - step0;
+                const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
+                tc_convert<TYPE, MC, true>(a, first[i], t, step * kTcStepCols, cols_here, b_ring + n * (Shape::kGroupsB * tc_group_b(TYPE)),
+                                           info_ring + n * tc_info_floats(TYPE, MC) * 4, n < step1 - step0 ? norm_parts + (n * MC + t) * 4 : 0u, lane);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[n]));
+            }
         }
 
         for (int tile = group; tile < n_tiles; tile += n_groups) {
@@ -793,8 +844,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
                             tc::bar_wait(tc::s32(&s_bempty[bs]), bphase ^ 1u, failed);
                             const uint32_t part = tile == group ? norm_parts + ((step - step0) * MC + t) * 4 : 0u;
-                            tc_convert<TYPE, MC, true>(a, at + kTcRows * kPitch + t * (kTcStepCols * 4), t, step * kTcStepCols, cols_here,
-                                                 b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)), info, part, lane);
+                            TcColumns c;
+                            const uint32_t xs = at + kTcRows * kPitch + t * (kTcStepCols * 4);
+                            int ca, cb;
+                            tc_columns<TYPE>(lane, ca, cb);
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(c.v[0]), "=f"(c.v[1]), "=f"(c.v[2]), "=f"(c.v[3]) : "r"(xs + ca * 4));
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(c.v[4]), "=f"(c.v[5]), "=f"(c.v[6]), "=f"(c.v[7]) : "r"(xs + cb * 4));
+                            if constexpr (chunk_block(TYPE) < kTcStepCols) {  // (else a step is whole)
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    c.v[i] = ca < cols_here ? c.v[i] : 0.0f;
+                                    c.v[4 + i] = cb < cols_here ? c.v[4 + i] : 0.0f;
+                                }
+                            }
+                            tc_convert<TYPE, MC, false>(a, c, t, step * kTcStepCols, cols_here, b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)), info, part, lane);
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                             __syncwarp();
                             if (lane == 0) tc::bar_arrive(tc::s32(&s_bfull[bs]));
@@ -879,6 +942,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             }
             pending = false;
             tc::fence_before();
+            if (tile + n_groups >= n_tiles) asm volatile("bar.arrive 7, %0;" ::"n"(kTcDecoders + 32) : "memory");  // tensor memory may go
             // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
             // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
             const int red_rows = a.tc_deal;
@@ -973,14 +1037,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             }
         }
     }
-    tc::fence_before();
-    __syncthreads();
     if (k_split > 1 && warp >= 16) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // (every thread takes part)
-    if (warp == 0) {
-        tc::fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-        if (lane == 0 && s_failed) atomicCAS(a.status, 0u, kStatusWaitExpired);
-    }
+    if (lane == 0 && *failed) atomicCAS(a.status, 0u, kStatusWaitExpired);
     if (a.out_idx != nullptr) tc_finish_argmax<MC>(a, m, best_v, best_i, warp, lane, s_best_v, s_best_i, &s_last);
 }
 
