@@ -74,7 +74,7 @@ def test_tiles_steps_and_splits_of_every_type(rt, codebooks, t, shapes, cols):
 
 
 @pytest.mark.parametrize("m", [1, 2, 4, 8, 16])
-@pytest.mark.parametrize("t", [T.Q3_K, T.Q2_K], ids=lambda t: t.name)
+@pytest.mark.parametrize("t", [T.Q3_K, T.Q2_K, T.Q8_0, T.IQ4_NL, T.IQ4_XS], ids=lambda t: t.name)
 def test_integer_sums_at_the_ends_of_their_range(rt, codebooks, t, m):
     """Types whose products are summed as integers: the largest and smallest weights times activations at both ends of the
     32-bit range they are rounded to, all of one sign, and activations at both ends of fp32's range."""

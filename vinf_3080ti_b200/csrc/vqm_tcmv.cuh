@@ -12,7 +12,8 @@
 //     are 2^-39 of it).  The planes are separate columns of the B operand, so M rows make 3M columns.  Products are exact,
 //     the tensor core adds in fp32.
 //     Q3_K and Q2_K: quant times sub-scale fits into 8 bits, and everything is a byte and an integer: a quarter of the multiplies
-//     that scale, half the stores to tensor memory, exact sums (see TcUnit<kQ3_K>, tc_convert_bytes).
+//     that scale, half the stores to tensor memory, exact sums (see TcUnit<kQ3_K>, tc_convert_bytes).  Q8_0, IQ4_NL and IQ4_XS: the
+//     weight without its scale is a byte already, and each block of 32 has its own sum.
 //   * A block owns 256 rows.  Thread = weight row (lane of tensor memory): scales are decoded once per row, by the one
 //     thread that needs them, and the A operand is written from registers to tensor memory with tcgen05.st (measured: an
 //     MMA of 128 x 16 with A in tensor memory takes 9.4 cycles at N = 16 and 16.4 at N = 32; with A in shared memory 40).
@@ -46,8 +47,7 @@
 
 namespace vqm {
 
-// (608 threads cap every thread at 96 registers.  Q8_0 and IQ4_XS with 8 rows, IQ4_XS with 2, IQ4_NL with 2 and 8, and the
-// 16-row kernels of Q2_K, Q4_K, Q5_K, Q6_K and IQ2_XS spill 20 to 150 bytes of sums and scales in the batch loop.)
+// (608 threads cap every thread at 96 registers.  IQ4_XS with 8 rows and the 16-row kernels of Q4_K and Q5_K spill 20 to 140 bytes.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums
@@ -67,14 +67,19 @@ __host__ __device__ constexpr int tc_pitch(int type) {
 __host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(type) < 8 && type != kQ6_K; }
 // A columns per weight: 2 where quant times sub-scale needs more than 11 bits and is split in two
 __host__ __device__ constexpr int tc_parts(int type) { return type == kQ6_K ? 2 : 1; }
-// types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit
+// types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit; with an integer scale the sums
+// stay integers until the super-scale
 __host__ __device__ constexpr bool tc_block32(int type) { return type == kQ8_0 || type == kIQ4_NL || type == kIQ4_XS; }
+__host__ __device__ constexpr bool tc_integer_scale(int type) { return type == kIQ4_XS; }
 __host__ __device__ constexpr int tc_groups(int type) { return type == kQ4_K || type == kQ5_K ? 8 : type == kQ2_K ? 16 : 0; }  // minimums per step
-// Types whose weights times sub-scale fit into 8 bits: the operands are bytes (kind::i8), see TcUnit<kQ3_K>.
-__host__ __device__ constexpr bool tc_bytes(int type) { return type == kQ3_K || type == kQ2_K; }
+// Types whose weights times sub-scale fit into 8 bits (see TcUnit<kQ3_K>; a step is one unit) ...
+__host__ __device__ constexpr bool tc_scaled_bytes(int type) { return type == kQ3_K || type == kQ2_K; }
 __host__ __device__ constexpr int tc_byte_offset(int type) { return type == kQ3_K ? 127 : 0; }  // what an A byte is above the weight
-__host__ __device__ constexpr int tc_mins(int type) { return tc_bytes(type) ? tc_groups(type) : tc_groups(type) / 2; }  // per half (bytes: whole) step
+// ... and types whose weights themselves are bytes (signed ones): their operands are bytes (kind::i8).
+__host__ __device__ constexpr bool tc_bytes(int type) { return tc_scaled_bytes(type) || tc_block32(type); }
+__host__ __device__ constexpr int tc_mins(int type) { return tc_scaled_bytes(type) ? tc_groups(type) : tc_groups(type) / 2; }  // per half (whole) step
 __host__ __device__ constexpr int tc_group_b(int type) { return (tc_bytes(type) ? 16 : 32) * kTcCore; }  // bytes of 8 B rows over a step
+__host__ __device__ constexpr int tc_chunk_regs(int type) { return tc_block32(type) ? 16 : 32; }  // tensor-memory columns of a chunk
 // order of a B core row's 8 columns, made of the column words a and b (4 columns each), see tc_columns
 enum : int { kOrderNibbles = 0, kOrderBytes = 1, kOrderGrid = 2 };
 __host__ __device__ constexpr int tc_order(int type) {
@@ -100,16 +105,17 @@ cudaError_t tc_encoder(TcEncode *out);
 // where two steps of weights in use and one in flight do not fit into shared memory.
 __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 176; }
 
-// activation rows a kernel is compiled for, their B rows (3 planes; bytes: 4 planes and a row of ones) in groups of 8, and the MMA's N
+// activation rows a kernel is compiled for, their B rows (3 planes; bytes: 4 planes, unsigned ones a row of ones too) in groups of 8, and
+// the MMA's N
 template <int TYPE, int MC>
 struct TcShape {
-    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + 1 : 3 * MC;
+    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + (tc_scaled_bytes(TYPE) ? 1 : 0) : 3 * MC;
     static constexpr int kGroupsB = (kRowsB + 7) / 8;
     static constexpr int kN = (kGroupsB + 1) / 2 * 16;
 };
-// per step: the activation rows' scales (bytes: and two integer sums each), then the sums of the column groups that share a minimum
+// per step: the activation rows' scales (scaled bytes: and two integer sums each), then the sums of the column groups that share a minimum
 __host__ __device__ constexpr int tc_info_rows(int mc) { return mc < 4 ? 4 : mc; }
-__host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_bytes(type) ? 3 : 1) * tc_info_rows(mc); }
+__host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_scaled_bytes(type) ? 3 : 1) * tc_info_rows(mc); }
 __host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(type, mc) + tc_groups(type) * mc; }
 // More than 8 activation rows: their B operand and infos come ready-made (tc_split_kernel), by bulk copies, because the stages
 // have no room for 16 KB of activations; the tile's sums go out 8 activation rows at a time.
@@ -211,7 +217,7 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // D (tensor memory) (+)= A (tensor memory, 128 x 32 bytes) * B (shared memory, N x 32 bytes, K-major core matrices); 16 fp16 or
-// 32 unsigned bytes along K, sums in fp32 or 32-bit integers
+// 32 bytes along K, sums in fp32 or 32-bit integers
 template <int TYPE>
 __device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     if constexpr (tc_bytes(TYPE)) {
@@ -230,9 +236,9 @@ __device__ __forceinline__ void mma(uint32_t d, uint32_t a, uint64_t b, uint32_t
             : "memory");
     }
 }
-// Instruction descriptor: 128 rows, N columns; fp32 += fp16 * fp16, or s32 += u8 * u8.
+// Instruction descriptor: 128 rows, N columns; fp32 += fp16 * fp16, s32 += u8 * u8 or s32 += s8 * s8.
 __host__ __device__ constexpr uint32_t instruction(int type, int n) {
-    return ((tc_bytes(type) ? 2u : 1u) << 4) | (static_cast<uint32_t>(n >> 3) << 17) | ((128u >> 4) << 24);
+    return ((tc_bytes(type) ? 2u : 1u) << 4) | (tc_bytes(type) && !tc_scaled_bytes(type) ? (1u << 7) | (1u << 10) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) | ((128u >> 4) << 24);
 }
 // Shared-memory descriptor without swizzle: 8 x 16-byte core matrices, kTcCore bytes apart along K, tc_group_b bytes along N.
 template <int TYPE>
@@ -252,6 +258,14 @@ __device__ __forceinline__ void st32(uint32_t at, const uint32_t (&r)[32]) {
 __device__ __forceinline__ void ld4(uint32_t at, float *v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "r"(at) : "memory");
 }
+__device__ __forceinline__ void st16(uint32_t at, const uint32_t (&r)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(at),
+                 "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+                 "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+                 : "memory");
+}
+__device__ __forceinline__ void st_chunk(uint32_t at, const uint32_t (&r)[32]) { st32(at, r); }
+__device__ __forceinline__ void st_chunk(uint32_t at, const uint32_t (&r)[16]) { st16(at, r); }
 __device__ __forceinline__ void ld1(uint32_t at, uint32_t &v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(at) : "memory");
 }

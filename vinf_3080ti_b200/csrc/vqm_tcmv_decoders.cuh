@@ -273,7 +273,11 @@ __device__ __forceinline__ void tc_words_at(uint32_t at, uint32_t (&w)[N]) {
     for (int i = 0; i < N; ++i) w[i] = __funnelshift_r(s[i], s[i + 1], sh);
 }
 
-// Q8_0: blocks of 32 int8 behind an fp16 scale; the scale stays outside, one sum per block.
+// Q8_0, IQ4_NL, IQ4_XS: the weights (quants, levels) are signed bytes as they are; a scale covers 32 of them, the K of one MMA, and
+// multiplies that MMA's sums.  Chunks of 64 weights, 16 registers.  1 / 4 / 8 rows, as fp16 and as bytes, us: IQ4_XS 17408 x 5120 23.4 /
+// 25.7 / 31.2 and 17.7 / 20.5 / 28.3; IQ4_NL 5120 x 17408 28.1 / 30.2 / 38.8 and 22.1 / 25.8 / 33.8; Q8_0 17408 x 5120 26.0 / 27.0 / 30.1
+// and 23.3 / 25.1 / 26.3 (of which its bytes take 14.5).
+// Q8_0: blocks of 32 int8 behind an fp16 scale.  Nothing to unpack: 4 integer instructions per 8 weights align the words.
 template <>
 struct TcUnit<kQ8_0> {
     float d[4];  // the half's four blocks
@@ -281,36 +285,32 @@ struct TcUnit<kQ8_0> {
     __device__ __forceinline__ void begin(uint32_t, uint32_t, int) {}
     __device__ __forceinline__ float scale(int g) const { return d[g]; }
     template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) {
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[16]) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const uint32_t at = row + 34 * (4 * kh + 2 * CH + g);
-            d[2 * CH + g] = half_bits_to_float(lds16(at)) * kTc24;
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * (1.0f / kTc24);
             uint32_t q[8];
             tc_words_at<8>(at + 2, q);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                uint32_t *r = a + 16 * g + 4 * i;  // int8 + 128 is the unsigned byte; 0x8080 is -128 * 2^-24
-                r[0] = tc::hadd2((q[2 * i] ^ 0x80808080u) & 0x00FF00FFu, 0x80808080u);
-                r[1] = tc::hadd2((q[2 * i + 1] ^ 0x80808080u) & 0x00FF00FFu, 0x80808080u);
-                r[2] = tc::hadd2(((q[2 * i] >> 8) ^ 0x00800080u) & 0x00FF00FFu, 0x80808080u);
-                r[3] = tc::hadd2(((q[2 * i + 1] >> 8) ^ 0x00800080u) & 0x00FF00FFu, 0x80808080u);
-            }
+            for (int i = 0; i < 8; ++i) a[8 * g + i] = q[i];
         }
     }
 };
 
-// The 8 nibbles of a word as a core row: the 16 levels of IQ4_NL / IQ4_XS sit in four registers, plus 128, one per byte.
+__device__ __forceinline__ uint32_t tc_prmt(uint32_t a, uint32_t b, uint32_t s) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(s));
+    return d;
+}
+// The 8 nibbles of a word as 8 levels, in the order of the nibbles: the 16 levels of IQ4_NL / IQ4_XS sit in four registers, one per
+// byte.  11 integer instructions.
 __device__ __forceinline__ void tc_iq4_word(uint32_t w, uint32_t *r) {
-    constexpr uint32_t L0 = 0x3F2D1801u, L1 = 0x766A5D4Fu, H0 = 0xA6998D81u, H1 = 0xF1D9C5B5u;
+    constexpr uint32_t L0 = 0xBFAD9881u, L1 = 0xF6EADDCFu, H0 = 0x26190D01u, H1 = 0x71594535u;
     const uint32_t sel = w & 0x77777777u;                          // entry within each half of the table
     const uint32_t pick = ((w >> 1) & 0x44444444u) | 0x32103210u;  // which half
-    const uint32_t x0 = __byte_perm(__byte_perm(L0, L1, sel), __byte_perm(H0, H1, sel), pick);
-    const uint32_t x1 = __byte_perm(__byte_perm(L0, L1, sel >> 16), __byte_perm(H0, H1, sel >> 16), pick >> 16);
-    r[0] = tc::hadd2(x0 & 0x00FF00FFu, 0x80808080u);               // low nibbles of bytes 0 and 1
-    r[1] = tc::hadd2(__byte_perm(x0, 0u, 0x4341), 0x80808080u);    // their high nibbles
-    r[2] = tc::hadd2(x1 & 0x00FF00FFu, 0x80808080u);
-    r[3] = tc::hadd2(__byte_perm(x1, 0u, 0x4341), 0x80808080u);
+    r[0] = tc_prmt(tc_prmt(L0, L1, sel), tc_prmt(H0, H1, sel), pick);
+    r[1] = tc_prmt(tc_prmt(L0, L1, sel >> 16), tc_prmt(H0, H1, sel >> 16), pick >> 16);
 }
 
 // IQ4_NL: blocks of 32 nibbles behind an fp16 scale.
@@ -321,15 +321,15 @@ struct TcUnit<kIQ4_NL> {
     __device__ __forceinline__ void begin(uint32_t, uint32_t, int) {}
     __device__ __forceinline__ float scale(int g) const { return d[g]; }
     template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) {
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[16]) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const uint32_t at = row + 18 * (4 * kh + 2 * CH + g);
-            d[2 * CH + g] = half_bits_to_float(lds16(at)) * kTc24;
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * (1.0f / kTc24);
             uint32_t q[4];
             tc_words_at<4>(at + 2, q);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) tc_iq4_word(q[i], a + 16 * g + 4 * i);
+            for (int i = 0; i < 4; ++i) tc_iq4_word(q[i], a + 8 * g + 2 * i);
         }
     }
 };
@@ -337,28 +337,23 @@ struct TcUnit<kIQ4_NL> {
 // IQ4_XS: d @0, high scale bits @2, low scale nibbles @4, nibbles @8; 32-column groups with a 6-bit scale.
 template <>
 struct TcUnit<kIQ4_XS> {
-    float d, dl[4];
+    float d;
     uint32_t sl, sh6;  // the half's four scale nibbles (16 bits) and bit pairs (8 bits)
     template <bool O>
     __device__ __forceinline__ void begin(uint32_t line, uint32_t, int kh) {
         const unsigned long long h = lds64(line);
-        d = half_bits_to_float(static_cast<uint32_t>(h) & 0xFFFFu) * kTc24;
+        d = half_bits_to_float(static_cast<uint32_t>(h) & 0xFFFFu) * (1.0f / kTc24);
         sl = static_cast<uint32_t>(h >> 32) >> (16 * kh);
         sh6 = static_cast<uint32_t>(h) >> (16 + 8 * kh);
     }
-    __device__ __forceinline__ float scale(int g) const { return dl[g]; }
+    __device__ __forceinline__ float scale(int) const { return d; }
+    __device__ __forceinline__ int integer_scale(int g) const { return static_cast<int>(((sl >> (4 * g)) & 15u) | (((sh6 >> (2 * g)) & 3u) << 4)) - 32; }
     template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[32]) {
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            const int i = 2 * CH + g;
-            const uint32_t ls = ((sl >> (4 * i)) & 15u) | (((sh6 >> (2 * i)) & 3u) << 4);
-            dl[i] = d * (__uint_as_float(0x4B000000u | ls) - (8388608.0f + 32.0f));
-        }
+    __device__ __forceinline__ void chunk(uint32_t line, uint32_t sh, int kh, uint32_t (&a)[16]) const {
         uint32_t q[8];
         tc::words<kIQ4_XS, false, 8 + 32 * CH, 8>(line + 64 * kh, sh, q);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) tc_iq4_word(q[i], a + 4 * i);
+        for (int i = 0; i < 8; ++i) tc_iq4_word(q[i], a + 2 * i);
     }
 };
 

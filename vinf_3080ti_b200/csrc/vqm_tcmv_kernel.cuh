@@ -17,7 +17,7 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
         a = 64 * (l >> 3) + 4 * (l & 7), b = a + 32;
     } else if constexpr (TYPE == kQ6_K) {            // half, word, pair of quarters
         a = 128 * (l >> 4) + 32 * (l & 1) + 4 * ((l >> 1) & 7), b = a + 64;
-    } else if constexpr (tc_bytes(TYPE)) {           // (half a row of 16 columns) chunk, half, word, pair of 32-column groups
+    } else if constexpr (tc_scaled_bytes(TYPE)) {    // (half a row of 16 columns) chunk, half, word, pair of 32-column groups
         a = 128 * ((l >> 3) & 1) + 16 * (l >> 4) + 4 * ((l >> 1) & 3) + 64 * (l & 1), b = a + 32;
     } else if constexpr (TYPE == kIQ4_NL || TYPE == kIQ4_XS) {
         a = 32 * (l >> 2) + 4 * (l & 3), b = a + 16;
@@ -26,32 +26,42 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
     }
 }
 
-// The B operand of bytes.  x = X * 2^-k exactly rounded to 32-bit integers, k from the chunk's largest magnitude (biased exponent
-// `big`): what is lost is below 2^-32 of it, 2^-28.8 of the chunk's 2-norm at most, where fp32 sums lose 2^-24.  The planes are the
-// four bytes of X + 2^31, most significant first; one row of ones behind them gives the sums of A that the 2^31 (and A's own offset)
-// are taken out with.  Sums of products are integers and exact.
-//   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(24 - k), then the integers -offset * sum of X's
-//   upper 16 bits (signed), and of its lower ones.
+// The B operand of bytes.  x = X * 2^-k, X rounded to a 32-bit integer (signed bytes: 31 bits), k from the chunk's largest magnitude
+// (biased exponent `big`): what is lost is below 2^-31 of it, 2^-27.8 of the chunk's 2-norm at most, where fp32 sums lose 2^-24.
+// Unsigned bytes: the planes are the four bytes of X + 2^31, most significant first; one row of ones behind them gives the sums of A that
+// the 2^31 (and A's own offset) are taken out with.  Signed bytes: the planes are X's digits, -128 .. 127.  Sums of products are integers
+// and exact.
+//   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(24 - k); unsigned bytes, then: the integers
+//   -offset * sum of X's upper 16 bits (signed), and of its lower ones.
 template <int TYPE, int MC, bool ONES>
 __device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
-    const uint32_t e = big > 7u ? big : 7u;  // (2^-151 is the unit of X then: below every fp32 number's)
-    // X = v * 2^(157 - e), in two factors where the power is beyond fp32
-    const float up = __uint_as_float((e < 30u ? 254u : 284u - e) << 23), up2 = __uint_as_float((e < 30u ? 157u - e : 127u) << 23);
-    if (e < 30u) {
+    constexpr bool kSigned = !tc_scaled_bytes(TYPE);
+    constexpr uint32_t kBits = kSigned ? 30u : 31u;
+    const uint32_t e = big > 7u ? big : 7u;  // (the unit of X is 2^-149 then, or less: no fp32 number's is smaller)
+    // X = v * 2^(126 + kBits - e), in two factors where the power is beyond fp32
+    const float up = __uint_as_float((e < kBits - 1u ? 254u : 253u + kBits - e) << 23), up2 = __uint_as_float((e < kBits - 1u ? 126u + kBits - e : 127u) << 23);
+    if (e < kBits - 1u) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] *= up2;
     }
+    constexpr int order[2][8] = {{0, 1, 2, 3, 4, 5, 6, 7}, {0, 4, 1, 5, 2, 6, 3, 7}};  // (IQ4: low and high nibbles in turn)
     uint32_t x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = static_cast<uint32_t>(__float2int_rn(v[i] * up));
+    for (int i = 0; i < 8; ++i) {
+        x[i] = static_cast<uint32_t>(__float2int_rn(v[order[tc_order(TYPE) == kOrderBytes][i]] * up));
+        if constexpr (kSigned) x[i] += 0x00808080u;
+    }
     uint32_t plane[4][2];
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
         const uint32_t *c = x + 4 * w;
         const uint32_t l01 = __byte_perm(c[0], c[1], 0x5140), l23 = __byte_perm(c[2], c[3], 0x5140);
         const uint32_t h01 = __byte_perm(c[0], c[1], 0x7362), h23 = __byte_perm(c[2], c[3], 0x7362);
-        plane[0][w] = __byte_perm(h01, h23, 0x7632) ^ 0x80808080u, plane[1][w] = __byte_perm(h01, h23, 0x5410);
+        plane[0][w] = __byte_perm(h01, h23, 0x7632), plane[1][w] = __byte_perm(h01, h23, 0x5410);
         plane[2][w] = __byte_perm(l01, l23, 0x7632), plane[3][w] = __byte_perm(l01, l23, 0x5410);
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+            if (kSigned ? p > 0 : p == 0) plane[p][w] ^= 0x80808080u;
     }
     constexpr unsigned kOffset = tc_byte_offset(TYPE);
     unsigned hi = 0, lo = 0;  // sums of the upper halves of X + 2^31, and of the lower ones
@@ -62,8 +72,8 @@ __device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, in
         hi = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[0] + sum[1]), lo = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[2] + sum[3]);
     }
     if (lane == 0) {
-        // 2^(e - 133); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
-        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e - 6u) << 23);
+        // 2^(e - 102 - kBits); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
+        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e + 25u - kBits) << 23);
         asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
         if constexpr (kOffset != 0) {
             asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (tc_info_rows(MC) + t) * 4), "r"(kOffset * (32768u * kTcStepCols - hi)) : "memory");
@@ -76,7 +86,7 @@ __device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, in
         const int n = p * MC + t;
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(plane[p][0]), "r"(plane[p][1]) : "memory");
     }
-    if (ONES && t == 0) {
+    if (!kSigned && ONES && t == 0) {
         constexpr int n = 4 * MC;
         asm volatile("st.shared.v2.u32 [%0], {%1, %1};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(0x01010101u) : "memory");
     }
@@ -207,12 +217,12 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, TcColumns &c,
 }
 
 // A unit is what a group of warps takes of a step: one or two halves of 128 columns.  Its chunks go to the tensor cores in
-// batches; tensor memory holds one batch of a group (64 columns) and 64 columns of sums.  Types with a scale per 32 columns
-// have a sum per 32 columns: with N = 32 only one chunk's fit.
-// Bytes: a unit is a whole step, of two chunks.
-__host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) && !tc_bytes(type) ? 2 : 1; }
+// batches; tensor memory holds one batch of a group and its sums, 128 columns in all.  Types with a scale per 32 columns have a sum
+// per 32 columns: with N = 32 only one chunk's fit.
+// Scaled bytes: a unit is a whole step, of two chunks.
+__host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) && !tc_scaled_bytes(type) ? 2 : 1; }
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_bytes(TYPE) && MC > 8) ? 1 : 2; }
+__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_scaled_bytes(TYPE) && MC > 8) ? 1 : 2; }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_half_batches() { return 2 * tc_parts(TYPE) / tc_batch_chunks<TYPE, MC>(); }
 // sums per row that a batch leaves
@@ -224,7 +234,8 @@ __host__ __device__ constexpr bool tc_fresh_batches(int type) { return tc_block3
 // What sums have to be multiplied with when they come back from tensor memory, one batch later.
 template <int TYPE, int MC>
 struct TcPending {
-    float s[tc_sums<TYPE, MC>()];        // super-scales of the sums
+    float s[tc_sums<TYPE, MC>()];        // scales of the sums (their bits are integers where tc_integer_scale)
+    float d;                             // the unit's super-scale then
     TcUnit<TYPE> unit[tc_halves(TYPE)];  // (only the minimums are used)
     uint32_t info;                       // the step's activation scales and group sums
     int kh;                              // the half, where a unit has one
@@ -344,9 +355,9 @@ __device__ __forceinline__ void tc_accumulate_bytes(const TcPending<TYPE, MC> &p
 // acc[t] += scale * (h0 + 2^-11 h1 + 2^-22 h2 sums) * activation scale  -  minimums * group sums
 template <int TYPE, int MC>
 __device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
-    constexpr int kSums = tc_sums<TYPE, MC>(), kMins = tc_mins(TYPE);
+    static_assert(tc_sums<TYPE, MC>() == 1, "one sum per unit");
+    constexpr int kMins = tc_mins(TYPE);
     if constexpr (MC > 8) {  // eight activation rows at a time, for the registers' sake
-        static_assert(kSums == 1, "one sum per unit");
         const f32x2 s2 = pack2(p.s[0], p.s[0]), c1 = pack2(0x1p-11f, 0x1p-11f), c2 = pack2(0x1p-22f, 0x1p-22f);
 #pragma unroll
         for (int t0 = 0; t0 < MC; t0 += 8) {
@@ -386,9 +397,8 @@ __device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &
         }
         return;
     }
-    float v[kSums][3 * MC + 1];
-#pragma unroll
-    for (int g = 0; g < kSums; ++g) tc::ld_sums<MC>(d_at + g * TcShape<TYPE, MC>::kN, v[g]);
+    float v[3 * MC + 1];
+    tc::ld_sums<MC>(d_at, v);
     f32x2 inv[(MC + 1) / 2];
     if constexpr (MC == 1) {
         inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
@@ -402,23 +412,20 @@ __device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &
         }
     }
     tc::wait_ld();
+    const float s = p.s[0];
+    if constexpr (MC == 1) {
+        float a, b, k, unused;
+        unpack2(acc.v[0], a, b);
+        unpack2(inv[0], k, unused);
+        a = fmaf(fmaf(v[2], 0x1p-22f, fmaf(v[1], 0x1p-11f, v[0])) * s, k, a);
+        acc.v[0] = pack2(a, b);
+    } else {
+        const f32x2 s2 = pack2(s, s), c1 = pack2(0x1p-11f, 0x1p-11f), c2 = pack2(0x1p-22f, 0x1p-22f);
 #pragma unroll
-    for (int g = 0; g < kSums; ++g) {
-        const float s = p.s[g];
-        if constexpr (MC == 1) {
-            float a, b, k, unused;
-            unpack2(acc.v[0], a, b);
-            unpack2(inv[0], k, unused);
-            a = fmaf(fmaf(v[g][2], 0x1p-22f, fmaf(v[g][1], 0x1p-11f, v[g][0])) * s, k, a);
-            acc.v[0] = pack2(a, b);
-        } else {
-            const f32x2 s2 = pack2(s, s), c1 = pack2(0x1p-11f, 0x1p-11f), c2 = pack2(0x1p-22f, 0x1p-22f);
-#pragma unroll
-            for (int t = 0; t < MC; t += 2) {
-                f32x2 u = fma2(pack2(v[g][MC + t], v[g][MC + t + 1]), c1, pack2(v[g][t], v[g][t + 1]));
-                u = fma2(pack2(v[g][2 * MC + t], v[g][2 * MC + t + 1]), c2, u);
-                acc.v[t / 2] = fma2(mul2(u, s2), inv[t / 2], acc.v[t / 2]);
-            }
+        for (int t = 0; t < MC; t += 2) {
+            f32x2 u = fma2(pack2(v[MC + t], v[MC + t + 1]), c1, pack2(v[t], v[t + 1]));
+            u = fma2(pack2(v[2 * MC + t], v[2 * MC + t + 1]), c2, u);
+            acc.v[t / 2] = fma2(mul2(u, s2), inv[t / 2], acc.v[t / 2]);
         }
     }
     if constexpr (kMins > 0) {
@@ -450,9 +457,117 @@ __device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &
     }
 }
 
+// Integer sums of a unit over the planes and activation rows, for types with integer scales.
 template <int TYPE, int MC>
-__device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
-    if constexpr (tc_bytes(TYPE)) tc_accumulate_bytes<TYPE, MC>(p, d_at, acc);
+struct TcUnitSums {
+    int v[tc_integer_scale(TYPE) ? 4 * MC : 1];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int &x : v) x = 0;
+    }
+};
+// The sums of signed bytes, one per 32 columns: with D_p the sums over plane p, scale * (2^24 D_0 + 2^16 D_1 + 2^8 D_2 + D_3).  Exact
+// up to the unit's end with an integer scale (|D_p| <= 2^19, times 32, times 8 groups), up to its own with an fp16 one.
+//   last: these are a unit's last sums
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_accumulate_blocks(const TcPending<TYPE, MC> &p, uint32_t d_at, bool last, TcUnitSums<TYPE, MC> &unit, TcAcc<MC> &acc) {
+    constexpr int kSums = tc_sums<TYPE, MC>(), kN = TcShape<TYPE, MC>::kN;
+    f32x2 inv[(MC + 1) / 2];
+    if (!tc_integer_scale(TYPE) || last) {
+        if constexpr (MC == 1) {
+            inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
+        } else if constexpr (MC == 2) {
+            inv[0] = lds64(p.info);
+        } else {
+#pragma unroll
+            for (int t = 0; t < MC; t += 4) {
+                const ulonglong2 w = lds128(p.info + t * 4);
+                inv[t / 2] = w.x, inv[t / 2 + 1] = w.y;
+            }
+        }
+    }
+    auto add = [&](float s, const float (&u)[MC]) {
+        if constexpr (MC == 1) {
+            float a, b, k, unused;
+            unpack2(acc.v[0], a, b);
+            unpack2(inv[0], k, unused);
+            acc.v[0] = pack2(fmaf(u[0] * s, k, a), b);
+        } else {
+            const f32x2 s2 = pack2(s, s);
+#pragma unroll
+            for (int t = 0; t < MC; t += 2) acc.v[t / 2] = fma2(mul2(pack2(u[t], u[t + 1]), s2), inv[t / 2], acc.v[t / 2]);
+        }
+    };
+    if constexpr (tc_integer_scale(TYPE)) {
+        constexpr int kPiece = MC > 4 ? 16 : 4 * MC, kAtOnce = MC > 4 ? 1 : kSums;  // (registers)
+#pragma unroll
+        for (int g0 = 0; g0 < kSums; g0 += kAtOnce) {
+#pragma unroll
+            for (int i0 = 0; i0 < 4 * MC; i0 += kPiece) {
+                uint32_t v[kAtOnce][kPiece];
+#pragma unroll
+                for (int g = 0; g < kAtOnce; ++g) {
+                    if constexpr (MC == 1) {
+                        tc::ld4(d_at + (g0 + g) * kN, v[g]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < kPiece; i += 8) tc::ld8(d_at + (g0 + g) * kN + i0 + i, v[g] + i);
+                    }
+                }
+                tc::wait_ld();
+#pragma unroll
+                for (int g = 0; g < kAtOnce; ++g) {
+                    const int k = __float_as_int(p.s[g0 + g]);
+#pragma unroll
+                    for (int i = 0; i < kPiece; ++i) unit.v[i0 + i] += k * static_cast<int>(v[g][i]);
+                }
+            }
+        }
+    } else {
+        constexpr int kAtOnce = MC > 4 ? 1 : kSums;  // (registers)
+#pragma unroll
+        for (int g0 = 0; g0 < kSums; g0 += kAtOnce) {
+            uint32_t v[kAtOnce][4 * MC];
+#pragma unroll
+            for (int g = 0; g < kAtOnce; ++g) {
+                if constexpr (MC == 1) {
+                    tc::ld4(d_at + (g0 + g) * kN, v[g]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4 * MC; i += 8) tc::ld8(d_at + (g0 + g) * kN + i, v[g] + i);
+                }
+            }
+            tc::wait_ld();
+#pragma unroll
+            for (int g = 0; g < kAtOnce; ++g) {
+                float u[MC];
+#pragma unroll
+                for (int t = 0; t < MC; ++t)
+                    u[t] = fmaf(static_cast<float>(static_cast<int>(v[g][t] * 256u + v[g][MC + t])), 65536.0f,
+                                static_cast<float>(static_cast<int>(v[g][2 * MC + t] * 256u + v[g][3 * MC + t])));
+                add(p.s[g0 + g], u);
+            }
+        }
+    }
+    if (tc_integer_scale(TYPE) && last) {
+        if constexpr (tc_integer_scale(TYPE)) {
+            float u[MC];
+#pragma unroll
+            for (int t = 0; t < MC; ++t) {
+                u[t] = static_cast<float>(unit.v[t]);
+#pragma unroll
+                for (int i = 1; i < 4; ++i) u[t] = fmaf(u[t], 256.0f, static_cast<float>(unit.v[i * MC + t]));
+            }
+            add(p.d, u);
+            unit.clear();
+        }
+    }
+}
+
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_accumulate(const TcPending<TYPE, MC> &p, uint32_t d_at, bool last, TcUnitSums<TYPE, MC> &unit, TcAcc<MC> &acc) {
+    if constexpr (tc_scaled_bytes(TYPE)) tc_accumulate_bytes<TYPE, MC>(p, d_at, acc);
+    else if constexpr (tc_bytes(TYPE)) tc_accumulate_blocks<TYPE, MC>(p, d_at, last, unit, acc);
     else tc_accumulate_halves<TYPE, MC>(p, d_at, acc);
 }
 
@@ -564,7 +679,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     constexpr int kNB = tc_b_stages<TYPE, MC>();
     constexpr bool kWide = tc_wide(TYPE), kPresplit = tc_presplit(MC);
     constexpr int kOut = tc_out_rows(MC);  // activation rows whose sums go out together
-    constexpr uint32_t kTmD = 32 * tc_batch_chunks<TYPE, MC>();  // a group's sums start at this column of its 128
+    constexpr uint32_t kTmD = tc_chunk_regs(TYPE) * tc_batch_chunks<TYPE, MC>();  // a group's sums start at this column of its 128
     constexpr uint32_t kIdesc = tc::instruction(TYPE, Shape::kN);
     static_assert(kTmD + tc_sums<TYPE, MC>() * Shape::kN <= 128, "tensor memory of a group");
     static_assert(kStages >= (kWide ? 3 : 2) && kStages + 2 <= kTcInfoSlots, "stage ring");
@@ -755,7 +870,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         __syncwarp();
     } else if (warp > 16) {
         // ---- MMA issue: warp 17 for groups 0 and 1, warp 18 for groups 2 and 3 ----
-        constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_halves(TYPE) * tc_half_batches<TYPE, MC>(), kMmas = 4 * kBC;
+        constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_halves(TYPE) * tc_half_batches<TYPE, MC>(), kMmas = tc_chunk_regs(TYPE) / 8 * kBC;
         const int pair = warp - 17;
         const uint32_t tmem = s_tmem;
         int bs = 0, st = 0;
@@ -763,7 +878,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         for (int tile = group; tile < n_tiles; tile += n_groups)
             for (int step = step0; step < step1; ++step) {
                 if (!kWide || (st & 1) == pair) {
-                    const uint64_t b_unit = tc::b_desc<TYPE>(b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)) + (kWide ? 0 : pair * (16 * kTcCore)));
+                    const uint64_t b_unit = tc::b_desc<TYPE>(b_ring + bs * (Shape::kGroupsB * tc_group_b(TYPE)) + (kWide ? 0 : pair * (tc_group_b(TYPE) / 2)));
                     tc::bar_wait(tc::s32(&s_bfull[bs]), bphase, failed);
 #pragma unroll
                     for (int b = 0; b < kBatches; ++b) {
@@ -778,8 +893,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                 for (int j = 0; j < kMmas; ++j) {
                                     // the B tile of 16 columns behind the batch's j-th 16 A columns (two A tiles per B tile with two parts)
                                     const int i = tc_parts(TYPE) == 2 ? ((b * kBC + (j >> 2)) * 2 + ((j & 3) >> 1)) : b * kMmas + j;
-                                    const int sum = tc_block32(TYPE) ? j >> 1 : 0;
-                                    const bool fresh = tc_block32(TYPE) ? (j & 1) == 0 : b == 0 && j == 0;
+                                    const int sum = tc_block32(TYPE) ? j : 0;
+                                    const bool fresh = tc_block32(TYPE) || (b == 0 && j == 0);
                                     tc::mma<TYPE>(tm + kTmD + sum * Shape::kN, tm + j * 8, b_unit + static_cast<uint64_t>(i * (2 * kTcCore / 16)), kIdesc,
                                             fresh ? 0u : 1u);
                                 }
@@ -809,6 +924,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         bool announced = false;                 // the cluster's barriers are known to exist
         bool pending = false;    // a unit's sums have not been read yet
         TcPending<TYPE, MC> pend;
+        TcUnitSums<TYPE, MC> unit_sums;
+        unit_sums.clear();
         TcAcc<MC> acc;
         acc.clear();
 
@@ -877,7 +994,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             const bool first = first_half && B == 0, last = last_half && B == kBatches - 1;
                             if constexpr (grid_is_codebook(TYPE)) v.table = table;
                             if constexpr (B == 0) v.template begin<O>(line, sh, half);
-                            uint32_t r[32];
+                            uint32_t r[tc_chunk_regs(TYPE)];
                             v.template chunk<O, B * kBC>(line, sh, half, r);
                             if (kBC == 1 && last) {  // everything of the stage has been read
                                 __syncwarp();
@@ -887,15 +1004,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             tc::bar_wait(mma_done, dphase, failed);
                             dphase ^= 1u;
                             tc::fence_after();
-                            tc::st32(tm_mine, r);
-                            if ((first || tc_fresh_batches(TYPE)) && pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
+                            tc::st_chunk(tm_mine, r);
+                            if ((first || tc_fresh_batches(TYPE)) && pending) tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, first, unit_sums, acc);
                             if constexpr (kBC == 2) {
                                 v.template chunk<O, B * kBC + 1>(line, sh, half, r);
                                 if (last) {
                                     __syncwarp();
                                     if (lane == 0) tc::bar_arrive(wempty);
                                 }
-                                tc::st32(tm_mine + 32, r);
+                                tc::st_chunk(tm_mine + tc_chunk_regs(TYPE), r);
                             }
                             tc::wait_st();
                             tc::fence_before();
@@ -907,8 +1024,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                     for (int h = 0; h < tc_halves(TYPE); ++h) pend.unit[h] = u[h];
                                 }
                                 pend.info = info, pend.kh = kh;
+                                if constexpr (tc_integer_scale(TYPE)) {
+                                    pend.d = v.scale(0);
 #pragma unroll
-                                for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = v.scale(tc_block32(TYPE) ? 2 * B * kBC + g : 0);
+                                    for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = __int_as_float(v.integer_scale(2 * B * kBC + g));
+                                } else {
+#pragma unroll
+                                    for (int g = 0; g < tc_sums<TYPE, MC>(); ++g) pend.s[g] = v.scale(tc_block32(TYPE) ? 2 * B * kBC + g : 0);
+                                }
                                 pending = true;
                             }
                         };
@@ -938,7 +1061,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             if (pending) {
                 tc::bar_wait(mma_done, dphase, failed);
                 tc::fence_after();
-                tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, acc);
+                tc_accumulate<TYPE, MC>(pend, tm_mine + kTmD, true, unit_sums, acc);
             }
             pending = false;
             tc::fence_before();
