@@ -69,6 +69,16 @@ __host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(
 __host__ __device__ constexpr int tc_parts(int type) { return type == kQ6_K ? 2 : 1; }
 // types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit; with an integer scale the sums
 // stay integers until the super-scale
+// types that look up four signed weights at a time (see TcSigned)
+__host__ __device__ constexpr bool tc_signed_table(int type) { return type == kIQ2_XXS || type == kIQ3_XXS || type == kIQ3_S; }
+// Copies of the signed table, word by word: 32 lanes that pick words at random from 32 banks take 3.5 turns, 16 from every other bank 3.1,
+// 8 from every fourth 2.6.  As many as there is room for.
+__host__ __device__ constexpr int tc_table_copies(int type, int mc) {
+    return type == kIQ3_XXS ? (mc <= 4 ? 4 : 2) : type == kIQ2_XXS ? 2 : type == kIQ3_S && mc <= 4 ? 2 : 1;
+}
+__host__ __device__ constexpr int tc_table_bytes(int type, int mc) {
+    return tc_signed_table(type) ? (type == kIQ3_XXS ? 16384 : 32768) * tc_table_copies(type, mc) : grid_bytes(type);
+}
 __host__ __device__ constexpr bool tc_block32(int type) { return type == kQ8_0 || type == kIQ4_NL || type == kIQ4_XS; }
 __host__ __device__ constexpr bool tc_integer_scale(int type) { return type == kIQ4_XS; }
 __host__ __device__ constexpr int tc_groups(int type) { return type == kQ4_K || type == kQ5_K ? 8 : type == kQ2_K ? 16 : 0; }  // minimums per step
@@ -126,7 +136,7 @@ __host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(T
 // Shared memory beside the weight stages, with `b` B stages (an MMA may read one group of rows further).
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_fixed_bytes(int b) {
-    return (grid_bytes(TYPE) + 127) / 128 * 128 + (b * TcShape<TYPE, MC>::kGroupsB + 1) * tc_group_b(TYPE) + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
+    return (tc_table_bytes(TYPE, MC) + 127) / 128 * 128 + (b * TcShape<TYPE, MC>::kGroupsB + 1) * tc_group_b(TYPE) + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
            2 * 264 * tc_out_rows(MC) * 4 + (tc_presplit(MC) ? 0 : (kTcMaxNormSteps + 2) * MC * 4) + 256;
 }
 template <int TYPE, int MC>

@@ -382,44 +382,16 @@ struct TcGrid {
         emit(m0, m1, signs7, k, r);
         r[3] ^= eighth & 0x80000000u;
     }
-    // bit 7 l: the parity of bits 7 l .. 7 l + 6
-    static __device__ __forceinline__ uint32_t parities(uint32_t x) {
-        const uint32_t x1 = x ^ (x >> 1), x2 = x1 ^ (x1 >> 2);
-        return x2 ^ (x1 >> 4) ^ (x >> 6);
-    }
     __device__ __forceinline__ void entry8(uint32_t index, uint32_t &m0, uint32_t &m1) const {
         const unsigned long long e = lds64(table + index * 8);
         m0 = static_cast<uint32_t>(e), m1 = static_cast<uint32_t>(e >> 32);
     }
-    __device__ __forceinline__ uint32_t entry4(uint32_t index) const { return lds32(table + index * 4); }
 };
 template <int K>
 __device__ __forceinline__ uint32_t tc_byte(uint32_t w) { return __byte_perm(w, 0u, 0x4440 | K); }
 // (everything behind the two bytes of d: the words() offsets of these types count from there)
 __device__ __forceinline__ uint32_t tc_line2(uint32_t row) { return (row + 2) & ~3u; }
 __device__ __forceinline__ uint32_t tc_shift2(uint32_t row) { return ((row + 2) & 2u) * 8u; }
-
-// IQ2_XXS: per 32 weights four index bytes and a word of 4 x 7 signs and a 4-bit scale.
-template <>
-struct TcUnit<kIQ2_XXS> : TcGrid {
-    template <bool O>
-    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int) { d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f); }
-    template <bool O, int CH>
-    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
-        uint32_t w[4];
-        tc::words<kIQ2_XXS, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
-#pragma unroll
-        for (int g = 0; g < 2; ++g) {
-            const uint32_t idx = w[2 * g], aux = w[2 * g + 1], par = parities(aux), k = odd_scale((aux >> 27) | 1u);
-            uint32_t m0, m1;
-            uint32_t *r = a + 16 * g;
-            entry8(tc_byte<0>(idx), m0, m1), emit7(m0, m1, aux & 127u, par << 31, k, r);
-            entry8(tc_byte<1>(idx), m0, m1), emit7(m0, m1, (aux >> 7) & 127u, par << 24, k, r + 4);
-            entry8(tc_byte<2>(idx), m0, m1), emit7(m0, m1, (aux >> 14) & 127u, par << 17, k, r + 8);
-            entry8(tc_byte<3>(idx), m0, m1), emit7(m0, m1, (aux >> 21) & 127u, par << 10, k, r + 12);
-        }
-    }
-};
 
 // IQ2_XS: 32 x (9-bit index, 7 signs) @2, 4-bit scale pairs @66.
 template <>
@@ -449,6 +421,7 @@ struct TcUnit<kIQ2_XS> : TcGrid {
     }
 };
 
+// (8-byte loads of the rows: 17408 x 5120, 1 row, 22.1 -> 21.3 us; IQ2_XS, which loads less, loses 1 %, Q2_K 4 %, Q3_K gains nothing.)
 // IQ2_S: index low bytes @2, sign bytes @34, index high bits @66, scale pairs @74.
 template <>
 struct TcUnit<kIQ2_S> : TcGrid {
@@ -457,16 +430,16 @@ struct TcUnit<kIQ2_S> : TcGrid {
     __device__ __forceinline__ void begin(uint32_t row, uint32_t, int kh) {
         d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f);
         uint32_t w[1];
-        tc::words<kIQ2_S, false, 72, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        tc_words_at<1>(row + 2 + 4 * kh + 72, w);
         sc = w[0];
-        tc::words<kIQ2_S, false, 64, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        tc_words_at<1>(row + 2 + 4 * kh + 64, w);
         hi = w[0];
     }
     template <bool O, int CH>
     __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
         uint32_t w[2], s[2];
-        tc::words<kIQ2_S, false, 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), w);
-        tc::words<kIQ2_S, false, 32 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), s);
+        tc_words_at<2>(row + 2 + 16 * kh + 8 * CH, w);
+        tc_words_at<2>(row + 2 + 16 * kh + 32 + 8 * CH, s);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const uint32_t b = sc >> (8 * (2 * CH + g)), q = hi >> (8 * (2 * CH + g));
@@ -481,54 +454,131 @@ struct TcUnit<kIQ2_S> : TcGrid {
     }
 };
 
+// ---- codebook types with a signed table ---------------------------------------------------------------------------------------
+// IQ2_XXS, IQ3_XXS, IQ3_S: the codebook lies in shared memory with every combination of four signs applied, as bytes weight + 128, so ONE
+// permute makes the index of four weights out of its index byte and a byte with their signs (and a ninth index bit, or which half of an
+// 8-weight entry):
+//   word idx + 256 * (signs + 16 * upper) of the table
+// A byte masked out is an fp16 subnormal, and one FMA takes the 128 out and applies the scale, exactly.  8 to 11 integer instructions + 4 FMAs
+// per 8 weights.  What bounds them then is shared memory (80 % busy before): random words of a table conflict (see tc_table_copies), and
+// 4-byte loads of the rows take four turns for 128 bytes where 8-byte ones take four for 256 and a select per word.  IQ3_S, IQ3_XXS, IQ2_XXS
+// 17408 x 5120, 1 row, us: masks and shifts for the signs 24.6 / 23.2 / 20.3, signed table 23.9 / 22.4 / 20.1, 8-byte loads 22.3 / 20.9 / 19.4,
+// copies of the table 21.8 / 20.1 / 18.8.  (As signed bytes with a sum per 32 columns, like Q8_0: 22.8 / 21.5 / 18.9 with 1 row, but 31.6 / 29.9 / 28.0
+// with 8 and twice that with 16, where these take 26.0 / 23.7 / 22.2 and 31.2 / 27.5 / 27.5.)
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_make_signed_table(const uint8_t *codebook, uint32_t table) {  // the decoder threads
+    constexpr int kWords = TYPE == kIQ3_XXS ? 256 : 512, kSigns = 16 * kWords / kTcDecoders;
+    const int word = threadIdx.x % kWords, sign0 = threadIdx.x / kWords * kSigns, idx = word & 255, upper = word >> 8;
+    const uint32_t m = reinterpret_cast<const uint32_t *>(codebook)[TYPE == kIQ2_XXS ? 2 * idx + upper : word];
+#pragma unroll
+    for (int i = 0; i < kSigns; ++i) {
+        const uint32_t s = static_cast<uint32_t>(sign0 + i), neg = (s * 0x00204081u) & 0x01010101u;
+        const uint32_t v = ((m ^ (neg * 0x7Fu)) + neg) ^ (neg << 7) ^ 0x80808080u;  // (magnitudes below 128; no carries, a zero stays one)
+        constexpr int kCopies = tc_table_copies(TYPE, MC);
+        const uint32_t at = table + (idx + 256 * (static_cast<int>(s) + 16 * upper)) * (4 * kCopies);
+        if constexpr (kCopies == 1) asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+        else if constexpr (kCopies == 2) asm volatile("st.shared.v2.u32 [%0], {%1, %1};" ::"r"(at), "r"(v) : "memory");
+        else asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(at), "r"(v) : "memory");
+    }
+}
+struct TcSigned {
+    float d;
+    uint32_t table, pitch;  // this lane's copy, and bytes from a word of it to the next
+    __device__ __forceinline__ float scale(int) const { return d; }
+    // what an entry's bytes are multiplied by, and what is added: k and -128 k, times 2^-24 both
+    struct Scale {
+        uint32_t k, b;
+        __device__ __forceinline__ explicit Scale(uint32_t odd) : k(TcGrid::odd_scale(odd)), b(tc::hmul2(k, 0x80808080u)) {}
+    };
+    // half a core row: the four weights of index byte I of `idx`, signs and upper bit in byte S of `signs`
+    template <int I, int S>
+    __device__ __forceinline__ void entry(uint32_t idx, uint32_t signs, const Scale &s, uint32_t *r) const {
+        uint32_t at;  // (bytes 2 and 3: the sign of `signs`' byte, which is below 32)
+        asm("prmt.b32 %0, %1, %2, %3;" : "=r"(at) : "r"(idx), "r"(signs), "n"(I | (4 + S) << 4 | (12 + S) << 8 | (12 + S) << 12));
+        const uint32_t w = lds32(table + at * pitch);
+        r[0] = tc::hfma2(w & 0x00FF00FFu, s.k, s.b);
+        r[1] = tc::hfma2(__byte_perm(w, 0u, 0x4341), s.k, s.b);
+    }
+    // Four 7-bit fields, each into a byte with its parity on top: the signs of 8 weights, of which the eighth is implied.
+    static __device__ __forceinline__ uint32_t signs8(uint32_t aux) {
+        const uint32_t y = (aux & 0x7Fu) | ((aux << 1) & 0x7F00u) | ((aux << 2) & 0x7F0000u) | ((aux << 3) & 0x7F000000u);
+        uint32_t p = y ^ (y >> 4);
+        p ^= p >> 2;
+        p ^= p >> 1;
+        return y | ((p << 7) & 0x80808080u);
+    }
+};
+
+// IQ2_XXS: per 32 weights four index bytes and a word of 4 x 7 signs and a 4-bit scale.
+template <>
+struct TcUnit<kIQ2_XXS> : TcSigned {
+    template <bool O>
+    __device__ __forceinline__ void begin(uint32_t row, uint32_t, int) { d = half_bits_to_float(lds16(row)) * (kTc24 * 0.125f); }
+    template <bool O, int CH>
+    __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
+        uint32_t w[4];
+        tc_words_at<4>(row + 2 + 32 * kh + 16 * CH, w);
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const uint32_t idx = w[2 * g], y = signs8(w[2 * g + 1]), lo = y & 0x0F0F0F0Fu, hi = ((y >> 4) & 0x0F0F0F0Fu) | 0x10101010u;
+            const Scale k((w[2 * g + 1] >> 27) | 1u);
+            uint32_t *r = a + 16 * g;
+            entry<0, 0>(idx, lo, k, r), entry<0, 0>(idx, hi, k, r + 2), entry<1, 1>(idx, lo, k, r + 4), entry<1, 1>(idx, hi, k, r + 6);
+            entry<2, 2>(idx, lo, k, r + 8), entry<2, 2>(idx, hi, k, r + 10), entry<3, 3>(idx, lo, k, r + 12), entry<3, 3>(idx, hi, k, r + 14);
+        }
+    }
+};
+
 // IQ3_XXS: two index bytes per 8 weights @2, per 32 weights a word of 4 x 7 signs and a 4-bit scale @66.
 template <>
-struct TcUnit<kIQ3_XXS> : TcGrid {
+struct TcUnit<kIQ3_XXS> : TcSigned {
     template <bool O>
     __device__ __forceinline__ void begin(uint32_t row, uint32_t, int) { d = half_bits_to_float(lds16(row)) * (kTc24 * 0.25f); }
     template <bool O, int CH>
     __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
         uint32_t w[4], x[2];
-        tc::words<kIQ3_XXS, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
-        tc::words<kIQ3_XXS, false, 64 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), x);
+        tc_words_at<4>(row + 2 + 32 * kh + 16 * CH, w);
+        tc_words_at<2>(row + 2 + 16 * kh + 64 + 8 * CH, x);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-            const uint32_t aux = x[g], par = parities(aux), k = odd_scale((aux >> 27) | 1u), i0 = w[2 * g], i1 = w[2 * g + 1];
+            const uint32_t i0 = w[2 * g], i1 = w[2 * g + 1], y = signs8(x[g]), lo = y & 0x0F0F0F0Fu, hi = (y >> 4) & 0x0F0F0F0Fu;
+            const Scale k((x[g] >> 27) | 1u);
             uint32_t *r = a + 16 * g;
-            emit7(entry4(tc_byte<0>(i0)), entry4(tc_byte<1>(i0)), aux & 127u, par << 31, k, r);
-            emit7(entry4(tc_byte<2>(i0)), entry4(tc_byte<3>(i0)), (aux >> 7) & 127u, par << 24, k, r + 4);
-            emit7(entry4(tc_byte<0>(i1)), entry4(tc_byte<1>(i1)), (aux >> 14) & 127u, par << 17, k, r + 8);
-            emit7(entry4(tc_byte<2>(i1)), entry4(tc_byte<3>(i1)), (aux >> 21) & 127u, par << 10, k, r + 12);
+            entry<0, 0>(i0, lo, k, r), entry<1, 0>(i0, hi, k, r + 2), entry<2, 1>(i0, lo, k, r + 4), entry<3, 1>(i0, hi, k, r + 6);
+            entry<0, 2>(i1, lo, k, r + 8), entry<1, 2>(i1, hi, k, r + 10), entry<2, 3>(i1, lo, k, r + 12), entry<3, 3>(i1, hi, k, r + 14);
         }
     }
 };
 
 // IQ3_S: index low bytes @2, index high bits @66, sign bytes @74, 4-bit scales @106.
 template <>
-struct TcUnit<kIQ3_S> : TcGrid {
+struct TcUnit<kIQ3_S> : TcSigned {
     uint32_t sc, hi;
     template <bool O>
     __device__ __forceinline__ void begin(uint32_t row, uint32_t, int kh) {
         d = half_bits_to_float(lds16(row)) * kTc24;
         uint32_t w[1];
-        tc::words<kIQ3_S, false, 104, 1>(tc_line2(row), tc_shift2(row), w);
+        tc_words_at<1>(row + 2 + 104, w);
         sc = w[0] >> (16 * kh);
-        tc::words<kIQ3_S, false, 64, 1>(tc_line2(row) + 4 * kh, tc_shift2(row), w);
+        tc_words_at<1>(row + 2 + 4 * kh + 64, w);
         hi = w[0];
     }
     template <bool O, int CH>
     __device__ __forceinline__ void chunk(uint32_t row, uint32_t, int kh, uint32_t (&a)[32]) const {
         uint32_t w[4], s[2];
-        tc::words<kIQ3_S, false, 16 * CH, 4>(tc_line2(row) + 32 * kh, tc_shift2(row), w);
-        tc::words<kIQ3_S, false, 72 + 8 * CH, 2>(tc_line2(row) + 16 * kh, tc_shift2(row), s);
+        tc_words_at<4>(row + 2 + 32 * kh + 16 * CH, w);
+        tc_words_at<2>(row + 2 + 16 * kh + 72 + 8 * CH, s);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-            const uint32_t k = odd_scale(((sc >> (4 * (2 * CH + g))) & 15u) * 2u + 1u), q = hi >> (8 * (2 * CH + g)), i0 = w[2 * g], i1 = w[2 * g + 1];
+            const uint32_t q = hi >> (8 * (2 * CH + g)), i0 = w[2 * g], i1 = w[2 * g + 1];
+            // the high bits of the even and of the odd entries, at bit 4 of the bytes of their signs (a multiply spreads them: bit 2 k goes to
+            // 8 k + 4; what the other products leave lies elsewhere, and carries stay on odd bits)
+            const uint32_t even = (s[g] & 0x0F0F0F0Fu) | (((q & 0x55u) * 0x00410410u) & 0x10101010u);
+            const uint32_t odd = ((s[g] >> 4) & 0x0F0F0F0Fu) | (((q & 0xAAu) * 0x00208208u) & 0x10101010u);
+            const Scale k(((sc >> (4 * (2 * CH + g))) & 15u) * 2u + 1u);
             uint32_t *r = a + 16 * g;
-            emit(entry4(tc_byte<0>(i0) | ((q << 8) & 256u)), entry4(tc_byte<1>(i0) | ((q << 7) & 256u)), tc_byte<0>(s[g]), k, r);
-            emit(entry4(tc_byte<2>(i0) | ((q << 6) & 256u)), entry4(tc_byte<3>(i0) | ((q << 5) & 256u)), tc_byte<1>(s[g]), k, r + 4);
-            emit(entry4(tc_byte<0>(i1) | ((q << 4) & 256u)), entry4(tc_byte<1>(i1) | ((q << 3) & 256u)), tc_byte<2>(s[g]), k, r + 8);
-            emit(entry4(tc_byte<2>(i1) | ((q << 2) & 256u)), entry4(tc_byte<3>(i1) | ((q << 1) & 256u)), tc_byte<3>(s[g]), k, r + 12);
+            entry<0, 0>(i0, even, k, r), entry<1, 0>(i0, odd, k, r + 2), entry<2, 1>(i0, even, k, r + 4), entry<3, 1>(i0, odd, k, r + 6);
+            entry<0, 2>(i1, even, k, r + 8), entry<1, 2>(i1, odd, k, r + 10), entry<2, 3>(i1, even, k, r + 12), entry<3, 3>(i1, odd, k, r + 14);
         }
     }
 };

@@ -695,7 +695,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     // layout: stages (1024-byte aligned) | table | B ring | per-step info | sums of the tile | sums of squares
     const uint32_t stages = (tc::s32(tc_raw) + 1023u) & ~1023u;
     [[maybe_unused]] const uint32_t table = stages + kStages * kStageBytes;
-    const uint32_t b_ring = table + (grid_bytes(TYPE) + 127) / 128 * 128;
+    const uint32_t b_ring = table + (tc_table_bytes(TYPE, MC) + 127) / 128 * 128;
     const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * tc_group_b(TYPE);
     const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
     const uint32_t norm_parts = red + 2 * 264 * kOut * 4;
@@ -788,7 +788,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
             tc::fence_before();
         } else {
-            if constexpr (grid_is_codebook(TYPE)) {
+            if constexpr (tc_signed_table(TYPE)) {
+                tc_make_signed_table<TYPE, MC>(a.codebook, table);
+            } else if constexpr (grid_is_codebook(TYPE)) {
                 for (int i = threadIdx.x; i < grid_bytes(TYPE) / 16; i += kTcDecoders) {
                     const uint4 w = *reinterpret_cast<const uint4 *>(a.codebook + i * 16);
                     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(table + i * 16), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w) : "memory");
@@ -992,7 +994,12 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         auto batch = [&](TcUnit<TYPE> &v, int half, auto batch_tag, bool first_half, bool last_half) {
                             constexpr int B = decltype(batch_tag)::value;
                             const bool first = first_half && B == 0, last = last_half && B == kBatches - 1;
-                            if constexpr (grid_is_codebook(TYPE)) v.table = table;
+                            if constexpr (tc_signed_table(TYPE)) {
+                                constexpr int kCopies = tc_table_copies(TYPE, MC);
+                                v.table = table + lane / (32 / kCopies) * 4, v.pitch = 4 * kCopies;
+                            } else if constexpr (grid_is_codebook(TYPE)) {
+                                v.table = table;
+                            }
                             if constexpr (B == 0) v.template begin<O>(line, sh, half);
                             uint32_t r[tc_chunk_regs(TYPE)];
                             v.template chunk<O, B * kBC>(line, sh, half, r);
