@@ -127,6 +127,21 @@ def test_prologues_residual_and_argmax(rt, codebooks, t, rows, cols, ntok):
     assert ids == [int(v) for v in logits.argmax(axis=1)]
 
 
+@pytest.mark.parametrize("ntok", [17, 24, 25, 63])
+@pytest.mark.parametrize("t,rows,cols", [(t, 2305, 2304) for t in TYPES] + [(T.Q4_K, 39000, 256), (T.Q6_K, 9473, 512), (T.Q3_K, 1025, 17408)],
+                         ids=lambda v: getattr(v, "name", str(v)))
+def test_twenty_four_rows_at_a_time_equal_eight_bit_for_bit(rt, t, rows, cols, ntok):
+    rng = np.random.default_rng(int(t) + rows + ntok)
+    rt.upload("w", synthetic_blocks(t, rows, cols, rng), int(t), cols, rows)
+    x = synthetic_activations(ntok, cols, rng)
+    x[1] *= 1e-5
+    x[ntok - 1, 7] = np.inf
+    (got,) = _run(rt, ["w"], ["y"], (rows,), x)
+    for c in range(0, ntok, 8):
+        (part,) = _run(rt, ["w"], ["y"], (rows,), x[c:c + 8])
+        assert np.array_equal(part.view(np.uint32), got[c:c + 8].view(np.uint32)), c
+
+
 @pytest.mark.parametrize("ntok", [9, 16, 37])
 @pytest.mark.parametrize("t,rows,cols", [(t, 2305, 2304) for t in TYPES] + [(T.Q4_K, 39000, 256), (T.Q6_K, 9473, 512)],
                          ids=lambda v: getattr(v, "name", str(v)))

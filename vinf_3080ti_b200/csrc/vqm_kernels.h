@@ -101,16 +101,17 @@ constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matve
     X(20, IQ4_NL) X(21, IQ3_S) X(22, IQ2_S) X(23, IQ4_XS)
 // split_tcmv_*: into how many column ranges the launch would be split (to go into a.k_split), 0 = the CUDA-core kernel is better.
 // launch_tcmv_*: x_split holds the B operands of more than 8 activation rows; n_launched (may be null) is counted up by the
-// kernels launched, one or two.
+// kernels launched, one or two (split: one for 16 rows).
 #define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
     int split_tcmv_##name(const MatvecArgs &a, int sm_count);                                                                    \
     cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m, \
                                    int sm_count, cudaStream_t stream, int *n_launched);
-// split_bytes_*: size of x_split for a launch of 9..16 rows over so many columns, 0 if the type takes 8 at most;
-// launch_split_*: makes it from a.x.
+// wide_rows_*: how many activation rows a launch takes, 24, 16 or 8; split_bytes_*: size of x_split for a launch of more than 8 rows over so
+// many columns, 0 if the type takes 8 at most; launch_split_*: makes it from a.x.
 #define VQM_DECLARE_SPLIT(id, name)                   \
+    int wide_rows_##name();                            \
     size_t split_bytes_##name(int cols);               \
-    cudaError_t launch_split_##name(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream);
+    cudaError_t launch_split_##name(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream, int *n_launched);
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_SPLIT)
 #undef VQM_DECLARE_SPLIT
 VQM_FOR_EACH_TC_TYPE(VQM_DECLARE_TC_LAUNCHER)

@@ -99,7 +99,7 @@ struct vqm_runtime {
     float *scratch_x = nullptr;
     unsigned *scratch_y = nullptr;  // kStatusWords, then the outputs, of more than kDirectRows rows
     size_t scratch_x_n = 0, scratch_y_n = 0;
-    uint8_t *x_split = nullptr;     // ready-made B operands of 9..16 activation rows
+    uint8_t *x_split = nullptr;     // ready-made B operands of more than 8 activation rows
     size_t x_split_bytes = 0;
     size_t split_need = 0;                      // what the widest tensor so far needs of it
     std::unordered_set<size_t> split_cols;      // columns of the tensors that use it
@@ -270,9 +270,18 @@ size_t split_bytes(int type, int cols) {
         default: return 0;
     }
 }
-cudaError_t dispatch_split(int type, const vqm::MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
+// Activation rows that a launch of the type takes.
+int wide_rows(int type) {
     switch (type) {
-#define VQM_CASE(id, name) case id: return vqm::launch_split_##name(a, x_split, m, stream);
+#define VQM_CASE(id, name) case id: return vqm::wide_rows_##name();
+        VQM_FOR_EACH_TC_TYPE(VQM_CASE)
+#undef VQM_CASE
+    default: return 8;
+    }
+}
+cudaError_t dispatch_split(int type, const vqm::MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream, int *n_launched) {
+    switch (type) {
+#define VQM_CASE(id, name) case id: return vqm::launch_split_##name(a, x_split, m, stream, n_launched);
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
         default: return cudaErrorInvalidValue;
@@ -405,8 +414,7 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         }
         if (err == cudaSuccess && m > 8) err = claim_split(rt);
         if (err == cudaSuccess && m > 8) {
-            err = dispatch_split(t0.type, a, rt->x_split, m, rt->stream);
-            ++launched;
+            err = dispatch_split(t0.type, a, rt->x_split, m, rt->stream, &launched);
         }
         if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, rt->x_split, m, rt->sm_count, rt->stream, &launched);
     } else {
@@ -424,12 +432,12 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
     return launch_parts(rt, 1, ts, x, ys, m, with_argmax, push);
 }
 
-// Room for the B operands of 9..16 activation rows of every tensor so far.  The allocator is entered in relaxed capture mode: the
+// Room for the B operands of more than 8 activation rows of every tensor so far.  The allocator is entered in relaxed capture mode: the
 // pass that finds the room missing may be one that is being captured, by this runtime or by another library.
 bool make_split_room(vqm_runtime *rt) {
     if (rt->split_need <= rt->x_split_bytes) return true;
-    // 28 KB per 256 columns; 2 MB hold up to 17920 columns of any type, so that a runtime allocates once
-    size_t bytes = rt->split_need < (2u << 20) ? 2u << 20 : rt->split_need;
+    // 42 KB per 256 columns; 3 MB hold up to 18432 columns of any type, so that a runtime allocates once
+    size_t bytes = rt->split_need < (3u << 20) ? 3u << 20 : rt->split_need;
     if (bytes < rt->x_split_bytes + rt->x_split_bytes / 2) bytes = rt->x_split_bytes + rt->x_split_bytes / 2;
     uint8_t *p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -446,8 +454,8 @@ bool make_split_room(vqm_runtime *rt) {
     return true;
 }
 
-// Whether the tensor takes 9..16 activation rows in one launch.
-bool takes_sixteen(vqm_runtime *rt, const Tensor &t) {
+// Whether the tensor takes more than 8 activation rows in one launch.
+bool takes_wide(vqm_runtime *rt, const Tensor &t) {
     if (split_bytes(t.type, t.cols) == 0) return false;
     vqm::MatvecArgs a{};
     set_single_part(a, t.data, nullptr, t.rows);
@@ -462,7 +470,7 @@ void see_buffer(vqm_runtime *rt, const Buffer &b) {
 
 // What the passes of a new tensor or buffer will need is made here, so that the first of them does not pay for it: the maps of a
 // tensor of the tensor-core matvec, and, once there is a buffer that holds more than 8 rows of some such tensor's activations, the
-// room for their B operands.  (An allocation of 2 MB takes 0.4 ms, which programs without such passes need not pay.)  Where
+// room for their B operands.  (That allocation takes 0.4 ms, which programs without such passes need not pay.)  Where
 // something fails the launches make up for it, and passes of more than 8 rows run 8 at a time.
 // First pass of 24 rows over three tensors in a new runtime: 530 us without this, 155 with it (later ones alone: 154).
 void prepare_tensor(vqm_runtime *rt, Tensor &t) {
@@ -1072,10 +1080,14 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
         count_launch(rt, 2);
         return VQM_OK;
     }
-    // every group of 8 or 16 activation rows re-reads the weight (from L2 when it fits)
-    const int widest = ntok > 8 && takes_sixteen(rt, *t) ? 16 : 8;
+    // Every group of 8, 16 or 24 activation rows re-reads the weight (from L2 when it fits) and unpacks it again.  24 rows in one launch instead
+    // of 16 and 8: Q4_K 5120 x 17408 43.0 instead of 48.8 us, Q3_K 17408 x 5120 34.9 and 44.1, Q6_K 6144 x 5120 30.2 and 34.7 (17 rows: 41.9
+    // and 43.1, 34.1 and 39.5, 29.6 and 31.9).  Only for the last 17 to 24 rows: before that, 16 at a time are cheaper per row (48 rows of
+    // Q4_K 73 us as 16 + 16 + 16, 84 as 24 + 24; 32 rows 49 as 16 + 16, 67 as 24 + 8).
+    const int widest = ntok > 8 && takes_wide(rt, *t) ? wide_rows(t->type) : 8;
     for (int c = 0, m = 0; c < ntok; c += m) {
-        m = ntok - c < widest ? ntok - c : widest;
+        m = ntok - c;
+        if (m > widest || m > 24) m = widest < 16 ? widest : 16;
         rc = launch_group(rt, *t, xp + static_cast<size_t>(c) * t->cols, yp + static_cast<size_t>(c) * t->rows, m, false);
         if (rc != VQM_OK) return rc;
     }

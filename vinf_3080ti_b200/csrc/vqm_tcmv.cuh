@@ -47,7 +47,8 @@
 
 namespace vqm {
 
-// (608 threads cap every thread at 96 registers.  IQ4_XS with 8 rows and the 16-row kernels of Q4_K and Q5_K spill 20 to 140 bytes.)
+// (608 threads cap every thread at 96 registers.  IQ4_XS with 8 rows and the 16-row kernels of Q4_K, Q5_K and IQ2_S spill 16 to 140 bytes, all
+// 24-row kernels 40 to 90.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums
@@ -115,11 +116,13 @@ cudaError_t tc_encoder(TcEncode *out);
 // where two steps of weights in use and one in flight do not fit into shared memory.
 __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 176; }
 
+// (24 rows of scaled bytes fill a group's tensor memory; the decoders add their bytes up themselves then.)
+__host__ __device__ constexpr bool tc_ones_row(int type, int mc) { return tc_scaled_bytes(type) && mc <= 16; }
 // activation rows a kernel is compiled for, their B rows (3 planes; bytes: 4 planes, unsigned ones a row of ones too) in groups of 8, and
 // the MMA's N
 template <int TYPE, int MC>
 struct TcShape {
-    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + (tc_scaled_bytes(TYPE) ? 1 : 0) : 3 * MC;
+    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + (tc_ones_row(TYPE, MC) ? 1 : 0) : 3 * MC;
     static constexpr int kGroupsB = (kRowsB + 7) / 8;
     static constexpr int kN = (kGroupsB + 1) / 2 * 16;
 };
@@ -128,9 +131,9 @@ __host__ __device__ constexpr int tc_info_rows(int mc) { return mc < 4 ? 4 : mc;
 __host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_scaled_bytes(type) ? 3 : 1) * tc_info_rows(mc); }
 __host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(type, mc) + tc_groups(type) * mc; }
 // More than 8 activation rows: their B operand and infos come ready-made (tc_split_kernel), by bulk copies, because the stages
-// have no room for 16 KB of activations; the tile's sums go out 8 activation rows at a time.
+// have no room for 16 KB of activations; the tile's sums go out 8 (of 24: 4) activation rows at a time.
 __host__ __device__ constexpr bool tc_presplit(int mc) { return mc > 8; }
-__host__ __device__ constexpr int tc_out_rows(int mc) { return mc > 8 ? 8 : mc; }
+__host__ __device__ constexpr int tc_out_rows(int mc) { return mc > 16 ? 4 : mc > 8 ? 8 : mc; }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(TYPE) + (tc_presplit(MC) ? 0 : MC * kTcStepCols * 4); }
 // Shared memory beside the weight stages, with `b` B stages (an MMA may read one group of rows further).
@@ -158,6 +161,9 @@ template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_split_bytes() { return TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE) + tc_info_floats(TYPE, MC) * 4; }
 // 16 activation rows at a time: not the types with a sum per 32 columns (96 columns of sums do not fit beside A in tensor memory)
 __host__ __device__ constexpr bool tc_sixteen(int type) { return !tc_block32(type); }
+// 24 at a time: where their B operands leave room for the stages
+template <int TYPE>
+__host__ __device__ constexpr bool tc_twenty_four() { return tc_sixteen(TYPE) && tc_stages_beside<TYPE, 24>(2) >= (tc_wide(TYPE) ? 3 : 2); }
 
 // ---- primitives --------------------------------------------------------------------------------------------------------
 namespace tc {

@@ -86,7 +86,7 @@ __device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, in
         const int n = p * MC + t;
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(plane[p][0]), "r"(plane[p][1]) : "memory");
     }
-    if (!kSigned && ONES && t == 0) {
+    if (tc_ones_row(TYPE, MC) && ONES && t == 0) {
         constexpr int n = 4 * MC;
         asm volatile("st.shared.v2.u32 [%0], {%1, %1};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(0x01010101u) : "memory");
     }
@@ -222,7 +222,7 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, TcColumns &c,
 // Scaled bytes: a unit is a whole step, of two chunks.
 __host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) && !tc_scaled_bytes(type) ? 2 : 1; }
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_scaled_bytes(TYPE) && MC > 8) ? 1 : 2; }
+__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_scaled_bytes(TYPE) && MC > 8) || MC > 16 ? 1 : 2; }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_half_batches() { return 2 * tc_parts(TYPE) / tc_batch_chunks<TYPE, MC>(); }
 // sums per row that a batch leaves
@@ -236,6 +236,7 @@ template <int TYPE, int MC>
 struct TcPending {
     float s[tc_sums<TYPE, MC>()];        // scales of the sums (their bits are integers where tc_integer_scale)
     float d;                             // the unit's super-scale then
+    uint32_t ones;                       // the sum of a unit's A bytes, where no row of ones makes it
     TcUnit<TYPE> unit[tc_halves(TYPE)];  // (only the minimums are used)
     uint32_t info;                       // the step's activation scales and group sums
     int kh;                              // the half, where a unit has one
@@ -267,8 +268,8 @@ template <int TYPE, int MC>
 __device__ __forceinline__ void tc_accumulate_bytes(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
     static_assert(tc_sums<TYPE, MC>() == 1, "one sum per unit");
     constexpr int kStep = MC > 8 ? 8 : MC, kMins = tc_mins(TYPE);  // activation rows at a time, for the registers' sake
-    uint32_t ones;
-    tc::ld1(d_at + 4 * MC, ones);
+    uint32_t ones = p.ones;
+    if constexpr (tc_ones_row(TYPE, MC)) tc::ld1(d_at + 4 * MC, ones);
 #pragma unroll
     for (int t0 = 0; t0 < MC; t0 += kStep) {
         uint32_t v[4][kStep < 4 ? 4 : kStep];
@@ -652,14 +653,15 @@ __device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, f
     if (threadIdx.x == 0) *a.done_counter = 0;
 }
 
-// B operands and infos of up to MC activation rows, one block per step: what every block of the matvec would work out for itself.
+// B operands and infos of the activation rows t0 .. t0 + 15 below m, of MC, one block per step: what every block of the matvec would work
+// out for itself.
 template <int TYPE, int MC>
-__global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant__ MatvecArgs a, uint8_t *out, const int m) {
+__global__ void __launch_bounds__(16 * 32) tc_split_kernel(const __grid_constant__ MatvecArgs a, uint8_t *out, const int t0, const int m) {
     constexpr int kOperand = TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE), kBytes = tc_split_bytes<TYPE, MC>();
     __shared__ __align__(16) uint8_t image[kBytes];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int step = blockIdx.x, t = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int step = blockIdx.x, t = t0 + static_cast<int>(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
     if (t < m) {
         TcColumns c;
@@ -667,8 +669,14 @@ __global__ void __launch_bounds__(MC * 32) tc_split_kernel(const __grid_constant
         tc_convert<TYPE, MC, true>(a, c, t, step * kTcStepCols, cols_here, tc::s32(image), tc::s32(image) + kOperand, 0u, lane);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kBytes / 16; i += MC * 32)
-        reinterpret_cast<uint4 *>(out + static_cast<size_t>(step) * kBytes)[i] = reinterpret_cast<const uint4 *>(image)[i];
+    uint4 *to = reinterpret_cast<uint4 *>(out + static_cast<size_t>(step) * kBytes);
+    for (int i = threadIdx.x; i < kBytes / 16; i += 16 * 32) {
+        if constexpr (MC > 16) {  // a launch's share: whole groups of 8 B rows, and 4 of every MC floats at a time
+            const int row = i < kOperand / 16 ? i / (tc_group_b(TYPE) / 16) * 8 % MC : (i - kOperand / 16) * 4 % MC;
+            if (row < t0 || row >= t0 + 16) continue;
+        }
+        to[i] = reinterpret_cast<const uint4 *>(image)[i];
+    }
 }
 
 template <int TYPE, int MC, typename MAPS>
@@ -991,6 +999,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         const uint32_t line = kRowAddress ? row : row & (tc_word_loads(TYPE) ? ~3u : ~7u), sh = (row & 2u) * 8u;
                         constexpr int kBC = tc_batch_chunks<TYPE, MC>(), kBatches = tc_half_batches<TYPE, MC>();
                         TcUnit<TYPE> u[tc_halves(TYPE)];
+                        [[maybe_unused]] uint32_t ones = 0;
                         auto batch = [&](TcUnit<TYPE> &v, int half, auto batch_tag, bool first_half, bool last_half) {
                             constexpr int B = decltype(batch_tag)::value;
                             const bool first = first_half && B == 0, last = last_half && B == kBatches - 1;
@@ -1003,6 +1012,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                             if constexpr (B == 0) v.template begin<O>(line, sh, half);
                             uint32_t r[tc_chunk_regs(TYPE)];
                             v.template chunk<O, B * kBC>(line, sh, half, r);
+                            if constexpr (tc_scaled_bytes(TYPE) && !tc_ones_row(TYPE, MC)) {
+                                static_assert(kBC == 1, "one chunk at a time");
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) ones = __dp4a(r[i], 0x01010101u, B == 0 && i == 0 ? 0u : ones);
+                            }
                             if (kBC == 1 && last) {  // everything of the stage has been read
                                 __syncwarp();
                                 if (lane == 0) tc::bar_arrive(wempty);
@@ -1031,6 +1045,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                                     for (int h = 0; h < tc_halves(TYPE); ++h) pend.unit[h] = u[h];
                                 }
                                 pend.info = info, pend.kh = kh;
+                                if constexpr (tc_scaled_bytes(TYPE) && !tc_ones_row(TYPE, MC)) pend.ones = ones;
                                 if constexpr (tc_integer_scale(TYPE)) {
                                     pend.d = v.scale(0);
 #pragma unroll
@@ -1045,6 +1060,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         auto half_unit = [&](TcUnit<TYPE> &v, int half, bool first, bool last) {
                             batch(v, half, TcInt<0>{}, first, last);
                             if constexpr (kBatches > 1) batch(v, half, TcInt<1>{}, first, last);
+                            if constexpr (kBatches > 2) batch(v, half, TcInt<2>{}, first, last), batch(v, half, TcInt<3>{}, first, last);
+                            static_assert(kBatches <= 2 || kBatches == 4, "batches of a half");
                         };
                         if constexpr (tc_halves(TYPE) == 1) {
                             half_unit(u[0], kh, true, true);

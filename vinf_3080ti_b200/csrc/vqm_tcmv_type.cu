@@ -1,5 +1,5 @@
 // One translation unit per GGUF type (-DVQM_TYPE=<id> -DVQM_TYPE_NAME=<name>): instantiates the tensor-core matvec for 1, 2,
-// up to 4, up to 8 and (most types) up to 16 activation rows and exports its launcher.
+// up to 4, up to 8 and (most types) up to 16 and 24 activation rows and exports its launcher.
 #include "vqm_tcmv_kernel.cuh"
 
 #ifndef VQM_TYPE
@@ -146,17 +146,19 @@ inline int choose_tc_split(int n_tiles, int cols, int sm_count, bool single) {
 
 // More than 8 activation rows (templates, so that types without the variant do not compile it)
 template <int TYPE>
-cudaError_t launch_sixteen(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
-    if constexpr (tc_sixteen(TYPE)) {
+constexpr int wide_rows() { return tc_twenty_four<TYPE>() ? 24 : tc_sixteen(TYPE) ? 16 : 8; }
+template <int TYPE, int MC>
+cudaError_t launch_wide(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+    if constexpr (MC <= wide_rows<TYPE>()) {
         if (a.x_split == nullptr || a.fuse != 0 || a.out_idx != nullptr) return cudaErrorInvalidValue;
-        return TcVariant<(TYPE >= 0 ? 16 : 0), TcMaps1>::launch(a, maps, 1, n_tiles, m, sm_count, stream);
+        return TcVariant<(TYPE >= 0 ? MC : 0), TcMaps1>::launch(a, maps, 1, n_tiles, m, sm_count, stream);
     } else {
         return cudaErrorInvalidValue;
     }
 }
-template <int TYPE>
-cudaError_t split_sixteen(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
-    if constexpr (tc_sixteen(TYPE)) {
+template <int TYPE, int MC>
+cudaError_t split_wide(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream, int *n_launched) {
+    if constexpr (MC <= wide_rows<TYPE>()) {
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[1];
         cfg.gridDim = dim3(static_cast<unsigned>((a.cols + kTcStepCols - 1) / kTcStepCols));
@@ -166,7 +168,12 @@ cudaError_t split_sixteen(const MatvecArgs &a, uint8_t *x_split, int m, cudaStre
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = a.overlap_launch ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, tc_split_kernel<TYPE, 16>, a, x_split, m);
+        cudaError_t err = cudaSuccess;
+        for (int t0 = 0; t0 < m && err == cudaSuccess; t0 += 16) {
+            if (n_launched != nullptr) ++*n_launched;
+            err = cudaLaunchKernelEx(&cfg, tc_split_kernel<TYPE, MC>, a, x_split, t0, m);
+        }
+        return err;
     } else {
         return cudaErrorInvalidValue;
     }
@@ -191,7 +198,8 @@ inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const
     if (m == 2) return VQM_LAUNCH(2);
     if (m <= 4) return VQM_LAUNCH(4);
     if (m <= 8) return VQM_LAUNCH(8);
-    if (m <= 16 && n_parts == 1) return launch_sixteen<VQM_TYPE>(a, maps, end - first, m, sm_count, stream);
+    if (m <= 16 && n_parts == 1) return launch_wide<VQM_TYPE, 16>(a, maps, end - first, m, sm_count, stream);
+    if (m <= 24 && n_parts == 1) return launch_wide<VQM_TYPE, 24>(a, maps, end - first, m, sm_count, stream);
     return cudaErrorInvalidValue;
 #undef VQM_LAUNCH
 }
@@ -205,12 +213,15 @@ int VQM_CAT(split_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &a, int sm_count) {
     return choose_tc_split(tc_tiles(a), a.cols, sm_count, takes_tail(a));
 }
 
+int VQM_CAT(wide_rows_, VQM_TYPE_NAME)() { return wide_rows<VQM_TYPE>(); }
+
 size_t VQM_CAT(split_bytes_, VQM_TYPE_NAME)(int cols) {
-    return tc_sixteen(VQM_TYPE) ? static_cast<size_t>((cols + kTcStepCols - 1) / kTcStepCols) * tc_split_bytes<VQM_TYPE, 16>() : 0;
+    constexpr int kRows = wide_rows<VQM_TYPE>();
+    return kRows > 8 ? static_cast<size_t>((cols + kTcStepCols - 1) / kTcStepCols) * tc_split_bytes<VQM_TYPE, kRows>() : 0;
 }
 
-cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream) {
-    return split_sixteen<VQM_TYPE>(a, x_split, m, stream);
+cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_t stream, int *n_launched) {
+    return m <= 16 ? split_wide<VQM_TYPE, 16>(a, x_split, m, stream, n_launched) : split_wide<VQM_TYPE, 24>(a, x_split, m, stream, n_launched);
 }
 
 cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m,
