@@ -1,9 +1,11 @@
 """CPU checks of the boundary: the library loads and exports exactly what include/vinf_b200.h declares."""
 from __future__ import annotations
 
+import ctypes
 import re
 from pathlib import Path
 
+import numpy as np
 import pytest
 
 from vinf_3080ti_b200 import _capi
@@ -58,3 +60,27 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_capi, "LIB_PATH", tmp_path / "libvinf_b200.so")
     with pytest.raises(_capi.ExtensionMissingError):
         _capi.load()
+
+
+@pytest.mark.parametrize("ntok,seen", [(3, 3), (np.int64(7), 7), (2.9, 2), ("5", 5), (True, 1), (-1, -1), (2**32 + 9, 9)])
+def test_pycall_hands_its_arguments_on_as_ctypes_does(ntok, seen):
+    got = []
+
+    @ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_char_p, ctypes.c_char_p, ctypes.c_char_p, ctypes.c_int)
+    def fn(*args):
+        got.append(args)
+        return 4
+
+    address = ctypes.cast(fn, ctypes.c_void_p).value
+    assert _capi.pycall().qmv(address, 123, "w", "größe", "y\0z", ntok) == 4
+    assert got == [(123, b"w", "größe".encode(), b"y", seen)]
+    for bad in ((b"w", "x", "y", 1), ("w", None, "y", 1)):
+        with pytest.raises(AttributeError):
+            _capi.pycall().qmv(address, 123, *bad)
+    with pytest.raises(UnicodeEncodeError):
+        _capi.pycall().qmv(address, 123, "w", "\udc80", "y", 1)
+    with pytest.raises((TypeError, ValueError)):
+        _capi.pycall().qmv(address, 123, "w", "x", "y", None)
+    with pytest.raises((TypeError, ValueError)):  # a closed runtime
+        _capi.pycall().qmv(address, None, "w", "x", "y", 1)
+    assert len(got) == 1

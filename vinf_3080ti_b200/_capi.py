@@ -87,6 +87,22 @@ _RESTYPES = {"vqm_last_error": c_char_p, "vqm_runtime_destroy": None, "vqm_strea
 _lib: ctypes.CDLL | None = None
 
 
+_pycall = None
+
+
+def pycall():
+    """The module that calls vqm_qmv without ctypes, loaded once."""
+    global _pycall
+    if _pycall is not None:
+        return _pycall
+    path = Path(__file__).resolve().parent / "_vqm_pycall.so"
+    if not path.exists():
+        raise ExtensionMissingError(f"{path} is not built; run `python -m vinf_3080ti_b200.build`")
+    from . import _vqm_pycall
+    _pycall = _vqm_pycall
+    return _pycall
+
+
 def load() -> ctypes.CDLL:
     """Loads the library once and types every entry point."""
     global _lib

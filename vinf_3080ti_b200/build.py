@@ -9,7 +9,7 @@ results are wrong on purpose.
 Such a build goes to --out (objects beside it) and is loaded with VINF_B200_LIB=<path>.
 
 Two translation units per GGUF type (the matvec kernel instantiations, plain and with the fused prologues) plus the small kernels and the
-runtime; objects go to csrc/build/, the library next to this file.  Cross-compiles without a GPU.
+runtime; objects go to csrc/build/, the library next to this file, and beside it _vqm_pycall.so (gcc).  Cross-compiles without a GPU.
 """
 from __future__ import annotations
 
@@ -18,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -25,6 +26,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = CSRC / "build"
 LIB = HERE / "libvinf_b200.so"
+PYCALL = HERE / "_vqm_pycall.so"  # vqm_qmv for Python without ctypes
 
 TYPES = [(0, "F32"), (1, "F16"), (8, "Q8_0"), (10, "Q2_K"), (11, "Q3_K"), (12, "Q4_K"), (13, "Q5_K"), (14, "Q6_K"),
          (16, "IQ2_XXS"), (17, "IQ2_XS"), (18, "IQ3_XXS"), (20, "IQ4_NL"), (21, "IQ3_S"), (22, "IQ2_S"), (23, "IQ4_XS")]
@@ -45,6 +47,16 @@ def _nvcc() -> str:
 def _sources() -> list[Path]:
     return sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) +
                   [HERE.parent / "include" / "vinf_b200.h"])
+
+
+def build_pycall() -> Path:
+    src = CSRC / "vqm_pycall.c"
+    if not PYCALL.exists() or src.stat().st_mtime > PYCALL.stat().st_mtime:
+        cmd = ["gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(PYCALL)]
+        done = subprocess.run(cmd, capture_output=True, text=True)
+        if done.returncode != 0:
+            raise RuntimeError(f"gcc failed for {src.name}:\n{done.stdout}\n{done.stderr}")
+    return PYCALL
 
 
 def up_to_date() -> bool:
@@ -72,6 +84,7 @@ def _compile(job: tuple[str, list[str], Path]) -> tuple[str, str]:
 
 def build(force: bool = False, jobs: int | None = None, verbose: bool = False, defines: list[str] | None = None, out: Path | None = None) -> Path:
     global OBJ, LIB
+    build_pycall()
     if defines or out:
         if out is None:
             raise ValueError("an experimental build (--define) needs --out, it must not replace the library")

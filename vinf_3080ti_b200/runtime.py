@@ -67,6 +67,7 @@ class Runtime:
 
     def __init__(self, iq3s_grid: bytes | None = None, codebooks: dict[str, bytes] | None = None) -> None:
         self._lib = _capi.load()
+        self._qmv, self._qmv_fn = _capi.pycall().qmv, ctypes.cast(self._lib.vqm_qmv, ctypes.c_void_p).value
         self._h = ctypes.c_void_p()
         if iq3s_grid is not None and len(iq3s_grid) != 2048:
             raise ValueError("iq3s_grid must be 2048 bytes (512 entries x 4 values)")
@@ -203,7 +204,9 @@ class Runtime:
     # ---- the hot path --------------------------------------------------------------------------------
     def qmv(self, weight: str, x: str, y: str, ntok: int = 1) -> None:
         """y[t][r] = sum_k W[r][k] x[t][k]; asynchronous."""
-        _capi.check(self._lib.vqm_qmv(self._h, _name(weight), _name(x), _name(y), int(ntok)))
+        status = self._qmv(self._qmv_fn, self._h.value, weight, x, y, ntok)
+        if status:
+            _capi.check(status)
 
     def matvec(self, name: str, x) -> bytes:
         """matvec(name, x_f32_bytes) -> y_f32_bytes; synchronous single-row entry."""
