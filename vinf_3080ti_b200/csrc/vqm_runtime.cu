@@ -436,8 +436,9 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
 // pass that finds the room missing may be one that is being captured, by this runtime or by another library.
 bool make_split_room(vqm_runtime *rt) {
     if (rt->split_need <= rt->x_split_bytes) return true;
-    // 42 KB per 256 columns; 3 MB hold up to 18432 columns of any type, so that a runtime allocates once
-    size_t bytes = rt->split_need < (3u << 20) ? 3u << 20 : rt->split_need;
+    // At most 42 KB per 256 columns; 2 MB hold 12288 columns of any type.  (3 MB at once, enough for 18432: a new runtime's first buffers take 0.3 to
+    // 0.6 ms longer, more than the second allocation that wider tensors ask for.)
+    size_t bytes = rt->split_need < (2u << 20) ? 2u << 20 : rt->split_need;
     if (bytes < rt->x_split_bytes + rt->x_split_bytes / 2) bytes = rt->x_split_bytes + rt->x_split_bytes / 2;
     uint8_t *p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
