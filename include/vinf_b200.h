@@ -106,7 +106,7 @@ int vqm_buffer_len(vqm_runtime *rt, const char *name, size_t *n);
 int vqm_buffer_bytes(vqm_runtime *rt, size_t *out);
 
 /* qmv(weight, x, y[, ntok]) - qwen_runtime.cu:1861-1912: y[t][r] = sum_k W[r][k] x[t][k], x = [ntok][cols],
- * y = [ntok][rows], both fp32 buffers.  Asynchronous.  More than 8 rows run as groups of 16 or 8. */
+ * y = [ntok][rows], both fp32 buffers.  Asynchronous.  More than 8 rows run as groups of 24, 16 or 8. */
 int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, int ntok);
 /* matvec(name, x) -> y - qwen_runtime.cu:2281-2315: synchronous single-row entry with host vectors. */
 int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t x_bytes, float *y_host, size_t y_bytes);
