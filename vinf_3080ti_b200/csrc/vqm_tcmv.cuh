@@ -63,7 +63,7 @@ __host__ __device__ constexpr int tc_pitch(int type) {
     return (lines | 1) * 16;
 }
 // Rows that are not 8-byte aligned are read either in 8-byte loads, by one of two copies of the decoder (rows that start in the
-// lower and in the upper word), or in 4-byte loads, which have twice the bank conflicts.  Q3_K 75776 x 5120, 1 row: 74 us with
+// lower and in the upper word), or in 4-byte loads, which have twice the bank conflicts.  As fp16, Q3_K 75776 x 5120, 1 row: 74 us with
 // two copies (they do not fit into the instruction cache), 64 us with word loads; Q6_K, which loads twice as much: 84 and 88.
 __host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(type) < 8 && type != kQ6_K; }
 // A columns per weight: 2 where quant times sub-scale needs more than 11 bits and is split in two

@@ -26,7 +26,7 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
     }
 }
 
-// The B operand of bytes.  x = X * 2^-k, X rounded to a 32-bit integer (signed bytes: 31 bits), k from the chunk's largest magnitude
+// The B operand of bytes.  x = X * 2^-k, X a 32-bit integer, rounded (signed bytes: 31 bits), k from the chunk's largest magnitude
 // (biased exponent `big`): what is lost is below 2^-31 of it, 2^-27.8 of the chunk's 2-norm at most, where fp32 sums lose 2^-24.
 // Unsigned bytes: the planes are the four bytes of X + 2^31, most significant first; one row of ones behind them gives the sums of A that
 // the 2^31 (and A's own offset) are taken out with.  Signed bytes: the planes are X's digits, -128 .. 127.  Sums of products are integers
