@@ -103,6 +103,47 @@ def test_integer_sums_at_the_ends_of_their_range(rt, codebooks, t, m):
             assert np.linalg.norm(got[k] - ref[k]) <= bound, (first + k, np.linalg.norm(got[k] - ref[k]) / np.linalg.norm(ref[k]))
 
 
+# The field that a row's first sub-scale (Q8_0: the weight of column 5) is made zero with: (byte, bits kept, bits set)
+ZERO_FIRST = {T.Q3_K: [(96, 0xF0, 0), (104, 0xFC, 2)], T.Q2_K: [(0, 0, 0)], T.Q8_0: [(7, 0, 0)], T.IQ4_NL: [(0, 0, 0), (1, 0, 0)],
+              T.IQ4_XS: [(4, 0xF0, 0), (2, 0xFC, 2)]}
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("t", list(ZERO_FIRST), ids=lambda t: t.name)
+def test_a_row_without_weight_at_an_outlier_is_as_exact_as_without_it(rt, codebooks, t, m):
+    """One activation is 10^3 to 10^6 times the others, and every other row's weight there is zero: such a row's error is measured
+    against its own products, row by row."""
+    rows, cols = 39000, 256
+    rng = np.random.default_rng(int(t))
+    block, size = TRAITS[t]
+    raw = np.frombuffer(synthetic_blocks(t, rows, cols, rng), dtype=np.uint8).reshape(rows, cols // block, size).copy()
+    for byte, keep, put in ZERO_FIRST[t]:
+        raw[1::2, 0, byte] = raw[1::2, 0, byte] & keep | put
+
+    def weights():
+        return O.dequantize(raw.tobytes(), int(t), rows * cols, codebooks).reshape(rows, cols).astype(np.float64)[1::2]
+
+    w, least = weights(), 0.0
+    assert not w[:, 5].any()
+    rt.upload("w", raw.tobytes(), int(t), cols, rows)
+    if t is T.Q2_K:  # a sum over quants and one over minimums, which may cancel
+        raw[:, :, 16:80] = 0
+        least = weights()
+    x = synthetic_activations(16, cols, rng)
+    x[:, 5] = 10.0 ** (3 + np.arange(16) % 4) * np.where(np.arange(16) % 8 < 4, 1.0, -1.0)
+    rest = x.astype(np.float64)
+    rest[:, 5] = 0.0
+    for first in range(0, 16, m):
+        (got,) = _run(rt, ["w"], ["y"], (rows,), x[first:first + m])
+        for k in range(m):
+            # fp32: some 40 independent roundings, each of at most 2^-24 of a sum of the order of the products' 2-norm: sqrt(40) of
+            # them, and 2.5 times that for the worst of 300000 outputs
+            size = np.linalg.norm((w - least) * rest[first + k], axis=1) + np.linalg.norm(least * rest[first + k] + 0 * w, axis=1)
+            bound = 2.0**-24 * 16 * size
+            error = np.abs(got[k, 1::2] - w @ rest[first + k])
+            assert np.all(error <= bound), (first + k, float((error / bound).max()))
+
+
 @pytest.mark.parametrize("t,rows,cols,ntok", [(T.Q6_K, 9473, 512, 1), (T.Q4_K, 2305, 2304, 4), (T.IQ4_XS, 2305, 2304, 8)],
                          ids=lambda v: getattr(v, "name", str(v)))
 def test_prologues_residual_and_argmax(rt, codebooks, t, rows, cols, ntok):

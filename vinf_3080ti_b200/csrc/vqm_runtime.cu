@@ -261,7 +261,7 @@ cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap 
     }
 }
 
-// Ready-made B operands of 9..16 activation rows: their size (0: the type takes 8 rows at most), and the kernel that makes them.
+// Ready-made B operands of more than 8 activation rows: their size (0: the type takes 8 rows at most), and the kernel that makes them.
 size_t split_bytes(int type, int cols) {
     switch (type) {
 #define VQM_CASE(id, name) case id: return vqm::split_bytes_##name(cols);
@@ -1082,8 +1082,7 @@ int vqm_qmv(vqm_runtime *rt, const char *weight, const char *x, const char *y, i
         return VQM_OK;
     }
     // Every group of 8, 16 or 24 activation rows re-reads the weight (from L2 when it fits) and unpacks it again.  24 rows in one launch instead
-    // of 16 and 8: Q4_K 5120 x 17408 43.0 instead of 48.8 us, Q3_K 17408 x 5120 34.9 and 44.1, Q6_K 6144 x 5120 30.2 and 34.7 (17 rows: 41.9
-    // and 43.1, 34.1 and 39.5, 29.6 and 31.9).  Only for the last 17 to 24 rows: before that, 16 at a time are cheaper per row (48 rows of
+    // of 16 and 8: Q4_K 5120 x 17408 43.0 instead of 48.8 us, Q6_K 6144 x 5120 30.2 and 34.7 (17 rows: 41.9 and 43.1, 29.6 and 31.9).  Only for the last 17 to 24 rows: before that, 16 at a time are cheaper per row (48 rows of
     // Q4_K 73 us as 16 + 16 + 16, 84 as 24 + 24; 32 rows 49 as 16 + 16, 67 as 24 + 8).
     const int widest = ntok > 8 && takes_wide(rt, *t) ? wide_rows(t->type) : 8;
     for (int c = 0, m = 0; c < ntok; c += m) {

@@ -8,12 +8,12 @@
 //     weights; one packed fp16 multiply (or FMA, for a bias) makes them (q - bias) * sub-scale * 2^-24, exactly.  fp16
 //     super-scales stay outside: the sums of a unit of columns are multiplied by them in fp32.
 //   * An activation is split exactly into three fp16 values, x = s * (h0 + 2^-11 h1 + 2^-22 h2), s a power of two chosen
-//     per 256 columns (33 bits for a 24-bit number; values far below the chunk's largest lose nothing either until they
-//     are 2^-39 of it).  The planes are separate columns of the B operand, so M rows make 3M columns.  Products are exact,
+//     per 256 columns (33 bits for a 24-bit number; values below the chunk's largest lose nothing either until they
+//     are 2^-32 of it).  The planes are separate columns of the B operand, so M rows make 3M columns.  Products are exact,
 //     the tensor core adds in fp32.
 //     Q3_K and Q2_K: quant times sub-scale fits into 8 bits, and everything is a byte and an integer: a quarter of the multiplies
 //     that scale, half the stores to tensor memory, exact sums (see TcUnit<kQ3_K>, tc_convert_bytes).  Q8_0, IQ4_NL and IQ4_XS: the
-//     weight without its scale is a byte already, and each block of 32 has its own sum.
+//     weight without its scale is a byte already, and each block of 32 has its own sum.  An activation is six bytes then.
 //   * A block owns 256 rows.  Thread = weight row (lane of tensor memory): scales are decoded once per row, by the one
 //     thread that needs them, and the A operand is written from registers to tensor memory with tcgen05.st (measured: an
 //     MMA of 128 x 16 with A in tensor memory takes 9.4 cycles at N = 16 and 16.4 at N = 32; with A in shared memory 40).
@@ -47,8 +47,8 @@
 
 namespace vqm {
 
-// (608 threads cap every thread at 96 registers.  IQ4_XS with 8 rows and the 16-row kernels of Q4_K, Q5_K and IQ2_S spill 16 to 140 bytes, all
-// 24-row kernels 40 to 90.)
+// (608 threads cap every thread at 96 registers.  IQ4_XS with 2 and 8 rows and the 16-row kernels of Q4_K, Q5_K, Q2_K and IQ2_S spill 16 to 30
+// bytes, all 24-row kernels 64 to 84.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums
@@ -116,19 +116,22 @@ cudaError_t tc_encoder(TcEncode *out);
 // where two steps of weights in use and one in flight do not fit into shared memory.
 __host__ __device__ constexpr bool tc_wide(int type) { return tc_pitch(type) <= 176; }
 
-// (24 rows of scaled bytes fill a group's tensor memory; the decoders add their bytes up themselves then.)
-__host__ __device__ constexpr bool tc_ones_row(int type, int mc) { return tc_scaled_bytes(type) && mc <= 16; }
-// activation rows a kernel is compiled for, their B rows (3 planes; bytes: 4 planes, unsigned ones a row of ones too) in groups of 8, and
+constexpr int kTcPlanes = 6;  // of activations as bytes
+// bits of their first two planes: with an integer scale the sums of a superblock must fit into 32 bits
+__host__ __device__ constexpr int tc_piece_bits(int type) { return tc_integer_scale(type) ? 11 : 14; }
+// (16 rows of scaled bytes fill a group's tensor memory; the decoders add their bytes up themselves then.)
+__host__ __device__ constexpr bool tc_ones_row(int type, int mc) { return tc_scaled_bytes(type) && mc <= 8; }
+// activation rows a kernel is compiled for, their B rows (3 planes; bytes: 6 planes, unsigned ones a row of ones too) in groups of 8, and
 // the MMA's N
 template <int TYPE, int MC>
 struct TcShape {
-    static constexpr int kRowsB = tc_bytes(TYPE) ? 4 * MC + (tc_ones_row(TYPE, MC) ? 1 : 0) : 3 * MC;
+    static constexpr int kRowsB = tc_bytes(TYPE) ? kTcPlanes * MC + (tc_ones_row(TYPE, MC) ? 1 : 0) : 3 * MC;
     static constexpr int kGroupsB = (kRowsB + 7) / 8;
     static constexpr int kN = (kGroupsB + 1) / 2 * 16;
 };
-// per step: the activation rows' scales (scaled bytes: and two integer sums each), then the sums of the column groups that share a minimum
+// per step: the activation rows' scales (bytes with an offset: and three integer sums each), then the sums of the column groups that share a minimum
 __host__ __device__ constexpr int tc_info_rows(int mc) { return mc < 4 ? 4 : mc; }
-__host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_scaled_bytes(type) ? 3 : 1) * tc_info_rows(mc); }
+__host__ __device__ constexpr int tc_info_scales(int type, int mc) { return (tc_byte_offset(type) != 0 ? 4 : 1) * tc_info_rows(mc); }
 __host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_info_scales(type, mc) + tc_groups(type) * mc; }
 // More than 8 activation rows: their B operand and infos come ready-made (tc_split_kernel), by bulk copies, because the stages
 // have no room for 16 KB of activations; the tile's sums go out 8 (of 24: 4) activation rows at a time.
@@ -159,11 +162,11 @@ __host__ __device__ constexpr int tc_smem_bytes() {
 // bytes of a step in the buffer of ready-made B operands: the operand, then the infos
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_split_bytes() { return TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE) + tc_info_floats(TYPE, MC) * 4; }
-// 16 activation rows at a time: not the types with a sum per 32 columns (96 columns of sums do not fit beside A in tensor memory)
+// 16 activation rows at a time: not the types with a sum per 32 columns (192 columns of sums do not fit beside A in tensor memory)
 __host__ __device__ constexpr bool tc_sixteen(int type) { return !tc_block32(type); }
-// 24 at a time: where their B operands leave room for the stages
+// 24 at a time: where their sums fit into a group's tensor memory (not six planes) and their B operands leave room for the stages
 template <int TYPE>
-__host__ __device__ constexpr bool tc_twenty_four() { return tc_sixteen(TYPE) && tc_stages_beside<TYPE, 24>(2) >= (tc_wide(TYPE) ? 3 : 2); }
+__host__ __device__ constexpr bool tc_twenty_four() { return tc_sixteen(TYPE) && !tc_bytes(TYPE) && tc_stages_beside<TYPE, 24>(2) >= (tc_wide(TYPE) ? 3 : 2); }
 
 // ---- primitives --------------------------------------------------------------------------------------------------------
 namespace tc {

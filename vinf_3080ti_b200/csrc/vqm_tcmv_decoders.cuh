@@ -14,6 +14,8 @@
 namespace vqm {
 
 constexpr float kTc24 = 16777216.0f;  // 2^24
+// Activations as bytes are integers times this and their factor (tc_convert_bytes).
+__host__ __device__ constexpr float tc_piece_unit(int type) { return 2.0f / static_cast<float>(1 << tc_piece_bits(type)); }
 
 template <int TYPE>
 struct TcUnit;
@@ -142,8 +144,8 @@ struct TcUnit<kQ6_K> {
 // Q3_K and Q2_K: quant times sub-scale fits into 8 bits, so an A column is a byte and ONE 32-bit multiply scales four weights: no
 // byte of the product carries into the next.  Half the registers and stores of fp16 and one integer instruction per four weights
 // less; a step is one batch.  Bound by unpacking as the others (warp instructions per 8 weights of Q3_K, 1 row: 31.5 as fp16, 21.2 so).
-// 17408 x 5120, 1 / 4 / 8 / 16 rows, fp16 and bytes, us: Q3_K 19.8 / 20.9 / 23.0 / 26.6 and 15.7 / 17.5 / 20.4 / 24.8, Q2_K 15.2 / 16.8 /
-// 20.6 / 26.6 and 12.7 / 14.8 / 18.5 / 26.0.  Error against 64 bits, Q3_K: 1.5e-7 and 7e-8; with outliers of 1000 times the rest 1e-6 and 7e-8.
+// 17408 x 5120, 1 / 4 / 8 / 16 rows, fp16 and bytes, us: Q3_K 19.8 / 20.9 / 23.0 / 26.6 and 15.3 / 17.3 / 20.4 / 27.0, Q2_K 15.2 / 16.8 /
+// 20.6 / 26.6 and 12.2 / 14.4 / 18.1 / 27.2.  Error against 64 bits, Q3_K: 1.5e-7 and 7e-8; with outliers of 1000 times the rest 1e-6 and 7e-8.
 // (Q4_K's products need 10 bits, Q6_K's 14: two and three bytes a weight.)
 // Chunk CH: byte columns 16 CH .. 16 CH + 15 of each of the eight 32-column groups (half * 4 + j);
 // register (half * 4 + i) * 4 + j holds columns 128 half + 32 j + 16 CH + 4 i .. + 3.
@@ -166,7 +168,7 @@ struct TcUnit<kQ3_K> {
     __device__ __forceinline__ void begin(uint32_t line, uint32_t sh, int) {
         uint32_t s[4];
         tc::words<kQ3_K, O, 96, 4>(line, sh, s);
-        d = half_bits_to_float(s[3] & 0xFFFFu) * (1.0f / kTc24);
+        d = half_bits_to_float(s[3] & 0xFFFFu) * tc_piece_unit(kQ3_K);
         sc[0] = (s[0] & 0x0F0F0F0Fu) | ((s[2] << 4) & 0x30303030u);
         sc[1] = (s[1] & 0x0F0F0F0Fu) | ((s[2] << 2) & 0x30303030u);
         sc[2] = ((s[0] >> 4) & 0x0F0F0F0Fu) | (s[2] & 0x30303030u);
@@ -225,7 +227,7 @@ struct TcUnit<kQ2_K> {
             sc[i] = (s[i] & 0x0F0F0000u) | ((s[i] << 2) & 0x00003C3Cu);
             mn[i] = (s[i] >> 4) & 0x0F0F0F0Fu;
         }
-        d = half_bits_to_float(w[0] & 0xFFFFu) * (0.25f / kTc24);
+        d = half_bits_to_float(w[0] & 0xFFFFu) * (0.25f * tc_piece_unit(kQ2_K));
         dm = half_bits_to_float(w[0] >> 16);
     }
     __device__ __forceinline__ float scale(int) const { return d; }
@@ -275,8 +277,8 @@ __device__ __forceinline__ void tc_words_at(uint32_t at, uint32_t (&w)[N]) {
 
 // Q8_0, IQ4_NL, IQ4_XS: the weights (quants, levels) are signed bytes as they are; a scale covers 32 of them, the K of one MMA, and
 // multiplies that MMA's sums.  Chunks of 64 weights, 16 registers.  1 / 4 / 8 rows, as fp16 and as bytes, us: IQ4_XS 17408 x 5120 23.4 /
-// 25.7 / 31.2 and 17.7 / 20.5 / 28.3; IQ4_NL 5120 x 17408 28.1 / 30.2 / 38.8 and 22.1 / 25.8 / 33.8; Q8_0 17408 x 5120 26.0 / 27.0 / 30.1
-// and 23.3 / 25.1 / 26.3 (of which its bytes take 14.5).
+// 25.7 / 31.2 and 18.3 / 23.6 / 31.6; IQ4_NL 5120 x 17408 28.1 / 30.2 / 38.8 and 22.4 / 28.5 / 38.4; Q8_0 17408 x 5120 26.0 / 27.0 / 30.1
+// and 23.7 / 24.3 / 29.0 (of which its bytes take 14.5).  Error against 64 bits, IQ4_XS: 1.5e-7 and 7e-8, Q8_0 1.4e-7 and 1.0e-7.
 // Q8_0: blocks of 32 int8 behind an fp16 scale.  Nothing to unpack: 4 integer instructions per 8 weights align the words.
 template <>
 struct TcUnit<kQ8_0> {
@@ -289,7 +291,7 @@ struct TcUnit<kQ8_0> {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const uint32_t at = row + 34 * (4 * kh + 2 * CH + g);
-            d[2 * CH + g] = half_bits_to_float(lds16(at)) * (1.0f / kTc24);
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * tc_piece_unit(kQ8_0);
             uint32_t q[8];
             tc_words_at<8>(at + 2, q);
 #pragma unroll
@@ -325,7 +327,7 @@ struct TcUnit<kIQ4_NL> {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             const uint32_t at = row + 18 * (4 * kh + 2 * CH + g);
-            d[2 * CH + g] = half_bits_to_float(lds16(at)) * (1.0f / kTc24);
+            d[2 * CH + g] = half_bits_to_float(lds16(at)) * tc_piece_unit(kIQ4_NL);
             uint32_t q[4];
             tc_words_at<4>(at + 2, q);
 #pragma unroll
@@ -342,7 +344,7 @@ struct TcUnit<kIQ4_XS> {
     template <bool O>
     __device__ __forceinline__ void begin(uint32_t line, uint32_t, int kh) {
         const unsigned long long h = lds64(line);
-        d = half_bits_to_float(static_cast<uint32_t>(h) & 0xFFFFu) * (1.0f / kTc24);
+        d = half_bits_to_float(static_cast<uint32_t>(h) & 0xFFFFu) * tc_piece_unit(kIQ4_XS);
         sl = static_cast<uint32_t>(h >> 32) >> (16 * kh);
         sh6 = static_cast<uint32_t>(h) >> (16 + 8 * kh);
     }

@@ -26,68 +26,76 @@ __device__ __forceinline__ void tc_columns(int l, int &a, int &b) {
     }
 }
 
-// The B operand of bytes.  x = X * 2^-k, X a 32-bit integer, rounded (signed bytes: 31 bits), k from the chunk's largest magnitude
-// (biased exponent `big`): what is lost is below 2^-31 of it, 2^-27.8 of the chunk's 2-norm at most, where fp32 sums lose 2^-24.
-// Unsigned bytes: the planes are the four bytes of X + 2^31, most significant first; one row of ones behind them gives the sums of A that
-// the 2^31 (and A's own offset) are taken out with.  Signed bytes: the planes are X's digits, -128 .. 127.  Sums of products are integers
-// and exact.
-//   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(24 - k); unsigned bytes, then: the integers
-//   -offset * sum of X's upper 16 bits (signed), and of its lower ones.
+// The B operand of bytes: six planes.  x = 2^(e - 126 - T) (p0 + 2^-15 p1 + 2^-30 p2), e the biased exponent of the largest magnitude of the
+// chunk (`big`), the pieces integers, p0 of at most 2^T (T = tc_piece_bits: 14 or 11), p1 and p2 of at most 2^14: each the rest of the one
+// before it, rounded to nearest.  An activation down to 2^-(T + 6) of the largest loses nothing, a smaller one at most 2^-(T + 30) of the
+// largest.  (Four planes of one 32-bit integer, 2^-31 of the largest: an output row whose weight is zero at an activation of 10^5 times the
+// rest was off by 2e-5 of its own products, now by 1e-7, as with three planes of fp16.)
+// Planes 2 q and 2 q + 1 are the upper and the lower byte of p_q: unsigned ones of p_q + 2^15, and one row of ones behind them gives the sum
+// of A that 2^15 is taken out with; signed ones its digits, -128 .. 127.  Sums of products are integers and exact.
+//   v: the lane's 2 x 4 columns (tc_columns), half a core row.  info: [rows] factors 2^(e - 127); with an offset of A's bytes, then: the
+//   three integers -offset * sum of p_q.
 template <int TYPE, int MC, bool ONES>
 __device__ __forceinline__ void tc_convert_bytes(float (&v)[8], uint32_t big, int t, uint32_t b_stage, uint32_t info, int lane) {
     constexpr bool kSigned = !tc_scaled_bytes(TYPE);
-    constexpr uint32_t kBits = kSigned ? 30u : 31u;
-    const uint32_t e = big > 7u ? big : 7u;  // (the unit of X is 2^-149 then, or less: no fp32 number's is smaller)
-    // X = v * 2^(126 + kBits - e), in two factors where the power is beyond fp32
-    const float up = __uint_as_float((e < kBits - 1u ? 254u : 253u + kBits - e) << 23), up2 = __uint_as_float((e < kBits - 1u ? 126u + kBits - e : 127u) << 23);
-    if (e < kBits - 1u) {
+    constexpr unsigned kOffset = tc_byte_offset(TYPE);
+    const uint32_t e = big > 1u ? big : 1u;
+    // 2^(126 + T - e), in two factors where the power is beyond fp32
+    constexpr uint32_t kTop = tc_piece_bits(TYPE);
+    const float up = __uint_as_float((e < kTop - 1u ? 254u : 253u + kTop - e) << 23);
+    if (e < kTop - 1u) {
+        const float up2 = __uint_as_float((126u + kTop - e) << 23);
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] *= up2;
     }
     constexpr int order[2][8] = {{0, 1, 2, 3, 4, 5, 6, 7}, {0, 4, 1, 5, 2, 6, 3, 7}};  // (IQ4: low and high nibbles in turn)
-    uint32_t x[8];
+    constexpr int kOrder = tc_order(TYPE) == kOrderBytes ? 1 : 0;
+    // added to a number below 2^15, this leaves its nearest integer in the low bits, and what is added to a piece for its bytes' sake
+    constexpr float kRound = 12582912.0f + (kSigned ? 128.0f : 32768.0f);
+    const f32x2 round = pack2(kRound, kRound), minus = pack2(-1.0f, -1.0f), next = pack2(32768.0f, 32768.0f), up_2 = pack2(up, up);
+    const uint32_t at = b_stage + (lane >> 1) * kTcCore + (lane & 1) * 8;
+    f32x2 r[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        x[i] = static_cast<uint32_t>(__float2int_rn(v[order[tc_order(TYPE) == kOrderBytes][i]] * up));
-        if constexpr (kSigned) x[i] += 0x00808080u;
-    }
-    uint32_t plane[4][2];
+    for (int i = 0; i < 4; ++i) r[i] = mul2(pack2(v[order[kOrder][2 * i]], v[order[kOrder][2 * i + 1]]), up_2);
 #pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        const uint32_t *c = x + 4 * w;
-        const uint32_t l01 = __byte_perm(c[0], c[1], 0x5140), l23 = __byte_perm(c[2], c[3], 0x5140);
-        const uint32_t h01 = __byte_perm(c[0], c[1], 0x7362), h23 = __byte_perm(c[2], c[3], 0x7362);
-        plane[0][w] = __byte_perm(h01, h23, 0x7632), plane[1][w] = __byte_perm(h01, h23, 0x5410);
-        plane[2][w] = __byte_perm(l01, l23, 0x7632), plane[3][w] = __byte_perm(l01, l23, 0x5410);
+    for (int q = 0; q < 3; ++q) {
+        uint32_t x[8], plane[2][2];
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-            if (kSigned ? p > 0 : p == 0) plane[p][w] ^= 0x80808080u;
-    }
-    constexpr unsigned kOffset = tc_byte_offset(TYPE);
-    unsigned hi = 0, lo = 0;  // sums of the upper halves of X + 2^31, and of the lower ones
-    if constexpr (kOffset != 0) {
-        unsigned sum[4];
+        for (int i = 0; i < 4; ++i) {
+            const f32x2 n = add2(r[i], round);
+            if (q < 2) r[i] = mul2(add2(r[i], fma2(n, minus, round)), next);  // the rest, exactly
+            float lo, hi;
+            unpack2(n, lo, hi);
+            x[2 * i] = __float_as_uint(lo), x[2 * i + 1] = __float_as_uint(hi);
+        }
 #pragma unroll
-        for (int p = 0; p < 4; ++p) sum[p] = __dp4a(plane[p][0], 0x01010101u, __dp4a(plane[p][1], 0x01010101u, 0u));
-        hi = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[0] + sum[1]), lo = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[2] + sum[3]);
-    }
-    if (lane == 0) {
-        // 2^(e - 102 - kBits); an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
-        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float((e + 25u - kBits) << 23);
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
+        for (int w = 0; w < 2; ++w) {
+            const uint32_t *c = x + 4 * w;
+            const uint32_t c01 = __byte_perm(c[0], c[1], 0x5140), c23 = __byte_perm(c[2], c[3], 0x5140);
+            plane[0][w] = __byte_perm(c01, c23, 0x7632), plane[1][w] = __byte_perm(c01, c23, 0x5410);
+            if constexpr (kSigned) plane[1][w] ^= 0x80808080u;
+        }
         if constexpr (kOffset != 0) {
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (tc_info_rows(MC) + t) * 4), "r"(kOffset * (32768u * kTcStepCols - hi)) : "memory");
-            asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + (2 * tc_info_rows(MC) + t) * 4), "r"(0u - kOffset * lo) : "memory");
+            unsigned sum[2];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) sum[p] = __dp4a(plane[p][0], 0x01010101u, __dp4a(plane[p][1], 0x01010101u, 0u));
+            const unsigned all = __reduce_add_sync(0xFFFFFFFFu, 256u * sum[0] + sum[1]);  // of p_q + 2^15
+            if (lane == 0)
+                asm volatile("st.shared.u32 [%0], %1;" ::"r"(info + ((q + 1) * tc_info_rows(MC) + t) * 4), "r"(kOffset * (32768u * kTcStepCols - all)) : "memory");
+        }
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int n = (2 * q + p) * MC + t;
+            asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(plane[p][0]), "r"(plane[p][1]) : "memory");
         }
     }
-    const uint32_t at = b_stage + (lane >> 1) * kTcCore + (lane & 1) * 8;
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const int n = p * MC + t;
-        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(plane[p][0]), "r"(plane[p][1]) : "memory");
+    if (lane == 0) {
+        // an infinite or undefined activation makes the outputs undefined: they are worked out again (tc_plain_sum)
+        const float down = big == 255u ? __uint_as_float(0x7FC00000u) : __uint_as_float(e << 23);
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(info + t * 4), "f"(down) : "memory");
     }
     if (tc_ones_row(TYPE, MC) && ONES && t == 0) {
-        constexpr int n = 4 * MC;
+        constexpr int n = kTcPlanes * MC;
         asm volatile("st.shared.v2.u32 [%0], {%1, %1};" ::"r"(at + (n >> 3) * tc_group_b(TYPE) + (n & 7) * 16), "r"(0x01010101u) : "memory");
     }
 }
@@ -218,11 +226,11 @@ __device__ __forceinline__ void tc_convert(const MatvecArgs &args, TcColumns &c,
 
 // A unit is what a group of warps takes of a step: one or two halves of 128 columns.  Its chunks go to the tensor cores in
 // batches; tensor memory holds one batch of a group and its sums, 128 columns in all.  Types with a scale per 32 columns have a sum
-// per 32 columns: with N = 32 only one chunk's fit.
+// per 32 columns: from N = 32 on only one chunk's fit.
 // Scaled bytes: a unit is a whole step, of two chunks.
 __host__ __device__ constexpr int tc_halves(int type) { return tc_wide(type) && !tc_scaled_bytes(type) ? 2 : 1; }
 template <int TYPE, int MC>
-__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 4) || (tc_scaled_bytes(TYPE) && MC > 8) || MC > 16 ? 1 : 2; }
+__host__ __device__ constexpr int tc_batch_chunks() { return (tc_block32(TYPE) && MC > 2) || (tc_scaled_bytes(TYPE) && MC > 8) || MC > 16 ? 1 : 2; }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_half_batches() { return 2 * tc_parts(TYPE) / tc_batch_chunks<TYPE, MC>(); }
 // sums per row that a batch leaves
@@ -261,38 +269,49 @@ struct TcAcc {
     }
 };
 
-// The sums of bytes: with D_p the sums over plane p and S the sum of A,
-//   sum of weight * X = 2^16 (2^8 D_0 + D_1 - 2^15 S - offset * upper halves of X) + (2^8 D_2 + D_3 - offset * lower halves of X),
-// both brackets exact in 32 bits (modulo 2^32 on the way): |weight| <= 128 or 0 <= weight <= 180 over 256 columns.
+// Sums over the six planes of bytes, of the K activation rows from t0 on, at tensor-memory column d_at.  (MC = 1: beside them the sum of A
+// where a row of ones makes it, for there is room for it in the load.)
+template <int MC, int K>
+__device__ __forceinline__ void tc_load_planes(uint32_t d_at, int t0, uint32_t (&v)[kTcPlanes][K], uint32_t &ones) {
+    if constexpr (MC == 1) {
+        uint32_t w[8];
+        tc::ld8(d_at, w);
+#pragma unroll
+        for (int i = 0; i < kTcPlanes; ++i) v[i][0] = w[i];
+        ones = w[kTcPlanes];
+    } else if constexpr (MC == 2) {
+        uint32_t w[16];
+        tc::ld8(d_at, w);
+        tc::ld8(d_at + 8, w + 8);
+#pragma unroll
+        for (int i = 0; i < 2 * kTcPlanes; ++i) v[i >> 1][i & 1] = w[i];
+        ones = w[2 * kTcPlanes];
+    } else {
+        static_assert(K == 4, "four activation rows");
+#pragma unroll
+        for (int i = 0; i < kTcPlanes; ++i) tc::ld4(d_at + i * MC + t0, v[i]);
+    }
+}
+// The sum over a piece (exact) and 2^-15 of the sum over the next.
+__device__ __forceinline__ float tc_join(uint32_t sum, uint32_t next) {
+    return fmaf(static_cast<float>(static_cast<int>(next)), 0x1p-15f, static_cast<float>(static_cast<int>(sum)));
+}
+
+// The sums of scaled bytes: with D_p the sums over plane p and S the sum of A,
+//   sum of weight * p_q = 2^8 D_2q + D_2q+1 - 2^15 S - offset * sum of p_q,
+// exact in 32 bits (modulo 2^32 on the way): |weight| <= 128 or 0 <= weight <= 180, |p_q| <= 2^14, 256 columns.
 template <int TYPE, int MC>
 __device__ __forceinline__ void tc_accumulate_bytes(const TcPending<TYPE, MC> &p, uint32_t d_at, TcAcc<MC> &acc) {
     static_assert(tc_sums<TYPE, MC>() == 1, "one sum per unit");
-    constexpr int kStep = MC > 8 ? 8 : MC, kMins = tc_mins(TYPE);  // activation rows at a time, for the registers' sake
+    constexpr int kStep = MC > 4 ? 4 : MC, kMins = tc_mins(TYPE);  // activation rows at a time, for the registers' sake
     uint32_t ones = p.ones;
-    if constexpr (tc_ones_row(TYPE, MC)) tc::ld1(d_at + 4 * MC, ones);
+    if constexpr (tc_ones_row(TYPE, MC) && MC > 2) tc::ld1(d_at + kTcPlanes * MC, ones);
 #pragma unroll
     for (int t0 = 0; t0 < MC; t0 += kStep) {
-        uint32_t v[4][kStep < 4 ? 4 : kStep];
-        if constexpr (MC == 1) {
-            uint32_t w[4];
-            tc::ld4(d_at, w);
+        uint32_t v[kTcPlanes][kStep], c[4][kStep];  // c: factors, -offset * sums of the pieces
+        tc_load_planes<MC, kStep>(d_at, t0, v, ones);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) v[i][0] = w[i];
-        } else if constexpr (MC == 2) {
-            uint32_t w[8];
-            tc::ld8(d_at, w);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v[i >> 1][i & 1] = w[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if constexpr (MC == 4) tc::ld4(d_at + i * MC, v[i]);
-                else tc::ld8(d_at + i * MC + t0, v[i]);
-            }
-        }
-        uint32_t c[3][kStep < 4 ? 4 : kStep];  // factors, sums of the upper and of the lower halves
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
+        for (int i = 0; i < 4; ++i) {
             if (i > 0 && tc_byte_offset(TYPE) == 0) {
 #pragma unroll
                 for (int t = 0; t < kStep; ++t) c[i][t] = 0u;
@@ -302,18 +321,16 @@ __device__ __forceinline__ void tc_accumulate_bytes(const TcPending<TYPE, MC> &p
                 const unsigned long long w = lds64(p.info + i * tc_info_rows(MC) * 4);
                 c[i][0] = static_cast<uint32_t>(w), c[i][1] = static_cast<uint32_t>(w >> 32);
             } else {
-#pragma unroll
-                for (int t = 0; t < kStep; t += 4) {
-                    const uint4 w = lds128u(p.info + (i * tc_info_rows(MC) + t0 + t) * 4);
-                    c[i][t] = w.x, c[i][t + 1] = w.y, c[i][t + 2] = w.z, c[i][t + 3] = w.w;
-                }
+                const uint4 w = lds128u(p.info + (i * tc_info_rows(MC) + t0) * 4);
+                c[i][0] = w.x, c[i][1] = w.y, c[i][2] = w.z, c[i][3] = w.w;
             }
         }
         tc::wait_ld();
         auto value = [&](int t) {
-            const uint32_t hi = v[0][t] * 256u + v[1][t] + (c[1][t] - 32768u * ones), lo = v[2][t] * 256u + v[3][t] + c[2][t];
-            // (with an offset the lower sums are signed)
-            return fmaf(static_cast<float>(static_cast<int>(hi)), 65536.0f, tc_byte_offset(TYPE) != 0 ? static_cast<float>(static_cast<int>(lo)) : static_cast<float>(lo));
+            uint32_t s[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) s[q] = v[2 * q][t] * 256u + v[2 * q + 1][t] + (c[1 + q][t] - 32768u * ones);
+            return fmaf(tc_join(s[1], s[2]), 0x1p-15f, static_cast<float>(static_cast<int>(s[0])));
         };
         if constexpr (MC == 1) {
             float a, b;
@@ -458,109 +475,83 @@ __device__ __forceinline__ void tc_accumulate_halves(const TcPending<TYPE, MC> &
     }
 }
 
-// Integer sums of a unit over the planes and activation rows, for types with integer scales.
+// Sums of a unit over its groups of 32 columns, for types with integer scales: scale * sum of weight * p0, exactly (127 * 2^11 * 32 columns
+// times 32, times 8 groups: below 2^31), and of the rest.
 template <int TYPE, int MC>
 struct TcUnitSums {
-    int v[tc_integer_scale(TYPE) ? 4 * MC : 1];
+    int top[tc_integer_scale(TYPE) ? MC : 1];
+    float rest[tc_integer_scale(TYPE) ? MC : 1];
     __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int &x : v) x = 0;
+        for (int &x : top) x = 0;
+#pragma unroll
+        for (float &x : rest) x = 0.0f;
     }
 };
-// The sums of signed bytes, one per 32 columns: with D_p the sums over plane p, scale * (2^24 D_0 + 2^16 D_1 + 2^8 D_2 + D_3).  Exact
-// up to the unit's end with an integer scale (|D_p| <= 2^19, times 32, times 8 groups), up to its own with an fp16 one.
+// The sums of signed bytes, one per 32 columns: with D_p the sums over plane p, sum of weight * p_q = 2^8 D_2q + D_2q+1, at most 2^26.
 //   last: these are a unit's last sums
 template <int TYPE, int MC>
 __device__ __forceinline__ void tc_accumulate_blocks(const TcPending<TYPE, MC> &p, uint32_t d_at, bool last, TcUnitSums<TYPE, MC> &unit, TcAcc<MC> &acc) {
     constexpr int kSums = tc_sums<TYPE, MC>(), kN = TcShape<TYPE, MC>::kN;
-    f32x2 inv[(MC + 1) / 2];
-    if (!tc_integer_scale(TYPE) || last) {
-        if constexpr (MC == 1) {
-            inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
-        } else if constexpr (MC == 2) {
-            inv[0] = lds64(p.info);
-        } else {
+    constexpr int kStep = MC > 4 ? 4 : MC, kAtOnce = MC == 1 ? kSums : MC == 2 && !tc_integer_scale(TYPE) ? 2 : 1;  // rows and sums at a time (registers)
 #pragma unroll
-            for (int t = 0; t < MC; t += 4) {
-                const ulonglong2 w = lds128(p.info + t * 4);
-                inv[t / 2] = w.x, inv[t / 2 + 1] = w.y;
+    for (int t0 = 0; t0 < MC; t0 += kStep) {
+        f32x2 inv[(kStep + 1) / 2];
+        if (!tc_integer_scale(TYPE) || last) {
+            if constexpr (MC == 1) {
+                inv[0] = pack2(__uint_as_float(lds32(p.info)), 0.0f);
+            } else if constexpr (MC == 2) {
+                inv[0] = lds64(p.info);
+            } else {
+                const ulonglong2 w = lds128(p.info + t0 * 4);
+                inv[0] = w.x, inv[1] = w.y;
             }
         }
-    }
-    auto add = [&](float s, const float (&u)[MC]) {
-        if constexpr (MC == 1) {
-            float a, b, k, unused;
-            unpack2(acc.v[0], a, b);
-            unpack2(inv[0], k, unused);
-            acc.v[0] = pack2(fmaf(u[0] * s, k, a), b);
-        } else {
-            const f32x2 s2 = pack2(s, s);
+        auto add = [&](float s, const float (&u)[kStep]) {
+            if constexpr (MC == 1) {
+                float a, b, k, none;
+                unpack2(acc.v[0], a, b);
+                unpack2(inv[0], k, none);
+                acc.v[0] = pack2(fmaf(u[0] * s, k, a), b);
+            } else {
 #pragma unroll
-            for (int t = 0; t < MC; t += 2) acc.v[t / 2] = fma2(mul2(pack2(u[t], u[t + 1]), s2), inv[t / 2], acc.v[t / 2]);
-        }
-    };
-    if constexpr (tc_integer_scale(TYPE)) {
-        constexpr int kPiece = MC > 4 ? 16 : 4 * MC, kAtOnce = MC > 4 ? 1 : kSums;  // (registers)
+                for (int t = 0; t < kStep; t += 2)
+                    acc.v[(t0 + t) / 2] = fma2(mul2(pack2(u[t], u[t + 1]), pack2(s, s)), inv[t / 2], acc.v[(t0 + t) / 2]);
+            }
+        };
 #pragma unroll
         for (int g0 = 0; g0 < kSums; g0 += kAtOnce) {
+            uint32_t v[kAtOnce][kTcPlanes][kStep], unused;
 #pragma unroll
-            for (int i0 = 0; i0 < 4 * MC; i0 += kPiece) {
-                uint32_t v[kAtOnce][kPiece];
-#pragma unroll
-                for (int g = 0; g < kAtOnce; ++g) {
-                    if constexpr (MC == 1) {
-                        tc::ld4(d_at + (g0 + g) * kN, v[g]);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < kPiece; i += 8) tc::ld8(d_at + (g0 + g) * kN + i0 + i, v[g] + i);
-                    }
-                }
-                tc::wait_ld();
-#pragma unroll
-                for (int g = 0; g < kAtOnce; ++g) {
-                    const int k = __float_as_int(p.s[g0 + g]);
-#pragma unroll
-                    for (int i = 0; i < kPiece; ++i) unit.v[i0 + i] += k * static_cast<int>(v[g][i]);
-                }
-            }
-        }
-    } else {
-        constexpr int kAtOnce = MC > 4 ? 1 : kSums;  // (registers)
-#pragma unroll
-        for (int g0 = 0; g0 < kSums; g0 += kAtOnce) {
-            uint32_t v[kAtOnce][4 * MC];
-#pragma unroll
-            for (int g = 0; g < kAtOnce; ++g) {
-                if constexpr (MC == 1) {
-                    tc::ld4(d_at + (g0 + g) * kN, v[g]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4 * MC; i += 8) tc::ld8(d_at + (g0 + g) * kN + i, v[g] + i);
-                }
-            }
+            for (int g = 0; g < kAtOnce; ++g) tc_load_planes<MC, kStep>(d_at + (g0 + g) * kN, t0, v[g], unused);
             tc::wait_ld();
 #pragma unroll
             for (int g = 0; g < kAtOnce; ++g) {
-                float u[MC];
+                float u[kStep];
 #pragma unroll
-                for (int t = 0; t < MC; ++t)
-                    u[t] = fmaf(static_cast<float>(static_cast<int>(v[g][t] * 256u + v[g][MC + t])), 65536.0f,
-                                static_cast<float>(static_cast<int>(v[g][2 * MC + t] * 256u + v[g][3 * MC + t])));
-                add(p.s[g0 + g], u);
+                for (int t = 0; t < kStep; ++t) {
+                    const uint32_t p0 = v[g][0][t] * 256u + v[g][1][t], p1 = v[g][2][t] * 256u + v[g][3][t], p2 = v[g][4][t] * 256u + v[g][5][t];
+                    if constexpr (tc_integer_scale(TYPE)) {
+                        const int k = __float_as_int(p.s[g0 + g]);
+                        unit.top[t0 + t] += k * static_cast<int>(p0);
+                        unit.rest[t0 + t] = fmaf(tc_join(p1, p2), static_cast<float>(k), unit.rest[t0 + t]);
+                    } else {
+                        u[t] = fmaf(tc_join(p1, p2), 0x1p-15f, static_cast<float>(static_cast<int>(p0)));
+                    }
+                }
+                if constexpr (!tc_integer_scale(TYPE)) add(p.s[g0 + g], u);
             }
         }
-    }
-    if (tc_integer_scale(TYPE) && last) {
         if constexpr (tc_integer_scale(TYPE)) {
-            float u[MC];
+            if (last) {
+                float u[kStep];
 #pragma unroll
-            for (int t = 0; t < MC; ++t) {
-                u[t] = static_cast<float>(unit.v[t]);
-#pragma unroll
-                for (int i = 1; i < 4; ++i) u[t] = fmaf(u[t], 256.0f, static_cast<float>(unit.v[i * MC + t]));
+                for (int t = 0; t < kStep; ++t) {
+                    u[t] = fmaf(unit.rest[t0 + t], 0x1p-15f, static_cast<float>(unit.top[t0 + t]));
+                    unit.rest[t0 + t] = 0.0f, unit.top[t0 + t] = 0;
+                }
+                add(p.d, u);
             }
-            add(p.d, u);
-            unit.clear();
         }
     }
 }
