@@ -265,6 +265,36 @@ def test_the_first_pass_of_sixteen_rows_may_be_captured(codebooks, extra):
             runtime.close()
 
 
+def test_the_room_for_wide_passes_is_allocated_once_and_not_for_prompts(codebooks):
+    import torch
+    from vinf_3080ti_b200.runtime import Runtime
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    shapes = [(T.Q4_K, 2305, 2304), (T.Q4_K, 1025, 17408), (T.Q6_K, 1025, 24576)]
+    weights = [torch.zeros(rows * (cols // 256) * TRAITS[t][1] + 256, dtype=torch.uint8, device="cuda") for t, rows, cols in shapes]
+    x = torch.zeros(512 * 2304, device="cuda")
+    runtime = Runtime(codebooks["iq3s_grid"], codebooks)
+    try:
+        runtime.bind_tensor("w0", weights[0].data_ptr(), int(T.Q4_K), 2304, 2305)
+        before = free()
+        runtime.bind("prompt", x.data_ptr(), 512 * 2304)
+        runtime.set_gemm_min_rows(64)
+        runtime.bind("more", x.data_ptr(), 64 * 2304)
+        assert free() == before
+        runtime.bind("x", x.data_ptr(), 24 * 2304)
+        made = free()
+        assert made < before
+        for i, (t, rows, cols) in enumerate(shapes):
+            runtime.bind_tensor(f"w{i}", weights[i].data_ptr(), int(t), cols, rows)
+        runtime.set_gemm_min_rows(0)
+        assert free() == made
+    finally:
+        runtime.close()
+
+
 @pytest.mark.parametrize("t", TYPES, ids=lambda t: t.name)
 def test_infinite_and_undefined_activations(rt, codebooks, t):
     """An output is infinite or undefined exactly where weight times activation makes it so, as on the CUDA cores; the other

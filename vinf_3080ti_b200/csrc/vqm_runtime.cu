@@ -103,7 +103,7 @@ struct vqm_runtime {
     size_t x_split_bytes = 0;
     size_t split_need = 0;                      // what the widest tensor so far needs of it
     std::unordered_set<size_t> split_cols;      // columns of the tensors that use it
-    bool wide_seen = false;                     // a buffer holds more than 8 rows of so many columns
+    bool wide_seen = false;                     // a buffer holds more than 8 rows of so many columns, but no prompt
     // x_split serves one stream at a time: split_event follows its last use on the stream before (see claim_split)
     bool split_used = false, split_wait = false;
     cudaStream_t split_stream = nullptr;
@@ -436,9 +436,10 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
 // pass that finds the room missing may be one that is being captured, by this runtime or by another library.
 bool make_split_room(vqm_runtime *rt) {
     if (rt->split_need <= rt->x_split_bytes) return true;
-    // At most 42 KB per 256 columns; 2 MB hold 12288 columns of any type.  (3 MB at once, enough for 18432: a new runtime's first buffers take 0.3 to
-    // 0.6 ms longer, more than the second allocation that wider tensors ask for.)
-    size_t bytes = rt->split_need < (2u << 20) ? 2u << 20 : rt->split_need;
+    // At most 42 KB per 256 columns; 4 MB hold 24576 columns of any type, so that a runtime allocates once.  (cudaMalloc takes 330 us for
+    // any size from 1 to 16 MB; with 2 MB, which tensors of more than 12288 columns outgrow, to bind three tensors and their buffers of 24 rows
+    // took 1720 us instead of 1480.)
+    size_t bytes = rt->split_need < (4u << 20) ? 4u << 20 : rt->split_need;
     if (bytes < rt->x_split_bytes + rt->x_split_bytes / 2) bytes = rt->x_split_bytes + rt->x_split_bytes / 2;
     uint8_t *p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -464,14 +465,18 @@ bool takes_wide(vqm_runtime *rt, const Tensor &t) {
     return use_tcmv(t.type, a, rt->sm_count, codebook_fits(rt, t.type)) && make_split_room(rt);
 }
 
+// (Buffers for prompt passes, which the GEMM takes, say nothing about wide passes of the matvec.  A program that has not turned prompt mode
+// on may do so once its buffers are there: until then 64 rows, the threshold that the reference's executor sets, count as a prompt.  Three
+// tensors and their buffers of 512 rows: 2020 us to bind with room for wide passes, 1380 without.)
 void see_buffer(vqm_runtime *rt, const Buffer &b) {
+    const size_t prompt = rt->gemm_min_rows > 0 ? static_cast<size_t>(rt->gemm_min_rows) : 64;
     if (b.elem == 4)
-        for (const size_t cols : rt->split_cols) rt->wide_seen |= b.n % cols == 0 && b.n / cols > 8;
+        for (const size_t cols : rt->split_cols) rt->wide_seen |= b.n % cols == 0 && b.n / cols > 8 && b.n / cols < prompt;
 }
 
 // What the passes of a new tensor or buffer will need is made here, so that the first of them does not pay for it: the maps of a
-// tensor of the tensor-core matvec, and, once there is a buffer that holds more than 8 rows of some such tensor's activations, the
-// room for their B operands.  (That allocation takes 0.4 ms, which programs without such passes need not pay.)  Where
+// tensor of the tensor-core matvec, and, once there is a buffer that holds more than 8 rows of some such tensor's activations, but no prompt,
+// the room for their B operands.  (That allocation takes 0.33 ms, which programs without such passes need not pay.)  Where
 // something fails the launches make up for it, and passes of more than 8 rows run 8 at a time.
 // First pass of 24 rows over three tensors in a new runtime: 530 us without this, 155 with it (later ones alone: 154).
 void prepare_tensor(vqm_runtime *rt, Tensor &t) {
@@ -1273,6 +1278,7 @@ int vqm_dequantize(vqm_runtime *rt, const char *weight, const char *out) {
 int vqm_set_gemm_min_rows(vqm_runtime *rt, int n) {
     if (n < 0) return fail(VQM_ERR_VALUE, "gemm_min_rows must be >= 0");
     rt->gemm_min_rows = n;
+    for (const auto &kv : rt->buffers) prepare_buffer(rt, kv.second);
     return VQM_OK;
 }
 
