@@ -76,8 +76,8 @@ def test_tiles_steps_and_splits_of_every_type(rt, codebooks, t, shapes, cols):
 @pytest.mark.parametrize("m", [1, 2, 4, 8, 16])
 @pytest.mark.parametrize("t", [T.Q3_K, T.Q2_K, T.Q8_0, T.IQ4_NL, T.IQ4_XS], ids=lambda t: t.name)
 def test_integer_sums_at_the_ends_of_their_range(rt, codebooks, t, m):
-    """Types whose products are summed as integers: the largest and smallest weights times activations at both ends of the
-    32-bit range they are rounded to, all of one sign, and activations at both ends of fp32's range."""
+    """Types whose products are summed as integers: the largest and smallest weights times activations whose integers are the largest
+    there are, all of one sign, and activations at both ends of fp32's range."""
     rows, cols = 2305, 2304
     block, size = TRAITS[t]
     raw = np.zeros((rows, cols // block, size), dtype=np.uint8)
@@ -94,6 +94,8 @@ def test_integer_sums_at_the_ends_of_their_range(rt, codebooks, t, m):
     x[5], x[6] = np.float32(2.0**100), np.float32(2.0**-95)
     x[7] = np.float32(2.0**-97) * np.arange(cols)
     x[8:] = x[:8][::-1]
+    bits = 11 if t is T.IQ4_XS else 14  # of the first integer: rounded up to 2^bits with a rest of -1/2, and to an even number with 1/2
+    x[8], x[15] = 2.0**bits - 0.5, 1.5 - 2.0**bits
     rt.upload("w", raw, int(t), cols, rows)
     for first in range(0, 16, m):
         (got,) = _run(rt, ["w"], ["y"], (rows,), x[first:first + m])
