@@ -84,3 +84,26 @@ def test_pycall_hands_its_arguments_on_as_ctypes_does(ntok, seen):
     with pytest.raises((TypeError, ValueError)):  # a closed runtime
         _capi.pycall().qmv(address, None, "w", "x", "y", 1)
     assert len(got) == 1
+
+
+def test_the_call_without_ctypes_is_optional(monkeypatch, tmp_path):
+    import sys
+
+    from vinf_3080ti_b200 import build
+
+    seen = []
+    monkeypatch.setattr(_capi, "load", lambda: type("Lib", (), {"vqm_qmv": staticmethod(lambda *a: seen.append(a) or 4)}))
+    monkeypatch.setitem(sys.modules, "vinf_3080ti_b200._vqm_pycall", None)  # as if this interpreter could not load it
+    monkeypatch.delattr("vinf_3080ti_b200._vqm_pycall", raising=False)
+    assert _capi.pycall() is None
+    call, address = _capi.qmv_caller()
+    assert call(address, 123, "w", "größe", "y", np.int64(7)) == 4
+    assert seen == [(123, b"w", "größe".encode(), b"y", 7)]
+    # a box without a C compiler gets the library all the same, and no stale module
+    stale = tmp_path / build.PYCALL.name
+    stale.write_bytes(b"")
+    monkeypatch.setattr(build, "PYCALL", stale)
+    monkeypatch.setattr(build, "up_to_date", lambda: True)
+    monkeypatch.setenv("PATH", str(tmp_path))
+    assert build.build_pycall(force=True) is None and not stale.exists()
+    assert build.build() == build.LIB

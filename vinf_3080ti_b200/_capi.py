@@ -87,20 +87,25 @@ _RESTYPES = {"vqm_last_error": c_char_p, "vqm_runtime_destroy": None, "vqm_strea
 _lib: ctypes.CDLL | None = None
 
 
-_pycall = None
-
-
 def pycall():
-    """The module that calls vqm_qmv without ctypes, loaded once."""
-    global _pycall
-    if _pycall is not None:
-        return _pycall
-    path = Path(__file__).resolve().parent / "_vqm_pycall.so"
-    if not path.exists():
-        raise ExtensionMissingError(f"{path} is not built; run `python -m vinf_3080ti_b200.build`")
-    from . import _vqm_pycall
-    _pycall = _vqm_pycall
-    return _pycall
+    """The module that calls vqm_qmv without ctypes; None where it was not built or this interpreter cannot load it."""
+    try:
+        from . import _vqm_pycall
+    except ImportError:
+        return None
+    return _vqm_pycall
+
+
+def qmv_caller():
+    """(call, address) such that call(address, handle, weight, x, y, ntok) is vqm_qmv on Python's str and int."""
+    fn, module = load().vqm_qmv, pycall()
+    if module is not None:
+        return module.qmv, ctypes.cast(fn, c_void_p).value
+
+    def call(_, handle, weight, x, y, ntok):
+        return fn(handle, weight.encode("utf-8"), x.encode("utf-8"), y.encode("utf-8"), int(ntok))
+
+    return call, None
 
 
 def load() -> ctypes.CDLL:

@@ -9,7 +9,8 @@ results are wrong on purpose.
 Such a build goes to --out (objects beside it) and is loaded with VINF_B200_LIB=<path>.
 
 Two translation units per GGUF type (the matvec kernel instantiations, plain and with the fused prologues) plus the small kernels and the
-runtime; objects go to csrc/build/, the library next to this file, and beside it _vqm_pycall.so (gcc).  Cross-compiles without a GPU.
+runtime; objects go to csrc/build/, the library next to this file.  Cross-compiles without a GPU.  Then, where gcc and Python's headers
+are there, _vqm_pycall.abi3.so beside the library: a faster way into it, which the package does without otherwise.
 """
 from __future__ import annotations
 
@@ -26,7 +27,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = CSRC / "build"
 LIB = HERE / "libvinf_b200.so"
-PYCALL = HERE / "_vqm_pycall.so"  # vqm_qmv for Python without ctypes
+PYCALL = HERE / "_vqm_pycall.abi3.so"  # vqm_qmv for Python without ctypes
 
 TYPES = [(0, "F32"), (1, "F16"), (8, "Q8_0"), (10, "Q2_K"), (11, "Q3_K"), (12, "Q4_K"), (13, "Q5_K"), (14, "Q6_K"),
          (16, "IQ2_XXS"), (17, "IQ2_XS"), (18, "IQ3_XXS"), (20, "IQ4_NL"), (21, "IQ3_S"), (22, "IQ2_S"), (23, "IQ4_XS")]
@@ -49,13 +50,20 @@ def _sources() -> list[Path]:
                   [HERE.parent / "include" / "vinf_b200.h"])
 
 
-def build_pycall() -> Path:
+def build_pycall(force: bool = False) -> Path | None:
+    """Optional: None, with a line on stderr, where it cannot be built."""
     src = CSRC / "vqm_pycall.c"
-    if not PYCALL.exists() or src.stat().st_mtime > PYCALL.stat().st_mtime:
+    if force or not PYCALL.exists() or src.stat().st_mtime > PYCALL.stat().st_mtime:
+        PYCALL.unlink(missing_ok=True)
         cmd = ["gcc", "-O2", "-shared", "-fPIC", "-Wall", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(PYCALL)]
-        done = subprocess.run(cmd, capture_output=True, text=True)
-        if done.returncode != 0:
-            raise RuntimeError(f"gcc failed for {src.name}:\n{done.stdout}\n{done.stderr}")
+        try:
+            done = subprocess.run(cmd, capture_output=True, text=True)
+            failure = done.stderr.strip() if done.returncode != 0 else None
+        except OSError as e:
+            failure = str(e)
+        if failure is not None:
+            print(f"{PYCALL.name} is not built, calls go through ctypes: {failure}", file=sys.stderr)
+            return None
     return PYCALL
 
 
@@ -84,7 +92,6 @@ def _compile(job: tuple[str, list[str], Path]) -> tuple[str, str]:
 
 def build(force: bool = False, jobs: int | None = None, verbose: bool = False, defines: list[str] | None = None, out: Path | None = None) -> Path:
     global OBJ, LIB
-    build_pycall()
     if defines or out:
         if out is None:
             raise ValueError("an experimental build (--define) needs --out, it must not replace the library")
@@ -92,6 +99,8 @@ def build(force: bool = False, jobs: int | None = None, verbose: bool = False, d
         OBJ = LIB.parent / (LIB.stem + "_obj")
         EXTRA_DEFINES[:] = [f"-D{d}" for d in (defines or [])]
         force = True
+    else:
+        build_pycall(force)
     if not force and up_to_date():
         return LIB
     OBJ.mkdir(parents=True, exist_ok=True)

@@ -67,7 +67,7 @@ class Runtime:
 
     def __init__(self, iq3s_grid: bytes | None = None, codebooks: dict[str, bytes] | None = None) -> None:
         self._lib = _capi.load()
-        self._qmv, self._qmv_fn = _capi.pycall().qmv, ctypes.cast(self._lib.vqm_qmv, ctypes.c_void_p).value
+        self._qmv, self._qmv_fn = _capi.qmv_caller()
         self._h = ctypes.c_void_p()
         if iq3s_grid is not None and len(iq3s_grid) != 2048:
             raise ValueError("iq3s_grid must be 2048 bytes (512 entries x 4 values)")
