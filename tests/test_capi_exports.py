@@ -107,3 +107,19 @@ def test_the_call_without_ctypes_is_optional(monkeypatch, tmp_path):
     monkeypatch.setenv("PATH", str(tmp_path))
     assert build.build_pycall(force=True) is None and not stale.exists()
     assert build.build() == build.LIB
+
+
+@pytest.mark.parametrize("call", ["qmv('w', 'x', 'y')", "matvec('w', bytes(4))", "has('w')", "qmv_argmax('w', 'x', None)", "argmax('x', 1)",
+                                  "write('x', bytes(4))", "synchronize()", "stream()", "capture_begin()", "graph_launch(0)",
+                                  "exchange_create(8)", "qmv_group(['w'], 'x', ['y'], 1)"])
+def test_calls_on_a_closed_runtime_are_errors(call):
+    from vinf_3080ti_b200.runtime import Runtime
+
+    rt = Runtime.__new__(Runtime)  # (a real one needs a GPU)
+    rt._lib = _capi.load()
+    rt._qmv, rt._qmv_fn = _capi.qmv_caller()
+    rt._h = ctypes.c_void_p()
+    rt.close()
+    rt.close()
+    with pytest.raises(ValueError, match="closed"):
+        eval(f"rt.{call}", {"rt": rt})

@@ -78,9 +78,15 @@ class Runtime:
                 self.set_codebook(name, data)
 
     def close(self) -> None:
-        if getattr(self, "_h", None) is not None and self._h.value:
-            self._lib.vqm_runtime_destroy(self._h)
-            self._h = ctypes.c_void_p()
+        """Gives everything back; every later call but this one is a ValueError."""
+        handle = self.__dict__.pop("_h", None)
+        if handle is not None and handle.value:
+            self._lib.vqm_runtime_destroy(handle)
+
+    def __getattr__(self, name: str):  # (looked up only for what is not there: costs the calls of an open runtime nothing)
+        if name == "_h":
+            raise ValueError("the runtime is closed")
+        raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
 
     def __del__(self) -> None:  # tp_dealloc: engine/csrc/megakernel/qwen_runtime.cu:1299-1336
         try:
