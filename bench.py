@@ -48,7 +48,7 @@ from vinf_3080ti_b200.synth import IQ_SWEEP, LAYER_SET, LM_HEAD, N_LAYERS, synth
 
 METRIC = "quant-matvec weight GB/s, synthetic-27B decode pass"
 # DRAM bytes (read + write) of one launch of the dominant kernel (tcmv_kernel, Q3_K 17408 x 5120, M = 4) from an ncu capture
-NCU_TRAFFIC_BYTES_PER_LAUNCH = 38455040
+NCU_TRAFFIC_BYTES_PER_LAUNCH = 38449152
 SM_COUNT, SM_LANES, SM_MAX_HZ = 148, 128, 1.965e9
 
 

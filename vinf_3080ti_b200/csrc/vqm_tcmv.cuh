@@ -1,4 +1,4 @@
-// Quantized matvec for 1..16 activation rows on the 5th-generation tensor cores:  y[t][r] = sum_k W[r][k] x[t][k].
+// Quantized matvec for 1..24 activation rows on the 5th-generation tensor cores:  y[t][r] = sum_k W[r][k] x[t][k].
 //
 // Same contract as the CUDA-core kernel (vqm_matvec.cuh): raw GGUF blocks read once for all activation rows, inputs and
 // sums of fp32 precision.  What bounds that kernel is instruction issue - a permute, half a packed FMA and half a packed
@@ -68,8 +68,6 @@ __host__ __device__ constexpr int tc_pitch(int type) {
 __host__ __device__ constexpr bool tc_word_loads(int type) { return block_align(type) < 8 && type != kQ6_K; }
 // A columns per weight: 2 where quant times sub-scale needs more than 11 bits and is split in two
 __host__ __device__ constexpr int tc_parts(int type) { return type == kQ6_K ? 2 : 1; }
-// types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit; with an integer scale the sums
-// stay integers until the super-scale
 // types that look up four signed weights at a time (see TcSigned)
 __host__ __device__ constexpr bool tc_signed_table(int type) { return type == kIQ2_XXS || type == kIQ3_XXS || type == kIQ3_S; }
 // Copies of the signed table, word by word: 32 lanes that pick words at random from 32 banks take 3.5 turns, 16 from every other bank 3.1,
@@ -80,6 +78,8 @@ __host__ __device__ constexpr int tc_table_copies(int type, int mc) {
 __host__ __device__ constexpr int tc_table_bytes(int type, int mc) {
     return tc_signed_table(type) ? (type == kIQ3_XXS ? 16384 : 32768) * tc_table_copies(type, mc) : grid_bytes(type);
 }
+// types whose scale covers 32 weights and stays outside: a sum per 32 columns instead of one per unit; with an integer scale the sums
+// (of the larger part of the activations) stay integers until the super-scale
 __host__ __device__ constexpr bool tc_block32(int type) { return type == kQ8_0 || type == kIQ4_NL || type == kIQ4_XS; }
 __host__ __device__ constexpr bool tc_integer_scale(int type) { return type == kIQ4_XS; }
 __host__ __device__ constexpr int tc_groups(int type) { return type == kQ4_K || type == kQ5_K ? 8 : type == kQ2_K ? 16 : 0; }  // minimums per step

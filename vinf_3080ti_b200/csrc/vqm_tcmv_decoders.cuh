@@ -1,10 +1,12 @@
-// Row decoders of the tensor-core matvec (vqm_tcmv.cuh): raw words of one row -> fp16 A columns.
+// Row decoders of the tensor-core matvec (vqm_tcmv.cuh): raw words of one row -> A columns, fp16 or bytes.
 //
-// begin() reads the scales of half a step (128 columns; `kh` = which half), chunk<CH>() fills the 32 registers (64 fp16
-// values) of chunk CH of the half.  Registers come in core rows of 4 (8 columns); the columns behind them are tc_columns() of
-// the kernel's header.  Masked fields are fp16 subnormals, field * 2^-24 times the field's place value; the multipliers undo
-// the place value, so every A value is (quant - bias) * sub-scale * 2^-24, exactly (at most 11 significant bits).  scale() is
-// the fp16 super-scale times 2^24.
+// begin() reads the scales of a unit (half a step of 128 columns, `kh` = which half; scaled bytes: a whole step), chunk<CH>() fills the
+// registers of its chunk CH: 32 of 64 fp16 values, 32 of 128 scaled bytes or 16 of 64 signed bytes.  Registers come in core rows of 4
+// (8 fp16 columns; 16 bytes); the columns behind them are tc_columns() of the kernel's header.
+//   fp16: masked fields are subnormals, field * 2^-24 times the field's place value; the multipliers undo the place value, so every A
+//   value is (quant - bias) * sub-scale * 2^-24, exactly (at most 11 significant bits).  scale() is the fp16 super-scale times 2^24.
+//   bytes: an A value is an integer, see the second part of this file.  scale() is the super-scale (signed bytes: the scale of 32
+//   weights) times tc_piece_unit().
 // The comments give the instructions per 8 weights: integer ones go to a pipe that takes a warp instruction every 2 cycles,
 // and so does packed fp16 arithmetic, but the two run side by side (measured 1.3 cycles per instruction when mixed).
 #pragma once
@@ -143,7 +145,7 @@ struct TcUnit<kQ6_K> {
 // ---- bytes ---------------------------------------------------------------------------------------------------------------
 // Q3_K and Q2_K: quant times sub-scale fits into 8 bits, so an A column is a byte and ONE 32-bit multiply scales four weights: no
 // byte of the product carries into the next.  Half the registers and stores of fp16 and one integer instruction per four weights
-// less; a step is one batch.  Bound by unpacking as the others (warp instructions per 8 weights of Q3_K, 1 row: 31.5 as fp16, 21.2 so).
+// less; a step is one batch.  Bound by unpacking as the others (warp instructions per 8 weights of Q3_K, 1 row: 31.5 as fp16, 21.0 so).
 // 17408 x 5120, 1 / 4 / 8 / 16 rows, fp16 and bytes, us: Q3_K 19.8 / 20.9 / 23.0 / 26.6 and 15.3 / 17.3 / 20.4 / 27.0, Q2_K 15.2 / 16.8 /
 // 20.6 / 26.6 and 12.2 / 14.4 / 18.1 / 27.2.  Error against 64 bits, Q3_K: 1.5e-7 and 7e-8; with outliers of 1000 times the rest 1e-6 and 7e-8.
 // (Q4_K's products need 10 bits, Q6_K's 14: two and three bytes a weight.)

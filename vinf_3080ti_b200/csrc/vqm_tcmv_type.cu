@@ -111,15 +111,16 @@ inline bool takes_tail(const MatvecArgs &a) { return a.part[1].rows == 0 && (a.o
 // where the line lies depends on what else the GPU does.  Measured with 1 / 4 / 8 rows, CUDA-core and this one (us):
 //   launches that wait for one another, on one stream:
 //     Q4_K 1024 x 5120:   5.0 /  6.9 / 10.1  and   6.5 /  7.5 / 10.0      2048 x 5120:  6.6 / 10.3 / 16.1  and   6.7 /  7.7 / 10.2
-//     Q6_K 1024 x 5120:   5.3 /  7.5 / 11.2  and   8.6 /  9.0 / 10.6      2048 x 5120:  7.0 / 10.8 / 16.4  and   8.8 /  9.1 / 10.7
-//     Q3_K 1024 x 5120:   5.3 /  7.5 / 11.1  and   7.8 /  8.5 / 10.4      2048 x 5120:  6.9 / 10.6 / 16.2  and   8.0 /  8.6 / 10.5
-//     IQ3_S 1024 x 5120:  6.8 / 11.1 / 17.0  and  10.1 / 10.7 / 12.6      2048 x 5120:  9.8 / 17.7 / 29.1  and  10.4 / 10.9 / 12.8
-//     IQ4_XS 1024 x 5120: 5.4 /  7.0 / 10.1  and   8.2 /  9.6 / 13.1      2048 x 5120:  7.3 / 10.2 / 15.6  and   8.4 /  9.8 / 13.3
+//     Q6_K 1024 x 5120:   5.3 /  7.5 / 11.2  and   8.6 /  9.0 / 10.6      2048 x 5120:  6.9 / 10.8 / 16.4  and   8.8 /  9.1 / 10.6
+//     Q3_K 1024 x 5120:   5.3 /  7.5 / 11.1  and   7.8 /  8.7 / 10.7      2048 x 5120:  6.9 / 10.6 / 16.2  and   7.9 /  8.9 / 10.8
+//     IQ3_S 1024 x 5120:  6.8 / 11.1 / 17.0  and  10.1 / 10.6 / 12.6      2048 x 5120:  9.8 / 17.7 / 29.2  and  10.4 / 10.9 / 12.8
+//     IQ4_XS 1024 x 5120: 5.4 /  7.1 / 10.1  and   8.4 / 10.7 / 13.9      2048 x 5120:  7.3 / 10.2 / 15.6  and   8.6 / 10.9 / 14.1
 //   three runtimes in turn, each on its stream (about 3 is the call itself):
-//     Q6_K 1024 x 5120:   4.9 /  6.4 /  8.9  and   5.8 /  5.1 /  5.1      2048 x 5120:  6.0 /  8.7 / 12.8  and   5.5 /  5.5 /  6.2
-//     IQ4_XS 1024 x 5120: 5.0 /  6.3 /  8.6  and   3.4 /  3.6 /  4.8      2048 x 5120:  6.3 /  8.4 / 13.1  and   3.3 /  3.8 /  5.0
-//   a decoder layer of the 27B model whose 1024 x 5120 projections run there or here (its blocks fit beside nothing of this kernel; before
-//   Q3_K went to the tensor cores as bytes): one stream, one graph: 96 / 104 / 123 and 101 / 105 / 120;  three streams, 1 row, and 4 with prologues: 84 to 92, 114 and 80, 89
+//     Q6_K 1024 x 5120:   4.9 /  6.4 /  8.9  and   5.8 /  5.0 /  5.1      2048 x 5120:  6.0 /  8.7 / 12.8  and   5.5 /  5.5 /  6.2
+//     IQ4_XS 1024 x 5120: 5.0 /  6.2 /  8.6  and   3.2 /  4.0 /  5.1      2048 x 5120:  6.3 /  8.4 / 13.1  and   3.3 /  4.0 /  5.4
+//   a decoder layer of the 27B model whose 1024 x 5120 projections run there or here (the blocks of the one kernel fit beside nothing of the
+//   other), 1 row, 4 with prologues, 8 in groups:  one stream, one graph: 85 / 119 / 93 and 90 / 110 / 93;  three streams: 78 / 106 / 80 and
+//   70 / 80 / 80
 // The choice must not depend on the number of rows.  From 72 pieces of 256 x 256 weights on, of which no block has to walk more
 // than one in 20, launches go here: single rows on one stream pay up to 2 times for the shortest of them (2 to 7 % of a layer),
 // 8 rows, and whatever shares the GPU, gain more.
