@@ -222,8 +222,8 @@ int vqm_qmv_push(vqm_runtime *rt, const char *weight, const char *x, const char 
  * vqm_qmv_push_group is the row-sharded form (see vqm_qmv_push): per tensor its place in the gathered vectors, one
  * flag slot for the whole launch. */
 int vqm_qmv_group(vqm_runtime *rt, int n, const char *const *weights, const char *x, const char *const *ys, int ntok);
-/* Column split on (default) or off.  On: a launch may share each row's columns among the up to 8 blocks of a
- * thread-block cluster, whose partial sums are added in column order, and all but small launches run on the tensor
+/* Column split on (default) or off.  On: a launch may share each row's columns among up to 8 blocks,
+ * whose partial sums are added in column order, and all but small launches run on the tensor
  * cores.  Off: every output is one warp's sum over all columns, so a tensor's outputs do not depend on what else is in
  * its launch.  (The environment variable VINF_B200_NO_SPLIT=1 sets the default to off.) */
 int vqm_set_column_split(vqm_runtime *rt, int enabled);

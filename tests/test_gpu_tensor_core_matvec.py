@@ -417,3 +417,96 @@ def test_wide_passes_on_two_streams_take_turns(rt, graph):
     assert waited
     for i in range(2):
         assert np.array_equal(rt.read_array(f"y{i}", m * rows).view(np.uint32), want[i].view(np.uint32)), i
+
+
+def _captured(rt, work):
+    """`work` as a graph, launched once: in a capture the blocks that share columns are clusters."""
+    rt.capture_begin()
+    work()
+    graph = rt.capture_end()
+    rt.graph_launch(graph)
+    rt.synchronize()
+    rt.graph_destroy(graph)
+
+
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 7, 8, 9, 16, 17, 24])
+@pytest.mark.parametrize("t", [T.Q6_K, T.Q3_K, T.Q8_0, T.IQ3_S], ids=lambda t: t.name)
+@pytest.mark.parametrize("rows,cols", [(2305, 2304), (1030, 5120), (4099, 1280)], ids=str)
+def test_sums_exchanged_through_memory_and_in_clusters_are_the_same(rt, t, rows, cols, m):
+    rng = np.random.default_rng(rows + cols + m)
+    rt.upload("w", synthetic_blocks(t, rows, cols, rng), int(t), cols, rows)
+    rt.alloc("x", m * cols)
+    rt.alloc("y", m * rows)
+    for _ in range(2):  # the second launch finds what the first has left behind
+        rt.write("x", synthetic_activations(m, cols, rng))
+        outs = []
+        for run in (lambda work: work(), lambda work: _captured(rt, work)):
+            rt.zero("y")
+            run(lambda: rt.qmv("w", "x", "y", m))
+            rt.synchronize()
+            outs.append(rt.read_array("y", m * rows).copy())
+        assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32))
+        assert np.abs(outs[0]).max() > 0
+
+
+@pytest.mark.parametrize("m", [1, 2, 4, 5, 8])
+def test_fused_sums_exchanged_through_memory_and_in_clusters_are_the_same(rt, m):
+    t, rows, cols = T.Q6_K, 2305, 2304
+    rng = np.random.default_rng(m)
+    rt.upload("w", synthetic_blocks(t, rows, cols, rng), int(t), cols, rows)
+    for name, n in (("x", m * cols), ("x2", m * cols), ("g", cols), ("y0", m * rows), ("y", m * rows)):
+        rt.alloc(name, n)
+    for name, n in (("x", m), ("x2", m), ("g", 1)):
+        rt.write(name, synthetic_activations(n, cols, rng))
+    rt.write("y0", synthetic_activations(m, rows, rng))
+    for options in ({"norm": "g"}, {"norm": "g", "add": True}, {"silu_mul": "x2", "add": True}):
+        outs = []
+        for run in (lambda work: work(), lambda work: _captured(rt, work)):
+            rt.copy("y", 0, "y0", 0, m * rows)
+            run(lambda: rt.qmv_fused("w", "x", "y", m, **options))
+            rt.synchronize()
+            outs.append(rt.read_array("y", m * rows).copy())
+        assert np.array_equal(outs[0].view(np.uint32), outs[1].view(np.uint32)), options
+    ids = []
+    for run in (lambda work: work(), lambda work: _captured(rt, work)):
+        run(lambda: rt.qmv_argmax("w", "x", "y", m, blocking=False))
+        ids.append(rt.argmax_fetch(m))
+    assert ids[0] == ids[1] == rt.read_array("y", m * rows).reshape(m, rows).argmax(axis=1).tolist()
+
+
+def test_overlapping_streams_and_more_runtimes_than_rooms_for_sums(codebooks):
+    import torch
+    from vinf_3080ti_b200.runtime import Runtime
+
+    t, rows, cols, m = T.Q4_K, 2305, 2304, 4
+    rng = np.random.default_rng(3)
+    raw, xs = synthetic_blocks(t, rows, cols, rng), [synthetic_activations(m, cols, rng) for _ in range(3)]
+    runtimes = [Runtime(codebooks["iq3s_grid"], codebooks) for _ in range(18)]
+    try:
+        want = None
+        for rt in runtimes:
+            rt.upload("w", raw, int(t), cols, rows)
+            for i, x in enumerate(xs):
+                rt.alloc(f"x{i}", m * cols)
+                rt.alloc(f"y{i}", m * rows)
+                rt.write(f"x{i}", x)
+        for rt in runtimes:
+            streams = [None] + [torch.cuda.Stream() for _ in range(5)]
+            for k in range(12):  # one runtime, launches on six streams that wait for nothing
+                stream = streams[k % 6]
+                rt.set_stream(stream.cuda_stream if stream is not None else None)
+                if k >= 3 and stream is not None:
+                    stream.synchronize()
+                rt.qmv("w", f"x{k % 3}", f"y{k % 3}", m)
+            torch.cuda.synchronize()
+            rt.set_stream(None)
+            rt.synchronize()
+            got = [rt.read_array(f"y{i}", m * rows).copy() for i in range(3)]
+            want = want or got
+            for g, w in zip(got, want):
+                assert np.array_equal(g.view(np.uint32), w.view(np.uint32))
+        ref = O.matvec(raw, int(t), rows, cols, xs[0], codebooks)
+        assert rel_l2(want[0].reshape(m, rows), ref) <= REL_L2
+    finally:
+        for rt in runtimes:
+            rt.close()

@@ -70,7 +70,10 @@ struct MatvecArgs {
 static_assert(sizeof(MatvecArgs) <= 384, "parameters of the CUDA-core kernel");
 struct TcMatvecArgs : MatvecArgs {
     const uint8_t *x_split;  // ready-made B operands of more than 8 activation rows
-    int tc_steps[9];         // block k of a cluster takes the 256-column steps [tc_steps[k], tc_steps[k + 1])
+    float *partials;         // sums of launches whose columns are split, see tc_finish_tile; null: clusters exchange them
+    unsigned *partial_counts;  // [tile]: how many column ranges are there; zero before and after a launch
+    int tc_groups, tc_split_recip;  // groups of k_split blocks, and 65536 / k_split rounded up
+    int tc_steps[9];         // block k of a group takes the 256-column steps [tc_steps[k], tc_steps[k + 1])
     int tc_deal, tc_deal_recip;  // rows of a tile that each block of a cluster finishes, and 65536 / tc_deal rounded up
     int tc_first, tc_end;        // tiles of this launch (a launch may take the last round of another, see choose_tc_tail)
     unsigned char tc_map_shift[kMaxParts];  // log2 of the number of tensor maps of each tensor
@@ -95,16 +98,27 @@ VQM_FOR_EACH_TYPE(VQM_DECLARE_LAUNCHER)
 
 constexpr int kTcTileRows = 256;   // rows of a tile of the tensor-core matvec
 constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matvec: times 31 it has to fit into the 11 bits of fp16
+// Room for the partial sums of a launch whose columns are split (at most sm_count / 2 tiles, sm_count blocks): the counts, then the records of
+// tc_finish_tile, 2 of a block for up to 8 activation rows, 12 smaller ones for 24.
+constexpr size_t tc_partial_count_bytes(int sm_count) { return (static_cast<size_t>(sm_count) * 4 + 255) / 256 * 256; }
+constexpr size_t tc_partial_bytes(int sm_count, int m) {
+    return tc_partial_count_bytes(sm_count) + static_cast<size_t>(sm_count) * (m <= 8 ? 2 * (4 * kTcTileRows + 32) : 12 * (2 * kTcTileRows + 32)) * 4;
+}
+struct TcScratch {
+    const uint8_t *x_split = nullptr;  // the B operands of more than 8 activation rows
+    // Room for partial sums, in use by one launch at a time: counts zero and sums empty (bytes of 0xFF) before and after it.  Null: the blocks that
+    // share columns are clusters and exchange sums in shared memory.  The outputs are the same, bit for bit.
+    uint8_t *partials = nullptr;
+};
 // The tensor-core matvec (vqm_tcmv_type.cu).  maps: per tensor of the launch its tensor maps (tc_encode_maps).
 #define VQM_FOR_EACH_TC_TYPE(X) \
     X(8, Q8_0) X(10, Q2_K) X(11, Q3_K) X(12, Q4_K) X(13, Q5_K) X(14, Q6_K) X(16, IQ2_XXS) X(17, IQ2_XS) X(18, IQ3_XXS) \
     X(20, IQ4_NL) X(21, IQ3_S) X(22, IQ2_S) X(23, IQ4_XS)
 // split_tcmv_*: into how many column ranges the launch would be split (to go into a.k_split), 0 = the CUDA-core kernel is better.
-// launch_tcmv_*: x_split holds the B operands of more than 8 activation rows; n_launched (may be null) is counted up by the
-// kernels launched, one or two (split: one for 16 rows).
+// launch_tcmv_*: n_launched (may be null) is counted up by the kernels launched, one or two (split: one for 16 rows).
 #define VQM_DECLARE_TC_LAUNCHER(id, name)                                                                                        \
     int split_tcmv_##name(const MatvecArgs &a, int sm_count);                                                                    \
-    cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m, \
+    cudaError_t launch_tcmv_##name(const MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const TcScratch &scratch, int m, \
                                    int sm_count, cudaStream_t stream, int *n_launched);
 // wide_rows_*: how many activation rows a launch takes, 24, 16 or 8; split_bytes_*: size of x_split for a launch of more than 8 rows over so
 // many columns, 0 if the type takes 8 at most; launch_split_*: makes it from a.x.

@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <unordered_map>
@@ -109,6 +110,12 @@ struct vqm_runtime {
     cudaStream_t split_stream = nullptr;
     cudaEvent_t split_event = nullptr;
     std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use (together at most twice the present one)
+    // Partial sums of matvecs whose columns are split (vqm::TcScratch).  Launches on different streams may overlap, so each stream has its own,
+    // known by the stream's id (ids, unlike handles, do not come again).  Of more than 8 activation rows: behind x_split, which one stream at a
+    // time uses.
+    std::vector<std::pair<unsigned long long, uint8_t *>> stream_partials;
+    uint8_t *partials = nullptr;  // of the present stream; null: none, clusters exchange the sums
+    bool split_emptied = false;   // those behind x_split are ready
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
     void *gemm_x = nullptr;  // fp16 copy of the activations of a prompt pass
@@ -250,11 +257,11 @@ bool use_tcmv(int type, vqm::MatvecArgs &a, int sm_count, bool codebook_small) {
     return split > 0;
 }
 
-cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m, int sm_count,
-                          cudaStream_t stream, int *n_launched) {
+cudaError_t dispatch_tcmv(int type, const vqm::MatvecArgs &a, const CUtensorMap *const *maps, int n_parts, const vqm::TcScratch &scratch, int m,
+                          int sm_count, cudaStream_t stream, int *n_launched) {
     switch (type) {
 #define VQM_CASE(id, name) \
-    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, x_split, m, sm_count, stream, n_launched);
+    case id: return vqm::launch_tcmv_##name(a, maps, n_parts, scratch, m, sm_count, stream, n_launched);
         VQM_FOR_EACH_TC_TYPE(VQM_CASE)
 #undef VQM_CASE
         default: return cudaErrorInvalidValue;
@@ -295,7 +302,7 @@ cudaError_t dispatch_raw(int type, vqm::MatvecArgs &a, int m, int sm_count, cuda
     const CUtensorMap *p[1] = {maps};
     const cudaError_t err = vqm::tc_encode_maps(type, a.part[0].w, a.rows, a.row_bytes, vqm::kTcTileRows / 8, maps);
     if (err != cudaSuccess) return err;
-    return dispatch_tcmv(type, a, p, 1, nullptr, m, sm_count, stream, nullptr);
+    return dispatch_tcmv(type, a, p, 1, vqm::TcScratch{}, m, sm_count, stream, nullptr);
 }
 
 cudaError_t encode_maps(Tensor &t) {
@@ -303,6 +310,94 @@ cudaError_t encode_maps(Tensor &t) {
     const cudaError_t err = vqm::tc_encode_maps(t.type, t.data, t.rows, static_cast<long long>(t.row_bytes), vqm::kTcTileRows / 8, t.maps);
     t.mapped = err == cudaSuccess;
     return err;
+}
+
+// Rooms for partial sums, of all runtimes: part of the library image, because an allocation of that size makes the creation of a runtime
+// 0.4 ms slower (0.7 ms; a program that runs out of them has clusters exchange the sums).  A room belongs to one stream of one runtime
+// until the runtime is destroyed.
+constexpr int kPartialRooms = 16, kPartialSms = 160;
+static __device__ __align__(256) uint8_t g_partial_rooms[kPartialRooms][(vqm::tc_partial_bytes(kPartialSms, 8) + 255) / 256 * 256];
+std::mutex g_partial_mutex;
+bool g_partial_taken[kPartialRooms];
+
+// A room's address, null if there is none left.
+uint8_t *take_partials(int sm_count) {
+    if (sm_count > kPartialSms) return nullptr;
+    const std::lock_guard<std::mutex> lock(g_partial_mutex);
+    static uint8_t *first = nullptr;  // (one device per process, see check_one_device)
+    if (first == nullptr) {
+        void *p = nullptr;
+        if (cudaGetSymbolAddress(&p, g_partial_rooms) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        first = static_cast<uint8_t *>(p);
+    }
+    for (int i = 0; i < kPartialRooms; ++i)
+        if (!g_partial_taken[i]) {
+            g_partial_taken[i] = true;
+            return first + i * sizeof(g_partial_rooms[0]);
+        }
+    return nullptr;
+}
+// (of a runtime all of whose work has ended)
+void give_partials_back(const uint8_t *room) {
+    const std::lock_guard<std::mutex> lock(g_partial_mutex);
+    void *first = nullptr;
+    if (cudaGetSymbolAddress(&first, g_partial_rooms) == cudaSuccess)
+        g_partial_taken[(room - static_cast<const uint8_t *>(first)) / sizeof(g_partial_rooms[0])] = false;
+}
+// As launches find and leave it.
+cudaError_t empty_partials(vqm_runtime *rt, uint8_t *p, int m, cudaStream_t stream) {
+    const size_t counts = vqm::tc_partial_count_bytes(rt->sm_count);
+    const cudaError_t err = cudaMemsetAsync(p, 0, counts, stream);
+    return err != cudaSuccess ? err : cudaMemsetAsync(p + counts, 0xFF, vqm::tc_partial_bytes(rt->sm_count, m) - counts, stream);
+}
+bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();
+    return true;
+}
+
+// The present stream's room for partial sums.  (Runtimes that keep changing streams have it for the first four.)
+constexpr size_t kMaxStreamPartials = 4;
+void find_partials(vqm_runtime *rt) {
+    rt->partials = nullptr;
+    unsigned long long id = 0;
+    if (is_capturing(rt->stream) || cudaStreamGetId(rt->stream, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return;
+    }
+    for (const auto &known : rt->stream_partials)
+        if (known.first == id) rt->partials = known.second;
+    if (rt->partials != nullptr || rt->stream_partials.size() >= kMaxStreamPartials) return;
+    uint8_t *const room = take_partials(rt->sm_count);
+    if (room == nullptr) return;
+    rt->stream_partials.emplace_back(id, room);
+    if (empty_partials(rt, room, 8, rt->stream) == cudaSuccess) rt->partials = room;
+}
+
+// Room for the partial sums of the next launch, none while a graph is captured: it may run beside other work, on any stream.  (Beside
+// nothing else, as a captured decode pass, clusters exchange them faster too: the 27B model's pass of 4 rows 4.84 ms, 4.94 through memory.)
+uint8_t *partials_now(vqm_runtime *rt, int m) {
+    if (rt->capturing || is_capturing(rt->stream)) return nullptr;
+    if (m <= 8) return rt->partials;
+    uint8_t *const room = rt->x_split + rt->x_split_bytes;  // (claim_split has been called)
+    if (!rt->split_emptied) rt->split_emptied = empty_partials(rt, room, 24, rt->stream) == cudaSuccess;
+    return rt->split_emptied ? room : nullptr;
+}
+// After a wait gave up, records may not be as launches leave them.  (What other streams still run may use theirs: those streams have clusters
+// from now on.)
+void renew_partials(vqm_runtime *rt) {
+    for (auto &known : rt->stream_partials) {
+        if (known.second == rt->partials && rt->partials != nullptr) {
+            if (empty_partials(rt, known.second, 8, rt->stream) != cudaSuccess) rt->partials = nullptr;
+        } else {
+            known.first = ULLONG_MAX;  // (no stream's id)
+        }
+    }
+    rt->split_emptied = false;
 }
 
 // Before x_split is used on the present stream: what used it on another one comes first.  (A capture must not wait for what is
@@ -416,7 +511,10 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         if (err == cudaSuccess && m > 8) {
             err = dispatch_split(t0.type, a, rt->x_split, m, rt->stream, &launched);
         }
-        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, rt->x_split, m, rt->sm_count, rt->stream, &launched);
+        vqm::TcScratch scratch;
+        scratch.x_split = rt->x_split;
+        if (a.k_split > 1) scratch.partials = partials_now(rt, m);
+        if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, scratch, m, rt->sm_count, rt->stream, &launched);
     } else {
         err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
         ++launched;
@@ -444,12 +542,15 @@ bool make_split_room(vqm_runtime *rt) {
     uint8_t *p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    const cudaError_t err = cudaMalloc(&p, bytes);
+    const cudaError_t err = cudaMalloc(&p, bytes + vqm::tc_partial_bytes(rt->sm_count, 24));
     cudaThreadExchangeStreamCaptureMode(&mode);
     if (err != cudaSuccess) {
         (void)cudaGetLastError();
         return false;
     }
+    // (beside a capture: by the first launch that needs it)
+    rt->split_emptied = !rt->capturing && !is_capturing(rt->stream) && empty_partials(rt, p + bytes, 24, rt->stream) == cudaSuccess;
+    if (rt->split_emptied) rt->split_used = true;  // (what uses it on another stream comes after that)
     if (rt->x_split != nullptr) rt->retired.push_back(rt->x_split);
     rt->x_split = p;
     rt->x_split_bytes = bytes;
@@ -527,6 +628,7 @@ int check_status_word(vqm_runtime *rt, const char *ctx) {
     if (err != cudaSuccess) return cuda_fail(ctx, err);
     if (host != 0) {
         cudaMemsetAsync(rt->status, 0, sizeof(unsigned), rt->stream);
+        renew_partials(rt);
         return status_failure(ctx, host);
     }
     return VQM_OK;
@@ -600,6 +702,7 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
         return rc;
     }
     rt->done_counter = rt->status + 16;
+    find_partials(rt);
     if (const char *e = getenv("VINF_B200_NO_PDL"); e != nullptr && e[0] == '1') rt->overlap_launch = 0;
     if (const char *e = getenv("VINF_B200_NO_SPLIT"); e != nullptr && e[0] == '1') rt->allow_split = 0;
     if (const char *e = getenv("VINF_B200_GEMM"); e != nullptr && strcmp(e, "mma") == 0) rt->gemm_tcgen05 = 0;
@@ -617,6 +720,10 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
 void vqm_runtime_destroy(vqm_runtime *rt) {
     if (rt == nullptr) return;
     if (rt->stream != nullptr) cudaStreamSynchronize(rt->stream);
+    for (const auto &known : rt->stream_partials) {
+        if (known.second != rt->partials) cudaDeviceSynchronize();  // (another stream's work)
+        give_partials_back(known.second);
+    }
     rt->stream = rt->own_stream;
     for (auto &g : rt->graphs)
         if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
@@ -1233,6 +1340,7 @@ int vqm_matvec(vqm_runtime *rt, const char *weight, const float *x_host, size_t 
     if (err != cudaSuccess) return cuda_fail("qmatvec", err);
     if (got[0] != 0) {
         if (out != got) cudaMemsetAsync(out, 0, sizeof(unsigned), rt->stream);
+        renew_partials(rt);
         return status_failure("qmatvec", got[0]);
     }
     memcpy(y_host, y_at, sizeof(float) * t.rows);
@@ -1304,7 +1412,9 @@ int vqm_set_stream(vqm_runtime *rt, void *stream) {
     const cudaStream_t next = stream != nullptr ? static_cast<cudaStream_t>(stream) : rt->own_stream;
     const cudaError_t err = leave_stream(rt, next);
     if (err != cudaSuccess) return cuda_fail("set_stream", err);
+    if (next == rt->stream) return VQM_OK;
     rt->stream = next;
+    find_partials(rt);
     return VQM_OK;
 }
 

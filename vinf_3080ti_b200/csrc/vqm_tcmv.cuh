@@ -34,9 +34,10 @@
 // misalignment, and tile copies of 32 rows of a class have a 16-byte aligned row stride.  The stage's row pitch is an odd
 // multiple of 16 bytes, free of bank conflicts for 16-byte loads.
 //
-// Columns are split over the k_split blocks of a cluster (each a contiguous range of steps); a tile's rows are dealt out to
-// the cluster's blocks, every block sends each its part of the sums (st.async) and the parts are added in the order of the
-// columns.  The split and the order of all additions depend on rows and columns only, never on M.
+// Columns are split over k_split blocks, each a contiguous range of steps.  The blocks exchange their sums through memory (tc_finish_tile) or,
+// where the launch has no room for them (a captured graph, a caller without a runtime), as a cluster: a tile's rows are dealt out to its blocks
+// and every block sends each its part (st.async).  Both add the parts in the order of the columns: the split and the order of all additions depend
+// on rows and columns only, never on M.
 #pragma once
 
 #include <cuda.h>
@@ -137,13 +138,15 @@ __host__ __device__ constexpr int tc_info_floats(int type, int mc) { return tc_i
 // have no room for 16 KB of activations; the tile's sums go out 8 (of 24: 4) activation rows at a time.
 __host__ __device__ constexpr bool tc_presplit(int mc) { return mc > 8; }
 __host__ __device__ constexpr int tc_out_rows(int mc) { return mc > 16 ? 4 : mc > 8 ? 8 : mc; }
+// pitch of the sums of a tile's rows in shared memory (tc_red_at; the parts of a cluster's blocks take at most 264 rows)
+constexpr int kTcRedRows = kTcRows + kTcRows / 8;
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_stage_bytes() { return kTcRows * tc_pitch(TYPE) + (tc_presplit(MC) ? 0 : MC * kTcStepCols * 4); }
 // Shared memory beside the weight stages, with `b` B stages (an MMA may read one group of rows further).
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_fixed_bytes(int b) {
     return (tc_table_bytes(TYPE, MC) + 127) / 128 * 128 + (b * TcShape<TYPE, MC>::kGroupsB + 1) * tc_group_b(TYPE) + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4 +
-           2 * 264 * tc_out_rows(MC) * 4 + (tc_presplit(MC) ? 0 : (kTcMaxNormSteps + 2) * MC * 4) + 256;
+           2 * kTcRedRows * tc_out_rows(MC) * 4 + (tc_presplit(MC) ? 0 : (kTcMaxNormSteps + 2) * MC * 4) + 256;
 }
 template <int TYPE, int MC>
 __host__ __device__ constexpr int tc_stages_beside(int b) {

@@ -592,27 +592,31 @@ __device__ __noinline__ float tc_plain_sum(const MatvecArgs &a, const uint8_t *r
 
 __device__ __forceinline__ bool tc_better(float v, int i, float bv, int bi) { return v > bv || (v == bv && i < bi); }
 
-// Fused argmax: block partials, then the last block to finish reduces them (ties to the lowest row, 0x7fffffff if nothing is
-// above -inf).  Warp w < 16 holds the best of activation row w % MC over its lanes' outputs.
-template <int MC>
-__device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, float bv, int bi, int warp, int lane, float *s_v, int *s_i, bool *s_last) {
-    auto warp_best = [&]() {
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-            if (tc_better(ov, oi, bv, bi)) bv = ov, bi = oi;
-        }
-    };
-    warp_best();
-    if (warp < 16 && lane == 0) s_v[warp] = bv, s_i[warp] = bi;
+// The order of floats as unsigned integers (no NaN).
+__device__ __forceinline__ uint32_t tc_ordered(float v) {
+    const uint32_t b = __float_as_uint(v);
+    return b ^ ((static_cast<uint32_t>(static_cast<int32_t>(b) >> 31)) | 0x80000000u);
+}
+// Fused argmax: what a warp's lanes have put out for an activation row (rows ascend with the lanes) against the warp's best so far.
+// NaN is no output; ties to the lower row.
+__device__ __forceinline__ void tc_note_best(bool exists, float v, int row, int lane, float *best_v, int *best_i) {
+    const uint32_t key = exists && v == v ? tc_ordered(v == 0.0f ? 0.0f : v) : 0u;
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, key);
+    const uint32_t who = __ballot_sync(0xFFFFFFFFu, key == top);
+    if (top != 0u && lane == __ffs(static_cast<int>(who)) - 1 && tc_better(v, row, *best_v, *best_i)) *best_v = v, *best_i = row;
+    __syncwarp();
+}
+
+// Block partials, then the last block to finish reduces them (ties to the lowest row, 0x7fffffff if nothing is above -inf).
+__device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, int warp, int lane, const float (*s_v)[8], const int (*s_i)[8], bool *s_last) {
     __syncthreads();
     const int grid = static_cast<int>(gridDim.x);
     if (threadIdx.x < static_cast<unsigned>(m)) {
         const int t = static_cast<int>(threadIdx.x);
-        bv = s_v[t], bi = s_i[t];
-        for (int w = t + MC; w < 16; w += MC)
-            if (tc_better(s_v[w], s_i[w], bv, bi)) bv = s_v[w], bi = s_i[w];
+        float bv = s_v[0][t];
+        int bi = s_i[0][t];
+        for (int w = 1; w < 16; ++w)
+            if (tc_better(s_v[w][t], s_i[w][t], bv, bi)) bv = s_v[w][t], bi = s_i[w][t];
         a.part_val[t * grid + blockIdx.x] = bv;
         a.part_idx[t * grid + blockIdx.x] = bi;
     }
@@ -625,13 +629,19 @@ __device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, f
     if (!*s_last) return;
     __threadfence();
     if (warp < m) {
-        bv = -INFINITY, bi = 0x7fffffff;
+        float bv = -INFINITY;
+        int bi = 0x7fffffff;
         for (int b = lane; b < grid; b += 32) {
             const float v = __ldcg(a.part_val + warp * grid + b);
             const int i = __ldcg(a.part_idx + warp * grid + b);
             if (tc_better(v, i, bv, bi)) bv = v, bi = i;
         }
-        warp_best();
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
+            const int oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
+            if (tc_better(ov, oi, bv, bi)) bv = ov, bi = oi;
+        }
         if (lane == 0) {
             bi = bi == 0x7fffffff ? bi : bi + a.row_base;
             // a launch that takes the last tiles of a tensor: the launch before it has left the best of the others, all lower rows
@@ -642,6 +652,167 @@ __device__ __forceinline__ void tc_finish_argmax(const TcMatvecArgs &a, int m, f
         }
     }
     if (threadIdx.x == 0) *a.done_counter = 0;
+}
+
+// An output: the sum over all columns, its epilogue, the store.
+template <int TYPE>
+__device__ __forceinline__ float tc_put(const TcMatvecArgs &a, const MatvecPart &part, int row, int t, float sum, float factor) {
+    if (a.fuse & kFuseNorm) sum *= factor;
+    if (sum != sum) sum = tc_plain_sum<TYPE>(a, part.w + static_cast<size_t>(row) * a.row_bytes, t, factor);
+    if (part.y != nullptr) {
+        float *y = part.y + static_cast<size_t>(t) * part.rows + row;
+        if (a.fuse & kFuseAdd) sum += *y;
+        *y = sum;
+    }
+    return sum;
+}
+
+// A word of a.partials that nobody has written: a NaN that no arithmetic gives.
+constexpr uint32_t kTcEmpty = 0xFFFFFFFFu;
+template <int N>
+__device__ __forceinline__ void tc_store_words(float *to, const uint32_t (&v)[N]) {
+    if constexpr (N == 1) asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(to), "r"(v[0]) : "memory");
+    else if constexpr (N == 2) asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(to), "r"(v[0]), "r"(v[1]) : "memory");
+    else asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(to), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tc_load_words(const float *from, uint32_t (&v)[N]) {
+    if constexpr (N == 1) asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v[0]) : "l"(from) : "memory");
+    else if constexpr (N == 2) asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "l"(from) : "memory");
+    else asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "l"(from) : "memory");
+}
+__device__ __forceinline__ uint32_t tc_word(float v) {
+    const uint32_t b = __float_as_uint(v);
+    return b == kTcEmpty ? 0x7FFFFFFFu : b;
+}
+
+// Where the sums of row r, activation row t of the exchange (of kOut) and a pair of groups lie in shared memory: a warp stores every eighth
+// row and reads 32 rows in turn, both without bank conflicts.
+template <int kOut>
+__device__ __forceinline__ uint32_t tc_red_at(uint32_t red, int pair, int t, int r) {
+    return red + ((pair * kOut + t) * kTcRedRows + r + (r >> 3)) * 4;
+}
+
+// Finishes a tile outside of a cluster: all decoder warps, thread = row, the two halves of the threads share the activation rows.
+// With columns split, the last of the k_split blocks to have counted itself in (each does so before its last sums are there) adds the
+// parts up in the order of the columns; the others leave theirs in a.partials.  They come with no fence: the last block reads words
+// until none is empty, and leaves them empty again.  It only waits for blocks that are about to store: blocks may run at any time and in any
+// place, and no cluster has to find room at once (120 blocks in clusters of 6 leave 28 SMs, of which other clusters cannot use most).
+// The way through L2 takes some 0.5 us longer than one through a cluster's shared memory, which a stream alone notices (a layer of 8 rows,
+// alone from launch to end, 109 -> 112 us; one of 1 row 100 -> 104) and three streams that share the GPU do not: clusters and this, each with
+// launch_dependents where it is now, layers of 1, 4 (fused) and 8 rows 67.3 / 81.9 / 81.2 and 60.8 / 73.3 / 75.0 us, 24 rows of three tensors
+// 101 and 84, six tensors of odd sizes with 2 rows 62 and 53.
+// (What was slower: a warp at a time, each with its own count, M=8 Q6_K 1024 x 5120 10.6 -> 11.8 us; counts that acquire and release, or fences on both
+// sides of a relaxed one, 0.6 and 1.4 us more.)
+// The loop over the outputs is rolled: this code runs once per tile, its instructions come from L2.
+template <int TYPE, int MC>
+__device__ __forceinline__ void tc_finish_tile(const TcMatvecArgs &a, int m, int p, int tile, int tile_row, int rank, bool more, uint32_t red, const float (&sums)[MC],
+                                               const float *norm, const int *s_last, float (*best_v)[8], int (*best_i)[8], volatile int *failed) {
+    constexpr int kOut = tc_out_rows(MC), kHalf = (kOut + 1) / 2, kVec = kHalf < 4 ? kHalf : 4;  // activation rows per exchange, a thread's part of them
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = threadIdx.x & 255, half = threadIdx.x >> 8, k_split = a.k_split;
+    const MatvecPart &part = a.part[p];
+    const int row = tile_row * kTcRows + r;
+    const bool exists = row < part.rows;
+    unsigned long long began = 0;
+#pragma unroll
+    for (int round = 0; round < MC / kOut; ++round) {
+        {
+            const int mine = ((warp >> 2) & 1) * 4 + (warp & 3) + 8 * lane;
+#pragma unroll
+            for (int t = 0; t < kOut; ++t)
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(tc_red_at<kOut>(red, warp >> 3, t, mine)), "f"(sums[round * kOut + t]) : "memory");
+        }
+        tc::decoders_sync();
+        const int t0 = round * kOut + half * kHalf;  // the thread's activation rows: kHalf from here on
+        if (t0 < m && (MC > 1 || half == 0)) {
+            const uint32_t at = tc_red_at<kOut>(red, 0, half * kHalf, r);
+            constexpr uint32_t kNext = kTcRedRows * 4, kPair = kOut * kNext;
+            float sq = 0.0f;  // lane i: the squares of activation row t0 + i
+            if (a.fuse & kFuseNorm) sq = lane < kHalf ? norm[t0 + lane] : 0.0f;
+            if (a.fuse & kFuseAdd) {  // what the outputs are added to, so that they do not wait for one row after the other
+#pragma unroll 1
+                for (int t = t0; t < t0 + kHalf && t < m; ++t)
+                    if (exists) asm volatile("prefetch.global.L1 [%0];" ::"l"(part.y + static_cast<size_t>(t) * part.rows + row));
+            }
+            bool out = true;
+            if (k_split > 1) {
+                // [round][column range][half]: [256 rows][kHalf], then for each of 8 warps the squares
+                constexpr int kRecord = kHalf * kTcRows + 32;
+                float *const first = a.partials + (((tile - a.tc_first) * (MC / kOut) + round) * k_split * 2 + half) * kRecord;
+                out = *s_last == k_split - 1;
+                uint32_t own[kHalf];
+#pragma unroll
+                for (int i = 0; i < kHalf; ++i) own[i] = tc_word(__uint_as_float(lds32(at + i * kNext)) + __uint_as_float(lds32(at + i * kNext + kPair)));
+                if (!out) {
+                    tc_store_words(first + rank * 2 * kRecord + r * kHalf, own);
+                    if ((a.fuse & kFuseNorm) && lane < kHalf) {
+                        const uint32_t w[1] = {tc_word(sq)};
+                        tc_store_words(first + rank * 2 * kRecord + kHalf * kTcRows + (warp & 7) * 4 + lane, w);
+                    }
+                } else {
+                    // the squares, lane 4 k + i: of column range k
+                    float *const squares = first + (lane >> 2) * 2 * kRecord + kHalf * kTcRows + (warp & 7) * 4 + (lane & 3);
+                    const bool there = (a.fuse & kFuseNorm) && lane < 4 * k_split && (lane & 3) < kHalf && (lane >> 2) != rank;
+                    uint32_t w[1] = {0u};
+                    uint32_t v[kMaxSplit][kVec];
+                    static_assert(kHalf == kVec, "one load per column range");
+                    float *const from = first + r * kHalf;
+#pragma unroll 1
+                    for (uint32_t i = 1;; ++i) {
+                        if (there) tc_load_words(squares, w);
+#pragma unroll
+                        for (int k = 0; k < kMaxSplit; ++k) {
+#pragma unroll
+                            for (int j = 0; j < kVec; ++j) v[k][j] = 0u;
+                            if (k < k_split && k != rank) tc_load_words(from + k * 2 * kRecord, v[k]);
+                        }
+                        bool empty = w[0] == kTcEmpty;
+#pragma unroll
+                        for (int k = 0; k < kMaxSplit; ++k)
+#pragma unroll
+                            for (int j = 0; j < kVec; ++j) empty |= v[k][j] == kTcEmpty;
+                        if (!__any_sync(0xFFFFFFFFu, empty) || ((i & 255u) == 0 && __any_sync(0xFFFFFFFFu, tc::give_up(&began, failed)))) break;
+                    }
+#pragma unroll
+                    for (int j = 0; j < kVec; ++j) {
+                        float sum = 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kMaxSplit; ++k) sum += __uint_as_float(k == rank ? own[j] : v[k][j]);
+                        asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + j * kNext), "f"(sum) : "memory");
+                    }
+                    if (a.fuse & kFuseNorm) {
+                        const uint32_t none[1] = {kTcEmpty};
+                        if (there) tc_store_words(squares, none);
+                        const float mine = __shfl_sync(0xFFFFFFFFu, sq, lane & 3);
+                        if ((lane >> 2) == rank) w[0] = __float_as_uint(mine);
+                        sq = 0.0f;
+#pragma unroll 1
+                        for (int k = 0; k < k_split; ++k) sq += __uint_as_float(__shfl_sync(0xFFFFFFFFu, w[0], 4 * k + (lane & 3)));
+                    }
+                    uint32_t none[kVec];
+#pragma unroll
+                    for (int j = 0; j < kVec; ++j) none[j] = kTcEmpty;
+#pragma unroll 1
+                    for (int k = 0; k < k_split; ++k) {
+                        if (k != rank) tc_store_words(from + k * 2 * kRecord, none);
+                    }
+                }
+            }
+            if (out) {
+                const float scale = (a.fuse & kFuseNorm) ? 1.0f / sqrtf(sq / static_cast<float>(a.cols) + a.eps) : 1.0f;
+                uint32_t from = at;
+#pragma unroll 1
+                for (int i = 0; i < kHalf && t0 + i < m; ++i, from += kNext) {
+                    float sum = __uint_as_float(lds32(from));
+                    if (k_split == 1) sum += __uint_as_float(lds32(from + kPair));
+                    const float factor = __shfl_sync(0xFFFFFFFFu, scale, i);
+                    if (exists) sum = tc_put<TYPE>(a, part, row, t0 + i, sum, factor);
+                    if (a.out_idx != nullptr) tc_note_best(exists, sum, row, lane, &best_v[warp][t0 + i], &best_i[warp][t0 + i]);
+                }
+            }
+        }
+        if (more || round + 1 < MC / kOut) tc::decoders_sync();  // the sums may be overwritten
+    }
 }
 
 // B operands and infos of the activation rows t0 .. t0 + 15 below m, of MC, one block per step: what every block of the matvec would work
@@ -687,9 +858,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
     __shared__ float s_norm[kMaxSplit][8];  // sums of squares of the activation rows, from every block of the cluster
-    __shared__ float s_best_v[16];
-    __shared__ int s_best_i[16];
+    __shared__ float s_best_v[16][8];  // fused argmax: the best outputs that each warp has seen, per activation row
+    __shared__ int s_best_i[16][8];
     __shared__ bool s_last;
+    __shared__ int s_count;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // layout: stages (1024-byte aligned) | table | B ring | per-step info | sums of the tile | sums of squares
     const uint32_t stages = (tc::s32(tc_raw) + 1023u) & ~1023u;
@@ -697,14 +869,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     const uint32_t b_ring = table + (tc_table_bytes(TYPE, MC) + 127) / 128 * 128;
     const uint32_t info_ring = b_ring + (kNB * Shape::kGroupsB + 1) * tc_group_b(TYPE);
     const uint32_t red = info_ring + kTcInfoSlots * tc_info_floats(TYPE, MC) * 4;
-    const uint32_t norm_parts = red + 2 * 264 * kOut * 4;
+    const uint32_t norm_parts = red + 2 * kTcRedRows * kOut * 4;
     volatile int *failed = &s_failed;
 
     const int k_split = a.k_split;
-    int rank, group, n_groups;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-    asm("mov.u32 %0, %%clusterid.x;" : "=r"(group));
-    asm("mov.u32 %0, %%nclusterid.x;" : "=r"(n_groups));
+    const bool clustered = k_split > 1 && a.partials == nullptr;
+    int group = static_cast<int>((blockIdx.x * static_cast<unsigned>(a.tc_split_recip)) >> 16), n_groups = a.tc_groups;
+    const int rank = static_cast<int>(blockIdx.x) - group * k_split;
     const int step0 = a.tc_steps[rank], step1 = a.tc_steps[rank + 1];
     auto tiles_of = [&](int p) { return (a.part[p].rows + kTcRows - 1) / kTcRows; };
     const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = a.tc_end;
@@ -809,13 +980,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         }
         asm volatile("bar.sync 6, %0;" ::"n"(kTcThreads) : "memory");
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // Announces this block's barriers to the cluster; whoever signals them waits for the announcements first.  (The barriers were
     // published by the fence behind their initialisation; a releasing arrive would wait for the copies in flight, 3 us.)
-    if (k_split > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (clustered) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     tc::fence_after();
-    float best_v = -INFINITY;
-    int best_i = 0x7fffffff;
 
     if (warp == 16) {
         if (tc::elect_one()) {
@@ -921,14 +1089,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
         const uint32_t tm_mine = s_tmem + wg * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
         const uint32_t a_full = tc::s32(&s_afull[wg]), mma_done = tc::s32(&s_done[wg]);
         int st = 0, stage = 0, bs = 0;  // step count, stage, B stage
-        uint32_t wphase = 0, bphase = 0, dphase = 1, rphase = 0, sphase = 0;  // (dphase: of the batch before the next one)
-        bool announced = false;                 // the cluster's barriers are known to exist
+        uint32_t wphase = 0, bphase = 0, dphase = 1;  // (dphase: of the batch before the next one)
         bool pending = false;    // a unit's sums have not been read yet
         TcPending<TYPE, MC> pend;
         TcUnitSums<TYPE, MC> unit_sums;
         unit_sums.clear();
         TcAcc<MC> acc;
         acc.clear();
+        uint32_t rounds = 0;  // in which sums have been handed over
+        if (lane < 8) s_best_v[warp][lane] = -INFINITY, s_best_i[warp][lane] = 0x7fffffff;
 
         // The first kNB steps' activations are converted by all warps at once, straight from global memory: the way through the
         // stages would put a copy and a turn of conversions (1 us) between the end of the previous kernel and the first MMAs.
@@ -1072,7 +1241,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                 if (++stage == kStages) stage = 0, wphase ^= 1u;
                 if (++bs == kNB) bs = 0, bphase ^= 1u;
             }
+            // The next kernel's blocks may come now.  Requested at the start of a block they take the SMs that this grid leaves, and those of its
+            // first blocks to end, and hold them until its last one has ended; clusters of the next but one find no room beside them.
+            // (With clusters, start of a block and here: the 27B model's pass of 4 rows 5.05 and 4.79 ms, a layer of 1 row on each of three streams
+            // 69.5 and 67.0 us, five IQ tensors of 1 row 96.5 and 91.3.  At the start of the last step: 4.81 ms, 68.3 us, 95.3.)
+            if (tile + n_groups >= n_tiles) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             // ---- the tile's last sums, then the outputs ----
+            unsigned counted = 0;  // thread 0: the column ranges of the tile that are ahead of this one
+            if (k_split > 1 && !clustered && threadIdx.x == 0) {
+                unsigned *const count = a.partial_counts + (tile - a.tc_first);
+                asm volatile("atom.inc.relaxed.gpu.global.u32 %0, [%1], %2;" : "=r"(counted) : "l"(count), "r"(static_cast<unsigned>(k_split) - 1u) : "memory");
+            }
             if (pending) {
                 tc::bar_wait(mma_done, dphase, failed);
                 tc::fence_after();
@@ -1081,9 +1260,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
             pending = false;
             tc::fence_before();
             if (tile + n_groups >= n_tiles) asm volatile("bar.arrive 7, %0;" ::"n"(kTcDecoders + 32) : "memory");  // tensor memory may go
-            // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
-            // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
-            const int red_rows = a.tc_deal;
             if ((a.fuse & kFuseNorm) && tile == group) {
                 tc::decoders_sync();  // (the last squares have been stored)
                 if (warp < m) {
@@ -1091,19 +1267,26 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                     for (int i = lane; i < step1 - step0; i += 32) sq += __uint_as_float(lds32(norm_parts + (i * MC + warp) * 4));
 #pragma unroll
                     for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, off);
-                    if (k_split == 1) {
+                    if (!clustered) {
                         if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(tc::s32(&s_norm[0][warp])), "f"(sq) : "memory");
                     } else {
-                        if (!announced) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-                        announced = true;
+                        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
                         if (lane < k_split) tc::st_async(tc::in_block(tc::s32(&s_norm[rank][warp]), lane), sq, tc::in_block(tc::s32(&s_cluster), lane));
                     }
                 }
             }
-            const int r0 = rank * red_rows, r1 = r0 + red_rows < kTcRows ? r0 + red_rows : kTcRows;
             float sums[MC];
             acc.get(sums);
             acc.clear();
+            if (!clustered) {
+                if (k_split > 1 && threadIdx.x == 0) s_count = static_cast<int>(counted);
+                tc_finish_tile<TYPE, MC>(a, m, p, tile, tile - tile0, rank, tile + n_groups < n_tiles, red, sums, s_norm[0], &s_count, s_best_v, s_best_i, failed);
+                continue;
+            }
+            // The tile's 256 rows are dealt out to the blocks of the cluster; every block sends each its part of the sums:
+            // red[column range][pair of groups][row of the receiver][activation row], counted in bytes on s_cluster
+            const int red_rows = a.tc_deal;
+            const int r0 = rank * red_rows, r1 = r0 + red_rows < kTcRows ? r0 + red_rows : kTcRows;
 #pragma unroll
             for (int round = 0; round < MC / kOut; ++round) {
             {
@@ -1112,25 +1295,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
 #pragma unroll
                 for (int t = 0; t < kOut; ++t) out[t] = sums[round * kOut + t];
                 const uint32_t to = red + ((rank * 2 + pair) * red_rows + (r - owner * red_rows)) * (kOut * 4);
-                if (k_split == 1) {
-#pragma unroll
-                    for (int t = 0; t < kOut; ++t) asm volatile("st.shared.f32 [%0], %1;" ::"r"(to + t * 4), "f"(out[t]) : "memory");
-                } else {
-                    if (!announced) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-                    announced = true;
-                    if (threadIdx.x == 0) {
-                        const int bytes = (r1 - r0) * (2 * kOut * 4) * k_split + ((a.fuse & kFuseNorm) && tile == group ? m * k_split * 4 : 0);
-                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::s32(&s_cluster)), "r"(bytes) : "memory");
-                    }
-                    tc::st_async_row<kOut>(tc::in_block(to, owner), out, tc::in_block(tc::s32(&s_cluster), owner));
+                // (once per thread: the cluster's barriers are known to exist)
+                if (rounds == 0 && !((a.fuse & kFuseNorm) && warp < m)) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+                if (threadIdx.x == 0) {
+                    const int bytes = (r1 - r0) * (2 * kOut * 4) * k_split + ((a.fuse & kFuseNorm) && tile == group ? m * k_split * 4 : 0);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::s32(&s_cluster)), "r"(bytes) : "memory");
                 }
+                tc::st_async_row<kOut>(tc::in_block(to, owner), out, tc::in_block(tc::s32(&s_cluster), owner));
             }
-            if (k_split == 1) {
-                tc::decoders_sync();
-            } else {
-                tc::bar_wait_cluster(tc::s32(&s_cluster), rphase, failed);
-                rphase ^= 1u;
-            }
+            tc::bar_wait_cluster(tc::s32(&s_cluster), rounds & 1u, failed);
             {
                 const int t = round * kOut + (warp & (kOut - 1));
                 const MatvecPart &part = a.part[p];
@@ -1141,43 +1314,37 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
                         for (int k = 0; k < k_split; ++k) sq += s_norm[k][t];
                         factor = 1.0f / sqrtf(sq / static_cast<float>(a.cols) + a.eps);
                     }
-                    for (int r = r0 + (warp / kOut) * 32 + lane; r < r1; r += 512 / kOut) {
-                        const int row = (tile - tile0) * kTcRows + r;
-                        if (row >= part.rows) break;
+                    for (int r = r0 + (warp / kOut) * 32; r < r1; r += 512 / kOut) {
+                        const int row = (tile - tile0) * kTcRows + r + lane;
+                        const bool exists = r + lane < r1 && row < part.rows;
                         float sum = 0.0f;
+                        if (exists) {
 #pragma unroll
-                        for (int k = 0; k < kMaxSplit; ++k)
-                            if (k < k_split) {
-                                const uint32_t at = red + ((2 * k * red_rows + (r - r0)) * kOut + (warp & (kOut - 1))) * 4;
-                                sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + kOut * red_rows * 4));
-                            }
-                        if (a.fuse & kFuseNorm) sum *= factor;
-                        if (sum != sum) sum = tc_plain_sum<TYPE>(a, part.w + static_cast<size_t>(row) * a.row_bytes, t, factor);
-                        if (part.y != nullptr) {
-                            float *y = part.y + static_cast<size_t>(t) * part.rows + row;
-                            if (a.fuse & kFuseAdd) sum += *y;
-                            *y = sum;
+                            for (int k = 0; k < kMaxSplit; ++k)
+                                if (k < k_split) {
+                                    const uint32_t at = red + ((2 * k * red_rows + (r + lane - r0)) * kOut + (warp & (kOut - 1))) * 4;
+                                    sum += __uint_as_float(lds32(at)) + __uint_as_float(lds32(at + kOut * red_rows * 4));
+                                }
+                            sum = tc_put<TYPE>(a, part, row, t, sum, factor);
                         }
-                        if (tc_better(sum, row, best_v, best_i)) best_v = sum, best_i = row;
+                        if (a.out_idx != nullptr) tc_note_best(exists, sum, row, lane, &s_best_v[warp][t], &s_best_i[warp][t]);
                     }
                 }
             }
             if (round + 1 < MC / kOut || tile + n_groups < n_tiles) {  // the sums may be overwritten once everybody has read them
                 tc::decoders_sync();
-                if (k_split > 1) {
-                    if (threadIdx.x < static_cast<unsigned>(k_split))
-                        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tc::in_block(tc::s32(&s_read), threadIdx.x))
-                                     : "memory");
-                    tc::bar_wait_cluster(tc::s32(&s_read), sphase, failed);
-                    sphase ^= 1u;
-                }
+                if (threadIdx.x < static_cast<unsigned>(k_split))
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tc::in_block(tc::s32(&s_read), threadIdx.x))
+                                 : "memory");
+                tc::bar_wait_cluster(tc::s32(&s_read), rounds & 1u, failed);
             }
+            ++rounds;
             }
         }
     }
-    if (k_split > 1 && warp >= 16) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // (every thread takes part)
+    if (clustered && warp >= 16) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");  // (every thread takes part)
     if (lane == 0 && *failed) atomicCAS(a.status, 0u, kStatusWaitExpired);
-    if (a.out_idx != nullptr) tc_finish_argmax<MC>(a, m, best_v, best_i, warp, lane, s_best_v, s_best_i, &s_last);
+    if (a.out_idx != nullptr) tc_finish_argmax(a, m, warp, lane, s_best_v, s_best_i, &s_last);
 }
 
 }  // namespace vqm

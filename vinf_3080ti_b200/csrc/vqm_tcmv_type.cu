@@ -40,7 +40,8 @@ struct TcVariant {
         return n;
     }
 
-    static void configure(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int grid, int k_split, int overlap, cudaStream_t stream) {
+    // cluster: blocks of a cluster
+    static void configure(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, int grid, int cluster, int overlap, cudaStream_t stream) {
         cfg.gridDim = dim3(static_cast<unsigned>(grid));
         cfg.blockDim = dim3(kTcThreads);
         cfg.dynamicSmemBytes = kSmem;
@@ -51,9 +52,9 @@ struct TcVariant {
             attr[n].val.programmaticStreamSerializationAllowed = 1;
             ++n;
         }
-        if (k_split > 1) {
+        if (cluster > 1) {
             attr[n].id = cudaLaunchAttributeClusterDimension;
-            attr[n].val.clusterDim.x = static_cast<unsigned>(k_split);
+            attr[n].val.clusterDim.x = static_cast<unsigned>(cluster);
             attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
             ++n;
         }
@@ -61,16 +62,18 @@ struct TcVariant {
         cfg.numAttrs = n;
     }
 
-    static cudaError_t launch(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int n_tiles, int m, int sm_count, cudaStream_t stream) {
-        const int fit = clusters(a.k_split, sm_count);
+    static cudaError_t launch(TcMatvecArgs &a, const CUtensorMap *const *maps, int n_parts, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+        const bool clustered = a.k_split > 1 && a.partials == nullptr;
+        const int fit = clustered ? clusters(a.k_split, sm_count) : clusters(1, sm_count) / a.k_split;
         if (fit == 0) return cudaErrorInvalidConfiguration;
-        const int grid = (n_tiles < fit ? n_tiles : fit) * a.k_split;
+        a.tc_groups = n_tiles < fit ? n_tiles : fit;
+        a.tc_split_recip = 65536 / a.k_split + 1;
         MAPS packed;
         for (int p = 0; p < static_cast<int>(sizeof(packed.m) / sizeof(packed.m[0])); ++p)
             for (int c = 0; c < 8; ++c) packed.m[p][c] = maps[p < n_parts ? p : 0][c];
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute attr[2];
-        configure(cfg, attr, grid, a.k_split, a.overlap_launch, stream);
+        configure(cfg, attr, a.tc_groups * a.k_split, clustered ? a.k_split : 1, a.overlap_launch, stream);
         return cudaLaunchKernelEx(&cfg, kKernel, a, packed, m);
     }
 };
@@ -149,7 +152,7 @@ inline int choose_tc_split(int n_tiles, int cols, int sm_count, bool single) {
 template <int TYPE>
 constexpr int wide_rows() { return tc_twenty_four<TYPE>() ? 24 : tc_sixteen(TYPE) ? 16 : 8; }
 template <int TYPE, int MC>
-cudaError_t launch_wide(const TcMatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
+cudaError_t launch_wide(TcMatvecArgs &a, const CUtensorMap *const *maps, int n_tiles, int m, int sm_count, cudaStream_t stream) {
     if constexpr (MC <= wide_rows<TYPE>()) {
         if (a.x_split == nullptr || a.fuse != 0 || a.out_idx != nullptr) return cudaErrorInvalidValue;
         return TcVariant<(TYPE >= 0 ? MC : 0), TcMaps1>::launch(a, maps, 1, n_tiles, m, sm_count, stream);
@@ -181,10 +184,15 @@ cudaError_t split_wide(const MatvecArgs &a, uint8_t *x_split, int m, cudaStream_
 }
 
 // Tiles [first, end) of a launch.
-inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int first, int end, int m,
+inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const TcScratch &scratch, int first, int end, int m,
                                 int sm_count, cudaStream_t stream, int *n_launched) {
     TcMatvecArgs a{args};
-    a.x_split = x_split;
+    a.x_split = scratch.x_split;
+    // (every block has a record: not where a block takes several tiles)
+    if (scratch.partials != nullptr && a.k_split > 1 && (end - first) * a.k_split <= sm_count) {
+        a.partial_counts = reinterpret_cast<unsigned *>(scratch.partials);
+        a.partials = reinterpret_cast<float *>(scratch.partials + tc_partial_count_bytes(sm_count));
+    }
     const int n_steps = (a.cols + kTcStepCols - 1) / kTcStepCols;
     for (int k = 0; k <= a.k_split; ++k) a.tc_steps[k] = k * n_steps / a.k_split;
     a.tc_deal = (kTcRows + a.k_split - 1) / a.k_split;
@@ -225,17 +233,17 @@ cudaError_t VQM_CAT(launch_split_, VQM_TYPE_NAME)(const MatvecArgs &a, uint8_t *
     return m <= 16 ? split_wide<VQM_TYPE, 16>(a, x_split, m, stream, n_launched) : split_wide<VQM_TYPE, 24>(a, x_split, m, stream, n_launched);
 }
 
-cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const uint8_t *x_split, int m,
+cudaError_t VQM_CAT(launch_tcmv_, VQM_TYPE_NAME)(const MatvecArgs &args, const CUtensorMap *const *maps, int n_parts, const TcScratch &scratch, int m,
                                                  int sm_count, cudaStream_t stream, int *n_launched) {
     const int n_tiles = tc_tiles(args);
     const TcTail tail = takes_tail(args) ? choose_tc_tail(n_tiles, args.cols, sm_count, args.k_split) : TcTail{};
-    if (tail.first == 0) return launch_tiles(args, maps, n_parts, x_split, 0, n_tiles, m, sm_count, stream, n_launched);
+    if (tail.first == 0) return launch_tiles(args, maps, n_parts, scratch, 0, n_tiles, m, sm_count, stream, n_launched);
     // the whole rounds, then the rest
-    const cudaError_t err = launch_tiles(args, maps, n_parts, x_split, 0, tail.first, m, sm_count, stream, n_launched);
+    const cudaError_t err = launch_tiles(args, maps, n_parts, scratch, 0, tail.first, m, sm_count, stream, n_launched);
     if (err != cudaSuccess) return err;
     MatvecArgs a = args;
     a.k_split = tail.k_split;
-    return launch_tiles(a, maps, n_parts, x_split, tail.first, n_tiles, m, sm_count, stream, n_launched);
+    return launch_tiles(a, maps, n_parts, scratch, tail.first, n_tiles, m, sm_count, stream, n_launched);
 }
 
 }  // namespace vqm
