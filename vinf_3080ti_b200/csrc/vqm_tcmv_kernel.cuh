@@ -877,12 +877,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tcmv_kernel(const __grid_consta
     int group = static_cast<int>((blockIdx.x * static_cast<unsigned>(a.tc_split_recip)) >> 16), n_groups = a.tc_groups;
     const int rank = static_cast<int>(blockIdx.x) - group * k_split;
     const int step0 = a.tc_steps[rank], step1 = a.tc_steps[rank + 1];
+    constexpr bool kSingle = sizeof(MAPS) == sizeof(TcMaps1);  // one tensor: nothing to look up
     auto tiles_of = [&](int p) { return (a.part[p].rows + kTcRows - 1) / kTcRows; };
-    const int end0 = tiles_of(0), end1 = end0 + tiles_of(1), end2 = end1 + tiles_of(2), n_tiles = a.tc_end;
+    const int end0 = kSingle ? 0 : tiles_of(0), end1 = kSingle ? 0 : end0 + tiles_of(1), end2 = kSingle ? 0 : end1 + tiles_of(2), n_tiles = a.tc_end;
     group += a.tc_first;
     // the tensor a tile belongs to, and that tensor's first tile
-    auto part_of = [&](int tile) { return (tile >= end0) + (tile >= end1) + (tile >= end2); };
-    auto first_tile = [&](int p) { return p == 0 ? 0 : p == 1 ? end0 : p == 2 ? end1 : end2; };
+    auto part_of = [&](int tile) { return kSingle ? 0 : (tile >= end0) + (tile >= end1) + (tile >= end2); };
+    auto first_tile = [&](int p) { return kSingle || p == 0 ? 0 : p == 1 ? end0 : p == 2 ? end1 : end2; };
 
     // ---- copy side: stage s of a step holds, per row class, 32 rows of kPitch bytes, then the activation rows ----
     auto class_mis = [&](const MatvecPart &p, int c) {
