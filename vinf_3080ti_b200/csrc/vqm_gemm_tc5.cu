@@ -49,12 +49,14 @@ constexpr int kAThreads = 512;             // decoder warps 0-15
 constexpr int kTThreads = kAThreads + 96;  // warp 16: activation tiles; warp 17: MMAs; warp 18: raw weights
 // Raw-block ring: a "run" is 256 weight columns of the 128 rows; a row's bytes of one run are contiguous.
 constexpr int kRawCols = 256, kStagesPerRun = kRawCols / kTK;
-__host__ __device__ constexpr int raw_buffers(int nh) { return nh == 1 ? 3 : 2; }
 __host__ __device__ constexpr int raw_run_bytes(int type) { return kRawCols / chunk_block(type) * chunk_block_bytes(type); }
 __host__ __device__ constexpr int raw_pitch(int type) { return tc_pitch(type); }  // bytes of a row in a buffer
+// (Q8_0, whose buffers are the largest, has two: three leave room for two stages of weights.  17408 x 5120, 64 and 256 rows: 53 and 61 us, 48 and
+// 56 so.)
+__host__ __device__ constexpr int raw_buffers(int type, int nh) { return nh == 1 && raw_pitch(type) < 256 ? 3 : 2; }
 __host__ __device__ constexpr int table_bytes16(int type) { return grid_bytes(type) > 0 ? (grid_bytes(type) + 15) / 16 * 16 : 16; }
 __host__ __device__ constexpr bool raw_staged(int type) { return raw_run_bytes(type) <= 288; }  // every quantised type
-__host__ __device__ constexpr int raw_ring_bytes(int type, int nh) { return raw_staged(type) ? raw_buffers(nh) * kTM * raw_pitch(type) + 16 : 0; }
+__host__ __device__ constexpr int raw_ring_bytes(int type, int nh) { return raw_staged(type) ? raw_buffers(type, nh) * kTM * raw_pitch(type) + 16 : 0; }
 // Activation tiles in flight (32 KB each in blocks of two accumulators), and as many weight tiles as fit beside them.
 __host__ __device__ constexpr int x_stages(int nh) { return nh == 1 ? 4 : 3; }
 __host__ __device__ constexpr int tc5_smem_bytes(int type, int nh, int stages) {
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
                                                                  unsigned *status) {
     constexpr int CPB = chunk_block(TYPE) / 8, BB = chunk_block_bytes(TYPE);
     constexpr int TABLE = table_bytes16(TYPE);
-    constexpr int kTStages = stages_for(TYPE, NH), kXStages = x_stages(NH), kRaw = raw_buffers(NH);
+    constexpr int kTStages = stages_for(TYPE, NH), kXStages = x_stages(NH) < kTStages ? x_stages(NH) : kTStages, kRaw = raw_buffers(TYPE, NH);
     constexpr bool kStaged = raw_staged(TYPE);
     // Decoder warps of a stage, and groups that take turns: a group must not run two uses of a stage ahead of another, the
     // parity of the barriers would not tell them apart, so there are no more groups than stages.
@@ -312,7 +314,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     static_assert(kGroups <= kTStages, "barrier phases");
     constexpr uint32_t kTmemCols = 256 * NH;
     extern __shared__ uint8_t tc5_raw[];
-    __shared__ __align__(8) uint64_t s_full[kMaxStages], s_empty[kMaxStages], s_xfull[4], s_xempty[4], s_done, s_raw_full[3], s_raw_empty[3];
+    __shared__ __align__(8) uint64_t s_full[kMaxStages], s_empty[kMaxStages], s_done, s_raw_full[3], s_raw_empty[3];
     __shared__ uint32_t s_tmem;
     __shared__ int s_failed;
     // table first, then the stages on a 1024-byte boundary (the swizzle works on absolute shared-memory address bits)
@@ -334,14 +336,10 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kTStages; ++s) {
-            // one arrive per decoder warp of the group that fills the stage, and in the first block of a pair one more for the
-            // second block's stage
-            bar_init(s32(&s_full[s]), kGroupWarps + (rank == 0 ? 1 : 0));
+            // one arrive per decoder warp of the group that fills the stage, the feeding thread's with the byte count of the activation tile
+            // that goes with it, and in the first block of a pair one more for the second block's stage
+            bar_init(s32(&s_full[s]), kGroupWarps + 1 + (rank == 0 ? 1 : 0));
             bar_init(s32(&s_empty[s]), 1);
-        }
-        for (int s = 0; s < kXStages; ++s) {
-            bar_init(s32(&s_xfull[s]), 1);  // the feeding thread's arrive with the tile's byte count
-            bar_init(s32(&s_xempty[s]), 1);
         }
         bar_init(s32(&s_done), 1);
         for (int b = 0; b < kRaw; ++b) {
@@ -367,8 +365,6 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     __syncthreads();
     cluster_sync_all();  // the other blocks' barriers and tensor memory exist before anybody signals or multiplies
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // (the next conversion of activations may be launched; it waits for this kernel's end before it touches anything)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem = s_tmem;
     volatile int *failed = &s_failed;
 
@@ -434,7 +430,9 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     } else if (warp == 16) {
         // ---- activation tiles: one thread, one TMA tile copy per accumulator and stage (64 columns x half of the
         //      accumulator's activation rows, in the same 128-byte swizzle; no multicast; rows beyond ntok arrive as zeros).
-        //      A buffer is refilled once its MMAs are done.
+        //      A buffer is refilled once its MMAs are done, which "empty" of their stage says; a tile's bytes are counted on "full" of its
+        //      stage.  (With barriers of their own for the activations the MMA warp waited and committed twice per stage.  64 rows of Q4_K
+        //      17408 x 5120 40.7 and 39.4 us so, 2048 rows of 5120 x 17408 347 and 341.)
         if (lane == 0) {
             // The kernel is launched while the conversion of the activations may still run (programmatic stream
             // serialization); this thread is the only reader of its output.
@@ -442,9 +440,9 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
             const int half = n_acc / 2;
             int k = 0;
             for (; k < n_k; ++k) {
-                const int stage = k % kXStages, use = k / kXStages;
-                if (!bar_wait(s32(&s_xempty[stage]), (use & 1) ^ 1, failed)) break;
-                const uint32_t bar = s32(&s_xfull[stage]);
+                const int stage = k % kXStages, before = k - kXStages;
+                if (before >= 0 && !bar_wait(s32(&s_empty[before % kTStages]), (before / kTStages) & 1, failed)) break;
+                const uint32_t bar = s32(&s_full[k % kTStages]);
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(NH * half * 128) : "memory");
 #pragma unroll
                 for (int nh = 0; nh < NH; ++nh)
@@ -455,7 +453,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
             }
             // the last tiles land before the block may leave, also when a wait gave up (bounded)
             for (int last = k > kXStages ? k - kXStages : 0; last < k; ++last)
-                for (int i = 0; i < (1 << 16) && !bar_try(s32(&s_xfull[last % kXStages]), (last / kXStages) & 1); ++i) __nanosleep(64);
+                for (int i = 0; i < (1 << 16) && !bar_try(s32(&s_full[last % kTStages]), (last / kTStages) & 1); ++i) __nanosleep(64);
         }
         __syncwarp();
     } else if (warp == 17) {
@@ -463,8 +461,6 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
             // ---- second block of a pair: tell the first block about every stage that is full here
             for (int q = 0; q < n_k; ++q) {
                 const int stage = q % kTStages;
-                // (and the activation tile that goes with it)
-                if (!warp_wait(s32(&s_xfull[q % kXStages]), (q / kXStages) & 1, failed)) break;
                 if (!warp_wait(s32(&s_full[stage]), (q / kTStages) & 1, failed)) break;
                 if (lane == 0) bar_arrive_cluster(in_block(s32(&s_full[stage]), static_cast<int>(in_cluster & ~1u)));
             }
@@ -473,7 +469,6 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
             const uint32_t idesc = (1u << 4) | (static_cast<uint32_t>(n_acc >> 3) << 17) | ((256u >> 4) << 24);
             for (int q = 0; q < n_k; ++q) {
                 const int stage = q % kTStages, xs = q % kXStages;
-                if (!warp_wait(s32(&s_xfull[xs]), (q / kXStages) & 1, failed)) break;  // the stage's activation tile
                 if (!__all_sync(0xFFFFFFFFu, bar_wait_cluster(s32(&s_full[stage]), (q / kTStages) & 1, failed) ? 1 : 0)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (tc::elect_one()) {
@@ -485,7 +480,6 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
                             mma_f16_pair(tmem + nh * 256, a_desc + 2 * j, b_desc + 2 * j + ((nh * kTB) >> 4), idesc, (q | j) != 0);
                     // the buffers are free again, in both blocks of the pair, once these MMAs have read them
                     mma_commit_pair(s32(&s_empty[stage]), static_cast<uint32_t>(pair));
-                    mma_commit_pair(s32(&s_xempty[xs]), static_cast<uint32_t>(pair));
                 }
                 __syncwarp();
             }
@@ -525,6 +519,10 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
     bool ok = true;
     if (warp < 16) {
         ok = warp_wait(s32(&s_done), 0, failed);
+        // (The next conversion of activations may be launched; it waits for this kernel's end before it touches anything.  Requested at the start
+        // of a block, that conversion and the GEMM behind it take SMs that other streams could use: three streams, 1500 rows of Q4_K 17408 x
+        // 5120 211 to 243 us, 200 so, 512 rows of four tensors 285 to 296 and 281 to 290.)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     auto read16 = [&](uint32_t at, float (&v)[16]) {
