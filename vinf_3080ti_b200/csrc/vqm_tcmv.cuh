@@ -48,8 +48,7 @@
 
 namespace vqm {
 
-// (608 threads cap every thread at 96 registers.  IQ4_XS with 2 and 8 rows and the 16-row kernels of Q4_K, Q5_K, Q2_K and IQ2_S spill 16 to 30
-// bytes, all 24-row kernels 64 to 84.)
+// (608 threads cap every thread at 96 registers.  The 16-row kernels of Q4_K, Q5_K, Q6_K and Q2_K spill 8 to 44 bytes, all 24-row kernels 8 to 52.)
 constexpr int kTcRows = kTcTileRows, kTcStepCols = 256, kTcDecoders = 512, kTcThreads = kTcDecoders + 96;
 constexpr int kTcCore = 144;                      // bytes from one 8-column core matrix of B to the next (128 + 16: no bank conflicts)
 constexpr int kTcInfoSlots = 8;                   // ring of per-step activation scales and group sums
