@@ -821,13 +821,8 @@ template <int TYPE, int MC>
 __global__ void __launch_bounds__(16 * 32) tc_split_kernel(const __grid_constant__ MatvecArgs a, uint8_t *out, const int t0, const int m) {
     constexpr int kOperand = TcShape<TYPE, MC>::kGroupsB * tc_group_b(TYPE), kBytes = tc_split_bytes<TYPE, MC>();
     __shared__ __align__(16) uint8_t image[kBytes];
-    // Of two launches (more than 16 rows) the second starts once the first has found its inputs there, so it need not wait for them; it waits for
-    // the first's end before its own, for whoever waits for it.  (Q6_K 6144 x 5120, Q3_K 17408 x 5120 and Q4_K 5120 x 17408, 24 rows, three
-    // streams: 82.3 us one after the other, 80.4 side by side; Q6_K alone 28.7 and 26.1.)
-    const bool first = t0 == 0, last = t0 + 16 >= m;
-    if (last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int step = blockIdx.x, t = t0 + static_cast<int>(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int cols_here = a.cols - step * kTcStepCols < kTcStepCols ? a.cols - step * kTcStepCols : kTcStepCols;
     if (t < m) {
@@ -844,7 +839,6 @@ __global__ void __launch_bounds__(16 * 32) tc_split_kernel(const __grid_constant
         }
         to[i] = reinterpret_cast<const uint4 *>(image)[i];
     }
-    if (!first) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <int TYPE, int MC, typename MAPS>
