@@ -104,10 +104,21 @@ constexpr size_t tc_partial_count_bytes(int sm_count) { return (static_cast<size
 constexpr size_t tc_partial_bytes(int sm_count, int m) {
     return tc_partial_count_bytes(sm_count) + static_cast<size_t>(sm_count) * (m <= 8 ? 2 * (4 * kTcTileRows + 32) : 12 * (2 * kTcTileRows + 32)) * 4;
 }
+constexpr size_t kTcPartialAlign = 256;  // of the room's address; the kernels' accesses to it are of up to 16 bytes
+// Size of the scratch for the B operands of more than 8 activation rows that is to hold `need` bytes where `present` do not: a multiple of
+// kTcPartialAlign, because room for partial sums lies behind it.  At most 42 KB per 256 columns; 4 MB hold 24576 columns of any type, so that a
+// runtime allocates once (with 3.9 MB for partial sums behind them).  (cudaMalloc takes 330 us for any size from 1 to 16 MB; with 2 MB, which
+// tensors of more than 12288 columns outgrow, to bind three tensors and their buffers of 24 rows took 1720 us instead of 1480.)  It grows by half
+// at least: what it has outgrown, which captured graphs may use, is together at most twice its size.
+constexpr size_t tc_grown_split_bytes(size_t need, size_t present) {
+    size_t bytes = need < (4u << 20) ? 4u << 20 : need;
+    if (bytes < present + present / 2) bytes = present + present / 2;
+    return (bytes + kTcPartialAlign - 1) / kTcPartialAlign * kTcPartialAlign;
+}
 struct TcScratch {
     const uint8_t *x_split = nullptr;  // the B operands of more than 8 activation rows
-    // Room for partial sums, in use by one launch at a time: counts zero and sums empty (bytes of 0xFF) before and after it.  Null: the blocks that
-    // share columns are clusters and exchange sums in shared memory.  The outputs are the same, bit for bit.
+    // Room for partial sums, aligned to kTcPartialAlign, in use by one launch at a time: counts zero and sums empty (bytes of 0xFF) before and
+    // after it.  Null: the blocks that share columns are clusters and exchange sums in shared memory.  The outputs are the same, bit for bit.
     uint8_t *partials = nullptr;
 };
 // The tensor-core matvec (vqm_tcmv_type.cu).  maps: per tensor of the launch its tensor maps (tc_encode_maps).

@@ -534,11 +534,7 @@ int launch_group(vqm_runtime *rt, Tensor &t, const float *x, float *y, int m, bo
 // pass that finds the room missing may be one that is being captured, by this runtime or by another library.
 bool make_split_room(vqm_runtime *rt) {
     if (rt->split_need <= rt->x_split_bytes) return true;
-    // At most 42 KB per 256 columns; 4 MB hold 24576 columns of any type, so that a runtime allocates once (with 3.9 MB for partial sums behind them).  (cudaMalloc takes 330 us for
-    // any size from 1 to 16 MB; with 2 MB, which tensors of more than 12288 columns outgrow, to bind three tensors and their buffers of 24 rows
-    // took 1720 us instead of 1480.)
-    size_t bytes = rt->split_need < (4u << 20) ? 4u << 20 : rt->split_need;
-    if (bytes < rt->x_split_bytes + rt->x_split_bytes / 2) bytes = rt->x_split_bytes + rt->x_split_bytes / 2;
+    const size_t bytes = vqm::tc_grown_split_bytes(rt->split_need, rt->x_split_bytes);
     uint8_t *p = nullptr;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);

@@ -188,6 +188,7 @@ inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const
                                 int sm_count, cudaStream_t stream, int *n_launched) {
     TcMatvecArgs a{args};
     a.x_split = scratch.x_split;
+    if (reinterpret_cast<uintptr_t>(scratch.partials) % kTcPartialAlign != 0) return cudaErrorInvalidValue;
     // (every block has a record: not where a block takes several tiles)
     if (scratch.partials != nullptr && a.k_split > 1 && (end - first) * a.k_split <= sm_count) {
         a.partial_counts = reinterpret_cast<unsigned *>(scratch.partials);
