@@ -544,8 +544,9 @@ bool make_split_room(vqm_runtime *rt) {
         (void)cudaGetLastError();
         return false;
     }
-    // (beside a capture: by the first launch that needs it)
-    rt->split_emptied = !rt->capturing && !is_capturing(rt->stream) && empty_partials(rt, p + bytes, 24, rt->stream) == cudaSuccess;
+    // (Beside a capture: by the first launch that needs it.  Likewise where another stream's last use of the scratch has not been waited for:
+    // to use it here would forget that one, and graphs may use what is retired.)
+    rt->split_emptied = !rt->split_wait && !rt->capturing && !is_capturing(rt->stream) && empty_partials(rt, p + bytes, 24, rt->stream) == cudaSuccess;
     if (rt->split_emptied) rt->split_used = true;  // (what uses it on another stream comes after that)
     if (rt->x_split != nullptr) rt->retired.push_back(rt->x_split);
     rt->x_split = p;
