@@ -70,6 +70,7 @@ SIGNATURES: dict[str, list] = {
     "vqm_graph_launch": [c_void_p, c_int],
     "vqm_graph_destroy": [c_void_p, c_int],
     "vqm_launch_count": [c_void_p, POINTER(c_uint64)],
+    "vqm_memory_exchange_count": [c_void_p, POINTER(c_uint64)],
     "vqm_exchange_create": [c_void_p, c_size_t, c_void_p, POINTER(c_uint64)],
     "vqm_exchange_open": [c_void_p, c_void_p, POINTER(c_uint64)],
     "vqm_exchange_config": [c_void_p, c_int, c_int, POINTER(c_uint64), c_size_t, c_size_t, c_int],

@@ -98,8 +98,14 @@ VQM_FOR_EACH_TYPE(VQM_DECLARE_LAUNCHER)
 
 constexpr int kTcTileRows = 256;   // rows of a tile of the tensor-core matvec
 constexpr int kTcMaxMagnitude = 66;  // of a codebook, for the tensor-core matvec: times 31 it has to fit into the 11 bits of fp16
-// Room for the partial sums of a launch whose columns are split (at most sm_count / 2 tiles, sm_count blocks): the counts, then the records of
-// tc_finish_tile, 2 of a block for up to 8 activation rows, 12 smaller ones for 24.
+inline int tc_tiles(const MatvecArgs &a) {
+    int n = 0;
+    for (int p = 0; p < kMaxParts; ++p) n += (a.part[p].rows + kTcTileRows - 1) / kTcTileRows;
+    return n;
+}
+// Room for the partial sums of a launch whose columns are split.  It holds a record of every block of one that takes each tile at once (not where
+// blocks take several tiles): at most sm_count / 2 tiles, sm_count blocks.  The counts, then the records of tc_finish_tile, 2 of a block for up to 8 activation rows, 12 smaller ones for 24.
+constexpr bool tc_partials_hold(int n_tiles, int k_split, int sm_count) { return static_cast<long long>(n_tiles) * k_split <= sm_count; }
 constexpr size_t tc_partial_count_bytes(int sm_count) { return (static_cast<size_t>(sm_count) * 4 + 255) / 256 * 256; }
 constexpr size_t tc_partial_bytes(int sm_count, int m) {
     return tc_partial_count_bytes(sm_count) + static_cast<size_t>(sm_count) * (m <= 8 ? 2 * (4 * kTcTileRows + 32) : 12 * (2 * kTcTileRows + 32)) * 4;

@@ -79,6 +79,13 @@ const int kCodebookTypes[5] = {vqm::kIQ2_XXS, vqm::kIQ2_XS, vqm::kIQ2_S, vqm::kI
 constexpr int kDirectRows = 16384;
 constexpr size_t kStatusWords = 4;  // status word of a synchronous matvec, padded to 16 bytes
 
+// A stream's room for partial sums (see find_partials).
+struct StreamPartials {
+    unsigned long long stream;  // its id: ids, unlike handles, do not come again
+    uint8_t *room;
+    bool emptied;  // the room is as launches find and leave it
+};
+
 struct vqm_runtime {
     int device = 0;
     int sm_count = 0;
@@ -110,12 +117,10 @@ struct vqm_runtime {
     cudaStream_t split_stream = nullptr;
     cudaEvent_t split_event = nullptr;
     std::vector<uint8_t *> retired;  // smaller ones, which captured graphs may use (together at most twice the present one)
-    // Partial sums of matvecs whose columns are split (vqm::TcScratch).  Launches on different streams may overlap, so each stream has its own,
-    // known by the stream's id (ids, unlike handles, do not come again).  Of more than 8 activation rows: behind x_split, which one stream at a
-    // time uses.
-    std::vector<std::pair<unsigned long long, uint8_t *>> stream_partials;
-    uint8_t *partials = nullptr;  // of the present stream; null: none, clusters exchange the sums
-    bool split_emptied = false;   // those behind x_split are ready
+    // Partial sums of matvecs whose columns are split (vqm::TcScratch).  Launches on different streams may overlap, so each stream has its own.
+    // Of more than 8 activation rows: behind x_split, which one stream at a time uses.
+    std::vector<StreamPartials> stream_partials;
+    bool split_emptied = false;   // those behind x_split are as launches find and leave them
     void *pinned = nullptr;  // host staging of the synchronous matvec: x on the way in, status and outputs on the way out
     size_t pinned_bytes = 0;
     void *gemm_x = nullptr;  // fp16 copy of the activations of a prompt pass
@@ -130,6 +135,7 @@ struct vqm_runtime {
     int overlap_launch = 1;  // programmatic dependent launch of consecutive matvecs (VINF_B200_NO_PDL=1 turns it off)
     bool capturing = false;
     uint64_t launches = 0, capture_launches = 0;
+    uint64_t memory_exchanges = 0;  // launches that exchanged partial sums through memory
     bool capture_uses_gemm_x = false, capture_uses_split = false;
     std::vector<Graph> graphs;
     // file loader: per reader thread two pinned staging slots, a copy stream and an event per slot (created on first use)
@@ -360,43 +366,45 @@ bool is_capturing(cudaStream_t stream) {
     return true;
 }
 
-// The present stream's room for partial sums.  (Runtimes that keep changing streams have it for the first four.)
+// The present stream's room for partial sums, null if there is none.  (Runtimes that keep changing streams have it for the first four.)  Looked
+// up by every launch, and made ready where a stream is set, so that its first launch need not: a handle says nothing about the stream behind
+// it (cudaStreamPerThread, a stream destroyed and another created), and what could not be done then (beside a capture, or with all rooms taken)
+// is done when it can be.
 constexpr size_t kMaxStreamPartials = 4;
-void find_partials(vqm_runtime *rt) {
-    rt->partials = nullptr;
+uint8_t *find_partials(vqm_runtime *rt) {
     unsigned long long id = 0;
     if (is_capturing(rt->stream) || cudaStreamGetId(rt->stream, &id) != cudaSuccess) {
         (void)cudaGetLastError();
-        return;
+        return nullptr;
     }
-    for (const auto &known : rt->stream_partials)
-        if (known.first == id) rt->partials = known.second;
-    if (rt->partials != nullptr || rt->stream_partials.size() >= kMaxStreamPartials) return;
-    uint8_t *const room = take_partials(rt->sm_count);
-    if (room == nullptr) return;
-    rt->stream_partials.emplace_back(id, room);
-    if (empty_partials(rt, room, 8, rt->stream) == cudaSuccess) rt->partials = room;
+    StreamPartials *mine = nullptr;
+    for (StreamPartials &known : rt->stream_partials)
+        if (known.stream == id) mine = &known;
+    if (mine == nullptr) {
+        if (rt->stream_partials.size() >= kMaxStreamPartials) return nullptr;
+        uint8_t *const room = take_partials(rt->sm_count);
+        if (room == nullptr) return nullptr;
+        rt->stream_partials.push_back(StreamPartials{id, room, false});
+        mine = &rt->stream_partials.back();
+    }
+    if (!mine->emptied) mine->emptied = empty_partials(rt, mine->room, 8, rt->stream) == cudaSuccess;
+    return mine->emptied ? mine->room : nullptr;
 }
 
 // Room for the partial sums of the next launch, none while a graph is captured: it may run beside other work, on any stream.  (Beside
 // nothing else, as a captured decode pass, clusters exchange them faster too: the 27B model's pass of 4 rows 4.84 ms, 4.94 through memory.)
 uint8_t *partials_now(vqm_runtime *rt, int m) {
-    if (rt->capturing || is_capturing(rt->stream)) return nullptr;
-    if (m <= 8) return rt->partials;
+    if (rt->capturing) return nullptr;
+    if (m <= 8) return find_partials(rt);
+    if (is_capturing(rt->stream)) return nullptr;
     uint8_t *const room = rt->x_split + rt->x_split_bytes;  // (claim_split has been called)
     if (!rt->split_emptied) rt->split_emptied = empty_partials(rt, room, 24, rt->stream) == cudaSuccess;
     return rt->split_emptied ? room : nullptr;
 }
-// After a wait gave up, records may not be as launches leave them.  (What other streams still run may use theirs: those streams have clusters
-// from now on.)
+// After a wait gave up, records may not be as launches leave them: the next launch on each stream empties them, behind what the stream
+// still runs.
 void renew_partials(vqm_runtime *rt) {
-    for (auto &known : rt->stream_partials) {
-        if (known.second == rt->partials && rt->partials != nullptr) {
-            if (empty_partials(rt, known.second, 8, rt->stream) != cudaSuccess) rt->partials = nullptr;
-        } else {
-            known.first = ULLONG_MAX;  // (no stream's id)
-        }
-    }
+    for (StreamPartials &known : rt->stream_partials) known.emptied = false;
     rt->split_emptied = false;
 }
 
@@ -513,7 +521,8 @@ int launch_parts(vqm_runtime *rt, int n, Tensor *const *ts, const float *x, floa
         }
         vqm::TcScratch scratch;
         scratch.x_split = rt->x_split;
-        if (a.k_split > 1) scratch.partials = partials_now(rt, m);
+        if (err == cudaSuccess && a.k_split > 1 && vqm::tc_partials_hold(vqm::tc_tiles(a), a.k_split, rt->sm_count)) scratch.partials = partials_now(rt, m);
+        if (scratch.partials != nullptr) ++rt->memory_exchanges;
         if (err == cudaSuccess) err = dispatch_tcmv(t0.type, a, maps, n, scratch, m, rt->sm_count, rt->stream, &launched);
     } else {
         err = dispatch_qmv(t0.type, a, m, rt->sm_count, rt->stream, nullptr);
@@ -699,7 +708,7 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
         return rc;
     }
     rt->done_counter = rt->status + 16;
-    find_partials(rt);
+    (void)find_partials(rt);
     if (const char *e = getenv("VINF_B200_NO_PDL"); e != nullptr && e[0] == '1') rt->overlap_launch = 0;
     if (const char *e = getenv("VINF_B200_NO_SPLIT"); e != nullptr && e[0] == '1') rt->allow_split = 0;
     if (const char *e = getenv("VINF_B200_GEMM"); e != nullptr && strcmp(e, "mma") == 0) rt->gemm_tcgen05 = 0;
@@ -717,10 +726,8 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
 void vqm_runtime_destroy(vqm_runtime *rt) {
     if (rt == nullptr) return;
     if (rt->stream != nullptr) cudaStreamSynchronize(rt->stream);
-    for (const auto &known : rt->stream_partials) {
-        if (known.second != rt->partials) cudaDeviceSynchronize();  // (another stream's work)
-        give_partials_back(known.second);
-    }
+    if (rt->stream_partials.size() > 1) cudaDeviceSynchronize();  // (other streams' work)
+    for (const StreamPartials &known : rt->stream_partials) give_partials_back(known.room);
     rt->stream = rt->own_stream;
     for (auto &g : rt->graphs)
         if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
@@ -1409,9 +1416,8 @@ int vqm_set_stream(vqm_runtime *rt, void *stream) {
     const cudaStream_t next = stream != nullptr ? static_cast<cudaStream_t>(stream) : rt->own_stream;
     const cudaError_t err = leave_stream(rt, next);
     if (err != cudaSuccess) return cuda_fail("set_stream", err);
-    if (next == rt->stream) return VQM_OK;
     rt->stream = next;
-    find_partials(rt);
+    (void)find_partials(rt);
     return VQM_OK;
 }
 
@@ -1464,6 +1470,11 @@ int vqm_graph_destroy(vqm_runtime *rt, int graph_id) {
 
 int vqm_launch_count(vqm_runtime *rt, uint64_t *out) {
     *out = rt->launches;
+    return VQM_OK;
+}
+
+int vqm_memory_exchange_count(vqm_runtime *rt, uint64_t *out) {
+    *out = rt->memory_exchanges;
     return VQM_OK;
 }
 

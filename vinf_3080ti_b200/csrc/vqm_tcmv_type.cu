@@ -78,12 +78,6 @@ struct TcVariant {
     }
 };
 
-inline int tc_tiles(const MatvecArgs &a) {
-    int n = 0;
-    for (int p = 0; p < kMaxParts; ++p) n += (a.part[p].rows + kTcRows - 1) / kTcRows;
-    return n;
-}
-
 // Tall tensors, whose blocks walk whole rows: the last round of tiles may occupy a few SMs only (LM head, 151936 rows: 594 tiles
 // on 148 SMs, 2 of them in a fifth round).  Its tiles then go to a second launch that splits their columns, if that saves more
 // than a launch costs (3.4 us, two to three steps).  first: its first tile, 0 if there is none.
@@ -188,9 +182,8 @@ inline cudaError_t launch_tiles(const MatvecArgs &args, const CUtensorMap *const
                                 int sm_count, cudaStream_t stream, int *n_launched) {
     TcMatvecArgs a{args};
     a.x_split = scratch.x_split;
-    if (reinterpret_cast<uintptr_t>(scratch.partials) % kTcPartialAlign != 0) return cudaErrorInvalidValue;
-    // (every block has a record: not where a block takes several tiles)
-    if (scratch.partials != nullptr && a.k_split > 1 && (end - first) * a.k_split <= sm_count) {
+    if (scratch.partials != nullptr && a.k_split > 1) {
+        if (reinterpret_cast<uintptr_t>(scratch.partials) % kTcPartialAlign != 0 || !tc_partials_hold(end - first, a.k_split, sm_count)) return cudaErrorInvalidValue;
         a.partial_counts = reinterpret_cast<unsigned *>(scratch.partials);
         a.partials = reinterpret_cast<float *>(scratch.partials + tc_partial_count_bytes(sm_count));
     }

@@ -315,6 +315,12 @@ class Runtime:
         _capi.check(self._lib.vqm_launch_count(self._h, ctypes.byref(out)))
         return out.value
 
+    def memory_exchange_count(self) -> int:
+        """Matvecs whose blocks exchanged partial sums through memory (the others with split columns: as clusters)."""
+        out = ctypes.c_uint64()
+        _capi.check(self._lib.vqm_memory_exchange_count(self._h, ctypes.byref(out)))
+        return out.value
+
     # ---- row-sharded tensors over several GPUs (no reference counterpart) -----------------------------------------
     def exchange_create(self, nbytes: int) -> tuple[bytes, int]:
         """Allocates this rank's exchange region; returns (64-byte CUDA IPC handle, device address)."""
