@@ -119,3 +119,39 @@ def test_threads_on_their_own_default_streams_have_rooms_of_their_own(two):
         thread.join()
     assert counts == {0: 8 * N // 2, 1: 8 * N // 2}
     p.check()
+
+
+def test_closing_a_runtime_of_two_streams_beside_an_open_capture(two):
+    import torch
+
+    gone, p = two
+    gone.rt.set_stream(torch.cuda.Stream().cuda_stream)
+    assert gone.exchanged(lambda: gone.launch(0)) == 1
+    opened, closed, failures = threading.Event(), threading.Event(), []
+
+    def capture():
+        try:
+            p.rt.capture_begin()
+            for i in range(N):
+                p.launch(i)
+            opened.set()
+            closed.wait(60)
+            graph = p.rt.capture_end()
+            p.rt.graph_launch(graph)
+            p.rt.synchronize()
+            p.rt.graph_destroy(graph)
+        except Exception as e:  # noqa: BLE001
+            failures.append(e)
+        finally:
+            opened.set()
+
+    thread = threading.Thread(target=capture)
+    thread.start()
+    assert opened.wait(60)
+    try:
+        gone.rt.close()
+    finally:
+        closed.set()
+        thread.join()
+    assert not failures
+    p.check()

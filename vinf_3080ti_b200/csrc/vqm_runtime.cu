@@ -7,6 +7,7 @@
 #include <fcntl.h>
 #include <unistd.h>
 
+#include <array>
 #include <atomic>
 #include <cerrno>
 #include <climits>
@@ -84,6 +85,7 @@ struct StreamPartials {
     unsigned long long stream;  // its id: ids, unlike handles, do not come again
     uint8_t *room;
     bool emptied;  // the room is as launches find and leave it
+    bool used;     // since the runtime last waited for the whole GPU
 };
 
 struct vqm_runtime {
@@ -325,33 +327,48 @@ constexpr int kPartialRooms = 16, kPartialSms = 160;
 static __device__ __align__(256) uint8_t g_partial_rooms[kPartialRooms][(vqm::tc_partial_bytes(kPartialSms, 8) + 255) / 256 * 256];
 std::mutex g_partial_mutex;
 bool g_partial_taken[kPartialRooms];
+// Rooms whose runtime is gone, but which work on a stream of the caller may still use: a number that says when it went, else 0.
+using PartialsLeft = std::array<uint64_t, kPartialRooms>;
+PartialsLeft g_partial_left{};
+uint64_t g_partial_gone = 0;
+uint8_t *g_partial_first = nullptr;  // room 0 (one device per process, see check_one_device)
 
 // A room's address, null if there is none left.
 uint8_t *take_partials(int sm_count) {
     if (sm_count > kPartialSms) return nullptr;
     const std::lock_guard<std::mutex> lock(g_partial_mutex);
-    static uint8_t *first = nullptr;  // (one device per process, see check_one_device)
-    if (first == nullptr) {
+    if (g_partial_first == nullptr) {
         void *p = nullptr;
         if (cudaGetSymbolAddress(&p, g_partial_rooms) != cudaSuccess) {
             (void)cudaGetLastError();
             return nullptr;
         }
-        first = static_cast<uint8_t *>(p);
+        g_partial_first = static_cast<uint8_t *>(p);
     }
     for (int i = 0; i < kPartialRooms; ++i)
         if (!g_partial_taken[i]) {
             g_partial_taken[i] = true;
-            return first + i * sizeof(g_partial_rooms[0]);
+            return g_partial_first + i * sizeof(g_partial_rooms[0]);
         }
     return nullptr;
 }
-// (of a runtime all of whose work has ended)
-void give_partials_back(const uint8_t *room) {
+// By a runtime that goes.  A room whose last work may not have ended is kept until some runtime has waited for the whole GPU: that wait is not
+// made here, it would break a capture that another thread has open.
+void give_partials_back(const uint8_t *room, bool ended) {
     const std::lock_guard<std::mutex> lock(g_partial_mutex);
-    void *first = nullptr;
-    if (cudaGetSymbolAddress(&first, g_partial_rooms) == cudaSuccess)
-        g_partial_taken[(room - static_cast<const uint8_t *>(first)) / sizeof(g_partial_rooms[0])] = false;
+    const size_t i = static_cast<size_t>(room - g_partial_first) / sizeof(g_partial_rooms[0]);
+    if (ended) g_partial_taken[i] = false;
+    else g_partial_left[i] = ++g_partial_gone;
+}
+// The rooms that are kept so, before such a wait, and back with them after it (those that have not come and gone again meanwhile).
+PartialsLeft partials_left() {
+    const std::lock_guard<std::mutex> lock(g_partial_mutex);
+    return g_partial_left;
+}
+void give_left_partials_back(const PartialsLeft &left) {
+    const std::lock_guard<std::mutex> lock(g_partial_mutex);
+    for (int i = 0; i < kPartialRooms; ++i)
+        if (left[i] != 0 && g_partial_left[i] == left[i]) g_partial_left[i] = 0, g_partial_taken[i] = false;
 }
 // As launches find and leave it.
 cudaError_t empty_partials(vqm_runtime *rt, uint8_t *p, int m, cudaStream_t stream) {
@@ -384,10 +401,11 @@ uint8_t *find_partials(vqm_runtime *rt) {
         if (rt->stream_partials.size() >= kMaxStreamPartials) return nullptr;
         uint8_t *const room = take_partials(rt->sm_count);
         if (room == nullptr) return nullptr;
-        rt->stream_partials.push_back(StreamPartials{id, room, false});
+        rt->stream_partials.push_back(StreamPartials{id, room, false, false});
         mine = &rt->stream_partials.back();
     }
     if (!mine->emptied) mine->emptied = empty_partials(rt, mine->room, 8, rt->stream) == cudaSuccess;
+    mine->used = true;
     return mine->emptied ? mine->room : nullptr;
 }
 
@@ -725,9 +743,14 @@ int vqm_runtime_create(const void *iq3s_grid, size_t nbytes, vqm_runtime **out) 
 
 void vqm_runtime_destroy(vqm_runtime *rt) {
     if (rt == nullptr) return;
-    if (rt->stream != nullptr) cudaStreamSynchronize(rt->stream);
-    if (rt->stream_partials.size() > 1) cudaDeviceSynchronize();  // (other streams' work)
-    for (const StreamPartials &known : rt->stream_partials) give_partials_back(known.room);
+    // What this runtime has launched on its own stream and on the present one has ended then.
+    unsigned long long ended[2] = {ULLONG_MAX, ULLONG_MAX};
+    const cudaStream_t streams[2] = {rt->stream, rt->own_stream};
+    for (int i = 0; i < (rt->stream == rt->own_stream ? 1 : 2); ++i)
+        if (streams[i] == nullptr || cudaStreamSynchronize(streams[i]) != cudaSuccess || cudaStreamGetId(streams[i], &ended[i]) != cudaSuccess)
+            ended[i] = ULLONG_MAX;
+    for (const StreamPartials &known : rt->stream_partials)
+        give_partials_back(known.room, !known.used || known.stream == ended[0] || known.stream == ended[1]);
     rt->stream = rt->own_stream;
     for (auto &g : rt->graphs)
         if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
@@ -1397,8 +1420,11 @@ int vqm_set_gemm_min_rows(vqm_runtime *rt, int n) {
 int vqm_synchronize(vqm_runtime *rt) {
     const int rc = no_capture(rt, "synchronize");
     if (rc != VQM_OK) return rc;
+    const PartialsLeft left = partials_left();
     const cudaError_t err = cudaDeviceSynchronize();
     if (err != cudaSuccess) return cuda_fail("synchronize", err);
+    give_left_partials_back(left);
+    for (StreamPartials &known : rt->stream_partials) known.used = false;
     return check_status_word(rt, "synchronize");
 }
 
