@@ -155,3 +155,84 @@ def test_closing_a_runtime_of_two_streams_beside_an_open_capture(two):
         thread.join()
     assert not failures
     p.check()
+
+
+@pytest.mark.parametrize("t,rows,cols,per_launch", [(T.Q6_K, 2305, 2304, 24), (T.Q3_K, 1030, 5120, 16), (T.Q8_0, 4099, 1280, 8)], ids=str)
+def test_every_row_count_goes_through_memory_and_gives_what_clusters_give(two, t, rows, cols, per_launch):
+    rt = two[0].rt
+    rng = np.random.default_rng(rows)
+    rt.upload("v", synthetic_blocks(t, rows, cols, rng), int(t), cols, rows)
+    rt.alloc("x", 24 * cols)
+    rt.alloc("y", 24 * rows)
+    for m in (1, 2, 4, 8, 16, 24):
+        rt.write("x", synthetic_activations(m, cols, rng))
+        rt.zero("y")
+        through_memory = two[0].exchanged(lambda: rt.qmv("v", "x", "y", m))
+        rt.synchronize()
+        assert through_memory == -(-m // per_launch), m
+        got = rt.read_array("y", m * rows).copy()
+        rt.zero("y")
+        rt.capture_begin()
+        rt.qmv("v", "x", "y", m)
+        graph = rt.capture_end()
+        rt.graph_launch(graph)
+        rt.synchronize()
+        rt.graph_destroy(graph)
+        assert np.abs(got).max() > 0 and np.array_equal(got.view(np.uint32), rt.read_array("y", m * rows).view(np.uint32)), m
+
+
+def test_streams_of_one_runtime_that_overlap(two):
+    import torch
+
+    p, streams = two[0], [torch.cuda.Stream() for _ in range(3)]
+    for _ in range(5):
+        p.clear()
+        for stream in streams:
+            with torch.cuda.stream(stream):
+                torch.cuda._sleep(2_000_000)  # some 1 ms: all launches are there before the first runs
+        before = p.rt.memory_exchange_count()
+        for i in range(N):
+            p.rt.set_stream(streams[i % 3].cuda_stream)
+            p.launch(i)
+        assert p.rt.memory_exchange_count() - before == N
+        p.check()
+
+
+def test_the_fifth_stream_of_a_runtime_has_clusters(two):
+    import torch
+
+    p, streams = two[0], [torch.cuda.Stream() for _ in range(4)]
+    for i, stream in enumerate(streams):  # (the first is the runtime's own)
+        p.rt.set_stream(stream.cuda_stream)
+        assert p.exchanged(lambda: [p.launch(k) for k in range(i, N, 4)]) == (N // 4 if i < 3 else 0)
+    p.check()
+
+
+def test_rooms_run_out_and_come_back(two, codebooks):
+    import torch
+
+    p, others = two[0], []
+    try:
+        while len(others) < 20:
+            others.append(Passes(codebooks))
+            if others[-1].exchanged(lambda: others[-1].launch(0)) == 0:
+                break
+        assert 2 <= len(others) < 20  # 16 rooms of a process
+        last = others[-1]
+        assert last.exchanged(lambda: [last.launch(i) for i in range(N)]) == 0
+        last.check()
+        last.clear()
+        others.pop(0).rt.close()
+        assert last.exchanged(lambda: [last.launch(i) for i in range(N)]) == N
+        last.check()
+    finally:
+        for other in others:
+            other.rt.close()
+    stream = torch.cuda.Stream()
+    for _ in range(18):  # whose last work is on a stream of the caller
+        gone = Passes(codebooks)
+        gone.rt.set_stream(stream.cuda_stream)
+        assert gone.exchanged(lambda: gone.launch(0)) == 1
+        gone.rt.set_stream(None)
+        gone.rt.close()
+        p.rt.synchronize()
