@@ -236,3 +236,38 @@ def test_rooms_run_out_and_come_back(two, codebooks):
         gone.rt.set_stream(None)
         gone.rt.close()
         p.rt.synchronize()
+
+
+ALONE = """
+import sys
+import numpy as np
+sys.path.insert(0, {repo!r})
+from tests.test_gpu_stream_partials import N, Passes
+with np.load({repo!r} + "/tests/golden/iq_codebooks.npz") as z:
+    books = {{k: z[k].tobytes() for k in z.files}}
+counts = []
+def run(p):
+    counts.append(p.exchanged(lambda: [p.launch(i) for i in range(N)]))
+    p.check()
+    p.clear()
+first = Passes(books)
+run(first)
+second = Passes(books)  # (nothing but captured launches yet)
+run(first)
+run(second)
+run(first)
+second.rt.close()
+run(first)
+print(counts)
+"""
+
+
+def test_clusters_while_one_stream_has_the_gpu_to_itself():
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    repo = str(Path(__file__).resolve().parent.parent)
+    done = subprocess.run([sys.executable, "-c", ALONE.format(repo=repo)], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    assert done.stdout.split("\n")[0] == str([0, 0, N, N, 0])

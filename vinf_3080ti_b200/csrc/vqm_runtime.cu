@@ -86,6 +86,7 @@ struct StreamPartials {
     uint8_t *room;
     bool emptied;  // the room is as launches find and leave it
     bool used;     // since the runtime last waited for the whole GPU
+    bool counted;  // in g_partial_streams
 };
 
 struct vqm_runtime {
@@ -331,6 +332,7 @@ bool g_partial_taken[kPartialRooms];
 using PartialsLeft = std::array<uint64_t, kPartialRooms>;
 PartialsLeft g_partial_left{};
 uint64_t g_partial_gone = 0;
+std::atomic<int> g_partial_streams{0};  // streams with rooms on which matvecs with split columns have been launched
 uint8_t *g_partial_first = nullptr;  // room 0 (one device per process, see check_one_device)
 
 // A room's address, null if there is none left.
@@ -388,7 +390,7 @@ bool is_capturing(cudaStream_t stream) {
 // it (cudaStreamPerThread, a stream destroyed and another created), and what could not be done then (beside a capture, or with all rooms taken)
 // is done when it can be.
 constexpr size_t kMaxStreamPartials = 4;
-uint8_t *find_partials(vqm_runtime *rt) {
+StreamPartials *find_partials(vqm_runtime *rt) {
     unsigned long long id = 0;
     if (is_capturing(rt->stream) || cudaStreamGetId(rt->stream, &id) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -401,19 +403,34 @@ uint8_t *find_partials(vqm_runtime *rt) {
         if (rt->stream_partials.size() >= kMaxStreamPartials) return nullptr;
         uint8_t *const room = take_partials(rt->sm_count);
         if (room == nullptr) return nullptr;
-        rt->stream_partials.push_back(StreamPartials{id, room, false, false});
+        rt->stream_partials.push_back(StreamPartials{id, room, false, false, false});
         mine = &rt->stream_partials.back();
     }
-    if (!mine->emptied) mine->emptied = empty_partials(rt, mine->room, 8, rt->stream) == cudaSuccess;
-    mine->used = true;
-    return mine->emptied ? mine->room : nullptr;
+    if (!mine->emptied) {
+        mine->emptied = empty_partials(rt, mine->room, 8, rt->stream) == cudaSuccess;
+        mine->used = true;
+    }
+    return mine->emptied ? mine : nullptr;
 }
 
-// Room for the partial sums of the next launch, none while a graph is captured: it may run beside other work, on any stream.  (Beside
-// nothing else, as a captured decode pass, clusters exchange them faster too: the 27B model's pass of 4 rows 4.84 ms, 4.94 through memory.)
+// Room for the partial sums of the next launch, null where clusters exchange them: the outputs are the same.  None while a graph is captured:
+// it may run beside other work, on any stream.  None either while only one stream of the process launches such matvecs: beside nothing
+// else clusters are faster, the way through L2 takes 0.3 to 1 us longer.  One runtime on one stream, clusters and memory, us: a layer with 1
+// row 87.7 and 88.6, with 4 rows 94.2 and 98.6, as fused calls 106.8 and 112.9, with 8 rows in groups 83.7 and 87.5; the 27B model's captured
+// pass of 4 rows 4840 and 4940.  Three runtimes on three streams: see tc_finish_tile.
 uint8_t *partials_now(vqm_runtime *rt, int m) {
     if (rt->capturing) return nullptr;
-    if (m <= 8) return find_partials(rt);
+    StreamPartials *const mine = find_partials(rt);
+    if (mine != nullptr && !mine->counted) {
+        mine->counted = true;
+        g_partial_streams.fetch_add(1, std::memory_order_relaxed);
+    }
+    if (g_partial_streams.load(std::memory_order_relaxed) < 2) return nullptr;
+    if (m <= 8) {
+        if (mine == nullptr) return nullptr;
+        mine->used = true;
+        return mine->room;
+    }
     if (is_capturing(rt->stream)) return nullptr;
     uint8_t *const room = rt->x_split + rt->x_split_bytes;  // (claim_split has been called)
     if (!rt->split_emptied) rt->split_emptied = empty_partials(rt, room, 24, rt->stream) == cudaSuccess;
@@ -749,8 +766,10 @@ void vqm_runtime_destroy(vqm_runtime *rt) {
     for (int i = 0; i < (rt->stream == rt->own_stream ? 1 : 2); ++i)
         if (streams[i] == nullptr || cudaStreamSynchronize(streams[i]) != cudaSuccess || cudaStreamGetId(streams[i], &ended[i]) != cudaSuccess)
             ended[i] = ULLONG_MAX;
-    for (const StreamPartials &known : rt->stream_partials)
+    for (const StreamPartials &known : rt->stream_partials) {
+        if (known.counted) g_partial_streams.fetch_sub(1, std::memory_order_relaxed);
         give_partials_back(known.room, !known.used || known.stream == ended[0] || known.stream == ended[1]);
+    }
     rt->stream = rt->own_stream;
     for (auto &g : rt->graphs)
         if (g.exec != nullptr) cudaGraphExecDestroy(g.exec);
