@@ -171,7 +171,8 @@ int vqm_graph_destroy(vqm_runtime *rt, int graph_id);
 /* Number of kernels this runtime has launched (graph launches count their kernels). */
 int vqm_launch_count(vqm_runtime *rt, uint64_t *out);
 /* Number of matvecs so far whose blocks exchanged the partial sums of split columns through memory.  All others with split
- * columns (captured ones, those of streams for which no room is left) exchanged them as clusters; outputs are the same. */
+ * columns (captured ones, those of a stream that alone in the process launches any, those of streams for which no room is
+ * left) exchanged them as clusters; outputs are the same. */
 int vqm_memory_exchange_count(vqm_runtime *rt, uint64_t *out);
 
 /* Stateless entry point for callers that own all memory: y = W x on `stream` (a cudaStream_t, NULL = legacy

@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(kTThreads, 1) qgemm_tc5_kernel(const __grid_co
         ok = warp_wait(s32(&s_done), 0, failed);
         // (The next conversion of activations may be launched; it waits for this kernel's end before it touches anything.  Requested at the start
         // of a block, that conversion and the GEMM behind it take SMs that other streams could use: three streams, 1500 rows of Q4_K 17408 x
-        // 5120 211 to 243 us, 200 so, 512 rows of four tensors 285 to 296 and 281 to 290.)
+        // 5120 211 to 243 us, 200 so, 512 rows of four tensors 290 and 284.  One stream alone: 512 rows 80.7 and 80.9, of four tensors 308 and 307.)
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }

@@ -35,7 +35,7 @@
 // multiple of 16 bytes, free of bank conflicts for 16-byte loads.
 //
 // Columns are split over k_split blocks, each a contiguous range of steps.  The blocks exchange their sums through memory (tc_finish_tile) or,
-// where the launch has no room for them (a captured graph, a caller without a runtime), as a cluster: a tile's rows are dealt out to its blocks
+// where the launch has been given no room for them (a captured graph, a caller without a runtime, a stream alone on the GPU), as a cluster: a tile's rows are dealt out to its blocks
 // and every block sends each its part (st.async).  Both add the parts in the order of the columns: the split and the order of all additions depend
 // on rows and columns only, never on M.
 #pragma once

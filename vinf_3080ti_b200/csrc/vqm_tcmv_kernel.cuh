@@ -698,8 +698,8 @@ __device__ __forceinline__ uint32_t tc_red_at(uint32_t red, int pair, int t, int
 // parts up in the order of the columns; the others leave theirs in a.partials.  They come with no fence: the last block reads words
 // until none is empty, and leaves them empty again.  It only waits for blocks that are about to store: blocks may run at any time and in any
 // place, and no cluster has to find room at once (120 blocks in clusters of 6 leave 28 SMs, of which other clusters cannot use most).
-// The way through L2 takes some 0.5 us longer than one through a cluster's shared memory, which a stream alone notices (a layer of 8 rows,
-// alone from launch to end, 109 -> 112 us; one of 1 row 100 -> 104) and three streams that share the GPU do not: clusters and this, each with
+// The way through L2 takes some 0.5 us longer than one through a cluster's shared memory, which a stream alone notices (back to back, a layer of
+// 4 rows 94.2 -> 98.6 us, one of 8 106.9 -> 114.2), so it has clusters; three streams that share the GPU do not: clusters and this, each with
 // launch_dependents where it is now, layers of 1, 4 (fused) and 8 rows 67.3 / 81.9 / 81.2 and 60.8 / 73.3 / 75.0 us, 24 rows of three tensors
 // 101 and 84, six tensors of odd sizes with 2 rows 62 and 53.
 // (What was slower: a warp at a time, each with its own count, M=8 Q6_K 1024 x 5120 10.6 -> 11.8 us; counts that acquire and release, or fences on both

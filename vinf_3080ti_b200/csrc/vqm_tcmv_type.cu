@@ -80,7 +80,7 @@ struct TcVariant {
 
 // Tall tensors, whose blocks walk whole rows: the last round of tiles may occupy a few SMs only (LM head, 151936 rows: 594 tiles
 // on 148 SMs, 2 of them in a fifth round).  Its tiles then go to a second launch that splits their columns, if that saves more
-// than a launch costs (3.4 us, two to three steps).  first: its first tile, 0 if there is none.
+// than a launch costs (3.4 us, two to three steps); that launch's blocks are clusters.  first: its first tile, 0 if there is none.
 struct TcTail {
     int first = 0, k_split = 0;
 };
@@ -102,25 +102,26 @@ inline bool takes_tail(const MatvecArgs &a) { return a.part[1].rows == 0 && (a.o
 // columns only.
 // Time of a launch in steps of 256 columns: every group of blocks walks `rounds` tiles of 256 rows, each block its share of the
 // steps (pairs of warp groups take whole steps in turn: an odd number costs as much as the next even one); a tile costs about
-// one step more for its sums, and another half for adding them up across a cluster.
+// one step more for its sums, and another half for adding them up across blocks.  As many groups run at once as clusters find room, also
+// where the sums go through memory, which needs none: a launch has to give the same bits either way, so it has the same split.
 // A launch has a fixed cost of about 3.4 us here and of 2.6 us on the CUDA-core kernel, which reads all columns of a short
 // tensor at once while a block here walks its steps; but it takes a quarter of the SMs, and more rows cost it little.  So
 // where the line lies depends on what else the GPU does.  Measured with 1 / 4 / 8 rows, CUDA-core and this one (us):
 //   launches that wait for one another, on one stream:
-//     Q4_K 1024 x 5120:   5.0 /  6.9 / 10.1  and   6.5 /  7.5 / 10.0      2048 x 5120:  6.6 / 10.3 / 16.1  and   6.7 /  7.7 / 10.2
-//     Q6_K 1024 x 5120:   5.3 /  7.5 / 11.2  and   8.6 /  9.0 / 10.6      2048 x 5120:  6.9 / 10.8 / 16.4  and   8.8 /  9.1 / 10.6
-//     Q3_K 1024 x 5120:   5.3 /  7.5 / 11.1  and   7.8 /  8.7 / 10.7      2048 x 5120:  6.9 / 10.6 / 16.2  and   7.9 /  8.9 / 10.8
-//     IQ3_S 1024 x 5120:  6.8 / 11.1 / 17.0  and  10.1 / 10.6 / 12.6      2048 x 5120:  9.8 / 17.7 / 29.2  and  10.4 / 10.9 / 12.8
-//     IQ4_XS 1024 x 5120: 5.4 /  7.1 / 10.1  and   8.4 / 10.7 / 13.9      2048 x 5120:  7.3 / 10.2 / 15.6  and   8.6 / 10.9 / 14.1
+//     Q4_K 1024 x 5120:   5.0 /  6.9 / 10.0  and   6.6 /  7.3 /  9.3      2048 x 5120:  6.6 / 10.3 / 16.2  and   6.7 /  7.4 /  9.5
+//     Q6_K 1024 x 5120:   5.3 /  7.5 / 11.1  and   8.6 /  8.9 / 10.1      2048 x 5120:  7.0 / 10.8 / 16.4  and   8.9 /  9.2 / 10.4
+//     Q3_K 1024 x 5120:   5.2 /  7.4 / 11.1  and   7.3 /  8.2 /  9.8      2048 x 5120:  6.9 / 10.5 / 16.1  and   7.4 /  8.3 /  9.8
+//     IQ3_S 1024 x 5120:  6.8 / 11.2 / 16.9  and   9.7 / 10.2 / 12.1      2048 x 5120:  9.8 / 17.8 / 29.1  and   9.8 / 10.4 / 12.2
+//     IQ4_XS 1024 x 5120: 5.3 /  7.0 / 10.0  and   8.1 / 10.5 / 13.3      2048 x 5120:  7.3 / 10.1 / 15.5  and   8.2 / 10.7 / 13.5
 //   three runtimes in turn, each on its stream (about 3 is the call itself):
-//     Q6_K 1024 x 5120:   4.9 /  6.4 /  8.9  and   5.8 /  5.0 /  5.1      2048 x 5120:  6.0 /  8.7 / 12.8  and   5.5 /  5.5 /  6.2
-//     IQ4_XS 1024 x 5120: 5.0 /  6.2 /  8.6  and   3.2 /  4.0 /  5.1      2048 x 5120:  6.3 /  8.4 / 13.1  and   3.3 /  4.0 /  5.4
+//     Q6_K 1024 x 5120:   4.8 /  6.1 /  8.7  and   3.5 /  3.7 /  4.2      2048 x 5120:  5.8 /  8.5 / 12.6  and   3.7 /  4.0 /  4.4
+//     IQ4_XS 1024 x 5120: 4.8 /  6.1 /  8.3  and   3.4 /  4.1 /  5.2      2048 x 5120:  6.1 /  8.3 / 12.9  and   3.6 /  4.3 /  5.4
 //   a decoder layer of the 27B model whose 1024 x 5120 projections run there or here (the blocks of the one kernel fit beside nothing of the
-//   other), 1 row, 4 with prologues, 8 in groups:  one stream, one graph: 85 / 119 / 93 and 90 / 110 / 93;  three streams: 78 / 106 / 80 and
-//   70 / 80 / 80
+//   other), 1 row, 4 with prologues, 8 in groups:  one stream, one graph: 80 / 113 / 86 and 86 / 104 / 85;  three streams: 66 / 94 / 70 and
+//   58 / 73 / 69
 // The choice must not depend on the number of rows.  From 72 pieces of 256 x 256 weights on, of which no block has to walk more
-// than one in 20, launches go here: single rows on one stream pay up to 2 times for the shortest of them (2 to 7 % of a layer),
-// 8 rows, and whatever shares the GPU, gain more.
+// than one in 20, launches go here: single rows on one stream pay up to 1.6 times for the shortest of them (8 % of a layer),
+// 4 rows and whatever shares the GPU gain more.
 inline int choose_tc_split(int n_tiles, int cols, int sm_count, bool single) {
     const int n_steps = (cols + kTcStepCols - 1) / kTcStepCols;
     if (static_cast<long long>(n_tiles) * n_steps < 72) return 0;
